@@ -366,13 +366,16 @@ def reference_main(args, metric, base_config, world, mat, scaling="weak"):
 # unique keys, |S| = 2^29 Zipf over R's keys, hot keys at small ranks (rank =
 # key) or scattered over the key range by a seeded permutation.
 LVR_CASES = [("z1", 1.0, 0), ("z1_scattered", 1.0, 1)]
-LVR_VARIANTS = [("lrn", "LRN", {}), ("rho_skew_split", "RHO", {}), ("rho_plain", "RHO", {"skew_split": 0})]
+# RHO partitioned (fixed passes) with and without the split, and under the
+# automatic plan (the direct counting join)
+LVR_VARIANTS = [("lrn", "LRN", {}), ("rho_skew_split", "RHO", {"passes": 2}),
+                ("rho_plain", "RHO", {"skew_split": 0}), ("rho_automatic", "RHO", {})]
 
 
 def learned_vs_radix(tbg, torch, dev, stream, steps, warmup, lr=26, ls=29, cases=LVR_CASES):
-    """Times LRN, RHO with its S-side skew split (the library default) and RHO
-    without it (the reference's behaviour) on the same device-resident
-    inputs, CUDA events on the join stream, the clock sampler running."""
+    """Times LRN, the partitioned RHO with its S-side skew split and without it
+    (the reference's behaviour), and RHO's automatic plan on the same
+    device-resident inputs, CUDA events on the join stream, the clock sampler running."""
     sh = stream.cuda_stream
     nR, nS = 1 << lr, 1 << ls
     tR = torch.empty(nR, dtype=torch.int64, device=dev)
@@ -628,8 +631,19 @@ def main():
     pipe_ms = ms / K
     peak_source = (f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                    else "fallback 6650 GB/s")
-    if algo in ("RHO", "RHT") and not mat:
-        scat_ms = (phase["ms_pass1"] + phase["ms_pass2"]) / K
+    scat_ms = (phase["ms_pass1"] + phase["ms_pass2"]) / K
+    if algo in ("RHO", "RHT") and not mat and scat_ms < 0.05 * pipe_ms:
+        # the direct counting join: S is joined in its histogram read, nothing
+        # is partitioned
+        achieved = 8 * rows / (pipe_ms / 1e3) / 1e9
+        roofline = {"bound": "hbm", "kernel": "all kernels of one join: k_hist_build (R's keys into the bit table) and "
+                                              "k_hist_probe (S's histogram and matches)",
+                    "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
+                    "peak_source": peak_source, "algorithmic_bytes_per_join": 8 * rows,
+                    "bytes_model": "every row of R and S read once (8 B); bound by one L1 line per clock and SM for "
+                                   "the lookups in the L2-resident table, not by HBM",
+                    "timing": "CUDA events around the timed joins on their stream"}
+    elif algo in ("RHO", "RHT") and not mat:
         scat_bytes = 16 * rows * passes
         achieved = scat_bytes / (scat_ms / 1e3) / 1e9 if scat_ms > 0 else None
         traffic, traffic_source = None, None

@@ -312,16 +312,23 @@ int ensure_radix_buffers(const RadixGeom &g, bool bypass, Workspace &w) {
     return TBG_OK;
 }
 
-// Histogram of one relation (with the heavy bypass for S when given), column
-// prefix and partition bases.
-int part_histogram(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w, cudaStream_t st,
-                   const SBypass *bypass) {
+// Per-chunk histograms of one relation (with the heavy bypass for S when
+// given).  With g.direct the read of R also enters its keys into the bit
+// table, and the read of S counts the matches when the join is direct.
+static int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w,
+                          cudaStream_t st, const SBypass *bypass) {
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     DevBuf &hist = rel ? w.histS : w.histR;
-    DevBuf &tot = rel ? w.totS : w.totR;
-    DevBuf &base = rel ? w.baseS : w.baseR;
     cudaError_t e;
-    if (!bypass) {
+    if (g.direct && rel == 0) {
+        e = launch_hist_build(d, g.n[0], g.ch[0], g.G[0], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), ctrl,
+                              st);
+        if (e == cudaSuccess)
+            e = launch_direct_decide(w.direct.as<uint32_t>(), direct_log2_max(g.n[0]), g.n[0], ctrl, st);
+    } else if (g.direct) {
+        e = launch_hist_probe(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(),
+                              g.n[0], ctrl, st);
+    } else if (!bypass) {
         const bool check = rel == 1 && g.s_range_max != 0xFFFFFFFFu;
         e = launch_hist_chunks(d, g.n[rel], g.ch[rel], g.G[rel], hist.as<uint32_t>(), g.B, g.rf, st,
                                check ? &ctrl->out_of_range : nullptr, g.s_range_max);
@@ -345,18 +352,84 @@ int part_histogram(int rel, const RadixGeom &g, const Row *d, const tbg_config &
         ba.heavy_rows = &ctrl->heavy_rows_S;
         e = launch_hist_bypass(ba, cfg.materialize != 0, st);
     }
-    if (e != cudaSuccess) return cuda_error(e, "histogram");
-    if ((e = launch_colscan(hist.as<uint32_t>(), g.G[rel], (int)g.P, tot.as<uint32_t>(), st)) != cudaSuccess)
-        return cuda_error(e, "colscan");
-    if ((e = launch_plan_bases(tot.as<uint32_t>(), base.as<uint64_t>(), g.B,
-                               rel ? &ctrl->max_part_S : &ctrl->max_part_R, st)) != cudaSuccess)
-        return cuda_error(e, "bases");
-    return TBG_OK;
+    return e == cudaSuccess ? TBG_OK : cuda_error(e, "histogram");
 }
 
-// Pass `which` (1 or 2) of one relation.  Pass 1 reads the relation (or, with
-// the bypass, the compacted S); the last pass writes partR / partS.
-int part_pass(int rel, int which, const RadixGeom &g, const Row *d, Workspace &w, cudaStream_t st, bool bypass) {
+static PlanArgs plan_args(const RadixGeom &g, Workspace &w) {
+    PlanArgs pa;
+    pa.r = RelPlan{w.totR.as<uint32_t>(), w.baseR.as<uint64_t>()};
+    pa.s = RelPlan{w.totS.as<uint32_t>(), w.baseS.as<uint64_t>()};
+    pa.nR = g.n[0];
+    pa.nS = g.n[1];
+    pa.P_log2 = g.B;
+    pa.b1 = g.b1;
+    pa.b2 = g.b2;
+    pa.passes = g.passes;
+    pa.capR = g.capR;
+    pa.capS = g.capS;
+    pa.items = w.items.as<Item>();
+    pa.item_cap = g.item_cap;
+    pa.ctrl = w.ctrl.as<Ctrl>();
+    return pa;
+}
+
+// Partitions up to which the column scan's last CTA also plans the work
+// items; above, one CTA would take longer over them than a launch of
+// P / 1024 CTAs.
+static constexpr uint64_t PLAN_TAIL_PARTS = 2048;
+
+// Column prefix of the histograms, partition totals and bases of the
+// relations in the mask `rels` (bit 0: R, bit 1: S) and, with `items`, the
+// join's work items (both relations' totals and bases must be there then).
+static int part_hist_plan(int rels, bool items, const RadixGeom &g, Workspace &w, cudaStream_t st) {
+    Ctrl *ctrl = w.ctrl.as<Ctrl>();
+    ColScan c[2];
+    if (rels & 1) c[0] = ColScan{w.histR.as<uint32_t>(), w.totR.as<uint32_t>(), g.G[0], (int)g.P};
+    if (rels & 2) c[1] = ColScan{w.histS.as<uint32_t>(), w.totS.as<uint32_t>(), g.G[1], (int)g.P};
+    PlanTail t;
+    t.rels = rels;
+    t.items = items && g.P <= PLAN_TAIL_PARTS;
+    t.done = &ctrl->done[rels == 1 ? 0 : 1];
+    t.plan = plan_args(g, w);
+    cudaError_t e = launch_colscan_plan(c[0], c[1], t, st);
+    if (e != cudaSuccess) return cuda_error(e, "column scan");
+    return items && !t.items ? plan_items(g, w, st) : TBG_OK;
+}
+
+int part_histogram(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w, cudaStream_t st,
+                   const SBypass *bypass) {
+    const int rc = part_hist_read(rel, g, d, cfg, w, st, bypass);
+    return rc ? rc : part_hist_plan(1 << rel, false, g, w, st);
+}
+
+// Counting joins try the direct join (direct.cu) under the automatic plan (the
+// passes and the build/probe are launched too and step aside when it is
+// direct: four empty launches take about 9 us, while reading the decision back
+// midway took 20 us from every join that is not direct); a
+// caller who fixes the radix bits or passes, or turns the skew split off, gets
+// the partitioned join.
+static bool tries_direct(const tbg_config &cfg) {
+    return !cfg.materialize && cfg.radix_bits <= 0 && (cfg.passes <= 0 || cfg.passes > 2) && cfg.skew_split;
+}
+
+// Start of a counting RHO or RHT: the control block cleared, and with g.direct
+// the bit table sized and cleared (dR is read).
+static int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st) {
+    cudaError_t e;
+    if (!g.direct) {
+        e = cudaMemsetAsync(w.ctrl.p, 0, sizeof(Ctrl), st);
+    } else {
+        const int lg = direct_log2_max(g.n[0]);
+        if ((e = w.direct.ensure((size_t)1 << (lg - 3))) != cudaSuccess) return cuda_error(e, "cudaMalloc");
+        e = launch_direct_prep(dR, g.n[0], w.direct.as<uint32_t>(), lg, w.ctrl.as<Ctrl>(), w.nsm, st);
+    }
+    return e == cudaSuccess ? TBG_OK : cuda_error(e, "start of the join");
+}
+
+// Arguments of pass `which` (1 or 2) of one relation.  Pass 1 reads the
+// relation (or, with the bypass, the compacted S); the last pass writes
+// partR / partS.
+static PartArgs pass_args(int rel, int which, const RadixGeom &g, const Row *d, Workspace &w, bool bypass) {
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     const uint64_t n = g.n[rel];
     PartArgs a;
@@ -381,43 +454,54 @@ int part_pass(int rel, int which, const RadixGeom &g, const Row *d, Workspace &w
     a.off1 = g.passes == 2 ? (rel ? w.off1S : w.off1R).as<uint32_t>() : nullptr;
     a.cnt1 = g.passes == 2 ? (rel ? w.cnt1S : w.cnt1R).as<uint32_t>() : nullptr;
     a.err = &ctrl->error;
+    a.skip = &ctrl->direct;
     Row *part = (rel ? w.partS : w.partR).as<Row>();
     Row *tmp = g.passes == 2 ? (rel ? w.tmpS : w.tmpR).as<Row>() : part;
-    cudaError_t e;
     if (which == 1) {
         a.in = bypass ? w.sc.as<Row>() : d;
         if (bypass) a.chunk_len = w.kept.as<uint32_t>();
         a.out = tmp;
-        e = launch_part_pass1(a, st);
     } else {
-        if (g.passes != 2) return TBG_OK;
         a.in = tmp;
         a.out = part;
-        e = launch_part_pass2(a, st);
     }
+    return a;
+}
+
+// Pass `which` of one relation.
+int part_pass(int rel, int which, const RadixGeom &g, const Row *d, Workspace &w, cudaStream_t st, bool bypass) {
+    if (which == 2 && g.passes != 2) return TBG_OK;
+    const PartArgs a = pass_args(rel, which, g, d, w, bypass);
+    const cudaError_t e = which == 1 ? launch_part_pass1(a, nullptr, st) : launch_part_pass2(a, nullptr, st);
+    return e == cudaSuccess ? TBG_OK : cuda_error(e, "partition pass");
+}
+
+// Pass `which` of S and R in one launch.
+static int part_pass_both(int which, const RadixGeom &g, const Row *dR, const Row *dS, Workspace &w, cudaStream_t st) {
+    if (which == 2 && g.passes != 2) return TBG_OK;
+    const PartArgs s = pass_args(1, which, g, dS, w, false), r = pass_args(0, which, g, dR, w, false);
+    const cudaError_t e = which == 1 ? launch_part_pass1(s, &r, st) : launch_part_pass2(s, &r, st);
     return e == cudaSuccess ? TBG_OK : cuda_error(e, "partition pass");
 }
 
 int plan_items(const RadixGeom &g, Workspace &w, cudaStream_t st) {
-    PlanArgs pa;
-    pa.r = RelPlan{w.totR.as<uint32_t>(), w.baseR.as<uint64_t>()};
-    pa.s = RelPlan{w.totS.as<uint32_t>(), w.baseS.as<uint64_t>()};
-    pa.nR = g.n[0];
-    pa.nS = g.n[1];
-    pa.P_log2 = g.B;
-    pa.b1 = g.b1;
-    pa.b2 = g.b2;
-    pa.passes = g.passes;
-    pa.capR = g.capR;
-    pa.capS = g.capS;
-    pa.items = w.items.as<Item>();
-    pa.item_cap = g.item_cap;
-    pa.ctrl = w.ctrl.as<Ctrl>();
-    cudaError_t e = launch_plan(pa, st);
+    cudaError_t e = launch_plan(plan_args(g, w), st);
     return e == cudaSuccess ? TBG_OK : cuda_error(e, "plan");
 }
 
-// Single-stream radix partitioning of R and S (RHO, RHT, RSM).
+// Both partitioning passes of R and S.
+static int both_passes(const tbg_config &cfg, const RadixGeom &g, const Row *dR, const Row *dS, Workspace &w,
+                       cudaStream_t st) {
+    const bool timing = cfg.timing != 0;
+    int rc;
+    if ((rc = part_pass_both(1, g, dR, dS, w, st))) return rc;
+    mark(w, timing, 2, st);
+    if ((rc = part_pass_both(2, g, dR, dS, w, st))) return rc;
+    mark(w, timing, 3, st);
+    return TBG_OK;
+}
+
+// Single-stream radix partitioning of R and S (RSM).
 int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
                     int capR, Workspace &w, cudaStream_t st, JoinRun *run, int *join_grid_out) {
     const bool timing = cfg.timing != 0;
@@ -431,28 +515,34 @@ int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row
     mark(w, timing, 0, st);
     cudaError_t e = cudaMemsetAsync(w.ctrl.p, 0, sizeof(Ctrl), st);
     if (e != cudaSuccess) return cuda_error(e, "memset");
-    if ((rc = part_histogram(0, g, dR, cfg, w, st, nullptr))) return rc;
-    if ((rc = part_histogram(1, g, dS, cfg, w, st, nullptr))) return rc;
-    if ((rc = plan_items(g, w, st))) return rc;
+    if ((rc = part_hist_read(0, g, dR, cfg, w, st, nullptr))) return rc;
+    if ((rc = part_hist_read(1, g, dS, cfg, w, st, nullptr))) return rc;
+    if ((rc = part_hist_plan(3, true, g, w, st))) return rc;
     mark(w, timing, 1, st);
-    if ((rc = part_pass(0, 1, g, dR, w, st, false))) return rc;
-    if ((rc = part_pass(1, 1, g, dS, w, st, false))) return rc;
-    mark(w, timing, 2, st);
-    if ((rc = part_pass(0, 2, g, dR, w, st, false))) return rc;
-    if ((rc = part_pass(1, 2, g, dS, w, st, false))) return rc;
-    mark(w, timing, 3, st);
-    return TBG_OK;
+    return both_passes(cfg, g, dR, dS, w, st);
 }
 
 // The radix-partitioned join: RHO (layout 0) and RHT (layout 1).
 int run_radix_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
                    tbg_row_out *d_rows, uint64_t cap, Workspace &w, cudaStream_t st,
                    JoinRun *run) {
+    const bool timing = cfg.timing != 0;
     const int capR = join_capacity(nR, !cfg.materialize);
-    int join_grid = 0;
-    int rc = radix_partition(cfg, dR, nR, dS, nS, capR, w, st, run, &join_grid);
+    RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
+    g.direct = tries_direct(cfg);
+    run->B = g.B;
+    run->passes = g.passes;
+    run->P = g.P;
+    int rc = ensure_radix_buffers(g, false, w);
     if (rc) return rc;
-    return radix_join_phase(cfg, d_rows, cap, w, st, run, capR, join_grid);
+    mark(w, timing, 0, st);
+    if ((rc = start_radix_join(g, dR, w, st))) return rc;
+    if ((rc = part_hist_read(0, g, dR, cfg, w, st, nullptr))) return rc;
+    if ((rc = part_hist_read(1, g, dS, cfg, w, st, nullptr))) return rc;
+    if ((rc = part_hist_plan(3, true, g, w, st))) return rc;
+    mark(w, timing, 1, st);
+    if ((rc = both_passes(cfg, g, dR, dS, w, st))) return rc;
+    return radix_join_phase(cfg, d_rows, cap, w, st, run, capR, g.join_grid);
 }
 
 // RHO / RHT with S arriving in slices, for callers that copy S from the host
@@ -473,7 +563,8 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
     const int capR = join_capacity(nR, !cfg.materialize);
     uint64_t smax = 1;
     for (int k = 0; k < nslices; k++) smax = std::max(smax, s_lo[k + 1] - s_lo[k]);
-    const RadixGeom gmax = radix_geometry(cfg, nR, smax, capR, w);
+    RadixGeom gmax = radix_geometry(cfg, nR, smax, capR, w);
+    gmax.direct = tries_direct(cfg);
     run->B = gmax.B;
     run->passes = gmax.passes;
     run->P = gmax.P;
@@ -481,10 +572,11 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
     if (rc) return rc;
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     if ((rc = issue(-1)) || (nslices > 0 && (rc = issue(0)))) return rc;
-    cudaError_t e = cudaMemsetAsync(w.ctrl.p, 0, sizeof(Ctrl), st);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, r_ready, 0);
+    cudaError_t e = cudaStreamWaitEvent(st, r_ready, 0);
     if (e != cudaSuccess) return cuda_error(e, "sliced join: setup");
-    // R: histogram, bases and both passes, while S is still arriving
+    if ((rc = start_radix_join(gmax, dR, w, st))) return rc;
+    // R: histogram, bases and both passes (which step aside when the join is
+    // direct, as every slice's do), while S is still arriving
     if ((rc = part_histogram(0, gmax, dR, cfg, w, st, nullptr))) return rc;
     if ((rc = part_pass(0, 1, gmax, dR, w, st, false))) return rc;
     if ((rc = part_pass(0, 2, gmax, dR, w, st, false))) return rc;
@@ -493,10 +585,11 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
         const uint64_t n = s_lo[k + 1] - s_lo[k];
         if (!n) continue;
         const Row *d = dS + s_lo[k];
-        const RadixGeom g = radix_geometry(cfg, nR, n, capR, w);
+        RadixGeom g = radix_geometry(cfg, nR, n, capR, w);
+        g.direct = gmax.direct;
         if ((e = cudaStreamWaitEvent(st, s_ready[k], 0)) != cudaSuccess) return cuda_error(e, "sliced join: wait");
-        if ((rc = part_histogram(1, g, d, cfg, w, st, nullptr))) return rc;
-        if ((rc = plan_items(g, w, st))) return rc;
+        if ((rc = part_hist_read(1, g, d, cfg, w, st, nullptr))) return rc;
+        if ((rc = part_hist_plan(2, true, g, w, st))) return rc;
         if ((rc = part_pass(1, 1, g, d, w, st, false))) return rc;
         if ((rc = part_pass(1, 2, g, d, w, st, false))) return rc;
         // the join's work-item ticket restarts for every slice
@@ -525,6 +618,7 @@ int radix_join_phase(const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap, W
     ja.out = d_rows;
     ja.cap = d_rows ? cap : 0;
     ja.err = &ctrl->error;
+    ja.skip = &ctrl->direct;
     ja.gate = nullptr;
     ja.gate_max = 0;
     ja.gate_le = 0;

@@ -1,0 +1,382 @@
+// Direct counting join: when R's keys are distinct and lie in a compact
+// range, one bit per key value is a perfect hash table of R that fits the L2
+// cache (or shared memory), and S is joined while it is read for its
+// histogram, without being partitioned.
+//
+// The reference's counting RHO and RHT (Joins/radix_join.c:187-244, :374-440)
+// partition both relations so that every R partition's table fits a core's
+// cache.  Here the bit table does: 2^27 keys are 16.8 MB, a seventh of the
+// L2.  Counting needs no payloads, and a distinct key matches at most once,
+// so the bit is the whole table entry.
+//
+// Bit of key k: k mod 2^w.  With max - min < 2^w that is injective on
+// [min, max], so R can be entered while it is read for its histogram, before
+// its range is known:
+//   k_direct_prep   guesses w from a sample of R (no guess: not direct) and
+//                   clears the table;
+//   k_hist_build    R's chunk histograms (as k_hist_chunks), the key range,
+//                   and the bits;
+//   k_direct_decide counts the set bits: direct iff the range fits 2^w and
+//                   |R| bits are set (all keys distinct);
+//   k_hist_probe    S's chunk histograms, and with the decision the matches.
+// The histograms are the partitioned join's own, so when the decision is no,
+// the join continues with the passes, and the statistics (partition sizes,
+// work items) are the same either way.
+#include <algorithm>
+
+#include "part_dev.cuh"
+#include "tbg_runtime.h"
+
+namespace tbg {
+
+constexpr int DIRECT_THREADS = 1024;
+constexpr int DIRECT_MIN_LOG2 = 10;
+
+// log2 of the largest table considered for nR rows: 32 bits per row (a
+// filtered or sparse key range up to 1/32 full), at most 2^29 bits (67 MB).
+// Measured on 2^30 S rows: 4.02 ms for tables of 0.5 to 34 MB, 5.0 ms at
+// 67 MB, 10.9 ms at 134 MB (out of the L2), where the partitioned join takes
+// 11.4 ms or more.
+int direct_log2_max(uint64_t nR) {
+    int k = DIRECT_MIN_LOG2;
+    while (k < 29 && (1ull << k) < nR * 32) k++;
+    return k;
+}
+
+// Shared memory words for S's copy of the bit table: two bits per R row, at
+// most what a CTA can hold beside its histogram bins.  A table in shared
+// memory is read at the speed of S's stream (2^30 rows: 1.37 ms), one in L2
+// at one line per clock and SM (4.02 ms).  Zero when a table of one bit per
+// row would not fit: then every bit is read from L2 and the CTA keeps its
+// smaller footprint.
+uint32_t direct_smem_words(uint64_t nR, uint64_t nbins) {
+    constexpr uint64_t CAP = 220 * 1024 / 4;
+    if (nbins >= CAP) return 0;
+    const uint64_t cap = CAP - nbins;
+    if ((nR + 31) / 32 + 1 > cap) return 0;
+    const uint64_t want = std::max<uint64_t>(1024, (nR + 15) / 16);
+    return (uint32_t)std::min(want, cap);
+}
+
+// Clears the control block (CTA 0) and, when a sample of R allows a direct
+// join, the bit table.  Every CTA takes the same 1024 evenly spaced rows, so
+// all come to the same w: the sample's range plus an eighth (evenly spaced
+// rows of a relation in random or sorted order miss about 1/1024 of it at
+// either end; a range that is wider after all only means "not direct").
+__global__ void __launch_bounds__(DIRECT_THREADS) k_direct_prep(const Row *__restrict__ R, uint64_t nR,
+                                                                uint32_t *__restrict__ bits, int log2_max,
+                                                                Ctrl *ctrl) {
+    __shared__ uint32_t s_lo, s_hi;
+    const int tid = threadIdx.x;
+    if (blockIdx.x == 0)
+        for (int i = tid; i < (int)(sizeof(Ctrl) / 4); i += DIRECT_THREADS) reinterpret_cast<uint32_t *>(ctrl)[i] = 0;
+    if (tid == 0) {
+        s_lo = 0xFFFFFFFFu;
+        s_hi = 0;
+    }
+    __syncthreads();
+    const uint64_t i = nR <= DIRECT_THREADS ? tid : (uint64_t)tid * (nR - 1) / (DIRECT_THREADS - 1);
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+    if (i < nR) lo = hi = R[i].key;
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if ((tid & 31) == 0) {
+        atomicMin(&s_lo, lo);
+        atomicMax(&s_hi, hi);
+    }
+    __syncthreads();
+    const uint32_t span = s_hi - s_lo;
+    const uint64_t want = (uint64_t)span + span / 8 + 64;
+    const int w = max(DIRECT_MIN_LOG2, 64 - __clzll((long long)(want - 1)));
+    if (w > log2_max) return;
+    if (blockIdx.x == 0 && tid == 0) ctrl->direct_log2 = (unsigned)w;
+    uint4 *b4 = reinterpret_cast<uint4 *>(bits);
+    const uint64_t n4 = 1ull << (w - 7);
+    for (uint64_t q = (uint64_t)blockIdx.x * DIRECT_THREADS + tid; q < n4; q += (uint64_t)gridDim.x * DIRECT_THREADS)
+        b4[q] = make_uint4(0, 0, 0, 0);
+}
+
+// Streams rows [lo, hi) of `in` in rounds of 8 rows per thread: fn(x, ok)
+// with four row pairs and their validity, warp-uniform trip counts; edge(row)
+// for the rows outside the 16-byte aligned body (thread 0).
+template <class Fn, class Edge>
+__device__ __forceinline__ void stream_pairs(const Row *__restrict__ in, uint64_t lo, uint64_t hi, Fn fn, Edge edge) {
+    if (lo >= hi) return;
+    const uint64_t head = ((reinterpret_cast<uintptr_t>(in + lo) & 15) != 0) ? 1 : 0;
+    const uint64_t body = hi - lo - head;
+    const uint32_t nv = (uint32_t)(body / 2);
+    const uint4 *v = reinterpret_cast<const uint4 *>(in + lo + head);
+    for (uint32_t base = 0; base < nv; base += DIRECT_THREADS * 4) {
+        uint4 x[4];
+        bool ok[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t i = base + u * DIRECT_THREADS + threadIdx.x;
+            ok[u] = i < nv;
+            x[u] = ok[u] ? ldg_stream(v + i) : make_uint4(0, 0, 0, 0);
+        }
+        fn(x, ok);
+    }
+    if (threadIdx.x == 0) {
+        if (head) edge(in[lo]);
+        if (body & 1) edge(in[hi - 1]);
+    }
+}
+
+__device__ __forceinline__ void hist_pairs(uint32_t *sh, const RadixF &rf, const uint4 (&x)[4], const bool (&ok)[4]) {
+    const bool dup = warp_has_dups(radix_f(rf, x[0].x), ok[0]);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        hist_add_warp(sh, radix_f(rf, x[u].x), ok[u], dup);
+        hist_add_warp(sh, radix_f(rf, x[u].z), ok[u], dup);
+    }
+}
+
+// R: chunk histograms, key range, bits.  The first sixteenth of a chunk's
+// rounds enters its bits with a returning atomic and gives up (for the whole
+// grid, through ctrl->direct_dup) at the first key already there: a relation
+// with many duplicates costs little before it takes the passes.  The other
+// rounds use atomics without a result, and a duplicate there shows in the
+// count of set bits.  Bound by the L2's atomics: 2^27 rows take 0.80 ms
+// without results against 1.17 ms with; the histogram read alone 0.16 ms.
+__global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__restrict__ in, uint64_t n, uint64_t chunk,
+                                                                  uint32_t *__restrict__ hist, int nbins, RadixF rf,
+                                                                  uint32_t *__restrict__ bits, Ctrl *ctrl) {
+    extern __shared__ uint32_t sh[];
+    __shared__ uint32_t s_inv, s_hi;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < nbins; i += DIRECT_THREADS) sh[i] = 0;
+    if (tid == 0) s_inv = s_hi = 0;
+    __syncthreads();
+    const unsigned w = ctrl->direct_log2;
+    const uint32_t wmask = w ? (uint32_t)((1ull << w) - 1) : 0u;
+    const uint64_t lo = (uint64_t)blockIdx.x * chunk;
+    const uint64_t hi = umin64(n, lo + chunk);
+    volatile unsigned *gave_up = &ctrl->direct_dup;
+    bool enter = w != 0;  // the same for all lanes of a warp
+    uint32_t kinv = 0, kmax = 0;  // largest ~key (the smallest key) and largest key
+    const uint32_t careful = (uint32_t)(chunk / (16 * 8 * DIRECT_THREADS)) + 1;
+    uint32_t round = 0;
+    auto set_bit = [&](uint32_t key, bool ret) {
+        const uint32_t s = key & wmask;
+        kinv = max(kinv, ~key);
+        kmax = max(kmax, key);
+        if (!ret) {
+            atomicOr(bits + (s >> 5), 1u << (s & 31));
+            return false;
+        }
+        return ((atomicOr(bits + (s >> 5), 1u << (s & 31)) >> (s & 31)) & 1u) != 0;
+    };
+    stream_pairs(
+        in, lo, hi,
+        [&](const uint4(&x)[4], const bool(&ok)[4]) {
+            if (enter) {
+                if (round < careful) {
+                    bool dup = false;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        if (ok[u]) {
+                            dup |= set_bit(x[u].x, true);
+                            dup |= set_bit(x[u].z, true);
+                        }
+                    }
+                    // one lane per warp touches the flag: all of them storing
+                    // it took 0.5 ms from a 2^22 x 2^24 join with triplicate keys
+                    dup = __any_sync(0xffffffffu, dup);
+                    unsigned seen = 0;
+                    if ((tid & 31) == 0) {
+                        seen = *gave_up;
+                        if (dup && !seen) *gave_up = 1;
+                    }
+                    enter = !dup && __shfl_sync(0xffffffffu, seen, 0) == 0;
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        if (ok[u]) {
+                            set_bit(x[u].x, false);
+                            set_bit(x[u].z, false);
+                        }
+                    }
+                }
+                round++;
+            }
+            __syncwarp();
+            hist_pairs(sh, rf, x, ok);
+        },
+        [&](const Row &r) {
+            if (enter) set_bit(r.key, false);
+            atomicAdd(&sh[radix_f(rf, r.key)], 1u);
+        });
+    if (w) {
+        for (int o = 16; o > 0; o >>= 1) {
+            kinv = max(kinv, __shfl_xor_sync(0xffffffffu, kinv, o));
+            kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
+        }
+        if ((tid & 31) == 0) {
+            atomicMax(&s_inv, kinv);
+            atomicMax(&s_hi, kmax);
+        }
+    }
+    __syncthreads();
+    if (w && tid == 0 && lo < hi) {
+        atomicMax(&ctrl->direct_inv_min, s_inv);
+        atomicMax(&ctrl->direct_max, s_hi);
+    }
+    uint32_t *dst = hist + (uint64_t)blockIdx.x * nbins;
+    for (int i = tid; i < nbins; i += DIRECT_THREADS) dst[i] = sh[i];
+}
+
+// Counts the set bits; the last CTA decides.  The table is read from L2
+// (2^27 keys: 33.5 MB, half of it R's range).
+__global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t *__restrict__ bits, uint64_t nR,
+                                                                  Ctrl *ctrl) {
+    __shared__ unsigned s_count;
+    const unsigned w = ctrl->direct_log2;
+    if (!w || ctrl->direct_dup) return;
+    const int tid = threadIdx.x;
+    if (tid == 0) s_count = 0;
+    __syncthreads();
+    const uint4 *b4 = reinterpret_cast<const uint4 *>(bits);
+    const uint64_t n4 = 1ull << (w - 7);
+    unsigned c = 0;  // at most 2^29 bits in all
+#pragma unroll 4
+    for (uint64_t q = (uint64_t)blockIdx.x * DIRECT_THREADS + tid; q < n4; q += (uint64_t)gridDim.x * DIRECT_THREADS) {
+        const uint4 x = __ldcg(b4 + q);
+        c += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((tid & 31) == 0 && c) atomicAdd(&s_count, c);
+    __syncthreads();
+    if (tid == 0) {
+        atomicAdd(&ctrl->direct_bits, (unsigned long long)s_count);
+        __threadfence();
+        if (atomicAdd(&ctrl->done[2], 1u) == gridDim.x - 1) {
+            __threadfence();
+            const unsigned long long set = atomicAdd(&ctrl->direct_bits, 0ull);
+            if (set == nR && (uint64_t)(ctrl->direct_max - ~ctrl->direct_inv_min) < (1ull << w)) ctrl->direct = 1;
+        }
+    }
+}
+
+// One word of the bit table from L2, not kept in L1 (a line of it is rarely
+// asked for again before it would be replaced).
+__device__ __forceinline__ uint32_t ld_bits(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+// S: chunk histograms and, when the join is direct, the matches.  Two
+// launches, of which one does the work: SMEM reads the table from a copy in
+// shared memory (the words from R's smallest key to its largest, when they
+// fit `smem_words`), the other from L2, and it is the plain histogram when the
+// join is not direct.  (One launch for both would hold the copy's shared
+// memory, and so one CTA per SM, for the plain histogram too: a sparse 2^20 x
+// 2^22 join took 182 us instead of 140 us.)  Bound by the L1's one line per
+// clock and SM for the table in L2: 2^30 rows 4.13 ms (8 B/row: 2.1 TB/s; 4.02
+// ms without the histogram), and by S's read from HBM for the table in shared
+// memory.  The partitioned join reads and writes 40 more bytes per row of S.
+template <bool SMEM>
+__global__ void __launch_bounds__(DIRECT_THREADS, 2)
+    k_hist_probe(const Row *__restrict__ in, uint64_t n, uint64_t chunk, uint32_t *__restrict__ hist, int nbins, RadixF rf,
+                 const uint32_t *__restrict__ bits, uint32_t smem_words, Ctrl *ctrl) {
+    const bool direct = ctrl->direct != 0;
+    const uint32_t kmin = ~ctrl->direct_inv_min, span = ctrl->direct_max - kmin;
+    const uint32_t wordmask = direct ? (uint32_t)((1ull << (ctrl->direct_log2 - 5)) - 1) : 0u;
+    const uint32_t w0 = kmin >> 5;
+    const uint32_t words = ((kmin + span) >> 5) - w0 + 1;
+    if (SMEM != (direct && words <= smem_words)) return;
+    extern __shared__ uint32_t sh[];
+    uint32_t *copy = sh + nbins;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < nbins; i += DIRECT_THREADS) sh[i] = 0;
+    if (SMEM)
+        for (uint32_t i = tid; i < words; i += DIRECT_THREADS) copy[i] = ld_bits(bits + ((w0 + i) & wordmask));
+    __syncthreads();
+    const uint64_t lo = (uint64_t)blockIdx.x * chunk;
+    const uint64_t hi = umin64(n, lo + chunk);
+    uint32_t matches = 0;  // a chunk holds < 2^32 rows, and a row matches at most once
+    auto word = [&](uint32_t key, bool ok) -> uint32_t {
+        if (!ok || key - kmin > span) return 0;
+        return SMEM ? copy[(key >> 5) - w0] : ld_bits(bits + ((key >> 5) & wordmask));
+    };
+    auto bit = [](uint32_t word, uint32_t key) { return (word >> (key & 31)) & 1u; };
+    stream_pairs(
+        in, lo, hi,
+        [&](const uint4(&x)[4], const bool(&ok)[4]) {
+            if (SMEM || direct) {
+                uint32_t a[8];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    a[2 * u] = word(x[u].x, ok[u]);
+                    a[2 * u + 1] = word(x[u].z, ok[u]);
+                }
+                hist_pairs(sh, rf, x, ok);  // while the words arrive
+#pragma unroll
+                for (int u = 0; u < 4; u++) matches += bit(a[2 * u], x[u].x) + bit(a[2 * u + 1], x[u].z);
+            } else {
+                hist_pairs(sh, rf, x, ok);
+            }
+        },
+        [&](const Row &r) {
+            if (SMEM || direct) matches += bit(word(r.key, true), r.key);
+            atomicAdd(&sh[radix_f(rf, r.key)], 1u);
+        });
+    if (SMEM || direct) {
+        const unsigned long long ws = warp_sum_u64(matches);
+        if ((tid & 31) == 0 && ws) atomicAdd(&ctrl->matches, ws);
+    }
+    __syncthreads();
+    uint32_t *dst = hist + (uint64_t)blockIdx.x * nbins;
+    for (int i = tid; i < nbins; i += DIRECT_THREADS) dst[i] = sh[i];
+}
+
+cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *bits, int log2_max, Ctrl *ctrl, int nsm,
+                               cudaStream_t st) {
+    const uint64_t n4 = 1ull << (log2_max - 7);
+    const unsigned g = (unsigned)std::min<uint64_t>((n4 + DIRECT_THREADS - 1) / DIRECT_THREADS, (uint64_t)nsm * 2);
+    k_direct_prep<<<g, DIRECT_THREADS, 0, st>>>(R, nR, bits, log2_max, ctrl);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
+                              uint32_t *bits, Ctrl *ctrl, cudaStream_t st) {
+    const int nbins = 1 << P_log2;
+    const size_t smem = (size_t)nbins * 4;
+    cudaError_t e = smem_limit((const void *)k_hist_build, smem);
+    if (e != cudaSuccess) return e;
+    k_hist_build<<<G, DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, bits, ctrl);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, Ctrl *ctrl, cudaStream_t st) {
+    const uint64_t n4 = 1ull << (log2_max - 7);
+    // two 16-byte words per thread and CTA at least, one CTA per SM at most
+    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), 148));
+    k_direct_decide<<<g, DIRECT_THREADS, 0, st>>>(bits, nR, ctrl);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
+                              const uint32_t *bits, uint64_t nR, Ctrl *ctrl, cudaStream_t st) {
+    const int nbins = 1 << P_log2;
+    const uint32_t words = direct_smem_words(nR, (uint64_t)nbins);
+    const size_t smem = (size_t)nbins * 4, smem_copy = smem + (size_t)words * 4;
+    cudaError_t e;
+    if (words) {
+        if ((e = smem_limit((const void *)k_hist_probe<true>, smem_copy)) != cudaSuccess) return e;
+        k_hist_probe<true><<<G, DIRECT_THREADS, smem_copy, st>>>(in, n, chunk, hist, nbins, rf, bits, words, ctrl);
+        count_launch();
+    }
+    if ((e = smem_limit((const void *)k_hist_probe<false>, smem)) != cudaSuccess) return e;
+    k_hist_probe<false><<<G, DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, bits, words, ctrl);
+    count_launch();
+    return cudaGetLastError();
+}
+
+}  // namespace tbg

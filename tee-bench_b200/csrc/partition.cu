@@ -115,11 +115,18 @@ __global__ void __launch_bounds__(HIST_THREADS) k_hist_chunks(const Row *__restr
 // owns 32 consecutive partitions (threadIdx.x, coalesced) and splits the
 // chunks into 32 segments (threadIdx.y): segment sums, a prefix over the
 // segments, then each segment rewritten with running prefixes.
+// K3 planner: partition bases and join work items.  Replaces the task
+// creation of Joins/radix_join.c:946-1000 and :609-617 (pairs with both sides
+// non-empty); oversized S sides are split into several items.
+// One launch does K2 for both relations, and its last CTA K3: five launches
+// (two column scans, two base scans, the planner) took 24 us of the 120 us of
+// a 2^21 x 2^21 join.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_colscan(uint32_t *__restrict__ hist, int G, int P,
-                                                  uint32_t *__restrict__ totals) {
-    __shared__ uint32_t seg[32][33];
-    const int f = blockIdx.x * 32 + threadIdx.x;
+constexpr int PLAN_THREADS = 1024;
+
+__device__ void column_scan(uint32_t *__restrict__ hist, int G, int P, uint32_t *__restrict__ totals, int block,
+                            uint32_t (*seg)[33]) {
+    const int f = block * 32 + threadIdx.x;
     const int per = (G + 31) / 32;
     const int c0 = min(G, (int)threadIdx.y * per), c1 = min(G, c0 + per);
     uint32_t *col = hist + f;
@@ -168,64 +175,59 @@ __global__ void __launch_bounds__(1024) k_colscan(uint32_t *__restrict__ hist, i
     }
 }
 
-// ---------------------------------------------------------------------------
-// K3 planner (one CTA): partition bases and join work items.  Replaces the
-// task creation of Joins/radix_join.c:946-1000 and :609-617 (pairs with both
-// sides non-empty); oversized S sides are split into several items.
-// ---------------------------------------------------------------------------
-constexpr int PLAN_THREADS = 1024;
-
-// Shared-memory index of entry i when every thread scans 32 consecutive
-// entries: one word of padding per 32 keeps those reads conflict-free.
-__device__ __forceinline__ uint32_t skew32(uint32_t i) { return i + (i >> 5); }
-
-// Exclusive scan of hist[0..P) into base[0..P], base[P] = total, and the
-// largest entry into *maxp.  The counts are staged through shared memory
-// (`sh`, P + P / 32 words) so global reads and writes are coalesced.
-__device__ void plan_bases(const uint32_t *hist, uint64_t *base, int P, unsigned long long *maxp, uint64_t *scratch,
-                           uint32_t *sh) {
-    const int tid = threadIdx.x;
-    for (int i = tid; i < P; i += PLAN_THREADS) sh[skew32(i)] = hist[i];
-    __syncthreads();
-    const int C = (P + PLAN_THREADS - 1) / PLAN_THREADS;
-    const int lo = min(P, tid * C), hi = min(P, lo + C);
+// Exclusive scan of tot[0..P) into base[0..P], base[P] = total (rows counted:
+// n unless rows were bypassed), and the largest entry into *maxp, by one CTA
+// of PLAN_THREADS threads.  Warp w owns P / 32 consecutive entries and walks
+// them 32 at a time, so loads and stores are coalesced.
+__device__ void plan_bases(const uint32_t *tot, uint64_t *base, int P, unsigned long long *maxp, int tid,
+                           uint64_t *scratch) {
+    const int lane = tid & 31, w = tid >> 5;
+    const int per = ((P + 31) / 32 + 31) & ~31;
+    const int lo = min(P, w * per), hi = min(P, lo + per);
     uint64_t sum = 0;
     uint32_t mx = 0;
-    for (int f = lo; f < hi; f++) {
-        const uint32_t x = sh[skew32(f)];
+#pragma unroll 4
+    for (int f = lo + lane; f < hi; f += 32) {
+        const uint32_t x = __ldcg(tot + f);
         sum += x;
         mx = max(mx, x);
     }
-    uint64_t total;
-    uint64_t run = block_excl_scan<PLAN_THREADS>(sum, &total, scratch);
-    for (int f = lo; f < hi; f++) {  // prefixes fit 32 bits: a relation holds < 2^32 rows
-        const uint32_t x = sh[skew32(f)];
-        sh[skew32(f)] = (uint32_t)run;
-        run += x;
+    sum = warp_sum_u64(sum);
+    mx = warp_max_u32(mx);
+    if (lane == 0) {
+        scratch[w] = sum;
+        if (mx) atomicMax(maxp, (unsigned long long)mx);
     }
     __syncthreads();
-    for (int i = tid; i < P; i += PLAN_THREADS) base[i] = sh[skew32(i)];
-    if (tid == 0) base[P] = total;  // rows counted (n unless rows were bypassed)
-    unsigned wmax = warp_max_u32(mx);
-    if ((tid & 31) == 0 && wmax) atomicMax(maxp, (unsigned long long)wmax);
+    uint64_t run = 0, total = 0;
+    for (int k = 0; k < 32; k++) {
+        if (k == w) run = total;
+        total += scratch[k];
+    }
+#pragma unroll 4
+    for (int f0 = lo; f0 < hi; f0 += 32) {
+        const int f = f0 + lane;
+        const uint32_t x = f < hi ? __ldcg(tot + f) : 0;
+        uint32_t inc = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (f < hi) base[f] = run + inc - x;
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (tid == 0) base[P] = total;
+    __syncthreads();  // scratch is reused; base is complete for this CTA
 }
 
-__global__ void __launch_bounds__(PLAN_THREADS) k_plan_bases(const uint32_t *totals, uint64_t *base, int P_log2,
-                                                            unsigned long long *maxp) {
-    extern __shared__ uint32_t sh[];
-    __shared__ uint64_t scratch[PLAN_THREADS / 32 + 1];
-    plan_bases(totals, base, 1 << P_log2, maxp, scratch, sh);
-}
-
-// Join work items from both relations' totals and bases (written by
-// k_plan_bases), planned by P / PLAN_THREADS CTAs.  Every CTA first counts
-// the items of all partitions (one coalesced read of both totals, from L2) to
-// take the same split decision; then thread t of CTA c plans partition
-// c * PLAN_THREADS + t, and each warp reserves its items with one atomic on
-// ctrl->nitems (zeroed by the launcher).  The item list is in reservation
-// order, not sorted by partition.
-__global__ void __launch_bounds__(PLAN_THREADS) k_plan(PlanArgs a) {
-    __shared__ uint64_t scratch[PLAN_THREADS / 32 + 1];
+// Join work items from both relations' totals and bases, for partitions
+// block * PLAN_THREADS + tid.  Every call first counts the items of all
+// partitions (one coalesced read of both totals, from L2) to take the same
+// split decision; each warp then reserves its items with one atomic on
+// ctrl->nitems (zeroed before).  The item list is in reservation order, not
+// sorted by partition.
+__device__ void plan_block(const PlanArgs &a, int block, int tid, uint64_t *scratch) {
     const int P = 1 << a.P_log2;
     // S sides larger than capS are split (skew) for every R chunk of the
     // partition; if that would overflow the item buffer, partitions whose R
@@ -235,22 +237,26 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(PlanArgs a) {
         return (hs + a.capS - 1) / a.capS;
     };
     uint64_t cnt_all = 0;
-    for (int f = threadIdx.x; f < P; f += PLAN_THREADS) {
-        const uint32_t hr = a.r.hist[f], hs = a.s.hist[f];
+    for (int f = tid; f < P; f += PLAN_THREADS) {
+        const uint32_t hr = __ldcg(a.r.hist + f), hs = __ldcg(a.s.hist + f);
         if (hr == 0 || hs == 0) continue;
         const uint64_t nrc = (hr + (uint64_t)a.capR - 1) / a.capR;
         cnt_all += nrc * s_chunks(hs, nrc, true);
     }
-    uint64_t total_all;
-    block_excl_scan<PLAN_THREADS>(cnt_all, &total_all, scratch);
+    const int lane = tid & 31, w = tid >> 5;
+    cnt_all = warp_sum_u64(cnt_all);
+    if (lane == 0) scratch[w] = cnt_all;
+    __syncthreads();
+    uint64_t total_all = 0;
+    for (int k = 0; k < PLAN_THREADS / 32; k++) total_all += scratch[k];
+    __syncthreads();
     const bool split_all = total_all <= a.item_cap;
-    const int f = blockIdx.x * PLAN_THREADS + threadIdx.x;
-    const int lane = threadIdx.x & 31;
+    const int f = block * PLAN_THREADS + tid;
     uint32_t hr = 0, hs = 0;
     uint64_t nrc = 0, nsc = 0;
     if (f < P) {
-        hr = a.r.hist[f];
-        hs = a.s.hist[f];
+        hr = __ldcg(a.r.hist + f);
+        hs = __ldcg(a.s.hist + f);
         if (hr && hs) {
             nrc = (hr + (uint64_t)a.capR - 1) / a.capR;
             nsc = s_chunks(hs, nrc, split_all);
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(PlanArgs a) {
     if (mine && !fits) atomicCAS(&a.ctrl->error, 0u, (unsigned)TBG_ERR_CAPACITY);
     if (mine && fits) {
         const uint64_t sstep = (hs + nsc - 1) / nsc;
-        const uint64_t rb = a.r.base[f], sb = a.s.base[f];
+        const uint64_t rb = __ldcg(a.r.base + f), sb = __ldcg(a.s.base + f);
         for (uint64_t rc = 0; rc < nrc; rc++) {
             for (uint64_t sc = 0; sc < nsc; sc++) {
                 Item it;
@@ -290,14 +296,57 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(PlanArgs a) {
     if (lane == 0 && ne) atomicAdd(&a.ctrl->nonempty, (unsigned long long)ne);
 }
 
+// Column scans of relation 0 in CTAs [0, cols of it), of relation 1 in the
+// rest.  With t.rels, the last CTA to finish (a ticket on *t.done, which it
+// resets) scans the bases of the relations in the mask t.rels and, with
+// t.items, plans the work items.
+__global__ void __launch_bounds__(PLAN_THREADS) k_colscan(ColScan r, ColScan s, PlanTail t) {
+    __shared__ uint32_t seg[32][33];
+    __shared__ uint64_t scratch[PLAN_THREADS / 32 + 1];
+    __shared__ bool s_last;
+    const int cols_r = (r.P + 31) / 32;
+    if ((int)blockIdx.x < cols_r) column_scan(r.hist, r.G, r.P, r.totals, blockIdx.x, seg);
+    else column_scan(s.hist, s.G, s.P, s.totals, blockIdx.x - cols_r, seg);
+    if (!t.rels) return;
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(t.done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const int P = 1 << t.plan.P_log2;
+    if (t.rels & 1) plan_bases(t.plan.r.hist, t.plan.r.base, P, &t.plan.ctrl->max_part_R, tid, scratch);
+    if (t.rels & 2) plan_bases(t.plan.s.hist, t.plan.s.base, P, &t.plan.ctrl->max_part_S, tid, scratch);
+    if (tid == 0) {
+        *t.done = 0;
+        if (t.items) t.plan.ctrl->nitems = 0;
+    }
+    if (!t.items) return;
+    __threadfence();
+    __syncthreads();
+    for (int b = 0; b * PLAN_THREADS < P; b++) {
+        plan_block(t.plan, b, tid, scratch);
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(PLAN_THREADS) k_plan(PlanArgs a) {
+    __shared__ uint64_t scratch[PLAN_THREADS / 32 + 1];
+    plan_block(a, blockIdx.x, threadIdx.x, scratch);
+}
+
 // ---------------------------------------------------------------------------
 // K4 pass 1: CTA c scatters chunk c by d1.  With one pass, d1 is f itself.
+// Both passes take up to two relations (the second one null for one): S's
+// CTAs come first, and R's, fewer and shorter, fill the last wave.
 // ---------------------------------------------------------------------------
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_pass1(PartArgs a) {
+__device__ __forceinline__ void part_pass1(const PartArgs &a, const int c) {
+    if (a.skip && *a.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto &sm = *reinterpret_cast<PassSmem<THREADS> *>(smem_raw);
-    const int c = blockIdx.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     const int P = 1 << (a.b1 + a.b2);
     const int F = 1 << a.b1;
     const uint32_t *pre = a.pre + (uint64_t)c * P;
@@ -353,13 +402,13 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_pass1(PartArgs
 // K5 pass 2: unit (c, s), s-major, scatters by d2 within pass-1 partition s.
 // ---------------------------------------------------------------------------
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_pass2(PartArgs a) {
+__device__ __forceinline__ void part_pass2(const PartArgs &a, const unsigned unit) {
+    if (a.skip && *a.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto &sm = *reinterpret_cast<PassSmem<THREADS> *>(smem_raw);
     const int F1 = 1 << a.b1, F2 = 1 << a.b2;
     const int P = F1 * F2;
     const int ngroups = (a.G + a.group - 1) / a.group;
-    const uint64_t unit = blockIdx.x;
     const int s = (int)(unit / ngroups), g = (int)(unit % ngroups);
     const int c0 = g * a.group, c1 = min(a.G, c0 + a.group) - 1;
     // chunk c's rows of partition s follow chunk c-1's in the pass-1 output,
@@ -373,6 +422,24 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_pass2(PartArgs
     }
     __syncthreads();
     part_range<THREADS>(a.in, lo, hi, a.n, a.out, (uint32_t)a.n, a.d2, F2, sm, a.err);
+}
+
+// The two relations of a launch take two copies of the pass in the code:
+// reading the arguments through one selected pointer costs registers that the
+// pass does not have (64 of 64 in use; with it the passes ran 5% slower).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+    k_part_pass1(const __grid_constant__ PartArgs a, const __grid_constant__ PartArgs b) {
+    if (blockIdx.x < (unsigned)a.G) part_pass1<THREADS>(a, blockIdx.x);
+    else part_pass1<THREADS>(b, blockIdx.x - a.G);
+}
+
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+    k_part_pass2(const __grid_constant__ PartArgs a, const __grid_constant__ PartArgs b) {
+    const unsigned units = (unsigned)((a.G + a.group - 1) / a.group) << a.b1;
+    if (blockIdx.x < units) part_pass2<THREADS>(a, blockIdx.x);
+    else part_pass2<THREADS>(b, blockIdx.x - units);
 }
 
 // ---------------------------------------------------------------------------
@@ -398,18 +465,13 @@ cudaError_t launch_hist_chunks(const Row *in, uint64_t n, uint64_t chunk, int G,
 }
 
 cudaError_t launch_colscan(uint32_t *hist, int G, int P, uint32_t *totals, cudaStream_t st) {
-    k_colscan<<<(P + 31) / 32, dim3(32, 32), 0, st>>>(hist, G, P, totals);
+    k_colscan<<<(P + 31) / 32, dim3(32, 32), 0, st>>>(ColScan{hist, totals, G, P}, ColScan{}, PlanTail{});
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_plan_bases(const uint32_t *totals, uint64_t *base, int P_log2, unsigned long long *maxp,
-                              cudaStream_t st) {
-    const int P = 1 << P_log2;
-    const size_t smem = (size_t)(P + P / 32 + 1) * sizeof(uint32_t);
-    cudaError_t e = smem_limit((const void *)k_plan_bases, smem);
-    if (e != cudaSuccess) return e;
-    k_plan_bases<<<1, PLAN_THREADS, smem, st>>>(totals, base, P_log2, maxp);
+cudaError_t launch_colscan_plan(const ColScan &r, const ColScan &s, const PlanTail &t, cudaStream_t st) {
+    k_colscan<<<(r.P + 31) / 32 + (s.P + 31) / 32, dim3(32, 32), 0, st>>>(r, s, t);
     count_launch();
     return cudaGetLastError();
 }
@@ -423,23 +485,23 @@ cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_part_pass1(const PartArgs &a, cudaStream_t st) {
+cudaError_t launch_part_pass1(const PartArgs &a, const PartArgs *b, cudaStream_t st) {
     constexpr int T = PASS1_THREADS;
     const size_t smem = sizeof(PassSmem<T>);
     cudaError_t e = smem_limit((const void *)k_part_pass1<T>, smem);
     if (e != cudaSuccess) return e;
-    k_part_pass1<T><<<a.G, T, smem, st>>>(a);
+    k_part_pass1<T><<<a.G + (b ? b->G : 0), T, smem, st>>>(a, b ? *b : a);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_part_pass2(const PartArgs &a, cudaStream_t st) {
+cudaError_t launch_part_pass2(const PartArgs &a, const PartArgs *b, cudaStream_t st) {
     constexpr int T = PASS2_THREADS;
     const size_t smem = sizeof(PassSmem<T>);
     cudaError_t e = smem_limit((const void *)k_part_pass2<T>, smem);
     if (e != cudaSuccess) return e;
-    const uint64_t units = (uint64_t)((a.G + a.group - 1) / a.group) << a.b1;
-    k_part_pass2<T><<<(unsigned)units, T, smem, st>>>(a);
+    auto units = [](const PartArgs &p) { return (uint64_t)((p.G + p.group - 1) / p.group) << p.b1; };
+    k_part_pass2<T><<<(unsigned)(units(a) + (b ? units(*b) : 0)), T, smem, st>>>(a, b ? *b : a);
     count_launch();
     return cudaGetLastError();
 }

@@ -40,7 +40,15 @@ struct Ctrl {
     unsigned long long nonempty;  // partitions with both sides non-empty
     unsigned long long heavy_rows_S;
     unsigned long long heavy_keys;
-    unsigned long long pad[3];
+    // direct counting join (direct.cu)
+    unsigned long long direct_bits;  // bits set in the table
+    unsigned int direct;             // 1: S was joined in its histogram read, the passes have nothing to do
+    unsigned int direct_log2;        // log2 of the table's bits, 0: not tried
+    unsigned int direct_dup;         // a key of R occurred twice
+    unsigned int direct_inv_min;     // ~(smallest key of R), kept as a maximum so that it starts at 0
+    unsigned int direct_max;         // largest key of R
+    unsigned int done[4];            // CTA tickets: column scans of R and of S, the bit count
+    unsigned int pad;
 };
 
 // Digits per pass of the tile scatter (part_dev.cuh).
@@ -104,6 +112,7 @@ struct PartArgs {
     uint32_t *off1;           // [G][F1] start of unit (c, s) in the pass-1 output
     uint32_t *cnt1;           // [G][F1] rows of unit (c, s)
     unsigned *err;
+    const unsigned *skip;     // the launch steps aside when *skip is set (null: never)
 };
 
 struct JoinArgs {
@@ -120,6 +129,7 @@ struct JoinArgs {
     const unsigned long long *gate;
     unsigned long long gate_max;
     int gate_le;
+    const unsigned *skip;      // the launch steps aside when *skip is set (null: never)
     unsigned long long *matches;
     unsigned long long *rows_ctr;
     tbg_row_out *out;
@@ -138,20 +148,45 @@ struct PlanArgs {
     Ctrl *ctrl;
 };
 
+// One relation's chunk histograms [G][P] for the column scan (P = 0: none).
+struct ColScan {
+    uint32_t *hist = nullptr;
+    uint32_t *totals = nullptr;  // [P], written
+    int G = 0, P = 0;
+};
+
+// What the column scan's last CTA does (plan.r / plan.s hold the totals).
+struct PlanTail {
+    int rels = 0;              // bit 0: R's bases, bit 1: S's
+    int items = 0;             // also the work items
+    unsigned *done = nullptr;  // CTA ticket, zero before and after
+    PlanArgs plan{};
+};
+
 // ---- launchers (partition.cu, join.cu, gen.cu) ----
 cudaError_t launch_hist_chunks(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist,
                                int P_log2, RadixF rf, cudaStream_t st,
                                unsigned long long *out_of_range = nullptr, uint32_t range_max = 0);
 cudaError_t launch_colscan(uint32_t *hist, int G, int P, uint32_t *totals, cudaStream_t st);
+cudaError_t launch_colscan_plan(const ColScan &r, const ColScan &s, const PlanTail &t, cudaStream_t st);
 cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st);
-cudaError_t launch_plan_bases(const uint32_t *totals, uint64_t *base, int P_log2, unsigned long long *maxp,
-                              cudaStream_t st);
-cudaError_t launch_part_pass1(const PartArgs &a, cudaStream_t st);
-cudaError_t launch_part_pass2(const PartArgs &a, cudaStream_t st);
+// b: a second relation in the same launch (null: none)
+cudaError_t launch_part_pass1(const PartArgs &a, const PartArgs *b, cudaStream_t st);
+cudaError_t launch_part_pass2(const PartArgs &a, const PartArgs *b, cudaStream_t st);
 cudaError_t launch_join(const JoinArgs &a, bool materialize, int grid, cudaStream_t st);
 size_t join_smem_bytes(int capR);
 size_t join_launch_smem(int capR, bool materialize, int layout);
 int join_ctas_per_sm(int capR, bool materialize, int layout);
+
+// ---- direct counting join (direct.cu) ----
+int direct_log2_max(uint64_t nR);
+cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *bits, int log2_max, Ctrl *ctrl, int nsm,
+                               cudaStream_t st);
+cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
+                              uint32_t *bits, Ctrl *ctrl, cudaStream_t st);
+cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, Ctrl *ctrl, cudaStream_t st);
+cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
+                              const uint32_t *bits, uint64_t nR, Ctrl *ctrl, cudaStream_t st);
 
 cudaError_t launch_gen_pk(Row *d, uint64_t n, uint64_t seed, cudaStream_t st);
 cudaError_t launch_gen_fk(Row *d, uint64_t n, uint64_t maxid, uint64_t seed, cudaStream_t st);

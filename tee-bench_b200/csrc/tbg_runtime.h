@@ -33,6 +33,7 @@ struct Workspace {
     DevBuf chain_rows, chain_rel;  // chained join: first join's rows and the relation made of them
     DevBuf aux[8];              // algorithm-specific scratch (sort, learned model)
     DevBuf shard;               // shard split: per-chunk histograms and totals
+    DevBuf direct;              // direct counting join: R's bit table
     Ctrl *host_ctrl = nullptr;  // pinned mirror of the control block
     static constexpr size_t HOST_SMALL_BYTES = 4096;
     void *host_small = nullptr;  // pinned HOST_SMALL_BYTES: mid-call read-backs (LRN's decision, shard totals)
@@ -88,6 +89,7 @@ struct RadixGeom {
     // S's histogram also counts keys with key - rf.sub > s_range_max into
     // ctrl->out_of_range (S binned by R's key range); 0xFFFFFFFF: no check
     uint32_t s_range_max = 0xFFFFFFFFu;
+    bool direct = false;  // the histogram reads try the direct counting join
 };
 RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int capR, Workspace &w);
 RadixGeom radix_geometry_msd(uint64_t nR, uint64_t nS, uint32_t sub, int B, int lowbits, Workspace &w);

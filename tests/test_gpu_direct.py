@@ -1,0 +1,104 @@
+"""The direct counting join (one bit per key value, S joined while it is read
+for its histogram): RHO and RHT under the automatic plan, against the oracle
+and against the partitioned join that a fixed number of passes selects.
+Counts and partition statistics are whole numbers, so equality is exact."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from gpu_util import run_join, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def relations(oracle, rng, nR, nS, lo, step, miss):
+    """R: nR distinct keys lo + step * i in random order; S: a share `miss` of
+    its rows has a key that R lacks (around and between R's keys)."""
+    R = np.zeros(nR, dtype=oracle.ROW)
+    S = np.zeros(nS, dtype=oracle.ROW)
+    keys = (lo + step * np.arange(nR, dtype=np.uint64)) & 0xFFFFFFFF
+    R["key"] = rng.permutation(keys)
+    S["key"] = R["key"][rng.integers(0, nR, nS)]
+    other = (lo - 50 + rng.integers(0, step * nR + 100, nS).astype(np.int64)) % (1 << 32)
+    S["key"] = np.where(rng.random(nS) < miss, other, S["key"])
+    oracle.fill_payloads(R, 0)
+    oracle.fill_payloads(S, 1)
+    return R, S
+
+
+# |R|, |S|, smallest key, key step, misaligned: one row, sizes around a round of
+# a CTA (8192 rows) and around the table's words, the table in shared memory
+# (|R| up to 1.6 M) and in L2, ranges that start and end at the ends of 32 bits,
+# sparse ranges that just fit (step 24) and that do not (step 40)
+CASES = [(1, 1, 5, 1, 0), (1, 70000, 0, 1, 1), (31, 4097, 1, 1, 0), (33, 4095, 4294967295 - 32, 1, 1),
+         (8191, 16385, 1, 1, 0), (8193, 65537, 31, 3, 1), (100003, 300007, 0, 24, 0), (100003, 300007, 1, 40, 1),
+         (262144, 1 << 20, 1, 1, 0), (1500001, 3000017, 77, 1, 1), (3000001, 5000011, 1 << 31, 2, 0)]
+
+
+@pytest.mark.parametrize("algo", ["RHO", "RHT"])
+@pytest.mark.parametrize("nR,nS,lo,step,off", CASES)
+def test_direct_join(tbg, oracle, cuda, algo, nR, nS, lo, step, off):
+    rng = np.random.default_rng(nR + step)
+    R, S = relations(oracle, rng, nR, nS, lo, step, 0.3)
+    ref = oracle.rho(R, S)
+    m, _, st = run_join(tbg, cuda, algo, R, S, offset=off)
+    assert m == ref
+    m2, _, st2 = run_join(tbg, cuda, algo, R, S, offset=off, passes=st.passes)  # the partitioned join
+    assert m2 == ref
+    for f in ("partitions", "work_items", "max_part_R", "max_part_S", "mean_part_R", "mean_part_S", "imbalance",
+              "radix_bits", "passes"):
+        assert getattr(st, f) == getattr(st2, f), f
+
+
+@pytest.mark.parametrize("where", ["first", "last", "many", "all"])
+def test_duplicate_keys_of_R_take_the_passes(tbg, oracle, cuda, where):
+    """One duplicate that the careful first rounds see, one that only the
+    count of set bits shows, many, and a relation of one key."""
+    rng = np.random.default_rng(3)
+    R, S = relations(oracle, rng, 400009, 700001, 1, 1, 0.2)
+    if where == "first":
+        R["key"][1] = R["key"][0]
+    elif where == "last":
+        R["key"][-1] = R["key"][-2]
+    elif where == "many":
+        R["key"] = rng.integers(1, 150000, len(R))
+    else:
+        R["key"], S = 9, S[:2000].copy()
+        S["key"][::7] = 9
+    ref = oracle.rho(R, S)
+    m, _, st = run_join(tbg, cuda, "RHO", R, S)
+    assert m == ref
+
+
+def test_direct_outlier_outside_the_sample(tbg, oracle, cuda):
+    """A key far outside the sampled range: not direct, same count."""
+    rng = np.random.default_rng(4)
+    R, S = relations(oracle, rng, 300000, 500000, 1, 1, 0.1)
+    R["key"][7], S["key"][11] = 4000000000, 4000000000
+    ref = oracle.rho(R, S)
+    m, _, st = run_join(tbg, cuda, "RHO", R, S)
+    assert m == ref
+
+
+def test_direct_async_and_sliced(tbg, oracle, cuda):
+    """Nothing waits in the asynchronous call and between the slices of the
+    drop-in call: the passes are launched and step aside (or not)."""
+    rng = np.random.default_rng(5)
+    R, S = relations(oracle, rng, 60013, 250007, 1, 1, 0.25)
+    D = R.copy()
+    D["key"][0] = D["key"][1]
+    s = cuda.cuda.current_stream().cuda_stream
+    out = cuda.zeros(2, dtype=cuda.int64, device="cuda")
+    tS, pS = to_dev(cuda, S)
+    for k, rel in enumerate((R, D)):
+        tR, pR = to_dev(cuda, rel)
+        tbg.join_device_async(tbg.config("RHO"), pR, len(rel), pS, len(S), out.data_ptr() + 8 * k, stream=s)
+        assert tbg.lib().tbg_sync_status(s) == 0
+    refs = [oracle.rho(R, S), oracle.rho(D, S)]
+    assert out.tolist() == refs
+    prev = tbg.set_dropin_slices(5)
+    try:
+        assert [tbg.find("RHT").join(rel, S) for rel in (R, D)] == refs
+    finally:
+        tbg.set_dropin_slices(prev)
