@@ -315,8 +315,8 @@ int ensure_radix_buffers(const RadixGeom &g, bool bypass, Workspace &w) {
 // Per-chunk histograms of one relation (with the heavy bypass for S when
 // given).  With g.direct the read of R also enters its keys into the bit
 // table, and the read of S counts the matches when the join is direct.
-static int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w,
-                          cudaStream_t st, const SBypass *bypass) {
+int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w, cudaStream_t st,
+                   const SBypass *bypass) {
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     DevBuf &hist = rel ? w.histS : w.histR;
     cudaError_t e;
@@ -381,7 +381,7 @@ static constexpr uint64_t PLAN_TAIL_PARTS = 2048;
 // Column prefix of the histograms, partition totals and bases of the
 // relations in the mask `rels` (bit 0: R, bit 1: S) and, with `items`, the
 // join's work items (both relations' totals and bases must be there then).
-static int part_hist_plan(int rels, bool items, const RadixGeom &g, Workspace &w, cudaStream_t st) {
+int part_hist_plan(int rels, bool items, const RadixGeom &g, Workspace &w, cudaStream_t st) {
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     ColScan c[2];
     if (rels & 1) c[0] = ColScan{w.histR.as<uint32_t>(), w.totR.as<uint32_t>(), g.G[0], (int)g.P};
@@ -490,8 +490,7 @@ int plan_items(const RadixGeom &g, Workspace &w, cudaStream_t st) {
 }
 
 // Both partitioning passes of R and S.
-static int both_passes(const tbg_config &cfg, const RadixGeom &g, const Row *dR, const Row *dS, Workspace &w,
-                       cudaStream_t st) {
+int both_passes(const tbg_config &cfg, const RadixGeom &g, const Row *dR, const Row *dS, Workspace &w, cudaStream_t st) {
     const bool timing = cfg.timing != 0;
     int rc;
     if ((rc = part_pass_both(1, g, dR, dS, w, st))) return rc;

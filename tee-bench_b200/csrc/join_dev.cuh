@@ -184,15 +184,15 @@ __device__ void build_table(Table &t, const Row *__restrict__ R, uint64_t r_off,
     }
 }
 
-// Matches of S rows [0, len) (row pointer s, any 8-byte alignment) against
-// the table, this thread's share: 16-byte loads, four in flight, and with
+// Sum of fn(key) over rows [0, len) (row pointer s, any 8-byte alignment),
+// this thread's share: 16-byte loads, four in flight, and with
 // TBG_PROBE_AHEAD the next group of four issued before the current group is
-// probed (the loads of one group then overlap the probes of the previous).
+// looked up (the loads of one group then overlap the lookups of the previous).
 #ifndef TBG_PROBE_AHEAD
 #define TBG_PROBE_AHEAD 1
 #endif
-template <int THREADS, bool CG = false>
-__device__ __forceinline__ unsigned long long probe_count(const Table &t, const Row *s, uint64_t len) {
+template <int THREADS, bool CG = false, class Fn>
+__device__ __forceinline__ unsigned long long stream_sum(const Row *s, uint64_t len, Fn fn) {
     unsigned long long local = 0;
     const uint64_t head = ((reinterpret_cast<uintptr_t>(s) & 15) && len) ? 1 : 0;
     const uint64_t body = len - head;
@@ -200,8 +200,8 @@ __device__ __forceinline__ unsigned long long probe_count(const Table &t, const 
     const bool tail = body & 1;
     const uint4 *v = reinterpret_cast<const uint4 *>(s + head);
     const int tid = threadIdx.x;
-    if (head && tid == 0) local += t.count(ld_row<CG>(s, 0).x);
-    if (tail && tid == THREADS - 1) local += t.count(ld_row<CG>(s, len - 1).x);
+    if (head && tid == 0) local += fn(ld_row<CG>(s, 0).x);
+    if (tail && tid == THREADS - 1) local += fn(ld_row<CG>(s, len - 1).x);
     uint64_t i = tid;
     if (TBG_PROBE_AHEAD && i + 3 * THREADS < nv) {
         uint4 n0 = ld_pair<CG>(v + i), n1 = ld_pair<CG>(v + i + THREADS);
@@ -216,22 +216,28 @@ __device__ __forceinline__ unsigned long long probe_count(const Table &t, const 
                 n2 = ld_pair<CG>(v + i + 2 * THREADS);
                 n3 = ld_pair<CG>(v + i + 3 * THREADS);
             }
-            local += t.count(x0.x) + t.count(x0.z) + t.count(x1.x) + t.count(x1.z);
-            local += t.count(x2.x) + t.count(x2.z) + t.count(x3.x) + t.count(x3.z);
+            local += fn(x0.x) + fn(x0.z) + fn(x1.x) + fn(x1.z);
+            local += fn(x2.x) + fn(x2.z) + fn(x3.x) + fn(x3.z);
             if (!more) break;
         }
     }
     for (; i + 3 * THREADS < nv; i += 4 * THREADS) {
         uint4 x0 = ld_pair<CG>(v + i), x1 = ld_pair<CG>(v + i + THREADS);
         uint4 x2 = ld_pair<CG>(v + i + 2 * THREADS), x3 = ld_pair<CG>(v + i + 3 * THREADS);
-        local += t.count(x0.x) + t.count(x0.z) + t.count(x1.x) + t.count(x1.z);
-        local += t.count(x2.x) + t.count(x2.z) + t.count(x3.x) + t.count(x3.z);
+        local += fn(x0.x) + fn(x0.z) + fn(x1.x) + fn(x1.z);
+        local += fn(x2.x) + fn(x2.z) + fn(x3.x) + fn(x3.z);
     }
     for (; i < nv; i += THREADS) {
         uint4 x0 = ld_pair<CG>(v + i);
-        local += t.count(x0.x) + t.count(x0.z);
+        local += fn(x0.x) + fn(x0.z);
     }
     return local;
+}
+
+// Matches of S rows [0, len) against the table, this thread's share.
+template <int THREADS, bool CG = false>
+__device__ __forceinline__ unsigned long long probe_count(const Table &t, const Row *s, uint64_t len) {
+    return stream_sum<THREADS, CG>(s, len, [&](uint32_t k) { return t.count(k); });
 }
 
 }  // namespace tbg

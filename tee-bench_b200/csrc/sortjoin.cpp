@@ -5,7 +5,8 @@
 // PSM (Joins/psm/parallel_sortmerge_join.h:61-111) sorts both relations by key
 // and merges them.  The sort is MSD: RHO's histogram and passes partition by
 // the top bits of key - min (at most 15), then every bucket is sorted by the
-// remaining 12 or 13 bits in one counting pass.  Relations whose key range
+// remaining 12 or 13 bits in one counting pass (counting joins: every bucket's
+// R rows are counted per key value, k_bucket_count).  Relations whose key range
 // leaves more low bits, or with a bucket over a million rows (a heavy key),
 // take an LSD radix sort (7- to 9-bit digits, chunked stable passes).
 #include <algorithm>
@@ -130,6 +131,63 @@ cudaError_t launch_bucket_sort(const Row *in, Row *out, const uint64_t *base, ui
 static constexpr uint64_t kBucketMax = 1u << 20;
 static constexpr int kLowBits = 12, kLowBitsMax = 13;
 
+// Radix bits and low bits of an MSD sort of keys that span `span` bits; false
+// when the LSD sort takes them (no bits above the low ones, or too many low
+// bits).
+static bool msd_bits(int span, int *B, int *lowbits) {
+    *lowbits = std::min(span, kLowBits);
+    *B = span - *lowbits;
+    if (*B > 15) {
+        *B = 15;
+        *lowbits = span - *B;
+    }
+    return *B >= 1 && *lowbits <= kLowBitsMax;
+}
+
+cudaError_t launch_bucket_count(const JoinArgs &a, uint32_t sub, int lowbits, int nsm, cudaStream_t st);
+
+// Count-only PSM on MSD buckets: both relations partitioned by the top bits of
+// key - sub (sub: R's smallest key), then k_bucket_count.  Nothing waits, and
+// neither S's keys outside R's range nor heavy keys (S's buckets are split over
+// CTAs by the planner) need another plan.
+static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, uint32_t sub, int B,
+                     int lowbits, Workspace &w, cudaStream_t st, JoinRun *run) {
+    // one radix bit less where both plans take two passes: a pass costs more
+    // per bit above 7 than the larger buckets do (8 + 7 bits against 7 + 7 at
+    // 2^27 x 2^30: 4.64 against 3.79 ms for the second pass)
+    if (B > 9 && lowbits < kLowBitsMax) {
+        B--;
+        lowbits++;
+    }
+    RadixGeom g = radix_geometry_msd(nR, nS, sub, B, lowbits, w);
+    g.capR = 0x7FFFFFFF;  // counters take any number of R rows
+    g.capS = std::max<uint64_t>(65536, nS / ((uint64_t)w.nsm * 12));
+    g.item_cap = 2 * (nS / g.capS + 4 * g.P) + 16;
+    int rc = ensure_radix_buffers(g, false, w);
+    if (rc) return rc;
+    if ((rc = part_hist_read(0, g, dR, cfg, w, st, nullptr)) || (rc = part_hist_read(1, g, dS, cfg, w, st, nullptr)) ||
+        (rc = part_hist_plan(3, true, g, w, st)) || (rc = both_passes(cfg, g, dR, dS, w, st)))
+        return rc;
+    Ctrl *ctrl = w.ctrl.as<Ctrl>();
+    JoinArgs ja;
+    memset(&ja, 0, sizeof ja);
+    ja.R = w.partR.as<Row>();
+    ja.S = w.partS.as<Row>();
+    ja.items = w.items.as<Item>();
+    ja.nitems = &ctrl->nitems;
+    ja.item_ctr = &ctrl->item_ctr[0];
+    ja.matches = &ctrl->matches;
+    ja.err = &ctrl->error;
+    const cudaError_t e = launch_bucket_count(ja, sub, lowbits, w.nsm, st);
+    if (e != cudaSuccess) return cuda_error(e, "bucket count");
+    mark_ev(w, cfg.timing != 0, 4, st);
+    run->B = B;
+    run->passes = g.passes + 1;  // the count takes the place of the bucket sort
+    run->P = g.P;
+    run->timed = cfg.timing != 0;
+    return TBG_OK;
+}
+
 // With check_s, the range [sub, sub + 2^span) is R's alone: S's histogram
 // also counts S's keys outside it, and if there are any, nothing is sorted
 // and *s_outside is set (the caller then takes both relations' range).
@@ -138,12 +196,8 @@ static int msd_sort(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row
                     cudaStream_t st, JoinRun *run) {
     msd_done[0] = msd_done[1] = false;
     *s_outside = false;
-    int lowbits = std::min(span, kLowBits), B = span - lowbits;
-    if (B > 15) {
-        B = 15;
-        lowbits = span - B;
-    }
-    if (B < 1 || lowbits > kLowBitsMax) return TBG_OK;  // the LSD sort takes both
+    int B, lowbits;
+    if (!msd_bits(span, &B, &lowbits)) return TBG_OK;  // the LSD sort takes both
     RadixGeom g = radix_geometry_msd(nR, nS, sub, B, lowbits, w);
     if (check_s) g.s_range_max = (uint32_t)((1ull << span) - 1);
     int rc = ensure_radix_buffers(g, false, w);
@@ -193,13 +247,7 @@ int run_psm_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *d
         if (e != cudaSuccess) return cuda_error(e, "cudaMalloc"); \
     } while (0)
     ENSURE(w.ctrl, sizeof(Ctrl));
-    ENSURE(w.aux[0], nR * 8);
-    ENSURE(w.aux[1], nR * 8);
-    ENSURE(w.aux[2], nS * 8);
-    ENSURE(w.aux[3], nS * 8);
     ENSURE(w.aux[4], 64);
-    ENSURE(w.aux[6], (merge_ctas(nR, nS) + 2) * 8);
-#undef ENSURE
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     uint32_t *mm = w.aux[4].as<uint32_t>();  // min, max of R's keys, then of S's
     uint32_t *hm = static_cast<uint32_t *>(w.host_small);
@@ -223,6 +271,15 @@ int run_psm_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *d
     int rc = read_range(dR, nR, &rmin, &rmax);
     if (rc) return rc;
     mark_ev(w, timing, 1, st);
+    int B = 0, lowbits = 0;
+    if (!cfg.materialize && nR && nS && msd_bits(span_of(rmin, rmax), &B, &lowbits))
+        return msd_count(cfg, dR, nR, dS, nS, rmin, B, lowbits, w, st, run);
+    ENSURE(w.aux[0], nR * 8);
+    ENSURE(w.aux[1], nR * 8);
+    ENSURE(w.aux[2], nS * 8);
+    ENSURE(w.aux[3], nS * 8);
+    ENSURE(w.aux[6], (merge_ctas(nR, nS) + 2) * 8);
+#undef ENSURE
     Row *sorted[2] = {w.aux[0].as<Row>(), w.aux[2].as<Row>()};
     bool msd_done[2] = {false, false};
     run->B = 8;
