@@ -408,13 +408,13 @@ int part_histogram(int rel, const RadixGeom &g, const Row *d, const tbg_config &
 // midway took 20 us from every join that is not direct); a
 // caller who fixes the radix bits or passes, or turns the skew split off, gets
 // the partitioned join.
-static bool tries_direct(const tbg_config &cfg) {
+bool tries_direct(const tbg_config &cfg) {
     return !cfg.materialize && cfg.radix_bits <= 0 && (cfg.passes <= 0 || cfg.passes > 2) && cfg.skew_split;
 }
 
-// Start of a counting RHO or RHT: the control block cleared, and with g.direct
+// Start of a join: the control block cleared, and with g.direct
 // the bit table sized and cleared (dR is read).
-static int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st) {
+int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st) {
     cudaError_t e;
     if (!g.direct) {
         e = cudaMemsetAsync(w.ctrl.p, 0, sizeof(Ctrl), st);
@@ -500,11 +500,12 @@ int both_passes(const tbg_config &cfg, const RadixGeom &g, const Row *dR, const 
     return TBG_OK;
 }
 
-// Single-stream radix partitioning of R and S (RSM).
+// Single-stream radix partitioning of R and S (RHO, RHT, RSM).
 int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
                     int capR, Workspace &w, cudaStream_t st, JoinRun *run, int *join_grid_out) {
     const bool timing = cfg.timing != 0;
-    const RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
+    RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
+    g.direct = tries_direct(cfg);
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;
@@ -512,8 +513,7 @@ int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row
     int rc = ensure_radix_buffers(g, false, w);
     if (rc) return rc;
     mark(w, timing, 0, st);
-    cudaError_t e = cudaMemsetAsync(w.ctrl.p, 0, sizeof(Ctrl), st);
-    if (e != cudaSuccess) return cuda_error(e, "memset");
+    if ((rc = start_radix_join(g, dR, w, st))) return rc;
     if ((rc = part_hist_read(0, g, dR, cfg, w, st, nullptr))) return rc;
     if ((rc = part_hist_read(1, g, dS, cfg, w, st, nullptr))) return rc;
     if ((rc = part_hist_plan(3, true, g, w, st))) return rc;
@@ -525,23 +525,11 @@ int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row
 int run_radix_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
                    tbg_row_out *d_rows, uint64_t cap, Workspace &w, cudaStream_t st,
                    JoinRun *run) {
-    const bool timing = cfg.timing != 0;
     const int capR = join_capacity(nR, !cfg.materialize);
-    RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
-    g.direct = tries_direct(cfg);
-    run->B = g.B;
-    run->passes = g.passes;
-    run->P = g.P;
-    int rc = ensure_radix_buffers(g, false, w);
+    int join_grid = 0;
+    int rc = radix_partition(cfg, dR, nR, dS, nS, capR, w, st, run, &join_grid);
     if (rc) return rc;
-    mark(w, timing, 0, st);
-    if ((rc = start_radix_join(g, dR, w, st))) return rc;
-    if ((rc = part_hist_read(0, g, dR, cfg, w, st, nullptr))) return rc;
-    if ((rc = part_hist_read(1, g, dS, cfg, w, st, nullptr))) return rc;
-    if ((rc = part_hist_plan(3, true, g, w, st))) return rc;
-    mark(w, timing, 1, st);
-    if ((rc = both_passes(cfg, g, dR, dS, w, st))) return rc;
-    return radix_join_phase(cfg, d_rows, cap, w, st, run, capR, g.join_grid);
+    return radix_join_phase(cfg, d_rows, cap, w, st, run, capR, join_grid);
 }
 
 // RHO / RHT with S arriving in slices, for callers that copy S from the host

@@ -7,7 +7,9 @@
 // partition both relations so that every R partition's table fits a core's
 // cache.  Here the bit table does: 2^27 keys are 16.8 MB, a seventh of the
 // L2.  Counting needs no payloads, and a distinct key matches at most once,
-// so the bit is the whole table entry.
+// so the bit is the whole table entry.  For the sort-merge joins RSM and PSM
+// the set bits are R's distinct keys in order, and S's rows are merged with
+// them as they come.
 //
 // Bit of key k: k mod 2^w.  With max - min < 2^w that is injective on
 // [min, max], so R can be entered while it is read for its histogram, before

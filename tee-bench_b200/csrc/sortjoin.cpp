@@ -53,6 +53,7 @@ int run_sortmerge_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const 
     ja.out = d_rows;
     ja.cap = d_rows ? cap : 0;
     ja.err = &ctrl->error;
+    ja.skip = &ctrl->direct;
     cudaError_t e =
         launch_join_rsm(ja, cfg.materialize != 0, w.nsm * rsm_ctas_per_sm(capR, cfg.materialize != 0), st);
     if (e != cudaSuccess) return cuda_error(e, "rsm join");
@@ -160,12 +161,13 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
         lowbits++;
     }
     RadixGeom g = radix_geometry_msd(nR, nS, sub, B, lowbits, w);
+    g.direct = tries_direct(cfg);
     g.capR = 0x7FFFFFFF;  // counters take any number of R rows
     g.capS = std::max<uint64_t>(65536, nS / ((uint64_t)w.nsm * 12));
     g.item_cap = 2 * (nS / g.capS + 4 * g.P) + 16;
     int rc = ensure_radix_buffers(g, false, w);
     if (rc) return rc;
-    if ((rc = part_hist_read(0, g, dR, cfg, w, st, nullptr)) || (rc = part_hist_read(1, g, dS, cfg, w, st, nullptr)) ||
+    if ((rc = start_radix_join(g, dR, w, st)) || (rc = part_hist_read(0, g, dR, cfg, w, st, nullptr)) || (rc = part_hist_read(1, g, dS, cfg, w, st, nullptr)) ||
         (rc = part_hist_plan(3, true, g, w, st)) || (rc = both_passes(cfg, g, dR, dS, w, st)))
         return rc;
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
@@ -178,6 +180,7 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     ja.item_ctr = &ctrl->item_ctr[0];
     ja.matches = &ctrl->matches;
     ja.err = &ctrl->error;
+    ja.skip = &ctrl->direct;
     const cudaError_t e = launch_bucket_count(ja, sub, lowbits, w.nsm, st);
     if (e != cudaSuccess) return cuda_error(e, "bucket count");
     mark_ev(w, cfg.timing != 0, 4, st);

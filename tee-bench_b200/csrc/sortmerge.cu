@@ -594,6 +594,7 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm_count(JoinArgs a) {
     __shared__ uint32_t s_item;
     __shared__ uint64_t scan_scratch[RSM_THREADS / 32 + 1];
     __shared__ uint32_t red[2];
+    if (*a.skip) return;
     const int tid = threadIdx.x;
     const int shift = a.hash_shift;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
@@ -720,6 +721,7 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
     extern __shared__ __align__(16) uint32_t bc_smem[];
     uint32_t *h = bc_smem;
     __shared__ uint32_t s_item[2];
+    if (*a.skip) return;
     const int tid = threadIdx.x;
     const uint32_t bins = 1u << lowbits;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable

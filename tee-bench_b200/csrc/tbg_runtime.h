@@ -94,6 +94,8 @@ struct RadixGeom {
 RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int capR, Workspace &w);
 RadixGeom radix_geometry_msd(uint64_t nR, uint64_t nS, uint32_t sub, int B, int lowbits, Workspace &w);
 int ensure_radix_buffers(const RadixGeom &g, bool bypass, Workspace &w);
+bool tries_direct(const tbg_config &cfg);
+int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st);
 int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w, cudaStream_t st,
                    const SBypass *bypass);
 int part_hist_plan(int rels, bool items, const RadixGeom &g, Workspace &w, cudaStream_t st);
