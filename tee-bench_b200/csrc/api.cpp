@@ -320,12 +320,12 @@ int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     DevBuf &hist = rel ? w.histS : w.histR;
     cudaError_t e;
-    if (g.direct && rel == 0) {
+    if (g.direct && rel == 0 && !bypass) {
         e = launch_hist_build(d, g.n[0], g.ch[0], g.G[0], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), ctrl,
                               st);
         if (e == cudaSuccess)
             e = launch_direct_decide(w.direct.as<uint32_t>(), direct_log2_max(g.n[0]), g.n[0], ctrl, st);
-    } else if (g.direct) {
+    } else if (g.direct && !bypass) {
         e = launch_hist_probe(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(),
                               g.n[0], ctrl, st);
     } else if (!bypass) {
@@ -350,6 +350,10 @@ int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &
         ba.scnt = bypass->scnt;
         ba.matches = &ctrl->matches;
         ba.heavy_rows = &ctrl->heavy_rows_S;
+        if (g.direct) {
+            ba.bits = w.direct.as<uint32_t>();
+            ba.ctrl = ctrl;
+        }
         e = launch_hist_bypass(ba, cfg.materialize != 0, st);
     }
     return e == cudaSuccess ? TBG_OK : cuda_error(e, "histogram");

@@ -262,14 +262,6 @@ __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t
     }
 }
 
-// One word of the bit table from L2, not kept in L1 (a line of it is rarely
-// asked for again before it would be replaced).
-__device__ __forceinline__ uint32_t ld_bits(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-
 // S: chunk histograms and, when the join is direct, the matches.  Two
 // launches, of which one does the work: SMEM reads the table from a copy in
 // shared memory (the words from R's smallest key to its largest, when they

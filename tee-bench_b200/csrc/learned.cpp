@@ -66,7 +66,8 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
             (e = cudaEventCreateWithFlags(&w.fork, cudaEventDisableTiming)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&w.joined, cudaEventDisableTiming)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&w.table, cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&w.emit, cudaEventDisableTiming)) != cudaSuccess)
+            (e = cudaEventCreateWithFlags(&w.emit, cudaEventDisableTiming)) != cudaSuccess ||
+            (e = cudaEventCreateWithFlags(&w.decided, cudaEventDisableTiming)) != cudaSuccess)
             return cuda_error(e, "stream");
     }
     cudaStream_t s2 = w.side;
@@ -80,7 +81,8 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     uint32_t tslots = 1u << 16;
     while (tslots < m + m / 2 && tslots < (1u << 24)) tslots <<= 1;
     const int capR = join_capacity(nR, !cfg.materialize);
-    const RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
+    RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
+    g.direct = tries_direct(cfg);
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;
@@ -101,10 +103,13 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     ENSURE(w.aux[5], (size_t)g.G[1] * (8 + 8 + 4) + 16);  // materialising: per chunk heavy pairs, bases, rows
 #undef ENSURE
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
-    // main stream: R's partitioning needs nothing from the model
+    // main stream: R's partitioning needs nothing from the model (its passes
+    // step aside when the join is direct, which S's read waits to know)
     auto partition_r = [&]() -> int {
         int r;
-        if ((r = part_histogram(0, g, dR, cfg, w, st, nullptr))) return r;
+        if ((r = part_hist_read(0, g, dR, cfg, w, st, nullptr))) return r;
+        if (g.direct && (e = cudaEventRecord(w.decided, st)) != cudaSuccess) return cuda_error(e, "event");
+        if ((r = part_hist_plan(1, false, g, w, st))) return r;
         if ((r = part_pass(0, 1, g, dR, w, st, false))) return r;
         return part_pass(0, 2, g, dR, w, st, false);
     };
@@ -132,7 +137,7 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     uint32_t *hkeptc = reinterpret_cast<uint32_t *>(hbase + g.G[1]);
 
     if (timing) cudaEventRecord(w.ev[0], st);
-    if ((e = cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), st)) != cudaSuccess) return cuda_error(e, "memset");
+    if ((rc = start_radix_join(g, dR, w, st))) return rc;
     if ((e = cudaEventRecord(w.fork, st)) != cudaSuccess) return cuda_error(e, "event");
     if (!TBG_LRN_LEARN_FIRST && (rc = partition_r()))
         return rc;
@@ -201,7 +206,7 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
             if ((e = cudaEventRecord(w.table, s2)) != cudaSuccess ||
                 (e = cudaStreamWaitEvent(st, w.table, 0)) != cudaSuccess)
                 return cuda_error(e, "event");
-            if ((e = launch_heavy_r(dR, nR, hkeys, hcnt, nullptr, nullptr, nullptr, 0, w.nsm, st)) !=
+            if ((e = launch_heavy_r(dR, nR, hkeys, hcnt, nullptr, nullptr, nullptr, 0, w.nsm, st, &ctrl->direct)) !=
                 cudaSuccess)
                 return cuda_error(e, "heavy R");
         }
@@ -217,6 +222,7 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     }
     if (timing) cudaEventRecord(w.ev[6], s2);
     // S: histogram (heavy rows joined or set aside on the way), passes
+    if (g.direct && (e = cudaStreamWaitEvent(s2, w.decided, 0)) != cudaSuccess) return cuda_error(e, "event");
     if ((rc = part_histogram(1, g, dS, cfg, w, s2, bypass ? &bp : nullptr))) return rc;
     if (bypass && mat) {
         // the heavy pairs: output places reserved here, written on the main

@@ -1031,7 +1031,8 @@ cudaError_t launch_heavy_build(const LearnBufs &b, uint32_t *keys, unsigned *ins
 template <int PASS>
 __global__ void __launch_bounds__(512) k_heavy_r(const Row *__restrict__ R, uint64_t n, const uint32_t *__restrict__ gkeys,
                                                  unsigned *gcnt, const unsigned *__restrict__ start, unsigned *cur,
-                                                 uint32_t *rpay) {
+                                                 uint32_t *rpay, const unsigned *skip) {
+    if (skip && *skip) return;
     extern __shared__ __align__(16) unsigned char smem_hr[];
     uint32_t *keys = reinterpret_cast<uint32_t *>(smem_hr);
     unsigned *cnt = keys + HEAVY_CAP;
@@ -1087,7 +1088,8 @@ __global__ void k_heavy_prefix(const unsigned *cnt, unsigned *start, unsigned *c
 // stage 0: per-slot counts of R's heavy rows; stage 1 (materialisation):
 // prefix of the counts, then every heavy row's payload into rpay.
 cudaError_t launch_heavy_r(const Row *R, uint64_t n, const uint32_t *keys, unsigned *cnt, unsigned *start,
-                           unsigned *cur, uint32_t *rpay, int stage, int nsm, cudaStream_t st) {
+                           unsigned *cur, uint32_t *rpay, int stage, int nsm, cudaStream_t st,
+                           const unsigned *skip) {
     if (!n) return cudaSuccess;
     const unsigned g = (unsigned)umin64((n + 511) / 512, (uint64_t)nsm * 4);
     const size_t smem = (size_t)HEAVY_CAP * 8;
@@ -1095,11 +1097,11 @@ cudaError_t launch_heavy_r(const Row *R, uint64_t n, const uint32_t *keys, unsig
     if (e == cudaSuccess) e = smem_limit((const void *)k_heavy_r<1>, smem);
     if (e != cudaSuccess) return e;
     if (stage == 0) {
-        k_heavy_r<0><<<g, 512, smem, st>>>(R, n, keys, cnt, nullptr, nullptr, nullptr);
+        k_heavy_r<0><<<g, 512, smem, st>>>(R, n, keys, cnt, nullptr, nullptr, nullptr, skip);
         count_launch();
     } else {
         k_heavy_prefix<<<1, 1024, 0, st>>>(cnt, start, cur);
-        k_heavy_r<1><<<g, 512, smem, st>>>(R, n, keys, cnt, start, cur, rpay);
+        k_heavy_r<1><<<g, 512, smem, st>>>(R, n, keys, cnt, start, cur, rpay, skip);
         count_launch(2);
     }
     return cudaGetLastError();
@@ -1166,6 +1168,7 @@ __device__ __forceinline__ void warp_append(unsigned sel, unsigned *ctr, Put put
 
 template <bool MAT>
 __global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass(BypassArgs a) {
+    if (a.bits && a.ctrl->direct) return;
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t *hkeys = reinterpret_cast<uint32_t *>(smem);  // 8-byte aligned buckets
     unsigned *hcnt = hkeys + HEAVY_CAP;
@@ -1271,6 +1274,99 @@ __global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass(BypassArgs a) {
             if (s_pairs) atomicAdd(a.matches, s_pairs);
         }
     }
+    if (lane == 0 && wh) atomicAdd(a.heavy_rows, wh);
+}
+
+// The counting bypass when the join is direct (direct.cu): nothing is
+// compacted, since no row is partitioned.  A light row is counted in its radix
+// bin and looked up in the bit table (L2); a heavy row is counted, and matches
+// when its key's bit is set, which the CTA looks up once per heavy key.  The
+// bypass saves the heavy rows' L2 lookups, one L1 line per clock and SM each.
+__global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass_direct(BypassArgs a) {
+    if (!a.ctrl->direct) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint32_t *hkeys = reinterpret_cast<uint32_t *>(smem);  // 8-byte aligned buckets
+    uint32_t *hist = hkeys + HEAVY_CAP;
+    __shared__ uint32_t hbit[HEAVY_CAP / 32];  // the heavy keys that R holds
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t kmin = ~a.ctrl->direct_inv_min, span = a.ctrl->direct_max - kmin;
+    const uint32_t wordmask = (uint32_t)((1ull << (a.ctrl->direct_log2 - 5)) - 1);
+    auto word = [&](uint32_t key) { return key - kmin <= span ? ld_bits(a.bits + ((key >> 5) & wordmask)) : 0u; };
+    for (int i = tid; i < a.nbins; i += BYP_THREADS) hist[i] = 0;
+    for (int i = tid; i < HEAVY_CAP; i += BYP_THREADS) {
+        const uint32_t k = a.hkeys[i];
+        hkeys[i] = k;
+        const unsigned b = __ballot_sync(0xffffffffu, k != EMPTY_KEY && ((word(k) >> (k & 31)) & 1u));
+        if (lane == 0) hbit[i >> 5] = b;
+    }
+    __syncthreads();
+    const uint64_t lo = (uint64_t)blockIdx.x * a.chunk;
+    const uint64_t hi = umin64(a.n, lo + a.chunk);
+    const uint32_t len = hi > lo ? (uint32_t)(hi - lo) : 0u;  // a chunk holds < 2^32 rows
+    const Row *src = a.in + lo;
+    const uint32_t head = (len && (reinterpret_cast<uintptr_t>(src) & 15)) ? 1u : 0u;
+    const uint32_t npairs = (len - head) / 2;
+    const bool tail = ((len - head) & 1) != 0;
+    const uint4 *v = reinterpret_cast<const uint4 *>(src + head);
+    unsigned matches = 0, heavy_rows = 0;  // this thread's: below 2^32
+    constexpr uint32_t ROUND = BYP_U * BYP_THREADS;
+    uint4 nx[BYP_U];
+    auto load_round = [&](uint32_t base) {
+#pragma unroll
+        for (int u = 0; u < BYP_U; u++) {
+            const uint32_t p = base + u * BYP_THREADS + tid;
+            nx[u] = p < npairs ? ldg_stream(v + p) : make_uint4(EMPTY_KEY, 0, EMPTY_KEY, 0);
+        }
+    };
+    load_round(0);
+    for (uint32_t base = 0; base < npairs; base += ROUND) {
+        uint32_t k[2 * BYP_U];
+        unsigned valid = 0;
+#pragma unroll
+        for (int u = 0; u < BYP_U; u++) {
+            k[2 * u] = nx[u].x;
+            k[2 * u + 1] = nx[u].z;
+            if (base + u * BYP_THREADS + tid < npairs) valid |= 3u << (2 * u);
+        }
+        load_round(base + ROUND);  // the next round's loads go out before this round's work
+        uint32_t bw[2 * BYP_U];
+        unsigned hm = 0;
+#pragma unroll
+        for (int j = 0; j < 2 * BYP_U; j++) {
+            const int slot = heavy_lookup(hkeys, k[j]);
+            const bool heavy = slot >= 0 && (valid >> j & 1);
+            hm |= heavy ? 1u << j : 0u;
+            matches += heavy ? (hbit[slot >> 5] >> (slot & 31)) & 1u : 0u;
+            bw[j] = (valid >> j & 1) && !heavy ? word(k[j]) : 0u;
+        }
+        heavy_rows += __popc(hm);
+        const unsigned km = valid & ~hm;
+        const bool dup = warp_has_dups(radix_f(a.rf, k[0]), km & 1u);
+#pragma unroll
+        for (int j = 0; j < 2 * BYP_U; j++) hist_add_warp(hist, radix_f(a.rf, k[j]), km >> j & 1, dup);
+#pragma unroll
+        for (int j = 0; j < 2 * BYP_U; j++) matches += (bw[j] >> (k[j] & 31)) & 1u;
+    }
+    if (tid == 0) {
+        auto edge = [&](uint32_t key) {
+            const int slot = heavy_lookup(hkeys, key);
+            if (slot >= 0) {
+                heavy_rows++;
+                matches += (hbit[slot >> 5] >> (slot & 31)) & 1u;
+            } else {
+                atomicAdd(&hist[radix_f(a.rf, key)], 1u);
+                matches += (word(key) >> (key & 31)) & 1u;
+            }
+        };
+        if (head) edge(src[0].key);
+        if (tail) edge(src[len - 1].key);
+    }
+    const unsigned long long wm = warp_sum_u64((unsigned long long)matches);
+    const unsigned long long wh = warp_sum_u64((unsigned long long)heavy_rows);
+    __syncthreads();
+    uint32_t *hdst = a.hist + (uint64_t)blockIdx.x * a.nbins;
+    for (int i = tid; i < a.nbins; i += BYP_THREADS) hdst[i] = hist[i];
+    if (lane == 0 && wm) atomicAdd(a.matches, wm);
     if (lane == 0 && wh) atomicAdd(a.heavy_rows, wh);
 }
 
@@ -1411,6 +1507,12 @@ cudaError_t launch_hist_bypass(const BypassArgs &a, bool mat, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     kern<<<a.G, BYP_THREADS, smem, st>>>(a);
     count_launch();
+    if (!mat && a.bits) {
+        const size_t smem_d = (size_t)HEAVY_CAP * 4 + (size_t)a.nbins * 4;
+        if ((e = smem_limit((const void *)k_hist_bypass_direct, smem_d)) != cudaSuccess) return e;
+        k_hist_bypass_direct<<<a.G, BYP_THREADS, smem_d, st>>>(a);
+        count_launch();
+    }
     return cudaGetLastError();
 }
 

@@ -98,6 +98,10 @@ struct BypassArgs {
     unsigned *scnt;             // counting: S rows per heavy slot (added to)
     unsigned long long *matches;
     unsigned long long *heavy_rows;
+    // direct counting join (null bits: not tried): ctrl->direct says which of
+    // k_hist_bypass and k_hist_bypass_direct does the work
+    const uint32_t *bits = nullptr;
+    Ctrl *ctrl = nullptr;
 };
 
 // Output of a materialising bypass: heavy S rows (in the compacted S, from
@@ -148,7 +152,8 @@ cudaError_t launch_decide(const LearnBufs &b, int use_model, double nS, double m
                           cudaStream_t st);
 cudaError_t launch_heavy_build(const LearnBufs &b, uint32_t *keys, unsigned *inserted, cudaStream_t st);
 cudaError_t launch_heavy_r(const Row *R, uint64_t n, const uint32_t *keys, unsigned *cnt,
-                           unsigned *start, unsigned *cur, uint32_t *rpay, int stage, int nsm, cudaStream_t st);
+                           unsigned *start, unsigned *cur, uint32_t *rpay, int stage, int nsm, cudaStream_t st,
+                           const unsigned *skip = nullptr);
 cudaError_t launch_hist_bypass(const BypassArgs &a, bool mat, cudaStream_t st);
 cudaError_t launch_heavy_sum(const unsigned *rcnt, const unsigned *scnt, unsigned long long *matches, cudaStream_t st);
 // Exclusive prefix of the chunks' heavy output rows plus one reservation of

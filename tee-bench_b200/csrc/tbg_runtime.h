@@ -39,7 +39,8 @@ struct Workspace {
     void *host_small = nullptr;  // pinned HOST_SMALL_BYTES: mid-call read-backs (LRN's decision, shard totals)
     cudaEvent_t ev[8];
     cudaStream_t side = nullptr;       // second stream (learned path), created on first use
-    cudaEvent_t fork = nullptr, joined = nullptr, table = nullptr, emit = nullptr;
+    cudaEvent_t fork = nullptr, joined = nullptr, table = nullptr, emit = nullptr,
+                decided = nullptr;
 };
 
 // What one join call did (for stats).
