@@ -321,10 +321,14 @@ int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &
     DevBuf &hist = rel ? w.histS : w.histR;
     cudaError_t e;
     if (g.direct && rel == 0 && !bypass) {
-        e = launch_hist_build(d, g.n[0], g.ch[0], g.G[0], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), ctrl,
-                              st);
+        e = launch_hist_build(d, g.n[0], g.ch[0], g.G[0], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(),
+                              g.direct_rows, ctrl, st);
         if (e == cudaSuccess)
-            e = launch_direct_decide(w.direct.as<uint32_t>(), direct_log2_max(g.n[0]), g.n[0], ctrl, st);
+            e = launch_direct_decide(g.direct_rows ? nullptr : w.direct.as<uint32_t>(), direct_log2_max(g.n[0]), g.n[0],
+                                     ctrl, st);
+    } else if (g.direct && g.direct_rows && !bypass) {
+        e = launch_hist_emit(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), g.rows,
+                             g.rows_cap, g.s_range_max, ctrl, st);
     } else if (g.direct && !bypass) {
         e = launch_hist_probe(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(),
                               g.n[0], ctrl, st);
@@ -391,9 +395,8 @@ int part_hist_plan(int rels, bool items, const RadixGeom &g, Workspace &w, cudaS
     if (rels & 1) c[0] = ColScan{w.histR.as<uint32_t>(), w.totR.as<uint32_t>(), g.G[0], (int)g.P};
     if (rels & 2) c[1] = ColScan{w.histS.as<uint32_t>(), w.totS.as<uint32_t>(), g.G[1], (int)g.P};
     PlanTail t;
-    t.rels = rels;
     t.items = items && g.P <= PLAN_TAIL_PARTS;
-    t.done = &ctrl->done[rels == 1 ? 0 : 1];
+    t.done = ctrl->done;
     t.plan = plan_args(g, w);
     cudaError_t e = launch_colscan_plan(c[0], c[1], t, st);
     if (e != cudaSuccess) return cuda_error(e, "column scan");
@@ -406,26 +409,32 @@ int part_histogram(int rel, const RadixGeom &g, const Row *d, const tbg_config &
     return rc ? rc : part_hist_plan(1 << rel, false, g, w, st);
 }
 
-// Counting joins try the direct join (direct.cu) under the automatic plan (the
-// passes and the build/probe are launched too and step aside when it is
-// direct: four empty launches take about 9 us, while reading the decision back
-// midway took 20 us from every join that is not direct); a
-// caller who fixes the radix bits or passes, or turns the skew split off, gets
-// the partitioned join.
-bool tries_direct(const tbg_config &cfg) {
-    return !cfg.materialize && cfg.radix_bits <= 0 && (cfg.passes <= 0 || cfg.passes > 2) && cfg.skew_split;
+// Joins try the direct join (direct.cu) under the automatic plan (the passes
+// and the build/probe are launched too and step aside when it is direct: four
+// empty launches take about 9 us, while reading the decision back midway took
+// 20 us from every join that is not direct); a caller who fixes the radix bits
+// or passes, or turns the skew split off, gets the partitioned join.  A
+// materialising join tries it while R can fit the payload table at all.
+void try_direct(RadixGeom &g, const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap) {
+    g.direct = cfg.radix_bits <= 0 && (cfg.passes <= 0 || cfg.passes > 2) && cfg.skew_split;
+    if (!cfg.materialize) return;
+    g.direct = g.direct && d_rows && g.n[0] <= (1ull << direct_log2_max_rows(g.n[0]));
+    g.direct_rows = true;
+    g.rows = d_rows;
+    g.rows_cap = cap;
 }
 
 // Start of a join: the control block cleared, and with g.direct
-// the bit table sized and cleared (dR is read).
+// the table sized and cleared (dR is read).
 int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st) {
     cudaError_t e;
     if (!g.direct) {
         e = cudaMemsetAsync(w.ctrl.p, 0, sizeof(Ctrl), st);
     } else {
-        const int lg = direct_log2_max(g.n[0]);
-        if ((e = w.direct.ensure((size_t)1 << (lg - 3))) != cudaSuccess) return cuda_error(e, "cudaMalloc");
-        e = launch_direct_prep(dR, g.n[0], w.direct.as<uint32_t>(), lg, w.ctrl.as<Ctrl>(), w.nsm, st);
+        const int lg = g.direct_rows ? direct_log2_max_rows(g.n[0]) : direct_log2_max(g.n[0]);
+        if ((e = w.direct.ensure((size_t)1 << (g.direct_rows ? lg + 2 : lg - 3))) != cudaSuccess)
+            return cuda_error(e, "cudaMalloc");
+        e = launch_direct_prep(dR, g.n[0], w.direct.as<uint32_t>(), lg, g.direct_rows, w.ctrl.as<Ctrl>(), w.nsm, st);
     }
     return e == cudaSuccess ? TBG_OK : cuda_error(e, "start of the join");
 }
@@ -506,10 +515,11 @@ int both_passes(const tbg_config &cfg, const RadixGeom &g, const Row *dR, const 
 
 // Single-stream radix partitioning of R and S (RHO, RHT, RSM).
 int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
-                    int capR, Workspace &w, cudaStream_t st, JoinRun *run, int *join_grid_out) {
+                    tbg_row_out *d_rows, uint64_t cap, int capR, Workspace &w, cudaStream_t st, JoinRun *run,
+                    int *join_grid_out) {
     const bool timing = cfg.timing != 0;
     RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
-    g.direct = tries_direct(cfg);
+    try_direct(g, cfg, d_rows, cap);
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;
@@ -531,7 +541,7 @@ int run_radix_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row 
                    JoinRun *run) {
     const int capR = join_capacity(nR, !cfg.materialize);
     int join_grid = 0;
-    int rc = radix_partition(cfg, dR, nR, dS, nS, capR, w, st, run, &join_grid);
+    int rc = radix_partition(cfg, dR, nR, dS, nS, d_rows, cap, capR, w, st, run, &join_grid);
     if (rc) return rc;
     return radix_join_phase(cfg, d_rows, cap, w, st, run, capR, join_grid);
 }
@@ -555,7 +565,7 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
     uint64_t smax = 1;
     for (int k = 0; k < nslices; k++) smax = std::max(smax, s_lo[k + 1] - s_lo[k]);
     RadixGeom gmax = radix_geometry(cfg, nR, smax, capR, w);
-    gmax.direct = tries_direct(cfg);
+    try_direct(gmax, cfg, d_rows, cap);
     run->B = gmax.B;
     run->passes = gmax.passes;
     run->P = gmax.P;
@@ -577,7 +587,7 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
         if (!n) continue;
         const Row *d = dS + s_lo[k];
         RadixGeom g = radix_geometry(cfg, nR, n, capR, w);
-        g.direct = gmax.direct;
+        try_direct(g, cfg, d_rows, cap);
         if ((e = cudaStreamWaitEvent(st, s_ready[k], 0)) != cudaSuccess) return cuda_error(e, "sliced join: wait");
         if ((rc = part_hist_read(1, g, d, cfg, w, st, nullptr))) return rc;
         if ((rc = part_hist_plan(2, true, g, w, st))) return rc;
@@ -656,8 +666,8 @@ int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, const Join
         stats->matches = c.matches;
         stats->partitions = run.P;
         stats->work_items = c.nitems;
-        stats->max_part_R = c.max_part_R;
-        stats->max_part_S = c.max_part_S;
+        stats->max_part_R = run.P ? c.max_part_R : 0;
+        stats->max_part_S = run.P ? c.max_part_S : 0;
         stats->mean_part_R = run.P ? (double)nR / run.P : 0;
         stats->mean_part_S = run.P ? (double)nS / run.P : 0;
         double mr = stats->mean_part_R > 0 ? c.max_part_R / stats->mean_part_R : 0;

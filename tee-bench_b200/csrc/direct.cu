@@ -21,6 +21,9 @@
 //   k_direct_decide counts the set bits: direct iff the range fits 2^w and
 //                   |R| bits are set (all keys distinct);
 //   k_hist_probe    S's chunk histograms, and with the decision the matches.
+// A materialising join keeps R's payload per key value instead of a bit
+// (k_hist_build<true>, k_hist_emit): 2^22 keys are 16.8 MB.  A payload equal to
+// the empty mark, like a key that occurs twice, sends the join to the passes.
 // The histograms are the partitioned join's own, so when the decision is no,
 // the join continues with the passes, and the statistics (partition sizes,
 // work items) are the same either way.
@@ -33,6 +36,7 @@ namespace tbg {
 
 constexpr int DIRECT_THREADS = 1024;
 constexpr int DIRECT_MIN_LOG2 = 10;
+constexpr uint32_t EMPTY_PAYLOAD = 0xFFFFFFFFu;  // a key value that R does not hold
 
 // log2 of the largest table considered for nR rows: 32 bits per row (a
 // filtered or sparse key range up to 1/32 full), at most 2^29 bits (67 MB).
@@ -60,14 +64,25 @@ uint32_t direct_smem_words(uint64_t nR, uint64_t nbins) {
     return (uint32_t)std::min(want, cap);
 }
 
+// The same for the payload table of a materialising join: 16 entries per row,
+// at most 2^24 entries (67 MB).  Measured on 2^28 S rows, gather and 12 B rows
+// out: 2.2 ms for tables up to 17 MB, 4.3 ms at 67 MB, 5.6 ms at 134 MB; the
+// partitioned join takes about 5 ms.
+int direct_log2_max_rows(uint64_t nR) {
+    int k = DIRECT_MIN_LOG2;
+    while (k < 24 && (1ull << k) < nR * 16) k++;
+    return k;
+}
+
 // Clears the control block (CTA 0) and, when a sample of R allows a direct
-// join, the bit table.  Every CTA takes the same 1024 evenly spaced rows, so
-// all come to the same w: the sample's range plus an eighth (evenly spaced
-// rows of a relation in random or sorted order miss about 1/1024 of it at
-// either end; a range that is wider after all only means "not direct").
+// join, the table (bits to 0, payloads to the empty mark).  Every CTA takes the same 1024 evenly spaced rows, so
+// all come to the same w: the sample's range plus 1/32 (evenly spaced rows of
+// a relation in random or sorted order miss about 1/1024 of it at either end;
+// a range that is wider after all only means "not direct").  More rows than
+// the table has entries cannot be distinct.
 __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_prep(const Row *__restrict__ R, uint64_t nR,
-                                                                uint32_t *__restrict__ bits, int log2_max,
-                                                                Ctrl *ctrl) {
+                                                                uint32_t *__restrict__ table, int log2_max,
+                                                                bool payloads, Ctrl *ctrl) {
     __shared__ uint32_t s_lo, s_hi;
     const int tid = threadIdx.x;
     if (blockIdx.x == 0)
@@ -90,14 +105,15 @@ __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_prep(const Row *__res
     }
     __syncthreads();
     const uint32_t span = s_hi - s_lo;
-    const uint64_t want = (uint64_t)span + span / 8 + 64;
+    const uint64_t want = (uint64_t)span + span / 32 + 64;
     const int w = max(DIRECT_MIN_LOG2, 64 - __clzll((long long)(want - 1)));
-    if (w > log2_max) return;
+    if (w > log2_max || nR > (1ull << w)) return;
     if (blockIdx.x == 0 && tid == 0) ctrl->direct_log2 = (unsigned)w;
-    uint4 *b4 = reinterpret_cast<uint4 *>(bits);
-    const uint64_t n4 = 1ull << (w - 7);
+    uint4 *b4 = reinterpret_cast<uint4 *>(table);
+    const uint64_t n4 = 1ull << (payloads ? w - 2 : w - 7);
+    const uint32_t fill = payloads ? EMPTY_PAYLOAD : 0u;
     for (uint64_t q = (uint64_t)blockIdx.x * DIRECT_THREADS + tid; q < n4; q += (uint64_t)gridDim.x * DIRECT_THREADS)
-        b4[q] = make_uint4(0, 0, 0, 0);
+        b4[q] = make_uint4(fill, fill, fill, fill);
 }
 
 // Streams rows [lo, hi) of `in` in rounds of 8 rows per thread: fn(x, ok)
@@ -143,9 +159,12 @@ __device__ __forceinline__ void hist_pairs(uint32_t *sh, const RadixF &rf, const
 // rounds use atomics without a result, and a duplicate there shows in the
 // count of set bits.  Bound by the L2's atomics: 2^27 rows take 0.80 ms
 // without results against 1.17 ms with; the histogram read alone 0.16 ms.
+// PAYLOADS: every row exchanges its payload with the key's entry (2^22 rows:
+// 37 us), so a duplicate shows at once.
+template <bool PAYLOADS>
 __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__restrict__ in, uint64_t n, uint64_t chunk,
                                                                   uint32_t *__restrict__ hist, int nbins, RadixF rf,
-                                                                  uint32_t *__restrict__ bits, Ctrl *ctrl) {
+                                                                  uint32_t *__restrict__ table, Ctrl *ctrl) {
     extern __shared__ uint32_t sh[];
     __shared__ uint32_t s_inv, s_hi;
     const int tid = threadIdx.x;
@@ -159,17 +178,19 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
     volatile unsigned *gave_up = &ctrl->direct_dup;
     bool enter = w != 0;  // the same for all lanes of a warp
     uint32_t kinv = 0, kmax = 0;  // largest ~key (the smallest key) and largest key
-    const uint32_t careful = (uint32_t)(chunk / (16 * 8 * DIRECT_THREADS)) + 1;
+    const uint32_t careful = PAYLOADS ? 0xFFFFFFFFu : (uint32_t)(chunk / (16 * 8 * DIRECT_THREADS)) + 1;
     uint32_t round = 0;
-    auto set_bit = [&](uint32_t key, bool ret) {
+    // enters a row; with ret, true says that the join is not direct
+    auto set_bit = [&](uint32_t key, uint32_t payload, bool ret) {
         const uint32_t s = key & wmask;
         kinv = max(kinv, ~key);
         kmax = max(kmax, key);
+        if (PAYLOADS) return atomicExch(table + s, payload) != EMPTY_PAYLOAD || payload == EMPTY_PAYLOAD;
         if (!ret) {
-            atomicOr(bits + (s >> 5), 1u << (s & 31));
+            atomicOr(table + (s >> 5), 1u << (s & 31));
             return false;
         }
-        return ((atomicOr(bits + (s >> 5), 1u << (s & 31)) >> (s & 31)) & 1u) != 0;
+        return ((atomicOr(table + (s >> 5), 1u << (s & 31)) >> (s & 31)) & 1u) != 0;
     };
     stream_pairs(
         in, lo, hi,
@@ -180,8 +201,8 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         if (ok[u]) {
-                            dup |= set_bit(x[u].x, true);
-                            dup |= set_bit(x[u].z, true);
+                            dup |= set_bit(x[u].x, x[u].y, true);
+                            dup |= set_bit(x[u].z, x[u].w, true);
                         }
                     }
                     // one lane per warp touches the flag: all of them storing
@@ -197,8 +218,8 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         if (ok[u]) {
-                            set_bit(x[u].x, false);
-                            set_bit(x[u].z, false);
+                            set_bit(x[u].x, x[u].y, false);
+                            set_bit(x[u].z, x[u].w, false);
                         }
                     }
                 }
@@ -208,7 +229,7 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
             hist_pairs(sh, rf, x, ok);
         },
         [&](const Row &r) {
-            if (enter) set_bit(r.key, false);
+            if (enter && set_bit(r.key, r.payload, false)) *gave_up = 1;
             atomicAdd(&sh[radix_f(rf, r.key)], 1u);
         });
     if (w) {
@@ -231,13 +252,19 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
 }
 
 // Counts the set bits; the last CTA decides.  The table is read from L2
-// (2^27 keys: 33.5 MB, half of it R's range).
+// (2^27 keys: 33.5 MB, half of it R's range).  A payload table (null bits)
+// needs no count: its entries showed every duplicate.
 __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t *__restrict__ bits, uint64_t nR,
                                                                   Ctrl *ctrl) {
     __shared__ unsigned s_count;
     const unsigned w = ctrl->direct_log2;
     if (!w || ctrl->direct_dup) return;
     const int tid = threadIdx.x;
+    if (!bits) {
+        if (blockIdx.x == 0 && tid == 0 && (uint64_t)(ctrl->direct_max - ~ctrl->direct_inv_min) < (1ull << w))
+            ctrl->direct = 1;
+        return;
+    }
     if (tid == 0) s_count = 0;
     __syncthreads();
     const uint4 *b4 = reinterpret_cast<const uint4 *>(bits);
@@ -254,7 +281,7 @@ __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t
     if (tid == 0) {
         atomicAdd(&ctrl->direct_bits, (unsigned long long)s_count);
         __threadfence();
-        if (atomicAdd(&ctrl->done[2], 1u) == gridDim.x - 1) {
+        if (atomicAdd(&ctrl->done[3], 1u) == gridDim.x - 1) {
             __threadfence();
             const unsigned long long set = atomicAdd(&ctrl->direct_bits, 0ull);
             if (set == nR && (uint64_t)(ctrl->direct_max - ~ctrl->direct_inv_min) < (1ull << w)) ctrl->direct = 1;
@@ -327,22 +354,199 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2)
     for (int i = tid; i < nbins; i += DIRECT_THREADS) dst[i] = sh[i];
 }
 
-cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *bits, int log2_max, Ctrl *ctrl, int nsm,
-                               cudaStream_t st) {
-    const uint64_t n4 = 1ull << (log2_max - 7);
+// S of a materialising join: chunk histograms and, when the join is direct,
+// the output rows.  A round takes 8 rows per thread: their payloads are
+// gathered from the table in L2, the matching rows take places in (warp, row
+// slot, lane) order in shared memory, one atomic reserves the round's output,
+// and one bulk store writes it: staged at its destination's 16-byte phase, so
+// all but the at most 3 words at either end leave by the copy engine and the
+// stores cost the SM no load/store instructions.  Bound by L2 (one sector per
+// row gathered, 12 B out, 8 B in).
+constexpr int EMIT_DIRECT_THREADS = 512;
+constexpr int EMIT_ROUND = EMIT_DIRECT_THREADS * 8;
+
+struct EmitSmem {
+    alignas(16) uint32_t stage[EMIT_ROUND * 3 + 4];
+    uint32_t wtot[EMIT_DIRECT_THREADS / 32];
+    unsigned long long base;
+    uint32_t total;
+};
+
+__global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
+    k_hist_emit(const Row *__restrict__ in, uint64_t n, uint64_t chunk, uint32_t *__restrict__ hist, int nbins, RadixF rf,
+                const uint32_t *__restrict__ table, tbg_row_out *__restrict__ out, uint64_t cap, uint32_t range_max,
+                Ctrl *ctrl) {
+    constexpr int T = EMIT_DIRECT_THREADS, NW = T / 32;
+    extern __shared__ __align__(16) unsigned char esmem[];
+    EmitSmem &sm = *reinterpret_cast<EmitSmem *>(esmem);
+    uint32_t *sh = reinterpret_cast<uint32_t *>(esmem + sizeof(EmitSmem));
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    for (int i = tid; i < nbins; i += T) sh[i] = 0;
+    const bool direct = ctrl->direct != 0;
+    const uint32_t kmin = ~ctrl->direct_inv_min, span = ctrl->direct_max - kmin;
+    const uint32_t mask = direct ? (uint32_t)((1ull << ctrl->direct_log2) - 1) : 0u;
+    __syncthreads();
+    const uint64_t lo = (uint64_t)blockIdx.x * chunk;
+    const uint64_t hi = umin64(n, lo + chunk);
+    unsigned long long matches = 0;  // not direct: keys outside range_max
+    // one round: this thread's rows (k, p) of `valid`; every thread calls it
+    auto round = [&](const uint32_t (&k)[8], const uint32_t (&p)[8], unsigned valid) {
+        uint32_t r[8];
+        if (direct) {
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                r[j] = (valid >> j & 1) && k[j] - kmin <= span ? ld_bits(table + (k[j] & mask)) : EMPTY_PAYLOAD;
+        }
+        const bool dup = warp_has_dups(radix_f(rf, k[0]), valid & 1u);
+#pragma unroll
+        for (int j = 0; j < 8; j++) hist_add_warp(sh, radix_f(rf, k[j]), valid >> j & 1, dup);
+        if (!direct) {
+            if (range_max != 0xFFFFFFFFu) {  // as k_hist_chunks: keys outside the bins' range
+                unsigned o = 0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) o += (valid >> j & 1) && k[j] - rf.sub > range_max;
+                matches += o;
+            }
+            return;
+        }
+        unsigned m[8], wt = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            m[j] = __ballot_sync(0xffffffffu, r[j] != EMPTY_PAYLOAD);
+            wt += __popc(m[j]);
+        }
+        if (lane == 0) sm.wtot[w] = wt;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (int q = 0; q < NW; q++) {
+            const uint32_t x = sm.wtot[q];
+            before += q < w ? x : 0;
+            total += x;
+        }
+        if (tid == 0) {
+            sm.base = total ? atomicAdd(&ctrl->rows, (unsigned long long)total) : 0;
+            bulk_wait_read();  // the last round's rows have left the stage
+        }
+        __syncthreads();
+        const unsigned long long base = sm.base;
+        const uintptr_t dst = reinterpret_cast<uintptr_t>(out + base);
+        const uint32_t phase = (uint32_t)(dst & 15) / 4;  // the stage starts at the destination's phase
+        const uint32_t keep = base < cap ? (uint32_t)umin64(total, cap - base) : 0u;
+        const unsigned lt = lanemask_lt();
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (m[j] >> lane & 1) {
+                uint32_t *q = sm.stage + phase + 3 * (before + __popc(m[j] & lt));
+                q[0] = k[j];
+                q[1] = r[j];
+                q[2] = p[j];
+            }
+            before += __popc(m[j]);
+        }
+        fence_proxy_async_smem();
+        __syncthreads();
+        // words [phase, phase + 3 * keep) of the stage go to the 16-byte aligned
+        // address dst - 4 * phase, word for word
+        uint32_t *g = reinterpret_cast<uint32_t *>(dst) - phase;
+        const uint32_t end = phase + 3 * keep;
+        const uint32_t a0 = (phase + 3) & ~3u, a1 = end & ~3u;  // the aligned body
+        if (tid == 0) {
+            if (a0 < a1) {
+                bulk_s2g(g + a0, sm.stage + a0, (a1 - a0) * 4);
+                bulk_commit();
+            }
+            matches += total;
+        } else if (w == 1) {  // up to 3 words before the body and after it
+            const uint32_t head_end = min(a0, end), tail0 = max(a1, head_end);
+            if (phase + lane < head_end) g[phase + lane] = sm.stage[phase + lane];
+            if (tail0 + lane < end) g[tail0 + lane] = sm.stage[tail0 + lane];
+        }
+    };
+    if (lo < hi) {
+        const uint32_t head = ((reinterpret_cast<uintptr_t>(in + lo) & 15) != 0) ? 1 : 0;
+        const uint64_t body = hi - lo - head;
+        const uint32_t nv = (uint32_t)(body / 2);
+        const bool tail = body & 1;
+        const uint4 *v = reinterpret_cast<const uint4 *>(in + lo + head);
+        uint4 nx[4];
+        auto load_round = [&](uint32_t b) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t i = b + u * T + tid;
+                nx[u] = i < nv ? ldg_stream(v + i) : make_uint4(0, 0, 0, 0);
+            }
+        };
+        load_round(0);
+        for (uint32_t b = 0; b < nv; b += 4 * T) {
+            uint32_t k[8], p[8];
+            unsigned valid = 0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                k[2 * u] = nx[u].x;
+                p[2 * u] = nx[u].y;
+                k[2 * u + 1] = nx[u].z;
+                p[2 * u + 1] = nx[u].w;
+                if (b + u * T + tid < nv) valid |= 3u << (2 * u);
+            }
+            load_round(b + 4 * T);  // in flight during this round
+            round(k, p, valid);
+        }
+        if (head || tail) {  // the edge rows: one round of at most two rows
+            uint32_t k[8] = {}, p[8] = {};
+            unsigned valid = 0;
+            if ((tid == 0 && head) || (tid == 1 && tail)) {
+                const Row r = in[tid == 0 ? lo : hi - 1];
+                k[0] = r.key;
+                p[0] = r.payload;
+                valid = 1;
+            }
+            round(k, p, valid);
+        }
+    }
+    if (direct) {  // thread 0 counted the rounds' rows
+        if (tid == 0) {
+            bulk_wait_all();
+            if (matches) atomicAdd(&ctrl->matches, matches);
+        }
+    } else {
+        const unsigned long long o = warp_sum_u64(matches);
+        if (lane == 0 && o) atomicAdd(&ctrl->out_of_range, o);
+    }
+    __syncthreads();
+    uint32_t *hdst = hist + (uint64_t)blockIdx.x * nbins;
+    for (int i = tid; i < nbins; i += T) hdst[i] = sh[i];
+}
+
+cudaError_t launch_hist_emit(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
+                             const uint32_t *table, tbg_row_out *out, uint64_t cap, uint32_t range_max, Ctrl *ctrl,
+                             cudaStream_t st) {
+    const int nbins = 1 << P_log2;
+    const size_t smem = sizeof(EmitSmem) + (size_t)nbins * 4;
+    cudaError_t e = smem_limit((const void *)k_hist_emit, smem);
+    if (e != cudaSuccess) return e;
+    k_hist_emit<<<G, EMIT_DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, table, out, cap, range_max, ctrl);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *table, int log2_max, bool payloads, Ctrl *ctrl,
+                               int nsm, cudaStream_t st) {
+    const uint64_t n4 = 1ull << (payloads ? log2_max - 2 : log2_max - 7);
     const unsigned g = (unsigned)std::min<uint64_t>((n4 + DIRECT_THREADS - 1) / DIRECT_THREADS, (uint64_t)nsm * 2);
-    k_direct_prep<<<g, DIRECT_THREADS, 0, st>>>(R, nR, bits, log2_max, ctrl);
+    k_direct_prep<<<g, DIRECT_THREADS, 0, st>>>(R, nR, table, log2_max, payloads, ctrl);
     count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
-                              uint32_t *bits, Ctrl *ctrl, cudaStream_t st) {
+                              uint32_t *table, bool payloads, Ctrl *ctrl, cudaStream_t st) {
     const int nbins = 1 << P_log2;
     const size_t smem = (size_t)nbins * 4;
-    cudaError_t e = smem_limit((const void *)k_hist_build, smem);
+    auto kern = payloads ? k_hist_build<true> : k_hist_build<false>;
+    cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    k_hist_build<<<G, DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, bits, ctrl);
+    kern<<<G, DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, table, ctrl);
     count_launch();
     return cudaGetLastError();
 }
@@ -350,7 +554,7 @@ cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, 
 cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, Ctrl *ctrl, cudaStream_t st) {
     const uint64_t n4 = 1ull << (log2_max - 7);
     // two 16-byte words per thread and CTA at least, one CTA per SM at most
-    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), 148));
+    const unsigned g = bits ? (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), 148)) : 1u;
     k_direct_decide<<<g, DIRECT_THREADS, 0, st>>>(bits, nR, ctrl);
     count_launch();
     return cudaGetLastError();

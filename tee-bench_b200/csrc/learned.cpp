@@ -82,7 +82,7 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     while (tslots < m + m / 2 && tslots < (1u << 24)) tslots <<= 1;
     const int capR = join_capacity(nR, !cfg.materialize);
     RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
-    g.direct = tries_direct(cfg);
+    if (!mat) try_direct(g, cfg, nullptr, 0);
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;

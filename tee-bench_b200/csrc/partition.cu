@@ -118,9 +118,10 @@ __global__ void __launch_bounds__(HIST_THREADS) k_hist_chunks(const Row *__restr
 // K3 planner: partition bases and join work items.  Replaces the task
 // creation of Joins/radix_join.c:946-1000 and :609-617 (pairs with both sides
 // non-empty); oversized S sides are split into several items.
-// One launch does K2 for both relations, and its last CTA K3: five launches
-// (two column scans, two base scans, the planner) took 24 us of the 120 us of
-// a 2^21 x 2^21 join.
+// One launch does K2 for both relations; each relation's last CTA scans its
+// bases, and the second of them plans the items: as five launches (two column
+// scans, two base scans, the planner) it took 24 us of the 120 us of a
+// 2^21 x 2^21 join.
 // ---------------------------------------------------------------------------
 constexpr int PLAN_THREADS = 1024;
 
@@ -177,37 +178,43 @@ __device__ void column_scan(uint32_t *__restrict__ hist, int G, int P, uint32_t 
 
 // Exclusive scan of tot[0..P) into base[0..P], base[P] = total (rows counted:
 // n unless rows were bypassed), and the largest entry into *maxp, by one CTA
-// of PLAN_THREADS threads.  Warp w owns P / 32 consecutive entries and walks
-// them 32 at a time, so loads and stores are coalesced.
+// of PLAN_THREADS threads.  Warp w owns `per` consecutive entries and walks
+// them 32 at a time, so loads and stores are coalesced; up to PLAN_THREADS
+// entries that is one load per thread.
 __device__ void plan_bases(const uint32_t *tot, uint64_t *base, int P, unsigned long long *maxp, int tid,
                            uint64_t *scratch) {
     const int lane = tid & 31, w = tid >> 5;
     const int per = ((P + 31) / 32 + 31) & ~31;
     const int lo = min(P, w * per), hi = min(P, lo + per);
-    uint64_t sum = 0;
-    uint32_t mx = 0;
+    const uint32_t first = lo + lane < hi ? __ldcg(tot + lo + lane) : 0;
+    uint64_t sum = first;
+    uint32_t mx = first;
 #pragma unroll 4
-    for (int f = lo + lane; f < hi; f += 32) {
+    for (int f = lo + 32 + lane; f < hi; f += 32) {
         const uint32_t x = __ldcg(tot + f);
         sum += x;
         mx = max(mx, x);
     }
     sum = warp_sum_u64(sum);
-    mx = warp_max_u32(mx);
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) {
         scratch[w] = sum;
         if (mx) atomicMax(maxp, (unsigned long long)mx);
     }
     __syncthreads();
-    uint64_t run = 0, total = 0;
-    for (int k = 0; k < 32; k++) {
-        if (k == w) run = total;
-        total += scratch[k];
+    const uint64_t ws = scratch[lane];  // 32 warps
+    uint64_t winc = ws;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, winc, o);
+        if (lane >= o) winc += y;
     }
+    uint64_t run = __shfl_sync(0xffffffffu, winc - ws, w);
+    const uint64_t total = __shfl_sync(0xffffffffu, winc, 31);
 #pragma unroll 4
     for (int f0 = lo; f0 < hi; f0 += 32) {
         const int f = f0 + lane;
-        const uint32_t x = f < hi ? __ldcg(tot + f) : 0;
+        const uint32_t x = f0 == lo ? first : (f < hi ? __ldcg(tot + f) : 0);
         uint32_t inc = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -236,31 +243,28 @@ __device__ void plan_block(const PlanArgs &a, int block, int tid, uint64_t *scra
         if (!a.capS || (nrc > 1 && !split_all)) return 1;
         return (hs + a.capS - 1) / a.capS;
     };
-    uint64_t cnt_all = 0;
-    for (int f = tid; f < P; f += PLAN_THREADS) {
-        const uint32_t hr = __ldcg(a.r.hist + f), hs = __ldcg(a.s.hist + f);
-        if (hr == 0 || hs == 0) continue;
-        const uint64_t nrc = (hr + (uint64_t)a.capR - 1) / a.capR;
-        cnt_all += nrc * s_chunks(hs, nrc, true);
-    }
+    const int f = block * PLAN_THREADS + tid;
+    const uint32_t hr = f < P ? __ldcg(a.r.hist + f) : 0, hs = f < P ? __ldcg(a.s.hist + f) : 0;
+    auto count = [&](uint32_t r, uint32_t s) -> uint64_t {
+        if (r == 0 || s == 0) return 0;
+        const uint64_t nrc = (r + (uint64_t)a.capR - 1) / a.capR;
+        return nrc * s_chunks(s, nrc, true);
+    };
+    uint64_t cnt_all = count(hr, hs);
+    if (P > PLAN_THREADS)
+        for (int q = tid; q < P; q += PLAN_THREADS)
+            if (q != f) cnt_all += count(__ldcg(a.r.hist + q), __ldcg(a.s.hist + q));
     const int lane = tid & 31, w = tid >> 5;
     cnt_all = warp_sum_u64(cnt_all);
     if (lane == 0) scratch[w] = cnt_all;
     __syncthreads();
-    uint64_t total_all = 0;
-    for (int k = 0; k < PLAN_THREADS / 32; k++) total_all += scratch[k];
+    const uint64_t total_all = warp_sum_u64(scratch[lane]);  // 32 warps
     __syncthreads();
     const bool split_all = total_all <= a.item_cap;
-    const int f = block * PLAN_THREADS + tid;
-    uint32_t hr = 0, hs = 0;
     uint64_t nrc = 0, nsc = 0;
-    if (f < P) {
-        hr = __ldcg(a.r.hist + f);
-        hs = __ldcg(a.s.hist + f);
-        if (hr && hs) {
-            nrc = (hr + (uint64_t)a.capR - 1) / a.capR;
-            nsc = s_chunks(hs, nrc, split_all);
-        }
+    if (hr && hs) {
+        nrc = (hr + (uint64_t)a.capR - 1) / a.capR;
+        nsc = s_chunks(hs, nrc, split_all);
     }
     const uint64_t mine = nrc * nsc;
     // warp prefix of the item counts, one reservation per warp
@@ -296,39 +300,49 @@ __device__ void plan_block(const PlanArgs &a, int block, int tid, uint64_t *scra
     if (lane == 0 && ne) atomicAdd(&a.ctrl->nonempty, (unsigned long long)ne);
 }
 
-// Column scans of relation 0 in CTAs [0, cols of it), of relation 1 in the
-// rest.  With t.rels, the last CTA to finish (a ticket on *t.done, which it
-// resets) scans the bases of the relations in the mask t.rels and, with
-// t.items, plans the work items.
+
+// Takes a ticket of *ctr after this CTA's writes; true for all threads of the
+// CTA that takes the last of `n`, which then sees the others' writes, and
+// leaves the counter at zero.
+__device__ bool last_of(unsigned *ctr, unsigned n, int tid, bool *flag) {
+    __syncthreads();  // this CTA's writes come before its ticket
+    if (tid == 0) {
+        __threadfence();
+        const bool last = atomicAdd(ctr, 1u) == n - 1;
+        if (last) {
+            *ctr = 0;
+            __threadfence();
+        }
+        *flag = last;
+    }
+    __syncthreads();
+    return *flag;
+}
+
+// Column scans of relation R in CTAs [0, cols of it), of S in the rest.  With
+// t.plan, each relation's last CTA scans its bases; with t.items, the CTA that
+// finishes the last relation of the launch plans the work items.
 __global__ void __launch_bounds__(PLAN_THREADS) k_colscan(ColScan r, ColScan s, PlanTail t) {
     __shared__ uint32_t seg[32][33];
     __shared__ uint64_t scratch[PLAN_THREADS / 32 + 1];
-    __shared__ bool s_last;
-    const int cols_r = (r.P + 31) / 32;
-    if ((int)blockIdx.x < cols_r) column_scan(r.hist, r.G, r.P, r.totals, blockIdx.x, seg);
+    __shared__ bool flag;
+    const int cols_r = (r.P + 31) / 32, cols_s = (s.P + 31) / 32;
+    const bool is_s = (int)blockIdx.x >= cols_r;
+    if (!is_s) column_scan(r.hist, r.G, r.P, r.totals, blockIdx.x, seg);
     else column_scan(s.hist, s.G, s.P, s.totals, blockIdx.x - cols_r, seg);
-    if (!t.rels) return;
+    if (!t.done) return;
     const int tid = threadIdx.y * 32 + threadIdx.x;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_last = atomicAdd(t.done, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
+    if (!last_of(t.done + is_s, is_s ? cols_s : cols_r, tid, &flag)) return;
+    Ctrl *ctrl = t.plan.ctrl;
     const int P = 1 << t.plan.P_log2;
-    if (t.rels & 1) plan_bases(t.plan.r.hist, t.plan.r.base, P, &t.plan.ctrl->max_part_R, tid, scratch);
-    if (t.rels & 2) plan_bases(t.plan.s.hist, t.plan.s.base, P, &t.plan.ctrl->max_part_S, tid, scratch);
-    if (tid == 0) {
-        *t.done = 0;
-        if (t.items) t.plan.ctrl->nitems = 0;
-    }
+    const RelPlan &rel = is_s ? t.plan.s : t.plan.r;
+    plan_bases(rel.hist, rel.base, P, is_s ? &ctrl->max_part_S : &ctrl->max_part_R, tid, scratch);
     if (!t.items) return;
+    if (!last_of(t.done + 2, cols_r && cols_s ? 2 : 1, tid, &flag)) return;
+    if (tid == 0) ctrl->nitems = 0;
     __threadfence();
     __syncthreads();
-    for (int b = 0; b * PLAN_THREADS < P; b++) {
-        plan_block(t.plan, b, tid, scratch);
-        __syncthreads();
-    }
+    for (int b = 0; b * PLAN_THREADS < P; b++) plan_block(t.plan, b, tid, scratch);
 }
 
 __global__ void __launch_bounds__(PLAN_THREADS) k_plan(PlanArgs a) {

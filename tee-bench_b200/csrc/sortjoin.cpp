@@ -36,7 +36,7 @@ int run_sortmerge_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const 
     // one shared-memory radix-sorted tile (512 threads x 8 rows) of R per item
     const int capR = RSM_CAPR;
     int join_grid = 0;
-    int rc = radix_partition(cfg, dR, nR, dS, nS, capR, w, st, run, &join_grid);
+    int rc = radix_partition(cfg, dR, nR, dS, nS, d_rows, cap, capR, w, st, run, &join_grid);
     if (rc) return rc;
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     JoinArgs ja;
@@ -151,8 +151,14 @@ cudaError_t launch_bucket_count(const JoinArgs &a, uint32_t sub, int lowbits, in
 // key - sub (sub: R's smallest key), then k_bucket_count.  Nothing waits, and
 // neither S's keys outside R's range nor heavy keys (S's buckets are split over
 // CTAs by the planner) need another plan.
+// lsd_passes > 0: the range has no bits above the low ones, where the sort
+// would be an LSD sort of that many passes; the buckets do for it too.
 static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, uint32_t sub, int B,
-                     int lowbits, Workspace &w, cudaStream_t st, JoinRun *run) {
+                     int lowbits, int lsd_passes, Workspace &w, cudaStream_t st, JoinRun *run) {
+    if (lsd_passes) {  // a range of at most kLowBits bits: two buckets
+        B = 1;
+        lowbits = std::max(lowbits - 1, 2);
+    }
     // one radix bit less where both plans take two passes: a pass costs more
     // per bit above 7 than the larger buckets do (8 + 7 bits against 7 + 7 at
     // 2^27 x 2^30: 4.64 against 3.79 ms for the second pass)
@@ -161,7 +167,7 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
         lowbits++;
     }
     RadixGeom g = radix_geometry_msd(nR, nS, sub, B, lowbits, w);
-    g.direct = tries_direct(cfg);
+    try_direct(g, cfg, nullptr, 0);
     g.capR = 0x7FFFFFFF;  // counters take any number of R rows
     g.capS = std::max<uint64_t>(65536, nS / ((uint64_t)w.nsm * 12));
     g.item_cap = 2 * (nS / g.capS + 4 * g.P) + 16;
@@ -184,9 +190,9 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     const cudaError_t e = launch_bucket_count(ja, sub, lowbits, w.nsm, st);
     if (e != cudaSuccess) return cuda_error(e, "bucket count");
     mark_ev(w, cfg.timing != 0, 4, st);
-    run->B = B;
-    run->passes = g.passes + 1;  // the count takes the place of the bucket sort
-    run->P = g.P;
+    run->B = lsd_passes ? 8 : B;
+    run->passes = lsd_passes ? lsd_passes : g.passes + 1;  // the count takes the place of the bucket sort
+    run->P = lsd_passes ? 0 : g.P;
     run->timed = cfg.timing != 0;
     return TBG_OK;
 }
@@ -194,33 +200,44 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
 // With check_s, the range [sub, sub + 2^span) is R's alone: S's histogram
 // also counts S's keys outside it, and if there are any, nothing is sorted
 // and *s_outside is set (the caller then takes both relations' range).
+// The first sort (check_s) also tries the direct join during the histogram
+// reads: with *direct set the join is done.
 static int msd_sort(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, uint32_t sub,
-                    int span, bool check_s, Row *sorted[2], bool msd_done[2], bool *s_outside, Workspace &w,
-                    cudaStream_t st, JoinRun *run) {
+                    int span, bool check_s, tbg_row_out *d_rows, uint64_t cap, Row *sorted[2], bool msd_done[2],
+                    bool *s_outside, bool *direct, Workspace &w, cudaStream_t st, JoinRun *run) {
     msd_done[0] = msd_done[1] = false;
-    *s_outside = false;
+    *s_outside = *direct = false;
     int B, lowbits;
     if (!msd_bits(span, &B, &lowbits)) return TBG_OK;  // the LSD sort takes both
     RadixGeom g = radix_geometry_msd(nR, nS, sub, B, lowbits, w);
     if (check_s) g.s_range_max = (uint32_t)((1ull << span) - 1);
+    if (check_s) try_direct(g, cfg, d_rows, cap);
     int rc = ensure_radix_buffers(g, false, w);
     if (rc) return rc;
     Ctrl *ctrl = w.ctrl.as<Ctrl>();
     cudaError_t e;
-    if ((e = cudaMemsetAsync(&ctrl->max_part_R, 0, 24, st)) != cudaSuccess) return cuda_error(e, "memset");
-    if ((rc = part_histogram(0, g, dR, cfg, w, st, nullptr)) || (rc = part_histogram(1, g, dS, cfg, w, st, nullptr)))
+    if ((rc = start_radix_join(g, dR, w, st))) return rc;
+    if ((rc = part_hist_read(0, g, dR, cfg, w, st, nullptr)) || (rc = part_hist_read(1, g, dS, cfg, w, st, nullptr)) ||
+        (rc = part_hist_plan(3, false, g, w, st)))
         return rc;
     // the largest bucket of each relation decides between this sort and LSD;
     // S's keys outside R's range void the histograms
-    unsigned long long *hm = static_cast<unsigned long long *>(w.host_small);
-    if ((e = cudaMemcpyAsync(hm, &ctrl->max_part_R, 24, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+    if ((e = cudaMemcpyAsync(w.host_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
         return cuda_error(e, "bucket sizes");
-    if (check_s && hm[2]) {
+    const Ctrl &hc = *w.host_ctrl;
+    if (!hc.direct && check_s && hc.out_of_range) {
         *s_outside = true;
         return TBG_OK;
     }
-    const unsigned long long maxp[2] = {hm[0], hm[1]};
+    run->B = B;
+    run->passes = g.passes + 1;
+    run->P = g.P;
+    if (hc.direct) {
+        *direct = true;
+        return TBG_OK;
+    }
+    const unsigned long long maxp[2] = {hc.max_part_R, hc.max_part_S};
     const Row *in[2] = {dR, dS};
     for (int rel = 0; rel < 2; rel++) {
         if (maxp[rel] > kBucketMax) continue;
@@ -234,9 +251,32 @@ static int msd_sort(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row
         msd_done[rel] = true;
         mark_ev(w, cfg.timing != 0, 2 + rel, st);
     }
-    run->B = B;
-    run->passes = g.passes + 1;
-    run->P = g.P;
+    return TBG_OK;
+}
+
+// The direct join in front of the LSD sort (key ranges without MSD buckets,
+// when R's range fits the table): its histograms have two bins, only to be
+// thrown away.  *direct: the join is done.
+static int direct_or_lsd(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, uint32_t rmin,
+                         uint32_t rmax, tbg_row_out *d_rows, uint64_t cap, bool *direct, Workspace &w, cudaStream_t st) {
+    *direct = false;
+    RadixGeom g = radix_geometry_msd(nR, nS, rmin, 1, 31, w);
+    try_direct(g, cfg, d_rows, cap);
+    const int lg = g.direct_rows ? direct_log2_max_rows(nR) : direct_log2_max(nR);
+    // more rows than key values: not distinct
+    if (!g.direct || (uint64_t)(rmax - rmin) >= (1ull << lg) || nR > (uint64_t)(rmax - rmin) + 1) return TBG_OK;
+    cudaError_t e;
+    if ((e = w.histR.ensure((uint64_t)g.G[0] * g.P * 4)) != cudaSuccess ||
+        (e = w.histS.ensure((uint64_t)g.G[1] * g.P * 4)) != cudaSuccess)
+        return cuda_error(e, "cudaMalloc");
+    int rc;
+    if ((rc = start_radix_join(g, dR, w, st)) || (rc = part_hist_read(0, g, dR, cfg, w, st, nullptr)) ||
+        (rc = part_hist_read(1, g, dS, cfg, w, st, nullptr)))
+        return rc;
+    if ((e = cudaMemcpyAsync(w.host_ctrl, w.ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+        return cuda_error(e, "direct join");
+    *direct = w.host_ctrl->direct != 0;
     return TBG_OK;
 }
 
@@ -275,8 +315,29 @@ int run_psm_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *d
     if (rc) return rc;
     mark_ev(w, timing, 1, st);
     int B = 0, lowbits = 0;
-    if (!cfg.materialize && nR && nS && msd_bits(span_of(rmin, rmax), &B, &lowbits))
-        return msd_count(cfg, dR, nR, dS, nS, rmin, B, lowbits, w, st, run);
+    if (!cfg.materialize && nR && nS) {
+        if (msd_bits(span_of(rmin, rmax), &B, &lowbits))
+            return msd_count(cfg, dR, nR, dS, nS, rmin, B, lowbits, 0, w, st, run);
+        if (span_of(rmin, rmax) <= kLowBits)
+            return msd_count(cfg, dR, nR, dS, nS, rmin, 1, lowbits, std::max<int>(1, (int)sort_plan(rmin, rmax).size()), w,
+                             st, run);
+    }
+    bool direct = false;
+    run->B = 8;
+    run->P = 0;
+    run->passes = 0;
+    auto done_direct = [&]() -> int {
+        for (int i = 2; i <= 4; i++) mark_ev(w, timing, i, st);
+        run->timed = timing;
+        return TBG_OK;
+    };
+    if (nR && nS && !msd_bits(span_of(rmin, rmax), &B, &lowbits)) {
+        if ((rc = direct_or_lsd(cfg, dR, nR, dS, nS, rmin, rmax, d_rows, cap, &direct, w, st))) return rc;
+        if (direct) {
+            run->passes = (int)sort_plan(rmin, rmax).size();
+            return done_direct();
+        }
+    }
     ENSURE(w.aux[0], nR * 8);
     ENSURE(w.aux[1], nR * 8);
     ENSURE(w.aux[2], nS * 8);
@@ -285,20 +346,18 @@ int run_psm_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *d
 #undef ENSURE
     Row *sorted[2] = {w.aux[0].as<Row>(), w.aux[2].as<Row>()};
     bool msd_done[2] = {false, false};
-    run->B = 8;
-    run->P = 0;
-    run->passes = 0;
     if (nR && nS) {
         bool s_outside = false;
-        if ((rc = msd_sort(cfg, dR, nR, dS, nS, rmin, span_of(rmin, rmax), true, sorted, msd_done, &s_outside, w, st,
-                           run)))
+        if ((rc = msd_sort(cfg, dR, nR, dS, nS, rmin, span_of(rmin, rmax), true, d_rows, cap, sorted, msd_done, &s_outside,
+                           &direct, w, st, run)))
             return rc;
+        if (direct) return done_direct();
         if (s_outside) {  // both relations' range, histograms again
             if ((rc = read_range(dS, nS, &smin, &smax))) return rc;
             have_s = true;
             const uint32_t lo = std::min(rmin, smin), hi = std::max(rmax, smax);
-            if ((rc = msd_sort(cfg, dR, nR, dS, nS, lo, span_of(lo, hi), false, sorted, msd_done, &s_outside, w,
-                               st, run)))
+            if ((rc = msd_sort(cfg, dR, nR, dS, nS, lo, span_of(lo, hi), false, d_rows, cap, sorted, msd_done, &s_outside,
+                               &direct, w, st, run)))
                 return rc;
         }
     }

@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm(JoinArgs a) {
     __shared__ unsigned long long s_base;
     __shared__ uint64_t scan_scratch[RSM_THREADS / 32 + 1];
     __shared__ uint32_t red[2];
+    if (*a.skip) return;
     const int tid = threadIdx.x;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
     unsigned long long local = 0;

@@ -40,14 +40,14 @@ struct Ctrl {
     unsigned long long nonempty;  // partitions with both sides non-empty
     unsigned long long heavy_rows_S;
     unsigned long long heavy_keys;
-    // direct counting join (direct.cu)
+    // direct join (direct.cu)
     unsigned long long direct_bits;  // bits set in the table
     unsigned int direct;             // 1: S was joined in its histogram read, the passes have nothing to do
     unsigned int direct_log2;        // log2 of the table's bits, 0: not tried
     unsigned int direct_dup;         // a key of R occurred twice
     unsigned int direct_inv_min;     // ~(smallest key of R), kept as a maximum so that it starts at 0
     unsigned int direct_max;         // largest key of R
-    unsigned int done[4];            // CTA tickets: column scans of R and of S, the bit count
+    unsigned int done[4];            // CTA tickets: column scans of R and of S, relations scanned; the bit count
     unsigned int pad;
 };
 
@@ -155,11 +155,10 @@ struct ColScan {
     int G = 0, P = 0;
 };
 
-// What the column scan's last CTA does (plan.r / plan.s hold the totals).
+// What the column scan's last CTAs do (plan.r / plan.s hold the totals).
 struct PlanTail {
-    int rels = 0;              // bit 0: R's bases, bit 1: S's
     int items = 0;             // also the work items
-    unsigned *done = nullptr;  // CTA ticket, zero before and after
+    unsigned *done = nullptr;  // CTA tickets [3] (R, S, relations), zero before and after; null: column scans only
     PlanArgs plan{};
 };
 
@@ -178,12 +177,16 @@ size_t join_smem_bytes(int capR);
 size_t join_launch_smem(int capR, bool materialize, int layout);
 int join_ctas_per_sm(int capR, bool materialize, int layout);
 
-// ---- direct counting join (direct.cu) ----
+// ---- direct join (direct.cu) ----
 int direct_log2_max(uint64_t nR);
-cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *bits, int log2_max, Ctrl *ctrl, int nsm,
-                               cudaStream_t st);
+cudaError_t launch_hist_emit(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
+                             const uint32_t *table, tbg_row_out *out, uint64_t cap, uint32_t range_max, Ctrl *ctrl,
+                             cudaStream_t st);
+int direct_log2_max_rows(uint64_t nR);
+cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *table, int log2_max, bool payloads, Ctrl *ctrl,
+                               int nsm, cudaStream_t st);
 cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
-                              uint32_t *bits, Ctrl *ctrl, cudaStream_t st);
+                              uint32_t *table, bool payloads, Ctrl *ctrl, cudaStream_t st);
 cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, Ctrl *ctrl, cudaStream_t st);
 cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
                               const uint32_t *bits, uint64_t nR, Ctrl *ctrl, cudaStream_t st);

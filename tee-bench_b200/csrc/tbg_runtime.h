@@ -33,7 +33,7 @@ struct Workspace {
     DevBuf chain_rows, chain_rel;  // chained join: first join's rows and the relation made of them
     DevBuf aux[8];              // algorithm-specific scratch (sort, learned model)
     DevBuf shard;               // shard split: per-chunk histograms and totals
-    DevBuf direct;              // direct counting join: R's bit table
+    DevBuf direct;              // direct join: R's table
     Ctrl *host_ctrl = nullptr;  // pinned mirror of the control block
     static constexpr size_t HOST_SMALL_BYTES = 4096;
     void *host_small = nullptr;  // pinned HOST_SMALL_BYTES: mid-call read-backs (LRN's decision, shard totals)
@@ -90,12 +90,15 @@ struct RadixGeom {
     // S's histogram also counts keys with key - rf.sub > s_range_max into
     // ctrl->out_of_range (S binned by R's key range); 0xFFFFFFFF: no check
     uint32_t s_range_max = 0xFFFFFFFFu;
-    bool direct = false;  // the histogram reads try the direct counting join
+    bool direct = false;  // the histogram reads try the direct join (direct.cu)
+    bool direct_rows = false;      // ... of a materialising join: R's payloads instead of bits,
+    tbg_row_out *rows = nullptr;   // ... S's read writes the rows here
+    uint64_t rows_cap = 0;
 };
 RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int capR, Workspace &w);
 RadixGeom radix_geometry_msd(uint64_t nR, uint64_t nS, uint32_t sub, int B, int lowbits, Workspace &w);
 int ensure_radix_buffers(const RadixGeom &g, bool bypass, Workspace &w);
-bool tries_direct(const tbg_config &cfg);
+void try_direct(RadixGeom &g, const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap);
 int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st);
 int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w, cudaStream_t st,
                    const SBypass *bypass);
@@ -107,7 +110,8 @@ int part_pass(int rel, int which, const RadixGeom &g, const Row *d, Workspace &w
 int plan_items(const RadixGeom &g, Workspace &w, cudaStream_t st);
 void mark(Workspace &w, bool timing, int i, cudaStream_t st);
 int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
-                    int capR, Workspace &w, cudaStream_t st, JoinRun *run, int *join_grid_out);
+                    tbg_row_out *d_rows, uint64_t cap, int capR, Workspace &w, cudaStream_t st, JoinRun *run,
+                    int *join_grid_out);
 int radix_join_phase(const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap, Workspace &w, cudaStream_t st,
                      JoinRun *run, int capR, int join_grid);
 int lsd_sort_chunked(const Row *in, uint64_t n, uint32_t kmin, uint32_t kmax, DevBuf &a, DevBuf &b, Workspace &w,

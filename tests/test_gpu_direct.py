@@ -102,3 +102,78 @@ def test_direct_async_and_sliced(tbg, oracle, cuda):
         assert [tbg.find("RHT").join(rel, S) for rel in (R, D)] == refs
     finally:
         tbg.set_dropin_slices(prev)
+
+
+# ---------------------------------------------------------------- materialising
+@pytest.mark.parametrize("algo", ["RHO", "RHT", "RSM", "PSM"])
+@pytest.mark.parametrize("nR,nS,lo,step,off", [(1, 1, 5, 1, 0), (3, 70001, 0, 1, 1), (4095, 4097, 1, 1, 0),
+                                               (8193, 65537, 31, 3, 1), (100003, 300007, 4294967295 - 1200036, 12, 1),
+                                               (100003, 300007, 1, 40, 0), (1500001, 3000017, 77, 1, 1)])
+def test_direct_rows(tbg, oracle, cuda, algo, nR, nS, lo, step, off):
+    rng = np.random.default_rng(nR + step)
+    R, S = relations(oracle, rng, nR, nS, lo, step, 0.3)
+    ref, ref_rows = oracle.rho(R, S, materialize=True)
+    m, rows, _ = run_join(tbg, cuda, algo, R, S, materialize=True, offset=off, cap=max(ref, 1))
+    assert m == ref
+    assert np.array_equal(oracle.sort_rows(rows), oracle.sort_rows(ref_rows))
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+@pytest.mark.parametrize("short", [0, 1, 4097])
+def test_direct_rows_stay_inside_the_buffer(tbg, oracle, cuda, shift, short):
+    """Output buffers at every 4-byte phase of a 16-byte word and capacities
+    below the row count: exact count, no word outside the buffer written."""
+    rng = np.random.default_rng(7)
+    R, S = relations(oracle, rng, 5003, 30011, 9, 2, 0.4)
+    ref, ref_rows = oracle.rho(R, S, materialize=True)
+    cap = ref - short
+    tR, pR = to_dev(cuda, R, 1)
+    tS, pS = to_dev(cuda, S)
+    out = cuda.full((3 * ref + 64,), -7, dtype=cuda.int32, device="cuda")
+    rc, m, _ = tbg.join_device(tbg.config("RHO", materialize=1), pR, len(R), pS, len(S), out.data_ptr() + 4 * (16 + shift),
+                               cap, check=False)
+    assert m == ref and rc == (tbg.ERR_CAPACITY if short else tbg.OK)
+    host = out.cpu().numpy()
+    a = 16 + shift
+    assert (host[:a] == -7).all() and (host[a + 3 * cap:] == -7).all()
+    got = oracle.sort_rows(host[a:a + 3 * cap].view(np.uint32).reshape(-1, 3))
+    if not short:
+        assert np.array_equal(got, oracle.sort_rows(ref_rows))
+    else:  # cap distinct rows of the result
+        code = lambda r: (r[:, 0].astype(np.uint64) << np.uint64(32)) | r[:, 2]  # noqa: E731
+        assert len(np.unique(code(got))) == cap and np.isin(code(got), code(ref_rows)).all()
+
+
+@pytest.mark.parametrize("case", ["empty_mark", "duplicate", "outlier", "zipf"])
+@pytest.mark.parametrize("algo", ["RHO", "RSM", "PSM"])
+def test_direct_rows_fall_back(tbg, oracle, cuda, algo, case):
+    """A payload equal to the table's empty mark, a duplicate key and a key
+    outside the sampled range send the join to the partitioned plan; a skewed
+    S does not."""
+    rng = np.random.default_rng(8)
+    R, S = relations(oracle, rng, 20011, 90001, 1000, 1, 0.2)
+    if case == "empty_mark":
+        R["payload"][77] = 0xFFFFFFFF
+        S["key"][5] = R["key"][77]
+    elif case == "duplicate":
+        R["key"][-1] = R["key"][0]
+    elif case == "outlier":
+        R["key"][3], S["key"][4] = 3000000000, 3000000000
+    else:
+        S["key"] = 1000 + np.minimum(rng.zipf(1.3, len(S)), 20010)
+    ref, ref_rows = oracle.rho(R, S, materialize=True)
+    m, rows, _ = run_join(tbg, cuda, algo, R, S, materialize=True, cap=ref)
+    assert m == ref
+    assert np.array_equal(oracle.sort_rows(rows), oracle.sort_rows(ref_rows))
+
+
+def test_direct_rows_sliced(tbg, oracle, cuda):
+    rng = np.random.default_rng(9)
+    R, S = relations(oracle, rng, 60013, 250007, 1, 1, 0.25)
+    ref, ref_rows = oracle.rho(R, S, materialize=True)
+    prev = tbg.set_dropin_slices(3)
+    try:
+        c, rows = tbg.find("RHO").join(R, S, 2, materialize=True)
+    finally:
+        tbg.set_dropin_slices(prev)
+    assert c == ref and np.array_equal(oracle.sort_rows(rows), oracle.sort_rows(ref_rows))
