@@ -299,7 +299,10 @@ typedef struct tbg_batch tbg_batch; /* opaque plan: tuned, graph-captured */
  * item and chunk size per size class by timing the batch's own joins;
  * radix_bits > 0 partitions every join with that many bits (one pass, <= 8);
  * radix_bits < 0 uses the built-in heuristic without timing.  The whole
- * batch is captured as one CUDA graph.  Waits for `stream` (the inputs may be
+ * batch is captured as one CUDA graph.  Unless radix_bits > 0, joins whose R
+ * holds distinct keys in a compact range when the plan is made (one run of the
+ * batch tells) are first tried with a bit per key value on every run, and
+ * partitioned when that run's contents do not allow it.  Waits for `stream` (the inputs may be
  * written there), then works on a private stream; the relations must stay
  * allocated, at the same addresses, until tbg_batch_destroy (their contents
  * may change between runs).                                                */

@@ -7,7 +7,9 @@
 // no cache line is shared by two joins); and lists the tickets of the
 // persistent kernel.  The autotuner picks those choices per size class
 // (floor(log2 |R_i|)) by timing candidate plans over the batch's own joins
-// of that class.  The final plan is captured as one CUDA graph: a memset of
+// of that class, without the direct join (which the kernel tries first on
+// every run, and which needs no choice): the tuned plan is what takes over
+// when a run's contents are not direct.  The final plan is captured as one CUDA graph: a memset of
 // the progress counters and results, the persistent kernel, and a copy of
 // the device error word to pinned host memory.
 //
@@ -67,6 +69,7 @@ struct Plan {
     BatchArgs args{};
     uint64_t rows = 0;  // input rows covered by the plan
     uint32_t tickets = 0;
+    std::vector<int> order;  // caller's index of each join of the plan
 };
 
 int validate(const tbg_batch_join *joins, int njoins) {
@@ -83,19 +86,31 @@ int validate(const tbg_batch_join *joins, int njoins) {
     return TBG_OK;
 }
 
+// log2 of a join's bit table (0: none): room for a dense key range, twice that
+// while one CTA can build it whole.
+uint32_t bit_table_log2(uint64_t nR) {
+    if (nR > (1ull << BATCH_BITS_MAX_LOG2)) return 0;
+    uint32_t w = 12;
+    while ((1ull << w) < nR) w++;
+    if (w < (uint32_t)BATCH_PART_LOG2 && (1ull << w) < 2 * nR) w++;
+    return w;
+}
+
 // Builds the plan of joins `sel` (indices into `joins`) with choice
-// `ch[size_class]`; allocates and uploads everything the kernel reads.
+// `ch[size_class]`, with bit tables for the joins of `tables` (by index into
+// `joins`; empty: none) that may have one; allocates and uploads everything the kernel reads.
 // Uploads are ordered on `st` and complete when this returns.
 int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &sel, const Choice *ch,
-               int grid, Plan &p, cudaStream_t st) {
+               int grid, const std::vector<char> &tables, Plan &p, cudaStream_t st) {
     std::vector<int> order(sel);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return joins[a].nR + joins[a].nS > joins[b].nR + joins[b].nS;
     });
     std::vector<BatchJoin> bj;
-    std::vector<uint2> chunks, jt;
+    std::vector<uint2> builds, chunks, jt;
+    std::vector<uint2> dchunks;
     std::vector<uint32_t> scans;
-    struct Off { size_t rp, sp, hr, hs, br, bs, it; };
+    struct Off { size_t rp, sp, hr, hs, br, bs, it, bits; };
     std::vector<Off> off;
     size_t part_bytes = 0, meta2 = 0;  // partitioned rows | histograms, bases, items
     uint64_t rows = 0;
@@ -117,6 +132,14 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
         const uint32_t j = (uint32_t)bj.size();
         rows += in.nR + in.nS;
         Off o{};
+        J.bits_log2 = !tables.empty() && tables[idx] ? bit_table_log2(in.nR) : 0;
+        if (J.bits_log2) {
+            o.bits = meta2;
+            meta2 = align_up(meta2 + ((size_t)1 << (J.bits_log2 - 3)));
+            const uint32_t parts = J.bits_log2 > (uint32_t)BATCH_PART_LOG2 ? 1u << (J.bits_log2 - BATCH_PART_LOG2) : 1u;
+            for (uint32_t k = 0; k < parts; k++) builds.push_back(make_uint2(j, k));
+            for (uint64_t k = 0; k < ceil_div(in.nS, BATCH_DCHUNK); k++) dchunks.push_back(make_uint2(j, (uint32_t)k));
+        }
         if (c.B > 0) {
             J.GR = (uint32_t)ceil_div(in.nR, c.chunk);
             J.GS = (uint32_t)ceil_div(in.nS, c.chunk);
@@ -140,7 +163,7 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
         bj.push_back(J);
         off.push_back(o);
     }
-    if (chunks.size() >= (1u << 30) || jt.size() >= (1u << 30))
+    if (chunks.size() >= (1u << 30) || dchunks.size() >= (1u << 30) || jt.size() >= (1u << 30))
         return set_error(TBG_ERR_ARG, "batch too large: %zu chunks", chunks.size());
     // device memory: [partitioned rows][histograms, bases, items] and the plan arrays
     const size_t meta_off = part_bytes;
@@ -149,8 +172,9 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
     char *base = p.part.as<char>();
     for (size_t k = 0; k < bj.size(); k++) {
         BatchJoin &J = bj[k];
-        if (J.B == 0) continue;
         const Off &o = off[k];
+        if (J.bits_log2) J.bits = reinterpret_cast<uint32_t *>(base + meta_off + o.bits);
+        if (J.B == 0) continue;
         J.Rp = reinterpret_cast<Row *>(base + o.rp);
         J.Sp = reinterpret_cast<Row *>(base + o.sp);
         J.histR = reinterpret_cast<uint32_t *>(base + meta_off + o.hr);
@@ -168,12 +192,16 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
     const size_t m_chunks = align_up(m_joins + bj.size() * sizeof(BatchJoin));
     const size_t m_scans = align_up(m_chunks + chunks.size() * sizeof(uint2));
     const size_t m_jt = align_up(m_scans + scans.size() * sizeof(uint32_t));
-    const size_t m_end = align_up(m_jt + jt.size() * sizeof(uint2));
+    const size_t m_builds = align_up(m_jt + jt.size() * sizeof(uint2));
+    const size_t m_dchunks = align_up(m_builds + builds.size() * sizeof(uint2));
+    const size_t m_end = align_up(m_dchunks + dchunks.size() * sizeof(uint2));
     std::vector<char> host(m_end);
     if (!bj.empty()) memcpy(host.data() + m_joins, bj.data(), bj.size() * sizeof(BatchJoin));
     if (!chunks.empty()) memcpy(host.data() + m_chunks, chunks.data(), chunks.size() * sizeof(uint2));
     if (!scans.empty()) memcpy(host.data() + m_scans, scans.data(), scans.size() * sizeof(uint32_t));
     if (!jt.empty()) memcpy(host.data() + m_jt, jt.data(), jt.size() * sizeof(uint2));
+    if (!dchunks.empty()) memcpy(host.data() + m_dchunks, dchunks.data(), dchunks.size() * sizeof(uint2));
+    if (!builds.empty()) memcpy(host.data() + m_builds, builds.data(), builds.size() * sizeof(uint2));
     e = p.meta.ensure(std::max<size_t>(ALIGN, m_end));
     if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (batch plan)");
     if (m_end) {
@@ -195,18 +223,26 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
     a.chunks = reinterpret_cast<const uint2 *>(m + m_chunks);
     a.scans = reinterpret_cast<const uint32_t *>(m + m_scans);
     a.jt = reinterpret_cast<const uint2 *>(m + m_jt);
+    a.builds = reinterpret_cast<const uint2 *>(m + m_builds);
+    a.dchunks = reinterpret_cast<const uint2 *>(m + m_dchunks);
     a.ticket = reinterpret_cast<unsigned *>(c);
     a.err = reinterpret_cast<unsigned *>(c) + 1;
+    a.direct = reinterpret_cast<unsigned *>(c) + 2;
     a.sync = reinterpret_cast<BatchSync *>(c + sync_off);
     a.counts = reinterpret_cast<unsigned long long *>(c + p.counts_off);
+    a.n_builds = (uint32_t)builds.size();
     a.n_chunks = (uint32_t)chunks.size();
+    a.n_dchunks = (uint32_t)dchunks.size();
+    a.njoins = (uint32_t)bj.size();
     a.n_scans = (uint32_t)scans.size();
     a.n_jt = (uint32_t)jt.size();
     a.capR = BATCH_CAPR;
     p.grid = grid;
     p.njoins = njoins;
     p.rows = rows;
-    p.tickets = 2 * a.n_chunks + a.n_scans + a.n_jt;
+    p.order.clear();
+    for (const BatchJoin &J : bj) p.order.push_back((int)J.orig);
+    p.tickets = a.n_builds + a.n_dchunks + 2 * a.n_chunks + a.n_scans + a.n_jt;
     return TBG_OK;
 }
 
@@ -241,6 +277,44 @@ int time_plan(const Plan &p, cudaStream_t st, int reps, double *ms, unsigned *er
     *err_host = err;
     if (err) return set_error((int)err, "batch autotune run: device status %u", err);
     *ms = best;
+    return TBG_OK;
+}
+
+// Runs a plan with bit tables once and leaves in `tables` the joins that were
+// direct: the others' tables cost a build that comes to nothing.  A plan whose
+// direct joins hold less than a quarter of the rows keeps none, and runs the
+// kernel without the direct phases (their code costs its partitioning tickets
+// registers: a batch of sparse keys took 12% longer with it).  *changed: the
+// plan has to be made again.
+int keep_direct(const Plan &p, const tbg_batch_join *joins, std::vector<char> &tables, bool *changed, cudaStream_t st) {
+    *changed = false;
+    const size_t n = p.order.size();
+    std::vector<BatchSync> sync(n);
+    unsigned err = 0;
+    cudaError_t e = enqueue(p, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(sync.data(), p.args.sync, n * sizeof(BatchSync), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&err, p.args.err, sizeof err, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_error(e, "batch: first run");
+    if (err) return set_error((int)err, "batch: first run: device status %u", err);
+    uint64_t rows = 0, direct_rows = 0;
+    std::vector<char> keep(tables.size(), 0);
+    for (size_t k = 0; k < n; k++) {
+        const int i = p.order[k];
+        rows += joins[i].nR + joins[i].nS;
+        if (sync[k].decision != 1) {
+            *changed |= tables[i] && bit_table_log2(joins[i].nR);
+            continue;
+        }
+        direct_rows += joins[i].nR + joins[i].nS;
+        keep[i] = 1;
+    }
+    if (direct_rows * 4 < rows) {
+        *changed |= direct_rows > 0;
+        keep.clear();
+    }
+    tables.swap(keep);
     return TBG_OK;
 }
 
@@ -296,7 +370,7 @@ static int autotune(tbg_batch *b, const tbg_batch_join *joins, int njoins, int g
         auto run = [&](Choice cand) -> int {
             Choice tab[NCLASS];
             tab[c] = cand;
-            int rc = build_plan(joins, njoins, sample, tab, grid, trial, b->st);
+            int rc = build_plan(joins, njoins, sample, tab, grid, {}, trial, b->st);
             if (rc) return rc;
             double ms = 0;
             unsigned err = 0;
@@ -411,7 +485,15 @@ TBG_API int tbg_batch_create(const tbg_batch_join *joins, int njoins, const tbg_
     }
     std::vector<int> all(njoins);
     for (int i = 0; i < njoins; i++) all[i] = i;
-    rc = build_plan(joins, njoins, all, b->cls, grid, b->plan, b->st);
+    // bit tables under the automatic plan (a fixed radix partitions every join)
+    std::vector<char> tables;
+    if (c.radix_bits <= 0) tables.assign(njoins, 1);
+    rc = build_plan(joins, njoins, all, b->cls, grid, tables, b->plan, b->st);
+    if (!rc && b->plan.args.n_builds) {
+        bool changed = false;
+        rc = keep_direct(b->plan, joins, tables, &changed, b->st);
+        if (!rc && changed) rc = build_plan(joins, njoins, all, b->cls, grid, tables, b->plan, b->st);
+    }
     if (rc) {
         batch_free(b);
         return rc;

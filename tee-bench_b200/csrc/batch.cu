@@ -1,6 +1,8 @@
 // Batched joins in one persistent launch.
 //
 // Every CTA pulls tickets from one counter; the ticket ranges are, in order,
+//   build    one part of one join's bit table (direct joins, below);
+//   probe    one chunk of the S_i of a join with a bit table;
 //   hist     one chunk (`chunk` rows) of R_i or S_i: shared-memory histogram
 //            over the join's P = 2^B partitions (low key bits);
 //   scan     one join: column prefix of its chunk histograms (in place),
@@ -8,12 +10,22 @@
 //   scatter  one chunk: the TMA-fed digit-sorting tile scatter of the
 //            single-join partitioner, cursors = base[f] + prefix[chunk][f];
 //   join     one worker of a partitioned join (pulls that join's items) or
-//            one S slice of a direct join (B = 0, R_i loaded whole);
+//            one S slice of an unpartitioned join (B = 0, R_i loaded whole);
 // build/probe runs out of shared memory as in the single-join kernel.  A
 // ticket waits only on tickets handed out before it (per-join counters with
 // acquire/release), so there is no grid-wide barrier and no co-residency
 // requirement.  Data written earlier in the launch (histograms, bases,
 // items, partitioned rows) is read with L2-only loads.
+//
+// Direct joins: when R_i's keys are distinct and lie in a compact range, one
+// bit per key value is its whole hash table (direct.cu).  A build ticket
+// enters R_i's keys into shared memory, where a key that is already there
+// shows a duplicate, and writes the bits out; a probe ticket looks rows of S_i
+// up in a copy of the bits.  S_i is read once and nothing is written.  The
+// other tickets pass over the joins that are direct, and a CTA ends at the
+// first of them when all are.  Bound by reading R and S: 512 joins of 2^10 ..
+// 2^18 R rows, 228 M rows in all, take 0.46 ms (4.0 TB/s) against 1.89 ms
+// partitioned.
 //
 // Each join's count equals the reference's RHO count on that join
 // (Joins/radix_join.c:1558-1561, join_init_run :1237-1396; bucket
@@ -29,6 +41,7 @@ namespace tbg {
 namespace {
 
 using BPart = PartSmem<BATCH_THREADS>;
+static_assert(((size_t)1 << (BATCH_PART_LOG2 - 3)) <= sizeof(BPart), "a part of a bit table fits");
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
     unsigned v;
@@ -64,6 +77,142 @@ __device__ void cta_signal(unsigned *flag) {
 }
 
 __device__ __forceinline__ int ilog2(uint32_t p) { return 31 - __clz(p); }
+
+// ---------------------------------------------------------------------------
+// direct joins
+// ---------------------------------------------------------------------------
+
+// fn(key) for the rows [0, n) of s, this thread's share, 8 rows in flight (a
+// plain loop: the other tickets' code leaves few registers free).
+template <class Fn>
+__device__ __forceinline__ void stream_keys(const Row *s, uint32_t n, Fn fn) {
+    constexpr uint32_t T = BATCH_THREADS;
+    const uint32_t head = (reinterpret_cast<uintptr_t>(s) & 15) && n ? 1u : 0u;
+    const uint32_t nv = (n - head) / 2;
+    const uint4 *v = reinterpret_cast<const uint4 *>(s + head);
+    if (threadIdx.x == 0) {
+        if (head) fn(s[0].key);
+        if ((n - head) & 1) fn(s[n - 1].key);
+    }
+    uint32_t i = threadIdx.x;
+    for (; i + 3 * T < nv; i += 4 * T) {
+        const uint4 a = ldg_stream(v + i), b = ldg_stream(v + i + T), c = ldg_stream(v + i + 2 * T),
+                    d = ldg_stream(v + i + 3 * T);
+        fn(a.x), fn(a.z), fn(b.x), fn(b.z), fn(c.x), fn(c.z), fn(d.x), fn(d.z);
+    }
+    for (; i < nv; i += T) {
+        const uint4 a = ldg_stream(v + i);
+        fn(a.x), fn(a.z);
+    }
+}
+
+__device__ __forceinline__ void block_min_max(uint32_t lo, uint32_t hi, uint32_t *red) {
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&red[0], lo);
+        atomicMax(&red[1], hi);
+    }
+    __syncthreads();
+}
+
+// Part `bt.y` of a join's bit table: the bits [bt.y * 2^BATCH_PART_LOG2, ...) of it.
+// A sample of R (the same for every part) that is wider than the table ends
+// the attempt before R is read.  The last part to finish decides.
+__device__ void build_part(const BatchArgs &a, uint32_t q, uint32_t *bits, uint32_t *red) {
+    const uint2 bt = a.builds[q];
+    const BatchJoin &J = a.joins[bt.x];
+    BatchSync &sy = a.sync[bt.x];
+    const int tid = threadIdx.x;
+    const uint32_t w = J.bits_log2, mask = (1u << w) - 1;
+    const uint32_t part_log2 = min(w, (uint32_t)BATCH_PART_LOG2), words = 1u << (part_log2 - 5);
+    if (tid == 0) {
+        red[0] = ~0u;
+        red[1] = 0;
+    }
+    __syncthreads();
+    {
+        const uint64_t n = J.nR;
+        const uint64_t i = n <= BATCH_THREADS ? tid : (uint64_t)tid * (n - 1) / (BATCH_THREADS - 1);
+        const uint32_t k = i < n ? J.R[i].key : J.R[0].key;
+        block_min_max(k, k, red);
+    }
+    if (red[1] - red[0] > mask) {
+        if (tid == 0) atomicExch(&sy.off, 1u);
+    } else {
+        for (uint32_t i = tid; i < words; i += BATCH_THREADS) bits[i] = 0;
+        __syncthreads();
+        uint32_t lo = ~0u, hi = 0;
+        bool dup = false;
+        stream_keys(J.R, (uint32_t)J.nR, [&](uint32_t k) {
+            lo = min(lo, k);
+            hi = max(hi, k);
+            const uint32_t s = k & mask;
+            if (s >> part_log2 == bt.y) {
+                const uint32_t b = s & ((1u << part_log2) - 1), bit = 1u << (b & 31);
+                dup |= (atomicOr(&bits[b >> 5], bit) & bit) != 0;
+            }
+        });
+        if (dup) atomicExch(&sy.off, 1u);
+        __syncthreads();
+        block_min_max(lo, hi, red);  // the sample's range lies inside R's
+        if (tid == 0) {
+            atomicMax(&sy.inv_min, ~red[0]);
+            atomicMax(&sy.kmax, red[1]);
+        }
+        uint4 *dst = reinterpret_cast<uint4 *>(J.bits + (size_t)bt.y * words);
+        for (uint32_t i = tid; i < words / 4; i += BATCH_THREADS) __stcg(dst + i, reinterpret_cast<uint4 *>(bits)[i]);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        const uint32_t parts = 1u << (w - part_log2);
+        if (atomicAdd(&sy.build_done, 1u) == parts - 1) {
+            __threadfence();
+            const bool ok = !__ldcg(&sy.off) && __ldcg(&sy.kmax) - ~__ldcg(&sy.inv_min) <= mask;
+            if (ok) atomicAdd(a.direct, 1u);
+            __threadfence();
+            atomicExch(&sy.decision, ok ? 1u : 2u);
+        }
+    }
+}
+
+// Whether join j is direct (the same for every thread); waits for its bit
+// table's decision.
+template <bool DIRECT>
+__device__ __forceinline__ bool is_direct(const BatchArgs &a, uint32_t j) {
+    if (!DIRECT || !a.joins[j].bits) return false;
+    cta_wait(&a.sync[j].decision, 1, a.err);
+    return __ldcg(&a.sync[j].decision) == 1;
+}
+
+// Matches of one chunk of a direct join's S: bits from a copy in shared
+// memory (`cap` words), or from L2 when R's range is wider.
+__device__ void direct_chunk(const BatchArgs &a, uint32_t q, uint32_t *copy, uint32_t cap) {
+    const uint2 c = a.dchunks[q];
+    const uint32_t j = c.x;
+    if (!is_direct<true>(a, j)) return;
+    const BatchJoin &J = a.joins[j];
+    const uint64_t lo = (uint64_t)c.y * BATCH_DCHUNK, hi = umin64(J.nS, lo + BATCH_DCHUNK);
+    const uint32_t kmin = ~__ldcg(&a.sync[j].inv_min), span = __ldcg(&a.sync[j].kmax) - kmin;
+    const uint32_t wordmask = (1u << (J.bits_log2 - 5)) - 1, w0 = kmin >> 5;
+    const uint32_t words = ((kmin + span) >> 5) - w0 + 1;
+    const uint32_t *bits = J.bits;
+    uint32_t local = 0;  // a chunk holds BATCH_DCHUNK rows at most
+    if (words <= cap) {
+        for (uint32_t i = threadIdx.x; i < words; i += BATCH_THREADS) copy[i] = __ldcg(bits + ((w0 + i) & wordmask));
+        __syncthreads();
+        stream_keys(J.S + lo, (uint32_t)(hi - lo), [&](uint32_t k) {
+            if (k - kmin <= span) local += (copy[(k >> 5) - w0] >> (k & 31)) & 1u;
+        });
+    } else {
+        stream_keys(J.S + lo, (uint32_t)(hi - lo), [&](uint32_t k) {
+            if (k - kmin <= span) local += (__ldcg(bits + ((k >> 5) & wordmask)) >> (k & 31)) & 1u;
+        });
+    }
+    local = __reduce_add_sync(0xffffffffu, local);
+    if ((threadIdx.x & 31) == 0 && local) atomicAdd(a.counts + J.orig, (unsigned long long)local);
+}
 
 // ---------------------------------------------------------------------------
 // hist: chunk histogram over the join's partitions
@@ -314,29 +463,46 @@ static_assert(sizeof(Item) == 32, "join_ticket reads an item as two 16-byte word
 
 }  // namespace
 
-__global__ void __launch_bounds__(BATCH_THREADS, 2) k_batch(BatchArgs a) {
+// DIRECT: the plan has bit tables.
+template <bool DIRECT>
+__global__ void __launch_bounds__(BATCH_THREADS, 2) k_batch(BatchArgs a, uint32_t smem_words) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t mbar[PART_NBUF];
     __shared__ uint64_t scratch[BATCH_THREADS / 32 + 1];
-    __shared__ uint32_t s_ticket, s_item;
+    __shared__ uint32_t s_ticket, s_item, s_red[2];
     const int tid = threadIdx.x;
     if (tid == 0) {
         for (int i = 0; i < PART_NBUF; i++) mbar_init(&mbar[i], 1);
         fence_mbar_init();
     }
     uint32_t kseq = 0;
-    const uint32_t t_scan = a.n_chunks, t_scat = t_scan + a.n_scans, t_join = t_scat + a.n_chunks;
-    const uint32_t t_end = t_join + a.n_jt;
+    const uint32_t t_hist = DIRECT ? a.n_builds + a.n_dchunks : 0u, t_scan = t_hist + a.n_chunks;
+    const uint32_t t_scat = t_scan + a.n_scans, t_join = t_scat + a.n_chunks, t_end = t_join + a.n_jt;
     for (;;) {
-        if (tid == 0) s_ticket = atomicAdd(a.ticket, 1u);
+        if (tid == 0) {
+            uint32_t t = atomicAdd(a.ticket, 1u);
+            if (DIRECT && t >= t_hist && ld_acquire_u32(a.direct) == a.njoins) t = t_end;  // nothing is left to do
+            s_ticket = t;
+        }
         __syncthreads();
         const uint32_t t = s_ticket;
         __syncthreads();
         if (t >= t_end) break;
-        if (t < t_scan) hist_chunk(a, t, reinterpret_cast<uint32_t *>(smem));
-        else if (t < t_scat) scan_join(a, t - t_scan, reinterpret_cast<uint32_t *>(smem), scratch);
-        else if (t < t_join) scatter_chunk(a, t - t_scat, *reinterpret_cast<BPart *>(smem), mbar, kseq);
-        else join_ticket(a, t - t_join, smem, scratch, &s_item);
+        if (DIRECT && t < t_hist) {
+            if (t < a.n_builds) build_part(a, t, reinterpret_cast<uint32_t *>(smem), s_red);
+            else direct_chunk(a, t - a.n_builds, reinterpret_cast<uint32_t *>(smem), smem_words);
+        } else {
+            // the join of this ticket
+            const uint32_t j = t < t_scan ? a.chunks[t - t_hist].x
+                             : t < t_scat ? a.scans[t - t_scan]
+                             : t < t_join ? a.chunks[t - t_scat].x
+                                          : a.jt[t - t_join].x;
+            if (is_direct<DIRECT>(a, j)) continue;
+            if (t < t_scan) hist_chunk(a, t - t_hist, reinterpret_cast<uint32_t *>(smem));
+            else if (t < t_scat) scan_join(a, t - t_scan, reinterpret_cast<uint32_t *>(smem), scratch);
+            else if (t < t_join) scatter_chunk(a, t - t_scat, *reinterpret_cast<BPart *>(smem), mbar, kseq);
+            else join_ticket(a, t - t_join, smem, scratch, &s_item);
+        }
         __syncthreads();  // shared memory is reused by the next ticket
     }
 }
@@ -353,8 +519,9 @@ size_t batch_smem_bytes() {
 cudaError_t batch_occupancy(int *per_sm) {
     const size_t smem = batch_smem_bytes();
     int n = 0;
-    cudaError_t e = smem_limit((const void *)k_batch, smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch, BATCH_THREADS, smem);
+    cudaError_t e = smem_limit((const void *)k_batch<false>, smem);
+    if (e == cudaSuccess) e = smem_limit((const void *)k_batch<true>, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch<true>, BATCH_THREADS, smem);
     if (e != cudaSuccess) return e;
     *per_sm = n < 1 ? 1 : n;
     return cudaSuccess;
@@ -369,7 +536,9 @@ int batch_ctas_per_sm() {
 // batch_ctas_per_sm() (called when a plan is made, outside any stream
 // capture) sets the kernel's shared-memory attribute.
 cudaError_t launch_batch(const BatchArgs &a, int grid, cudaStream_t st) {
-    k_batch<<<grid, BATCH_THREADS, batch_smem_bytes(), st>>>(a);
+    const size_t smem = batch_smem_bytes();
+    auto kern = a.n_builds ? k_batch<true> : k_batch<false>;
+    kern<<<grid, BATCH_THREADS, smem, st>>>(a, (uint32_t)(smem / 4));
     count_launch();
     return cudaGetLastError();
 }

@@ -207,3 +207,46 @@ def test_batch_c4_full(tbg, oracle, cuda):
     if free < 120 * (1 << 30):
         pytest.skip("needs ~100 GB of free device memory")
     _c4_check(tbg, oracle, torch, 4096, 10, 20, seed=4, oracle_joins=3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, -1])
+def test_batch_direct_joins_follow_their_contents(tbg, oracle, cuda, mode):
+    """A plan made on distinct dense keys joins through bit tables (one CTA's
+    part: 2^19 key values; two parts at 600001 rows); new contents in the same
+    buffers -- duplicates, keys outside the table's range, keys that wrap at
+    2^32, misses around R's range -- give their own counts, and a plan made on
+    sparse keys takes dense ones too."""
+    torch = cuda
+    rs = np.random.RandomState(11)
+    sizes = [1, 33, 4096, 4097, 8192, 70001, 262144, 524288, 600001]
+
+    def contents(kind):
+        out = []
+        for n in sizes:
+            lo = {"dense": 1, "wrap": 2 ** 32 - n}.get(kind, 1000)
+            keys = lo + rs.permutation(n).astype(np.int64)
+            if kind == "dup" and n > 1:
+                keys[-1] = keys[0]
+            elif kind == "outlier":
+                keys[n // 2] = 4000000000
+            elif kind == "sparse":
+                keys = (keys * 2654435761) % 2 ** 32
+            S = np.where(rs.random_sample(2 * n + 3) < 0.7, keys[rs.randint(0, n, 2 * n + 3)],
+                         (lo - 50 + rs.randint(0, n + 100, 2 * n + 3)) % 2 ** 32)
+            out.append((_rel(keys), _rel(S)))
+        return out
+
+    for first in ("dense", "sparse"):
+        joins = contents(first)
+        buf, dj = upload(torch, joins)
+        b = tbg.Batch(dj, tbg.config("RHO", radix_bits=mode))
+        try:
+            assert run_batch(tbg, torch, b, len(dj)) == oracle_counts(oracle, joins), first
+            for kind in ("dup", "outlier", "wrap", "sparse", "dense"):
+                joins = contents(kind)
+                new, _ = upload(torch, joins)
+                buf.copy_(new)
+                assert run_batch(tbg, torch, b, len(dj)) == oracle_counts(oracle, joins), (first, kind)
+        finally:
+            b.close()
