@@ -10,7 +10,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <atomic>
 #include <mutex>
+#include <thread>
+#include <vector>
 
 #include "tbg_internal.h"
 #include "tbg_runtime.h"
@@ -51,9 +54,80 @@ static cudaError_t slice_streams() {
     return e;
 }
 
+// Copies from pageable memory.  The driver stages them through its own pinned
+// buffer on one core (11 GB/s); here up to STAGE_THREADS threads copy chunks
+// into pinned slots of their own and enqueue each chunk's transfer, so the
+// transfers follow one another at the link's rate as long as the cores keep up
+// (2^22 + 2^25 rows, 302 MB: 8.5 ms against 27.2 ms).  The slots (STAGE_BYTES
+// in all) are kept for the next call; calls are serialised by g_dropin_mu.
+constexpr int STAGE_THREADS = 8, STAGE_SLOTS = 3;
+constexpr size_t STAGE_CHUNK = 1u << 20;
+constexpr size_t STAGE_BYTES = STAGE_THREADS * STAGE_SLOTS * STAGE_CHUNK;
+// Below 24 MB the driver's copy is as fast (the source is still in the host's
+// caches, and starting the threads takes 0.1 ms each: 16 MB 1.1 ms against 1.2
+// to 1.5 ms; 32 MB 2.6 against 2.1 ms); one thread per 8 MB.
+constexpr size_t STAGE_MIN = 24u << 20, STAGE_PER_THREAD = 8u << 20;
+static char *g_stage = nullptr;
+static cudaEvent_t g_stage_free[STAGE_THREADS * STAGE_SLOTS];  // the slot's last transfer is done
+
+static bool stage_ready() {
+    if (g_stage) return true;
+    for (auto &ev : g_stage_free)
+        if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) ev = nullptr;
+    bool ok = cudaMallocHost(&g_stage, STAGE_BYTES) == cudaSuccess;
+    for (auto &ev : g_stage_free) ok = ok && ev;
+    if (!ok) {
+        cudaGetLastError();
+        if (g_stage) cudaFreeHost(g_stage);
+        g_stage = nullptr;
+    }
+    return ok;
+}
+
+static bool pageable(const void *p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
+}
+
+// Every byte's transfer is enqueued on `st` when it returns.
 static cudaError_t h2d(void *dst, const void *src, size_t bytes, cudaStream_t st) {
     if (!bytes) return cudaSuccess;
-    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
+    const int nt = (int)std::min<size_t>(std::min<unsigned>(STAGE_THREADS, cores), bytes / STAGE_PER_THREAD);
+    int dev = 0;
+    if (bytes < STAGE_MIN || nt < 2 || !pageable(src) || !stage_ready() || cudaGetDevice(&dev) != cudaSuccess)
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    const size_t nchunks = (bytes + STAGE_CHUNK - 1) / STAGE_CHUNK;
+    std::atomic<size_t> next{0};
+    std::atomic<int> failed{cudaSuccess};
+    auto work = [&](int t) {
+        cudaError_t e = cudaSetDevice(dev);
+        for (int k = 0; e == cudaSuccess && !failed.load(); k++) {
+            const size_t c = next.fetch_add(1);
+            if (c >= nchunks) break;
+            const int slot = t * STAGE_SLOTS + k % STAGE_SLOTS;
+            const size_t off = c * STAGE_CHUNK, len = std::min(STAGE_CHUNK, bytes - off);
+            char *buf = g_stage + (size_t)slot * STAGE_CHUNK;
+            if ((e = cudaEventSynchronize(g_stage_free[slot])) != cudaSuccess) break;
+            memcpy(buf, static_cast<const char *>(src) + off, len);
+            if ((e = cudaMemcpyAsync(static_cast<char *>(dst) + off, buf, len, cudaMemcpyHostToDevice, st)) == cudaSuccess)
+                e = cudaEventRecord(g_stage_free[slot], st);
+        }
+        if (e != cudaSuccess) failed.store(e);
+    };
+    std::vector<std::thread> helpers;
+    try {
+        helpers.reserve(nt - 1);
+        for (int t = 1; t < nt; t++) helpers.emplace_back(work, t);
+    } catch (...) {  // fewer helpers than wanted: the chunks are shared among those there are
+    }
+    work(0);
+    for (auto &h : helpers) h.join();
+    return (cudaError_t)failed.load();
 }
 
 static result_t *fail(int code) {
