@@ -415,8 +415,12 @@ int part_histogram(int rel, const RadixGeom &g, const Row *d, const tbg_config &
 // 20 us from every join that is not direct); a caller who fixes the radix bits
 // or passes, or turns the skew split off, gets the partitioned join.  A
 // materialising join tries it while R can fit the payload table at all.
+bool automatic_plan(const tbg_config &cfg) {
+    return cfg.radix_bits <= 0 && (cfg.passes <= 0 || cfg.passes > 2) && cfg.skew_split;
+}
+
 void try_direct(RadixGeom &g, const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap) {
-    g.direct = cfg.radix_bits <= 0 && (cfg.passes <= 0 || cfg.passes > 2) && cfg.skew_split;
+    g.direct = automatic_plan(cfg);
     if (!cfg.materialize) return;
     g.direct = g.direct && d_rows && g.n[0] <= (1ull << direct_log2_max_rows(g.n[0]));
     g.direct_rows = true;
@@ -540,6 +544,10 @@ int run_radix_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row 
                    tbg_row_out *d_rows, uint64_t cap, Workspace &w, cudaStream_t st,
                    JoinRun *run) {
     const int capR = join_capacity(nR, !cfg.materialize);
+    if (nR <= SMALL_R) {
+        const RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
+        if (is_small_join(cfg, g)) return run_small_join(cfg, g, dR, dS, d_rows, cap, w, st, run);
+    }
     int join_grid = 0;
     int rc = radix_partition(cfg, dR, nR, dS, nS, d_rows, cap, capR, w, st, run, &join_grid);
     if (rc) return rc;
@@ -656,7 +664,9 @@ int radix_join_phase(const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap, W
 // Reads back the control block and fills stats; waits for the stream.
 int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, const JoinRun &run,
                 uint64_t nR, uint64_t nS, uint64_t cap, uint64_t *matches, tbg_stats *stats) {
-    cudaError_t e = cudaMemcpyAsync(w.host_ctrl, w.ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, st);
+    cudaError_t e = run.ctrl_on_host
+                        ? cudaSuccess
+                        : cudaMemcpyAsync(w.host_ctrl, w.ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return cuda_error(e, "readback");
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_error(e, "join");
     const Ctrl &c = *w.host_ctrl;
@@ -772,6 +782,7 @@ int tbg_join_device(const tbg_config *cfg, const struct row_t *dR, uint64_t nR,
     t_err = TBG_OK;
     cudaStream_t st = (cudaStream_t)stream;
     JoinRun run;
+    run.waits = true;
     Workspace *w = nullptr;
     int rc = join_device_impl(cfg, reinterpret_cast<const Row *>(dR), nR,
                               reinterpret_cast<const Row *>(dS), nS, d_rows, rows_cap, st, &run, &w);

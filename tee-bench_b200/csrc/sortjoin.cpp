@@ -35,6 +35,10 @@ int run_sortmerge_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const 
                        tbg_row_out *d_rows, uint64_t cap, Workspace &w, cudaStream_t st, JoinRun *run) {
     // one shared-memory radix-sorted tile (512 threads x 8 rows) of R per item
     const int capR = RSM_CAPR;
+    if (nR <= SMALL_R) {
+        const RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
+        if (is_small_join(cfg, g)) return run_small_join(cfg, g, dR, dS, d_rows, cap, w, st, run);
+    }
     int join_grid = 0;
     int rc = radix_partition(cfg, dR, nR, dS, nS, d_rows, cap, capR, w, st, run, &join_grid);
     if (rc) return rc;

@@ -51,6 +51,14 @@ struct Ctrl {
     unsigned int pad;
 };
 
+// Sums of the CTAs of a small join (small.cu); zero between launches.
+struct SmallCtl {
+    unsigned long long matches, rows;
+    unsigned int hist[8];  // S rows per partition
+    unsigned int done;     // CTA ticket
+    unsigned int pad;
+};
+
 // Digits per pass of the tile scatter (part_dev.cuh).
 constexpr int SCATTER_FMAX = 256;
 

@@ -34,6 +34,7 @@ struct Workspace {
     DevBuf aux[8];              // algorithm-specific scratch (sort, learned model)
     DevBuf shard;               // shard split: per-chunk histograms and totals
     DevBuf direct;              // direct join: R's table
+    DevBuf small;               // small join: the CTAs' sums (SmallCtl)
     Ctrl *host_ctrl = nullptr;  // pinned mirror of the control block
     static constexpr size_t HOST_SMALL_BYTES = 4096;
     void *host_small = nullptr;  // pinned HOST_SMALL_BYTES: mid-call read-backs (LRN's decision, shard totals)
@@ -55,6 +56,8 @@ struct JoinRun {
     float ms_learn = 0;
     double heavy_pred = 0, heavy_sampled = 0;
     uint64_t launches = 0;
+    bool waits = false;         // the caller waits for the result
+    bool ctrl_on_host = false;  // the join's last kernel writes host_ctrl itself
 };
 
 Workspace *workspace_for(cudaStream_t st);
@@ -98,6 +101,7 @@ struct RadixGeom {
 RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int capR, Workspace &w);
 RadixGeom radix_geometry_msd(uint64_t nR, uint64_t nS, uint32_t sub, int B, int lowbits, Workspace &w);
 int ensure_radix_buffers(const RadixGeom &g, bool bypass, Workspace &w);
+bool automatic_plan(const tbg_config &cfg);
 void try_direct(RadixGeom &g, const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap);
 int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st);
 int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w, cudaStream_t st,
@@ -123,6 +127,11 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
                           int nslices, const std::function<int(int)> &issue, cudaEvent_t r_ready,
                           const cudaEvent_t *s_ready, tbg_row_out *d_rows, uint64_t cap, Workspace &w,
                           cudaStream_t st, JoinRun *run);
+// R rows of the largest small join (small.cu): one shared-memory table.
+constexpr uint64_t SMALL_R = 16384;
+bool is_small_join(const tbg_config &cfg, const RadixGeom &g);
+int run_small_join(const tbg_config &cfg, const RadixGeom &g, const Row *dR, const Row *dS, tbg_row_out *d_rows,
+                   uint64_t cap, Workspace &w, cudaStream_t st, JoinRun *run);
 int run_sortmerge_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
                        tbg_row_out *d_rows, uint64_t cap, Workspace &w, cudaStream_t st, JoinRun *run);
 int run_psm_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
