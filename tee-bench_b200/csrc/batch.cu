@@ -401,12 +401,18 @@ __device__ void scatter_chunk(const BatchArgs &a, uint32_t c, BPart &sm, uint64_
 // join: build/probe
 // ---------------------------------------------------------------------------
 template <bool CG>
-__device__ unsigned long long pair_count(Table &t, const Row *R, uint64_t rn, const Row *S, uint64_t sn,
+__device__ unsigned long long pair_count(Table &t, CellTable &ct, const Row *R, uint64_t rn, const Row *S, uint64_t sn,
                                          uint32_t capR, uint64_t *scratch) {
     unsigned long long c = 0;
     for (uint64_t r0 = 0; r0 < rn; r0 += capR) {
-        build_table<BATCH_THREADS, CG>(t, R, r0, (uint32_t)umin64(capR, rn - r0), scratch);
-        c += probe_count<BATCH_THREADS, CG>(t, S, sn);
+        const uint32_t n = (uint32_t)umin64(capR, rn - r0);
+        if (t.layout == 0) {
+            build_cells<BATCH_THREADS, CG>(ct, R, r0, n);
+            c += probe_count<BATCH_THREADS, CG>(ct, S, sn);
+        } else {
+            build_table<BATCH_THREADS, CG>(t, R, r0, n, scratch);
+            c += probe_count<BATCH_THREADS, CG>(t, S, sn);
+        }
         __syncthreads();  // table rebuilt by the next R slice
     }
     return c;
@@ -417,24 +423,25 @@ __device__ void join_ticket(const BatchArgs &a, uint32_t q, unsigned char *smem,
     const uint2 jt = a.jt[q];
     const BatchJoin &J = a.joins[jt.x];
     const uint32_t capR = a.capR;
-    Table t;
+    Table t;  // layout 1 (histogram table)
     t.key = reinterpret_cast<uint32_t *>(smem);
     t.pay = t.key + capR;
     t.heads = t.pay + capR;
-    t.next = reinterpret_cast<uint16_t *>(t.heads + capR + 2);
-    t.head64 = nullptr;
-    if (J.layout == 0) {  // counts only: keys, packed heads (capR * 4 is a multiple of 8), links
-        t.head64 = reinterpret_cast<uint64_t *>(t.key + capR);
-        t.next = reinterpret_cast<uint16_t *>(t.head64 + floor_pow2(capR + 2));
-    }
+    t.next = nullptr;
     t.hs = (int)J.B;
     t.layout = (int)J.layout;
     t.hcap = floor_pow2(capR + 2);
+    CellTable ct;  // layout 0 (bucket chains)
+    ct.link_bits = cell_link_bits(capR);
+    ct.hcap = 1u << ct.link_bits;  // an unpartitioned join (B = 0) needs them all
+    ct.heads = reinterpret_cast<uint32_t *>(smem);
+    ct.cells = ct.heads + ct.hcap;
+    ct.hs = (int)J.B;
     unsigned long long local = 0;
     if (J.B == 0) {
         const uint64_t lo = (uint64_t)jt.y * J.capS;
         const uint64_t hi = umin64(J.nS, lo + J.capS);
-        if (lo < hi) local = pair_count<false>(t, J.R, J.nR, J.S + lo, hi - lo, capR, scratch);
+        if (lo < hi) local = pair_count<false>(t, ct, J.R, J.nR, J.S + lo, hi - lo, capR, scratch);
     } else {
         BatchSync &sy = a.sync[jt.x];
         cta_wait(&sy.scat_done, J.GR + J.GS, a.err);
@@ -452,7 +459,7 @@ __device__ void join_ticket(const BatchArgs &a, uint32_t q, unsigned char *smem,
             const uint64_t s_len = (uint64_t)m1.x | ((uint64_t)m1.y << 32);
             const uint32_t r_len = m1.z;
             if (r_off + r_len <= J.nR && s_off + s_len <= J.nS)
-                local += pair_count<true>(t, J.Rp + r_off, r_len, J.Sp + s_off, s_len, capR, scratch);
+                local += pair_count<true>(t, ct, J.Rp + r_off, r_len, J.Sp + s_off, s_len, capR, scratch);
         }
     }
     const unsigned long long ws = warp_sum_u64(local);

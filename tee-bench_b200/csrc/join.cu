@@ -20,6 +20,10 @@
 
 namespace tbg {
 
+// Heads of a counting table: about one per row (partitions average half the
+// table or less, see join_capacity).
+__host__ __device__ __forceinline__ uint32_t count_heads(int capR) { return floor_pow2((uint32_t)capR); }
+
 template <bool MAT>
 __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -31,23 +35,22 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
         if (a.gate_le ? v > a.gate_max : v <= a.gate_max) return;
     }
     Table t;
-    t.key = reinterpret_cast<uint32_t *>(smem);
-    t.pay = t.key + a.capR;
-    t.heads = t.pay + a.capR;
-    t.next = reinterpret_cast<uint16_t *>(t.heads + a.capR + 2);
-    t.head64 = nullptr;
-    t.hcap = floor_pow2((uint32_t)a.capR + 2);
-    if (!MAT && a.layout == 0) {  // count only: keys, packed heads (capR * 4 is a multiple of 8), links
-        t.hcap = count_head_slots(a.capR);
-        t.head64 = reinterpret_cast<uint64_t *>(t.key + a.capR);
-        t.next = reinterpret_cast<uint16_t *>(t.head64 + t.hcap);
+    CellTable ct;
+    if (MAT) {
+        t.key = reinterpret_cast<uint32_t *>(smem);
+        t.pay = t.key + a.capR;
+        t.heads = t.pay + a.capR;
+        t.next = reinterpret_cast<uint16_t *>(t.heads + a.capR + 2);
+        t.hcap = floor_pow2((uint32_t)a.capR + 2);
+        t.hs = a.hash_shift;
+        t.layout = a.layout;
+    } else {
+        ct.hcap = count_heads(a.capR);
+        ct.heads = reinterpret_cast<uint32_t *>(smem);
+        ct.cells = ct.heads + ct.hcap;
+        ct.hs = a.hash_shift;
+        ct.link_bits = cell_link_bits((uint32_t)a.capR);
     }
-    if (!MAT && a.layout == 1) {  // count only: keys, then bucket starts and cursors (no payloads)
-        t.pay = nullptr;
-        t.heads = t.key + a.capR;
-    }
-    t.hs = a.hash_shift;
-    t.layout = a.layout;
     const int tid = threadIdx.x;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
     unsigned long long local = 0;
@@ -68,7 +71,8 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
             }
         }
         const Item m = a.items[it];
-        build_table<JOIN_THREADS>(t, a.R, m.r_off, m.r_len, scan_scratch);
+        if (MAT) build_table<JOIN_THREADS>(t, a.R, m.r_off, m.r_len, scan_scratch);
+        else build_cells<JOIN_THREADS>(ct, a.R, m.r_off, m.r_len);
 
         const Row *s = a.S + m.s_off;
         const uint64_t len = m.s_len;
@@ -79,7 +83,7 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
         const uint4 *v = reinterpret_cast<const uint4 *>(s + head);
 
         if (!MAT) {
-            local += probe_count<JOIN_THREADS>(t, s, len);
+            local += probe_count<JOIN_THREADS>(ct, s, len);
         } else {
             // block-synchronous rounds: 8 rows per thread, one reservation per round
             const uint64_t per_round = 4ull * JOIN_THREADS;
@@ -140,33 +144,24 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
 size_t join_smem_bytes(int capR) {
     return (size_t)capR * 4 * 2 + ((size_t)capR + 2) * 4 + (size_t)capR * 2 + 16;
 }
-// Shared memory of a k_join launch: counting bucket-chain tables hold keys,
-// packed heads and links only.
-// Counting histogram tables (RHT) hold keys, the bucket starts and cursors.
-size_t join_launch_smem(int capR, bool materialize, int layout) {
-    if (!materialize && layout == 0)
-        return (size_t)capR * 4 + (size_t)count_head_slots(capR) * 8 + (size_t)capR * 2 + 16;
-    if (!materialize && layout == 1) {
-        uint32_t p = 1;
-        while (p < (uint32_t)capR) p <<= 1;
-        const size_t nb = std::max<uint32_t>(p >> 2, 4);  // buckets of the largest partition
-        return (size_t)capR * 4 + (2 * nb + 1) * 4 + 16;
-    }
+// Shared memory of a k_join launch (counting: heads and cells).
+size_t join_launch_smem(int capR, bool materialize) {
+    if (!materialize) return ((size_t)count_heads(capR) + capR) * 4;
     return join_smem_bytes(capR);
 }
 
 // Resident CTAs per SM of a k_join launch at a table of capR rows, cached per
-// (device, capR, materialize, layout): the occupancy query runs once per size.
-int join_ctas_per_sm(int capR, bool materialize, int layout) {
+// (device, capR, materialize): the occupancy query runs once per size.
+int join_ctas_per_sm(int capR, bool materialize) {
     static std::mutex mu;
     static std::map<std::pair<int, int>, int> cache;
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> g(mu);
-    const int key = capR * 4 + (materialize ? 2 : 0) + (layout ? 1 : 0);
+    const int key = capR * 2 + (materialize ? 1 : 0);
     auto it = cache.find(std::make_pair(dev, key));
     if (it != cache.end()) return it->second;
-    const size_t smem = join_launch_smem(capR, materialize, layout);
+    const size_t smem = join_launch_smem(capR, materialize);
     int n = 0;
     if (smem_limit((const void *)k_join<false>, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_join<false>, JOIN_THREADS, smem) != cudaSuccess) {
@@ -179,7 +174,7 @@ int join_ctas_per_sm(int capR, bool materialize, int layout) {
 }
 
 cudaError_t launch_join(const JoinArgs &a, bool materialize, int grid, cudaStream_t st) {
-    const size_t smem = join_launch_smem(a.capR, materialize, a.layout);
+    const size_t smem = join_launch_smem(a.capR, materialize);
     auto kern = materialize ? k_join<true> : k_join<false>;
     cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;

@@ -14,25 +14,6 @@ __host__ __device__ __forceinline__ uint32_t floor_pow2(uint32_t x) {
     return p;
 }
 
-// Bucket heads of a count-only bucket-chain table of capR rows: the largest
-// power of two <= capR + 2, divided by TBG_COUNT_HEAD_DIV (a build option for
-// A/B timing: fewer heads, longer chains, a smaller table and so more CTAs
-// per SM).
-#ifndef TBG_COUNT_HEAD_DIV
-#define TBG_COUNT_HEAD_DIV 1
-#endif
-__host__ __device__ __forceinline__ uint32_t count_head_slots(int capR) {
-    const uint32_t h = floor_pow2((uint32_t)capR + 2) / TBG_COUNT_HEAD_DIV;
-    return h ? h : 1;
-}
-
-// Packed bucket head of a count-only bucket-chain table: the head entry's
-// key, its 1-based row and its 1-based next link in one 64-bit word, so a
-// probe whose chain has one entry costs one shared load.
-__device__ __forceinline__ uint64_t pack_head(uint32_t key, uint32_t row1, uint32_t next1) {
-    return ((uint64_t)key << 32) | (row1 << 16) | next1;
-}
-
 // Histogram-table probes read the bucket's keys four at a time (a build
 // option for A/B timing).
 #ifndef TBG_RHT_VEC_PROBE
@@ -41,10 +22,9 @@ __device__ __forceinline__ uint64_t pack_head(uint32_t key, uint32_t row1, uint3
 
 struct Table {
     uint32_t *key;    // [capR]
-    uint32_t *pay;    // [capR] (unused with head64)
+    uint32_t *pay;    // [capR]
     uint32_t *heads;  // layout 0: [N] 1-based chain heads; layout 1: [Nb+1] starts, then cursors
     uint16_t *next;   // layout 0: [capR] 1-based next links
-    uint64_t *head64; // layout 0, count only (else null): [N] packed heads instead of heads
     uint32_t mask;    // bucket mask
     uint32_t hcap;    // head slots available (a power of two <= capR + 2)
     int hs;           // hash shift (radix bits already consumed)
@@ -66,11 +46,7 @@ struct Table {
     __device__ __forceinline__ uint32_t count(uint32_t k) const {
         uint32_t c = 0;
         const uint32_t b = bucket(k);
-        if (head64) {
-            const uint64_t x = head64[b];
-            c = ((x >> 16) & 0xFFFF) != 0 && (uint32_t)(x >> 32) == k;
-            for (uint32_t h = (uint32_t)x & 0xFFFF; h; h = next[h - 1]) c += (key[h - 1] == k);
-        } else if (layout == 0) {
+        if (layout == 0) {
             for (uint32_t h = heads[b]; h; h = next[h - 1]) c += (key[h - 1] == k);
         } else if (TBG_RHT_VEC_PROBE) {
             // the bucket's keys read as 16-byte words (key[] starts 16-byte
@@ -91,6 +67,49 @@ struct Table {
 };
 
 
+// Count-only bucket chains of 32-bit cells.  With q = key >> hs, row i's
+// bucket is q mod N and its tag the bits of q above that, which with the
+// bucket and the low hs bits (shared by all rows of the join's partition)
+// make up the whole key: a cell needs no key beside it.  A cell holds {tag,
+// link}, link the 1-based place in `cells` of the next cell of the chain (0:
+// the end); a new row's cell becomes the bucket's head and the head it
+// displaces moves to cells[i].  The tag has 32 - link_bits bits, so N is at
+// least 2^(link_bits - hs).  Against 64-bit heads {key, row, link} with keys
+// and links in arrays of their own (112 KB at 8192 rows, two CTAs per SM) a
+// lookup reads one 4-byte word instead of 8 bytes, and 10240 rows take 72 KB,
+// three CTAs per SM.
+constexpr uint32_t CELL_EMPTY = 0xFFFFFFFFu;  // its link is past any row
+
+struct CellTable {
+    uint32_t *heads;  // [N <= hcap]
+    uint32_t *cells;  // [rows]
+    uint32_t hcap;    // a power of two
+    int hs, link_bits;
+    uint32_t mask;    // N - 1
+    int tag_shift;    // hs + log2 N
+
+    __device__ __forceinline__ uint32_t count(uint32_t k) const {
+        uint32_t c = heads[(k >> hs) & mask];
+        if (c == CELL_EMPTY) return 0;
+        const uint32_t tag = tag_shift < 32 ? k >> tag_shift : 0u;
+        const uint32_t lmask = (1u << link_bits) - 1;
+        uint32_t n = 0;
+        for (;;) {
+            n += (c >> link_bits) == tag;
+            const uint32_t l = c & lmask;
+            if (!l) return n;
+            c = cells[l - 1];
+        }
+    }
+};
+
+// Link bits of a table of `rows` rows: links 0 .. rows, and one value more.
+__host__ __device__ __forceinline__ int cell_link_bits(uint32_t rows) {
+    int b = 1;
+    while ((1u << b) < rows + 2) b++;
+    return b;
+}
+
 // R rows are read with plain loads, or with L2-only loads (CG) when they were
 // written earlier in the same kernel launch by other CTAs.
 template <bool CG>
@@ -105,33 +124,37 @@ __device__ __forceinline__ uint4 ld_pair(const uint4 *p) {
     return ldg_stream(p);
 }
 
+// Builds the cells of R rows [r_off, r_off + r_len); ends with a barrier.
+template <int THREADS, bool CG = false>
+__device__ __forceinline__ void build_cells(CellTable &t, const Row *__restrict__ R, uint64_t r_off, uint32_t r_len) {
+    const int tid = threadIdx.x;
+    const uint32_t least = t.link_bits > t.hs ? 1u << (t.link_bits - t.hs) : 1u;
+    const uint32_t N = min(max(next_pow2(r_len), max(least, 4u)), t.hcap);
+    t.mask = N - 1;
+    t.tag_shift = t.hs + 31 - __clz(N);
+    for (uint32_t i = tid; i < N / 4; i += THREADS)
+        reinterpret_cast<uint4 *>(t.heads)[i] = make_uint4(CELL_EMPTY, CELL_EMPTY, CELL_EMPTY, CELL_EMPTY);
+    __syncthreads();
+    for (uint32_t i = tid; i < r_len; i += THREADS) {
+        const uint32_t k = ld_row<CG>(R, r_off + i).x;
+        uint32_t *head = &t.heads[(k >> t.hs) & t.mask];
+        const uint32_t tag = t.tag_shift < 32 ? (k >> t.tag_shift) << t.link_bits : 0u;
+        uint32_t old = *head;
+        for (;;) {  // ends: each failed swap means another row entered this chain
+            const uint32_t seen = atomicCAS(head, old, old == CELL_EMPTY ? tag : tag | (i + 1));
+            if (seen == old) break;
+            old = seen;
+        }
+        if (old != CELL_EMPTY) t.cells[i] = old;
+    }
+    __syncthreads();
+}
+
 template <int THREADS, bool CG = false>
 __device__ void build_table(Table &t, const Row *__restrict__ R, uint64_t r_off, uint32_t r_len,
                             uint64_t *scan_scratch) {
     const int tid = threadIdx.x;
-    if (t.head64) {
-        // the same buckets and chains with packed heads: a row enters at
-        // the head of its chain by compare-and-swap, its next link being the
-        // head it displaced
-        const uint32_t N = min(next_pow2(r_len), t.hcap);
-        t.mask = N - 1;
-        for (uint32_t i = tid; i < r_len; i += THREADS) t.key[i] = ld_row<CG>(R, r_off + i).x;
-        for (uint32_t i = tid; i < N; i += THREADS) t.head64[i] = 0;
-        __syncthreads();
-        for (uint32_t i = tid; i < r_len; i += THREADS) {
-            const uint32_t k = t.key[i];
-            unsigned long long *slot = reinterpret_cast<unsigned long long *>(&t.head64[t.bucket(k)]);
-            unsigned long long old = *slot;
-            for (;;) {  // ends: each failed swap means another row entered this chain
-                const unsigned long long seen =
-                    atomicCAS(slot, old, (unsigned long long)pack_head(k, i + 1, (uint32_t)(old >> 16) & 0xFFFF));
-                if (seen == old) break;
-                old = seen;
-            }
-            t.next[i] = (uint16_t)((old >> 16) & 0xFFFF);
-        }
-        __syncthreads();
-    } else if (t.layout == 0) {
+    if (t.layout == 0) {
         // next_pow2(|R_p|) buckets as in the reference, at most hcap (a
         // longer average chain when capR is not a power of two)
         const uint32_t N = min(next_pow2(r_len), t.hcap);
@@ -235,8 +258,8 @@ __device__ __forceinline__ unsigned long long stream_sum(const Row *s, uint64_t 
 }
 
 // Matches of S rows [0, len) against the table, this thread's share.
-template <int THREADS, bool CG = false>
-__device__ __forceinline__ unsigned long long probe_count(const Table &t, const Row *s, uint64_t len) {
+template <int THREADS, bool CG = false, class T = Table>
+__device__ __forceinline__ unsigned long long probe_count(const T &t, const Row *s, uint64_t len) {
     return stream_sum<THREADS, CG>(s, len, [&](uint32_t k) { return t.count(k); });
 }
 

@@ -38,6 +38,12 @@ struct SmallArgs {
     uint64_t cap;
 };
 
+// Heads of the count-only table: two to four per row (the tag needs 2^15 of
+// them at 16384 rows, 2^14 below).
+__host__ __device__ __forceinline__ uint32_t small_heads(uint32_t table_rows) {
+    return 1u << cell_link_bits(table_rows);
+}
+
 // Adds the block's counts of digits [0, P) of this thread's key to cnt[8]
 // (shared); every lane of the warp calls it.
 __device__ __forceinline__ void count_digits(uint32_t *cnt, uint32_t key, bool valid, int P) {
@@ -68,19 +74,21 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
 
     // R's table
     Table t;
-    t.key = reinterpret_cast<uint32_t *>(smem);
-    t.hs = a.B;
-    t.layout = 0;
+    CellTable ct;
     if (MAT) {
+        t.key = reinterpret_cast<uint32_t *>(smem);
+        t.hs = a.B;
+        t.layout = 0;
         t.pay = t.key + a.table_rows;
         t.heads = t.pay + a.table_rows;
         t.next = reinterpret_cast<uint16_t *>(t.heads + a.table_rows + 2);
-        t.head64 = nullptr;
         t.hcap = floor_pow2(a.table_rows + 2);
     } else {
-        t.hcap = count_head_slots((int)a.table_rows);
-        t.head64 = reinterpret_cast<uint64_t *>(t.key + a.table_rows);
-        t.next = reinterpret_cast<uint16_t *>(t.head64 + t.hcap);
+        ct.hcap = small_heads(a.table_rows);
+        ct.heads = reinterpret_cast<uint32_t *>(smem);
+        ct.cells = ct.heads + ct.hcap;
+        ct.hs = 0;  // nothing is partitioned: keys differ in every bit
+        ct.link_bits = cell_link_bits(a.table_rows);
     }
     uint32_t *bits = reinterpret_cast<uint32_t *>(smem);
     uint32_t kmin = 0, span = 0;
@@ -114,7 +122,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
             by_bits = dup == 0;
         }
     }
-    if (!by_bits) build_table<T>(t, a.R, 0, a.nR, scratch);
+    if (MAT) build_table<T>(t, a.R, 0, a.nR, scratch);
+    else if (!by_bits) build_cells<T>(ct, a.R, 0, a.nR);
 
     // this CTA's slice of S
     const uint64_t s0 = (uint64_t)blockIdx.x * a.slice;
@@ -132,7 +141,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
         } else {
             local = stream_sum<T>(s, len, [&](uint32_t k) {
                 odd += k & 1;
-                return t.count(k);
+                return ct.count(k);
             });
         }
         odd = __reduce_add_sync(0xffffffffu, odd);
@@ -260,7 +269,7 @@ int run_small_join(const tbg_config &cfg, const RadixGeom &g, const Row *dR, con
     a.out = d_rows;
     a.cap = d_rows && mat ? cap : 0;
     const size_t smem = mat ? join_smem_bytes((int)a.table_rows)
-                            : std::max(join_launch_smem((int)a.table_rows, false, 0),
+                            : std::max(((size_t)small_heads(a.table_rows) + a.table_rows) * 4,
                                        std::min<size_t>(SMALL_SMEM_MAX, (size_t)nR * 4));  // 32 key values per row
     a.bit_words = mat ? 0 : (uint32_t)(smem / 4);
     auto kern = mat ? k_small<true> : k_small<false>;

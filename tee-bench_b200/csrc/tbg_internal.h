@@ -69,7 +69,9 @@ constexpr int PART_ITEMS = 8;
 // Shared-memory table capacity of the build/probe kernels (rows of R_p).
 constexpr int JOIN_THREADS = 512;
 constexpr int JOIN_CAPR_DEFAULT = 5120;
-constexpr int JOIN_CAPR_FIT = 8192;    // counting joins: the average R partition fills this table
+// counting joins: R's partitions aim at 8192 rows and fit this table (72 KB,
+// three CTAs per SM) while none is a quarter larger
+constexpr int JOIN_CAPR_FIT = 10240;
 constexpr int JOIN_CAPR_WIDE = 16384;  // ... and partitions up to this size are joined whole
 constexpr int JOIN_CAPR_SMALL = 4096;  // count-only tables when every R partition fits it
 
@@ -182,8 +184,8 @@ cudaError_t launch_part_pass1(const PartArgs &a, const PartArgs *b, cudaStream_t
 cudaError_t launch_part_pass2(const PartArgs &a, const PartArgs *b, cudaStream_t st);
 cudaError_t launch_join(const JoinArgs &a, bool materialize, int grid, cudaStream_t st);
 size_t join_smem_bytes(int capR);
-size_t join_launch_smem(int capR, bool materialize, int layout);
-int join_ctas_per_sm(int capR, bool materialize, int layout);
+size_t join_launch_smem(int capR, bool materialize);
+int join_ctas_per_sm(int capR, bool materialize);
 
 // ---- direct join (direct.cu) ----
 int direct_log2_max(uint64_t nR);
