@@ -165,6 +165,8 @@ template <bool PAYLOADS>
 __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__restrict__ in, uint64_t n, uint64_t chunk,
                                                                   uint32_t *__restrict__ hist, int nbins, RadixF rf,
                                                                   uint32_t *__restrict__ table, Ctrl *ctrl) {
+    dep_wait();
+    dep_trigger();
     extern __shared__ uint32_t sh[];
     __shared__ uint32_t s_inv, s_hi;
     const int tid = threadIdx.x;
@@ -256,6 +258,8 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
 // needs no count: its entries showed every duplicate.
 __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t *__restrict__ bits, uint64_t nR,
                                                                   Ctrl *ctrl) {
+    dep_wait();
+    dep_trigger();
     __shared__ unsigned s_count;
     const unsigned w = ctrl->direct_log2;
     if (!w || ctrl->direct_dup) return;
@@ -303,6 +307,8 @@ template <bool SMEM>
 __global__ void __launch_bounds__(DIRECT_THREADS, 2)
     k_hist_probe(const Row *__restrict__ in, uint64_t n, uint64_t chunk, uint32_t *__restrict__ hist, int nbins, RadixF rf,
                  const uint32_t *__restrict__ bits, uint32_t smem_words, Ctrl *ctrl) {
+    dep_wait();
+    dep_trigger();
     const bool direct = ctrl->direct != 0;
     const uint32_t kmin = ~ctrl->direct_inv_min, span = ctrl->direct_max - kmin;
     const uint32_t wordmask = direct ? (uint32_t)((1ull << (ctrl->direct_log2 - 5)) - 1) : 0u;
@@ -376,6 +382,8 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
     k_hist_emit(const Row *__restrict__ in, uint64_t n, uint64_t chunk, uint32_t *__restrict__ hist, int nbins, RadixF rf,
                 const uint32_t *__restrict__ table, tbg_row_out *__restrict__ out, uint64_t cap, uint32_t range_max,
                 Ctrl *ctrl) {
+    dep_wait();
+    dep_trigger();
     constexpr int T = EMIT_DIRECT_THREADS, NW = T / 32;
     extern __shared__ __align__(16) unsigned char esmem[];
     EmitSmem &sm = *reinterpret_cast<EmitSmem *>(esmem);
@@ -525,9 +533,10 @@ cudaError_t launch_hist_emit(const Row *in, uint64_t n, uint64_t chunk, int G, u
     const size_t smem = sizeof(EmitSmem) + (size_t)nbins * 4;
     cudaError_t e = smem_limit((const void *)k_hist_emit, smem);
     if (e != cudaSuccess) return e;
-    k_hist_emit<<<G, EMIT_DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, table, out, cap, range_max, ctrl);
+    e = launch_dep(k_hist_emit, G, EMIT_DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, table, out, cap, range_max,
+                   ctrl);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *table, int log2_max, bool payloads, Ctrl *ctrl,
@@ -546,18 +555,18 @@ cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, 
     auto kern = payloads ? k_hist_build<true> : k_hist_build<false>;
     cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    kern<<<G, DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, table, ctrl);
+    e = launch_dep(kern, G, DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, table, ctrl);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, Ctrl *ctrl, cudaStream_t st) {
     const uint64_t n4 = 1ull << (log2_max - 7);
     // two 16-byte words per thread and CTA at least, one CTA per SM at most
     const unsigned g = bits ? (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), 148)) : 1u;
-    k_direct_decide<<<g, DIRECT_THREADS, 0, st>>>(bits, nR, ctrl);
+    const cudaError_t e = launch_dep(k_direct_decide, g, DIRECT_THREADS, 0, st, bits, nR, ctrl);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
@@ -568,13 +577,14 @@ cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, 
     cudaError_t e;
     if (words) {
         if ((e = smem_limit((const void *)k_hist_probe<true>, smem_copy)) != cudaSuccess) return e;
-        k_hist_probe<true><<<G, DIRECT_THREADS, smem_copy, st>>>(in, n, chunk, hist, nbins, rf, bits, words, ctrl);
+        e = launch_dep(k_hist_probe<true>, G, DIRECT_THREADS, smem_copy, st, in, n, chunk, hist, nbins, rf, bits, words, ctrl);
         count_launch();
+        if (e != cudaSuccess) return e;
     }
     if ((e = smem_limit((const void *)k_hist_probe<false>, smem)) != cudaSuccess) return e;
-    k_hist_probe<false><<<G, DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, bits, words, ctrl);
+    e = launch_dep(k_hist_probe<false>, G, DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, bits, words, ctrl);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace tbg

@@ -29,6 +29,8 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_item[2];
     __shared__ uint64_t scan_scratch[JOIN_THREADS / 32 + 1];
+    dep_wait();
+    dep_trigger();
     if (a.skip && *a.skip) return;
     if (a.gate) {  // the same value for every thread: the whole launch steps aside
         const unsigned long long v = *a.gate;
@@ -178,9 +180,9 @@ cudaError_t launch_join(const JoinArgs &a, bool materialize, int grid, cudaStrea
     auto kern = materialize ? k_join<true> : k_join<false>;
     cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, JOIN_THREADS, smem, st>>>(a);
+    e = launch_dep(kern, grid, JOIN_THREADS, smem, st, a);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace tbg

@@ -323,6 +323,8 @@ __device__ bool last_of(unsigned *ctr, unsigned n, int tid, bool *flag) {
 // t.plan, each relation's last CTA scans its bases; with t.items, the CTA that
 // finishes the last relation of the launch plans the work items.
 __global__ void __launch_bounds__(PLAN_THREADS) k_colscan(ColScan r, ColScan s, PlanTail t) {
+    dep_wait();
+    dep_trigger();
     __shared__ uint32_t seg[32][33];
     __shared__ uint64_t scratch[PLAN_THREADS / 32 + 1];
     __shared__ bool flag;
@@ -444,6 +446,8 @@ __device__ __forceinline__ void part_pass2(const PartArgs &a, const unsigned uni
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     k_part_pass1(const __grid_constant__ PartArgs a, const __grid_constant__ PartArgs b) {
+    dep_wait();
+    dep_trigger();
     if (blockIdx.x < (unsigned)a.G) part_pass1<THREADS>(a, blockIdx.x);
     else part_pass1<THREADS>(b, blockIdx.x - a.G);
 }
@@ -451,6 +455,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     k_part_pass2(const __grid_constant__ PartArgs a, const __grid_constant__ PartArgs b) {
+    dep_wait();
+    dep_trigger();
     const unsigned units = (unsigned)((a.G + a.group - 1) / a.group) << a.b1;
     if (blockIdx.x < units) part_pass2<THREADS>(a, blockIdx.x);
     else part_pass2<THREADS>(b, blockIdx.x - units);
@@ -485,9 +491,9 @@ cudaError_t launch_colscan(uint32_t *hist, int G, int P, uint32_t *totals, cudaS
 }
 
 cudaError_t launch_colscan_plan(const ColScan &r, const ColScan &s, const PlanTail &t, cudaStream_t st) {
-    k_colscan<<<(r.P + 31) / 32 + (s.P + 31) / 32, dim3(32, 32), 0, st>>>(r, s, t);
+    const cudaError_t e = launch_dep(k_colscan, (r.P + 31) / 32 + (s.P + 31) / 32, dim3(32, 32), 0, st, r, s, t);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st) {
@@ -504,9 +510,9 @@ cudaError_t launch_part_pass1(const PartArgs &a, const PartArgs *b, cudaStream_t
     const size_t smem = sizeof(PassSmem<T>);
     cudaError_t e = smem_limit((const void *)k_part_pass1<T>, smem);
     if (e != cudaSuccess) return e;
-    k_part_pass1<T><<<a.G + (b ? b->G : 0), T, smem, st>>>(a, b ? *b : a);
+    e = launch_dep(k_part_pass1<T>, a.G + (b ? b->G : 0), T, smem, st, a, b ? *b : a);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_part_pass2(const PartArgs &a, const PartArgs *b, cudaStream_t st) {
@@ -515,9 +521,9 @@ cudaError_t launch_part_pass2(const PartArgs &a, const PartArgs *b, cudaStream_t
     cudaError_t e = smem_limit((const void *)k_part_pass2<T>, smem);
     if (e != cudaSuccess) return e;
     auto units = [](const PartArgs &p) { return (uint64_t)((p.G + p.group - 1) / p.group) << p.b1; };
-    k_part_pass2<T><<<(unsigned)(units(a) + (b ? units(*b) : 0)), T, smem, st>>>(a, b ? *b : a);
+    e = launch_dep(k_part_pass2<T>, (unsigned)(units(a) + (b ? units(*b) : 0)), T, smem, st, a, b ? *b : a);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace tbg

@@ -292,6 +292,8 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm(JoinArgs a) {
     __shared__ unsigned long long s_base;
     __shared__ uint64_t scan_scratch[RSM_THREADS / 32 + 1];
     __shared__ uint32_t red[2];
+    dep_wait();
+    dep_trigger();
     if (*a.skip) return;
     const int tid = threadIdx.x;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
@@ -595,6 +597,8 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm_count(JoinArgs a) {
     __shared__ uint32_t s_item;
     __shared__ uint64_t scan_scratch[RSM_THREADS / 32 + 1];
     __shared__ uint32_t red[2];
+    dep_wait();
+    dep_trigger();
     if (*a.skip) return;
     const int tid = threadIdx.x;
     const int shift = a.hash_shift;
@@ -692,16 +696,16 @@ cudaError_t launch_join_rsm(const JoinArgs &a, bool materialize, int grid, cudaS
         if ((e = smem_limit((const void *)k_join_rsm_count, smem)) !=
             cudaSuccess)
             return e;
-        k_join_rsm_count<<<grid, RSM_THREADS, smem, st>>>(a);
+        e = launch_dep(k_join_rsm_count, grid, RSM_THREADS, smem, st, a);
     } else {
         const size_t smem = rsm_smem_bytes(a.capR);
         if ((e = smem_limit((const void *)k_join_rsm<true>, smem)) !=
             cudaSuccess)
             return e;
-        k_join_rsm<true><<<grid, RSM_THREADS, smem, st>>>(a);
+        e = launch_dep(k_join_rsm<true>, grid, RSM_THREADS, smem, st, a);
     }
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 // ---------------------------------------------------------------------------
@@ -722,6 +726,8 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
     extern __shared__ __align__(16) uint32_t bc_smem[];
     uint32_t *h = bc_smem;
     __shared__ uint32_t s_item[2];
+    dep_wait();
+    dep_trigger();
     if (*a.skip) return;
     const int tid = threadIdx.x;
     const uint32_t bins = 1u << lowbits;
@@ -767,9 +773,9 @@ cudaError_t launch_bucket_count(const JoinArgs &a, uint32_t sub, int lowbits, in
     const size_t smem = (size_t)4 << lowbits;
     cudaError_t e = smem_limit((const void *)k_bucket_count, smem);
     if (e != cudaSuccess) return e;
-    k_bucket_count<<<nsm * BCOUNT_CTAS, BCOUNT_THREADS, smem, st>>>(a, sub, lowbits);
+    e = launch_dep(k_bucket_count, nsm * BCOUNT_CTAS, BCOUNT_THREADS, smem, st, a, sub, lowbits);
     count_launch();
-    return cudaGetLastError();
+    return e;
 }
 
 // ---------------------------------------------------------------------------

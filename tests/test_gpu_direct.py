@@ -177,3 +177,45 @@ def test_direct_rows_sliced(tbg, oracle, cuda):
     finally:
         tbg.set_dropin_slices(prev)
     assert c == ref and np.array_equal(oracle.sort_rows(rows), oracle.sort_rows(ref_rows))
+
+
+@pytest.mark.parametrize("materialize", [0, 1])
+@pytest.mark.parametrize("nR", [5000, 90001])
+def test_async_join_in_a_captured_graph(tbg, oracle, cuda, nR, materialize):
+    """The asynchronous call captured into a CUDA graph (after a first call that
+    sizes the scratch) and replayed on changing contents: distinct keys, then
+    duplicates."""
+    torch = cuda
+    rng = np.random.default_rng(nR)
+    R, S = relations(oracle, rng, nR, 120007, 1, 1, 0.3)
+    D = R.copy()
+    D["key"][0] = D["key"][1]
+    tR, pR = to_dev(torch, R)
+    tS, pS = to_dev(torch, S)
+    tD, _ = to_dev(torch, D)
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    cap = 2 * len(S)
+    rows = torch.zeros(3 * cap, dtype=torch.int32, device="cuda")
+    st = torch.cuda.Stream()
+
+    def call():
+        tbg.join_device_async(tbg.config("RHO", materialize=materialize), pR, len(R), pS, len(S), out.data_ptr(),
+                              rows.data_ptr() if materialize else 0, cap if materialize else 0, stream=st.cuda_stream)
+
+    call()
+    st.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        call()
+    for rel, dev in ((R, tR.clone()), (D, tD), (R, tR.clone())):
+        tR.copy_(dev)
+        torch.cuda.synchronize()
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        ref, ref_rows = oracle.rho(rel, S, materialize=True)
+        assert out.item() == ref
+        if materialize:
+            got = rows[: 3 * ref].cpu().numpy().view(np.uint32).reshape(-1, 3)
+            assert np.array_equal(oracle.sort_rows(got), oracle.sort_rows(ref_rows))
+    assert tbg.lib().tbg_sync_status(st.cuda_stream) == 0
