@@ -152,12 +152,12 @@ __device__ __forceinline__ void hist_pairs(uint32_t *sh, const RadixF &rf, const
     }
 }
 
-// R: chunk histograms, key range, bits.  The first sixteenth of a chunk's
-// rounds enters its bits with a returning atomic and gives up (for the whole
-// grid, through ctrl->direct_dup) at the first key already there: a relation
-// with many duplicates costs little before it takes the passes.  The other
-// rounds use atomics without a result, and a duplicate there shows in the
-// count of set bits.  Bound by the L2's atomics: 2^27 rows take 0.80 ms
+// R: chunk histograms, key range, bits.  A sixteenth of the rows is entered
+// first with a returning atomic, which gives up (for the whole grid, through
+// ctrl->direct_dup) at the first key already there: a relation with many
+// duplicates costs little before it takes the passes.  The other rows use
+// atomics without a result, and a duplicate there shows in the count of set
+// bits.  Bound by the L2's atomics: 2^27 rows take 0.80 ms
 // without results against 1.17 ms with; the histogram read alone 0.16 ms.
 // PAYLOADS: every row exchanges its payload with the key's entry (2^22 rows:
 // 37 us), so a duplicate shows at once.
@@ -180,7 +180,9 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
     volatile unsigned *gave_up = &ctrl->direct_dup;
     bool enter = w != 0;  // the same for all lanes of a warp
     uint32_t kinv = 0, kmax = 0;  // largest ~key (the smallest key) and largest key
-    const uint32_t careful = PAYLOADS ? 0xFFFFFFFFu : (uint32_t)(chunk / (16 * 8 * DIRECT_THREADS)) + 1;
+    // a sixteenth of the rounds of long chunks, of the chunks when they are short
+    const uint32_t rounds16 = (uint32_t)(chunk / (16 * 8 * DIRECT_THREADS));
+    const uint32_t careful = PAYLOADS ? 0xFFFFFFFFu : rounds16 ? rounds16 : (blockIdx.x & 15) == 0 ? 1u : 0u;
     uint32_t round = 0;
     // enters a row; with ret, true says that the join is not direct
     auto set_bit = [&](uint32_t key, uint32_t payload, bool ret) {

@@ -125,8 +125,10 @@ __global__ void __launch_bounds__(HIST_THREADS) k_hist_chunks(const Row *__restr
 // ---------------------------------------------------------------------------
 constexpr int PLAN_THREADS = 1024;
 
+// With totals_only (a direct join, which uses no prefix) the chunks' rows stay
+// as they are.
 __device__ void column_scan(uint32_t *__restrict__ hist, int G, int P, uint32_t *__restrict__ totals, int block,
-                            uint32_t (*seg)[33]) {
+                            uint32_t (*seg)[33], bool totals_only) {
     const int f = block * 32 + threadIdx.x;
     const int per = (G + 31) / 32;
     const int c0 = min(G, (int)threadIdx.y * per), c1 = min(G, c0 + per);
@@ -154,6 +156,7 @@ __device__ void column_scan(uint32_t *__restrict__ hist, int G, int P, uint32_t 
         }
         if (f < P) totals[f] = run;
     }
+    if (totals_only) return;
     __syncthreads();
     if (f < P) {
         uint32_t run = seg[threadIdx.y][threadIdx.x];
@@ -330,8 +333,9 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_colscan(ColScan r, ColScan s, 
     __shared__ bool flag;
     const int cols_r = (r.P + 31) / 32, cols_s = (s.P + 31) / 32;
     const bool is_s = (int)blockIdx.x >= cols_r;
-    if (!is_s) column_scan(r.hist, r.G, r.P, r.totals, blockIdx.x, seg);
-    else column_scan(s.hist, s.G, s.P, s.totals, blockIdx.x - cols_r, seg);
+    const bool totals_only = t.done && t.plan.ctrl->direct;
+    if (!is_s) column_scan(r.hist, r.G, r.P, r.totals, blockIdx.x, seg, totals_only);
+    else column_scan(s.hist, s.G, s.P, s.totals, blockIdx.x - cols_r, seg, totals_only);
     if (!t.done) return;
     const int tid = threadIdx.y * 32 + threadIdx.x;
     if (!last_of(t.done + is_s, is_s ? cols_s : cols_r, tid, &flag)) return;
