@@ -332,13 +332,13 @@ int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &
                               g.direct_rows, ctrl, st);
         if (e == cudaSuccess)
             e = launch_direct_decide(g.direct_rows ? nullptr : w.direct.as<uint32_t>(), direct_log2_max(g.n[0]), g.n[0],
-                                     ctrl, st);
+                                     g.sample_S, g.n[1], ctrl, st);
     } else if (g.direct && g.direct_rows && !bypass) {
         e = launch_hist_emit(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), g.rows,
                              g.rows_cap, g.s_range_max, ctrl, st);
     } else if (g.direct && !bypass) {
         e = launch_hist_probe(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(),
-                              g.n[0], ctrl, st);
+                              g.n[0], w.nsm, ctrl, st);
     } else if (!bypass) {
         const bool check = rel == 1 && g.s_range_max != 0xFFFFFFFFu;
         e = launch_hist_chunks(d, g.n[rel], g.ch[rel], g.G[rel], hist.as<uint32_t>(), g.B, g.rf, st,
@@ -531,6 +531,7 @@ int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row
     const bool timing = cfg.timing != 0;
     RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
     try_direct(g, cfg, d_rows, cap);
+    g.sample_S = dS;
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;

@@ -49,19 +49,19 @@ int direct_log2_max(uint64_t nR) {
     return k;
 }
 
-// Shared memory words for S's copy of the bit table: two bits per R row, at
-// most what a CTA can hold beside its histogram bins.  A table in shared
-// memory is read at the speed of S's stream (2^30 rows: 1.37 ms), one in L2
-// at one line per clock and SM (4.02 ms).  Zero when a table of one bit per
-// row would not fit: then every bit is read from L2 and the CTA keeps its
-// smaller footprint.
+// Shared memory words for a CTA's copy of the bit table or of one of two parts
+// of it: what a CTA can hold beside its histogram bins (one CTA per SM either
+// way).  A table in shared memory is read at the speed of S's stream (2^30
+// rows: 1.37 ms), one in L2 at one line per clock and SM (4.02 ms); in two
+// parts every row is read twice, which is still faster than L2 (2.5 M x 50 M
+// rows: 241 against 314 us), in three not (5 M x 100 M: 459 against 470 us,
+// 5 M x 20 M: 175 against 168 us).  Zero when one bit per row would not fit.
+constexpr uint32_t DIRECT_PARTS = 2;
 uint32_t direct_smem_words(uint64_t nR, uint64_t nbins) {
     constexpr uint64_t CAP = 220 * 1024 / 4;
-    if (nbins >= CAP) return 0;
+    if (nbins >= CAP / 2) return 0;
     const uint64_t cap = CAP - nbins;
-    if ((nR + 31) / 32 + 1 > cap) return 0;
-    const uint64_t want = std::max<uint64_t>(1024, (nR + 15) / 16);
-    return (uint32_t)std::min(want, cap);
+    return (nR + 31) / 32 + 1 <= cap * DIRECT_PARTS ? (uint32_t)cap : 0u;
 }
 
 // The same for the payload table of a materialising join: 16 entries per row,
@@ -257,9 +257,11 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
 
 // Counts the set bits; the last CTA decides.  The table is read from L2
 // (2^27 keys: 33.5 MB, half of it R's range).  A payload table (null bits)
-// needs no count: its entries showed every duplicate.
+// needs no count: its entries showed every duplicate.  CTA 0 also looks at 1024
+// evenly spaced rows of S (null: not there yet) for hot keys: under Zipf z = 1
+// over 16.8 M keys they hold thousands of equal pairs, uniform keys hardly any.
 __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t *__restrict__ bits, uint64_t nR,
-                                                                  Ctrl *ctrl) {
+                                                                  const Row *__restrict__ S, uint64_t nS, Ctrl *ctrl) {
     dep_wait();
     dep_trigger();
     __shared__ unsigned s_count;
@@ -272,6 +274,20 @@ __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t
         return;
     }
     if (tid == 0) s_count = 0;
+    if (blockIdx.x == 0) {
+        __shared__ uint32_t seen[4096];  // a sampled key at its hash: the later of two keys stays
+        __shared__ unsigned equal;
+        if (tid == 0) equal = 0;
+        for (int i = tid; i < 4096; i += DIRECT_THREADS) seen[i] = ~0u;
+        __syncthreads();
+        if (S && (uint64_t)tid < nS) {
+            const uint64_t i = nS <= DIRECT_THREADS ? tid : (uint64_t)tid * (nS - 1) / (DIRECT_THREADS - 1);
+            const uint32_t k = S[i].key;
+            if (k != ~0u && atomicExch(&seen[(k * 0x9E3779B1u) >> 20], k) == k) atomicAdd(&equal, 1u);
+        }
+        __syncthreads();
+        if (tid == 0) ctrl->direct_hot = !S || equal >= 16;
+    }
     __syncthreads();
     const uint4 *b4 = reinterpret_cast<const uint4 *>(bits);
     const uint64_t n4 = 1ull << (w - 7);
@@ -296,46 +312,50 @@ __global__ void __launch_bounds__(DIRECT_THREADS) k_direct_decide(const uint32_t
 }
 
 // S: chunk histograms and, when the join is direct, the matches.  Two
-// launches, of which one does the work: SMEM reads the table from a copy in
-// shared memory (the words from R's smallest key to its largest, when they
-// fit `smem_words`), the other from L2, and it is the plain histogram when the
-// join is not direct.  (One launch for both would hold the copy's shared
-// memory, and so one CTA per SM, for the plain histogram too: a sparse 2^20 x
-// 2^22 join took 182 us instead of 140 us.)  Bound by the L1's one line per
-// clock and SM for the table in L2: 2^30 rows 4.13 ms (8 B/row: 2.1 TB/s; 4.02
-// ms without the histogram), and by S's read from HBM for the table in shared
-// memory.  The partitioned join reads and writes 40 more bytes per row of S.
-template <bool SMEM>
+// launches, of which one does the work: k_hist_probe_smem reads the table from
+// shared memory when it fits there, in up to DIRECT_PARTS parts; k_hist_probe
+// reads it from L2, and is the plain histogram when the join is not direct.
+// (One launch for both would hold the copy's shared memory, and so one CTA per
+// SM, for the plain histogram too: a sparse 2^20 x 2^22 join took 182 us
+// instead of 140 us.)
+
+// The words of the table that R's range covers: first word, number of words.
+__device__ __forceinline__ uint2 direct_words(const Ctrl *ctrl) {
+    const uint32_t kmin = ~ctrl->direct_inv_min, kmax = ctrl->direct_max;
+    return make_uint2(kmin >> 5, (kmax >> 5) - (kmin >> 5) + 1);
+}
+// Whether they fit the copies of at most `parts_max` CTAs.
+__device__ __forceinline__ bool direct_fits(uint32_t words, uint32_t smem_words, uint32_t parts_max) {
+    return words <= (uint64_t)smem_words * parts_max;
+}
+
+// The table in L2: bound by the L1's one line per clock and SM (2^30 rows 4.13
+// ms, 8 B/row: 2.1 TB/s; 4.02 ms without the histogram).  The partitioned join
+// reads and writes 40 more bytes per row of S.
 __global__ void __launch_bounds__(DIRECT_THREADS, 2)
     k_hist_probe(const Row *__restrict__ in, uint64_t n, uint64_t chunk, uint32_t *__restrict__ hist, int nbins, RadixF rf,
-                 const uint32_t *__restrict__ bits, uint32_t smem_words, Ctrl *ctrl) {
+                 const uint32_t *__restrict__ bits, uint32_t smem_words, uint32_t parts_max, Ctrl *ctrl) {
     dep_wait();
     dep_trigger();
     const bool direct = ctrl->direct != 0;
     const uint32_t kmin = ~ctrl->direct_inv_min, span = ctrl->direct_max - kmin;
     const uint32_t wordmask = direct ? (uint32_t)((1ull << (ctrl->direct_log2 - 5)) - 1) : 0u;
-    const uint32_t w0 = kmin >> 5;
-    const uint32_t words = ((kmin + span) >> 5) - w0 + 1;
-    if (SMEM != (direct && words <= smem_words)) return;
+    if (direct && direct_fits(direct_words(ctrl).y, smem_words, parts_max)) return;
     extern __shared__ uint32_t sh[];
-    uint32_t *copy = sh + nbins;
     const int tid = threadIdx.x;
     for (int i = tid; i < nbins; i += DIRECT_THREADS) sh[i] = 0;
-    if (SMEM)
-        for (uint32_t i = tid; i < words; i += DIRECT_THREADS) copy[i] = ld_bits(bits + ((w0 + i) & wordmask));
     __syncthreads();
     const uint64_t lo = (uint64_t)blockIdx.x * chunk;
     const uint64_t hi = umin64(n, lo + chunk);
     uint32_t matches = 0;  // a chunk holds < 2^32 rows, and a row matches at most once
-    auto word = [&](uint32_t key, bool ok) -> uint32_t {
-        if (!ok || key - kmin > span) return 0;
-        return SMEM ? copy[(key >> 5) - w0] : ld_bits(bits + ((key >> 5) & wordmask));
-    };
     auto bit = [](uint32_t word, uint32_t key) { return (word >> (key & 31)) & 1u; };
-    stream_pairs(
-        in, lo, hi,
-        [&](const uint4(&x)[4], const bool(&ok)[4]) {
-            if (SMEM || direct) {
+    auto probe = [&](auto load) {
+        auto word = [&](uint32_t key, bool ok) -> uint32_t {
+            return ok && key - kmin <= span ? load(bits + ((key >> 5) & wordmask)) : 0u;
+        };
+        stream_pairs(
+            in, lo, hi,
+            [&](const uint4(&x)[4], const bool(&ok)[4]) {
                 uint32_t a[8];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
@@ -345,15 +365,28 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2)
                 hist_pairs(sh, rf, x, ok);  // while the words arrive
 #pragma unroll
                 for (int u = 0; u < 4; u++) matches += bit(a[2 * u], x[u].x) + bit(a[2 * u + 1], x[u].z);
-            } else {
-                hist_pairs(sh, rf, x, ok);
-            }
-        },
-        [&](const Row &r) {
-            if (SMEM || direct) matches += bit(word(r.key, true), r.key);
-            atomicAdd(&sh[radix_f(rf, r.key)], 1u);
-        });
-    if (SMEM || direct) {
+            },
+            [&](const Row &r) {
+                matches += bit(word(r.key, true), r.key);
+                atomicAdd(&sh[radix_f(rf, r.key)], 1u);
+            });
+    };
+    // Through the L1, hot keys are found there instead of queueing at their L2
+    // slice (16.8 M x 134 M rows, Zipf z = 1: 0.53 against 1.50 ms past it; z =
+    // 1.5: 0.43 against 2.18 ms).  Uniform keys gain from it in tables up to 4
+    // MB (9%) and above 28 MB, which crowd the L2 (5% at 34 MB, 18% at 67), and lose 2.5%
+    // between.
+    const uint32_t bytes = span / 8;
+    if (!direct) {
+        stream_pairs(
+            in, lo, hi, [&](const uint4(&x)[4], const bool(&ok)[4]) { hist_pairs(sh, rf, x, ok); },
+            [&](const Row &r) { atomicAdd(&sh[radix_f(rf, r.key)], 1u); });
+    } else if (ctrl->direct_hot || bytes <= (4u << 20) || bytes > (28u << 20)) {
+        probe([](const uint32_t *p) { return __ldg(p); });
+    } else {
+        probe([](const uint32_t *p) { return ldg_no_l1(p); });
+    }
+    if (direct) {
         const unsigned long long ws = warp_sum_u64(matches);
         if ((tid & 31) == 0 && ws) atomicAdd(&ctrl->matches, ws);
     }
@@ -362,22 +395,106 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2)
     for (int i = tid; i < nbins; i += DIRECT_THREADS) dst[i] = sh[i];
 }
 
+// The table in shared memory: CTA b holds part b mod `parts` of it and, with
+// the other CTAs of its part, reads all of S in rounds of 8192 rows; round u is
+// counted in the histogram by the part u mod `parts`.  A direct join uses the
+// histograms' column sums only, so a CTA's counts go to row b of the G rows
+// whatever chunks they are from, and it clears the rows b + gridDim, ....
+// 1.8 M x 36 M rows (two parts): 186 us against 270 us from L2.
+__global__ void __launch_bounds__(DIRECT_THREADS, 1)
+    k_hist_probe_smem(const Row *__restrict__ in, uint64_t n, int G, uint32_t *__restrict__ hist, int nbins, RadixF rf,
+                      const uint32_t *__restrict__ bits, uint32_t smem_words, uint32_t parts_max, Ctrl *ctrl) {
+    dep_wait();
+    dep_trigger();
+    constexpr uint32_t T = DIRECT_THREADS;
+    if (!ctrl->direct) return;
+    const uint2 all = direct_words(ctrl);
+    if (!direct_fits(all.y, smem_words, parts_max)) return;
+    extern __shared__ uint32_t sh[];
+    uint32_t *copy = sh + nbins;
+    const int tid = threadIdx.x;
+    const uint32_t parts = (all.y + smem_words - 1) / smem_words;  // <= parts_max <= gridDim.x
+    const uint32_t per = (all.y + parts - 1) / parts;              // <= smem_words
+    const uint32_t part = blockIdx.x % parts, member = blockIdx.x / parts;
+    const uint32_t members = (gridDim.x - part + parts - 1) / parts;
+    const uint32_t wordmask = (uint32_t)((1ull << (ctrl->direct_log2 - 5)) - 1);
+    const uint32_t w0 = all.x + min(part * per, all.y), words = min(per, all.x + all.y - w0);
+    // this part's keys: [klo, klo + kspan] (kspan: none for a part past the end)
+    const uint32_t kmin = ~ctrl->direct_inv_min, kmax = ctrl->direct_max;
+    const uint32_t klo = max(kmin, w0 << 5), khi = min(kmax, ((w0 + words - 1) << 5) | 31);
+    const bool none = words == 0;
+    const uint32_t kspan = none ? 0 : khi - klo;
+    for (int i = tid; i < nbins; i += T) sh[i] = 0;
+    for (uint32_t i = tid; i < words; i += T) copy[i] = __ldg(bits + ((w0 + i) & wordmask));
+    __syncthreads();
+    uint32_t matches = 0;  // this thread's: at most one per row
+    auto look = [&](uint32_t key) {
+        if (key - klo <= kspan && !none) matches += (copy[(key >> 5) - w0] >> (key & 31)) & 1u;
+    };
+    const uint32_t head = (reinterpret_cast<uintptr_t>(in) & 15) ? 1u : 0u;
+    const uint32_t nv = (uint32_t)((n - head) / 2);  // n >= 1
+    const uint4 *v = reinterpret_cast<const uint4 *>(in + head);
+    uint4 nx[4];
+    auto load = [&](uint64_t round) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint64_t i = round * (4 * T) + u * T + tid;
+            nx[u] = i < nv ? ldg_stream(v + i) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    load(member);
+    for (uint64_t round = member; round * (4 * T) < nv; round += members) {
+        uint4 x[4];
+        bool ok[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            x[u] = nx[u];
+            ok[u] = round * (4 * T) + u * T + tid < nv;
+        }
+        load(round + members);  // in flight during this round
+        if (round % parts == part) hist_pairs(sh, rf, x, ok);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (ok[u]) {
+                look(x[u].x);
+                look(x[u].z);
+            }
+        }
+    }
+    if (member == 0 && tid == 0) {  // the rows outside the 16-byte aligned body
+        auto edge = [&](uint32_t key) {
+            look(key);
+            if (part == 0) atomicAdd(&sh[radix_f(rf, key)], 1u);
+        };
+        if (head) edge(in[0].key);
+        if ((n - head) & 1) edge(in[n - 1].key);
+    }
+    const unsigned long long ws = warp_sum_u64(matches);
+    if ((tid & 31) == 0 && ws) atomicAdd(&ctrl->matches, ws);
+    __syncthreads();
+    for (int c = blockIdx.x; c < G; c += gridDim.x) {
+        uint32_t *dst = hist + (uint64_t)c * nbins;
+        const bool mine = c == (int)blockIdx.x;
+        for (int i = tid; i < nbins; i += T) dst[i] = mine ? sh[i] : 0u;
+    }
+}
+
 // S of a materialising join: chunk histograms and, when the join is direct,
 // the output rows.  A round takes 8 rows per thread: their payloads are
 // gathered from the table in L2, the matching rows take places in (warp, row
-// slot, lane) order in shared memory, one atomic reserves the round's output,
-// and one bulk store writes it: staged at its destination's 16-byte phase, so
-// all but the at most 3 words at either end leave by the copy engine and the
-// stores cost the SM no load/store instructions.  Bound by L2 (one sector per
-// row gathered, 12 B out, 8 B in).
+// slot, lane) order in shared memory, and one atomic reserves the round's
+// output.  A round's rows leave for memory while the next round's payloads
+// arrive, and the reservation returns while the rows are staged, so a round
+// waits for neither.  Bound by L2 (one sector per row gathered, 12 B out, 8 B
+// in): 16.8 M rows take XXX us, 161 us before the rounds overlapped (then
+// with a bulk store per round).
 constexpr int EMIT_DIRECT_THREADS = 512;
 constexpr int EMIT_ROUND = EMIT_DIRECT_THREADS * 8;
 
 struct EmitSmem {
-    alignas(16) uint32_t stage[EMIT_ROUND * 3 + 4];
+    alignas(16) uint32_t stage[EMIT_ROUND * 3];
     uint32_t wtot[EMIT_DIRECT_THREADS / 32];
     unsigned long long base;
-    uint32_t total;
 };
 
 __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
@@ -399,13 +516,23 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
     const uint64_t lo = (uint64_t)blockIdx.x * chunk;
     const uint64_t hi = umin64(n, lo + chunk);
     unsigned long long matches = 0;  // not direct: keys outside range_max
+    uint32_t staged = 0;             // rows of the last round in the stage, at sm.base
+    // writes the staged rows out, word by word (coalesced)
+    auto flush = [&]() {
+        const unsigned long long base = sm.base;
+        const uint32_t words = base < cap ? 3 * (uint32_t)umin64(staged, cap - base) : 0u;
+        uint32_t *g = reinterpret_cast<uint32_t *>(out + base);
+#pragma unroll 4
+        for (uint32_t i = tid; i < words; i += T) __stcs(g + i, sm.stage[i]);
+    };
     // one round: this thread's rows (k, p) of `valid`; every thread calls it
     auto round = [&](const uint32_t (&k)[8], const uint32_t (&p)[8], unsigned valid) {
         uint32_t r[8];
         if (direct) {
 #pragma unroll
             for (int j = 0; j < 8; j++)
-                r[j] = (valid >> j & 1) && k[j] - kmin <= span ? ld_bits(table + (k[j] & mask)) : EMPTY_PAYLOAD;
+                r[j] = (valid >> j & 1) && k[j] - kmin <= span ? __ldg(table + (k[j] & mask)) : EMPTY_PAYLOAD;
+            flush();  // the last round's rows, while the payloads arrive
         }
         const bool dup = warp_has_dups(radix_f(rf, k[0]), valid & 1u);
 #pragma unroll
@@ -426,7 +553,7 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
             wt += __popc(m[j]);
         }
         if (lane == 0) sm.wtot[w] = wt;
-        __syncthreads();
+        __syncthreads();  // totals written, the stage free
         uint32_t before = 0, total = 0;
 #pragma unroll
         for (int q = 0; q < NW; q++) {
@@ -434,44 +561,25 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
             before += q < w ? x : 0;
             total += x;
         }
-        if (tid == 0) {
-            sm.base = total ? atomicAdd(&ctrl->rows, (unsigned long long)total) : 0;
-            bulk_wait_read();  // the last round's rows have left the stage
-        }
-        __syncthreads();
-        const unsigned long long base = sm.base;
-        const uintptr_t dst = reinterpret_cast<uintptr_t>(out + base);
-        const uint32_t phase = (uint32_t)(dst & 15) / 4;  // the stage starts at the destination's phase
-        const uint32_t keep = base < cap ? (uint32_t)umin64(total, cap - base) : 0u;
+        unsigned long long base = 0;
+        if (tid == 0 && total) base = atomicAdd(&ctrl->rows, (unsigned long long)total);
         const unsigned lt = lanemask_lt();
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             if (m[j] >> lane & 1) {
-                uint32_t *q = sm.stage + phase + 3 * (before + __popc(m[j] & lt));
+                uint32_t *q = sm.stage + 3 * (before + __popc(m[j] & lt));
                 q[0] = k[j];
                 q[1] = r[j];
                 q[2] = p[j];
             }
             before += __popc(m[j]);
         }
-        fence_proxy_async_smem();
-        __syncthreads();
-        // words [phase, phase + 3 * keep) of the stage go to the 16-byte aligned
-        // address dst - 4 * phase, word for word
-        uint32_t *g = reinterpret_cast<uint32_t *>(dst) - phase;
-        const uint32_t end = phase + 3 * keep;
-        const uint32_t a0 = (phase + 3) & ~3u, a1 = end & ~3u;  // the aligned body
         if (tid == 0) {
-            if (a0 < a1) {
-                bulk_s2g(g + a0, sm.stage + a0, (a1 - a0) * 4);
-                bulk_commit();
-            }
+            sm.base = base;
             matches += total;
-        } else if (w == 1) {  // up to 3 words before the body and after it
-            const uint32_t head_end = min(a0, end), tail0 = max(a1, head_end);
-            if (phase + lane < head_end) g[phase + lane] = sm.stage[phase + lane];
-            if (tail0 + lane < end) g[tail0 + lane] = sm.stage[tail0 + lane];
         }
+        staged = total;
+        __syncthreads();  // staged, and its place known
     };
     if (lo < hi) {
         const uint32_t head = ((reinterpret_cast<uintptr_t>(in + lo) & 15) != 0) ? 1 : 0;
@@ -513,12 +621,10 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
             }
             round(k, p, valid);
         }
+        if (direct) flush();
     }
     if (direct) {  // thread 0 counted the rounds' rows
-        if (tid == 0) {
-            bulk_wait_all();
-            if (matches) atomicAdd(&ctrl->matches, matches);
-        }
+        if (tid == 0 && matches) atomicAdd(&ctrl->matches, matches);
     } else {
         const unsigned long long o = warp_sum_u64(matches);
         if (lane == 0 && o) atomicAdd(&ctrl->out_of_range, o);
@@ -562,29 +668,34 @@ cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, 
     return e;
 }
 
-cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, Ctrl *ctrl, cudaStream_t st) {
+cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, Ctrl *ctrl,
+                                 cudaStream_t st) {
     const uint64_t n4 = 1ull << (log2_max - 7);
     // two 16-byte words per thread and CTA at least, one CTA per SM at most
     const unsigned g = bits ? (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), 148)) : 1u;
-    const cudaError_t e = launch_dep(k_direct_decide, g, DIRECT_THREADS, 0, st, bits, nR, ctrl);
+    const cudaError_t e = launch_dep(k_direct_decide, g, DIRECT_THREADS, 0, st, bits, nR, S, nS, ctrl);
     count_launch();
     return e;
 }
 
 cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
-                              const uint32_t *bits, uint64_t nR, Ctrl *ctrl, cudaStream_t st) {
+                              const uint32_t *bits, uint64_t nR, int nsm, Ctrl *ctrl, cudaStream_t st) {
     const int nbins = 1 << P_log2;
     const uint32_t words = direct_smem_words(nR, (uint64_t)nbins);
+    const unsigned grid = (unsigned)std::min(G, nsm);  // every CTA writes a row of the histogram
+    const uint32_t parts_max = std::min<uint32_t>(DIRECT_PARTS, grid);
     const size_t smem = (size_t)nbins * 4, smem_copy = smem + (size_t)words * 4;
     cudaError_t e;
     if (words) {
-        if ((e = smem_limit((const void *)k_hist_probe<true>, smem_copy)) != cudaSuccess) return e;
-        e = launch_dep(k_hist_probe<true>, G, DIRECT_THREADS, smem_copy, st, in, n, chunk, hist, nbins, rf, bits, words, ctrl);
+        if ((e = smem_limit((const void *)k_hist_probe_smem, smem_copy)) != cudaSuccess) return e;
+        e = launch_dep(k_hist_probe_smem, grid, DIRECT_THREADS, smem_copy, st, in, n, G, hist, nbins, rf, bits, words,
+                       parts_max, ctrl);
         count_launch();
         if (e != cudaSuccess) return e;
     }
-    if ((e = smem_limit((const void *)k_hist_probe<false>, smem)) != cudaSuccess) return e;
-    e = launch_dep(k_hist_probe<false>, G, DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, bits, words, ctrl);
+    if ((e = smem_limit((const void *)k_hist_probe, smem)) != cudaSuccess) return e;
+    e = launch_dep(k_hist_probe, G, DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, bits, words, parts_max,
+                   ctrl);
     count_launch();
     return e;
 }

@@ -83,6 +83,7 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     const int capR = join_capacity(nR, !cfg.materialize);
     RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
     if (!mat) try_direct(g, cfg, nullptr, 0);
+    g.sample_S = dS;
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;

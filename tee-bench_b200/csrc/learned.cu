@@ -1291,7 +1291,7 @@ __global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass_direct(BypassArg
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t kmin = ~a.ctrl->direct_inv_min, span = a.ctrl->direct_max - kmin;
     const uint32_t wordmask = (uint32_t)((1ull << (a.ctrl->direct_log2 - 5)) - 1);
-    auto word = [&](uint32_t key) { return key - kmin <= span ? ld_bits(a.bits + ((key >> 5) & wordmask)) : 0u; };
+    auto word = [&](uint32_t key) { return key - kmin <= span ? ldg_no_l1(a.bits + ((key >> 5) & wordmask)) : 0u; };
     for (int i = tid; i < a.nbins; i += BYP_THREADS) hist[i] = 0;
     for (int i = tid; i < HEAVY_CAP; i += BYP_THREADS) {
         const uint32_t k = a.hkeys[i];

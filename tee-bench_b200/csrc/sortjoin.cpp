@@ -172,6 +172,7 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     }
     RadixGeom g = radix_geometry_msd(nR, nS, sub, B, lowbits, w);
     try_direct(g, cfg, nullptr, 0);
+    g.sample_S = dS;
     g.capR = 0x7FFFFFFF;  // counters take any number of R rows
     g.capS = std::max<uint64_t>(65536, nS / ((uint64_t)w.nsm * 12));
     g.item_cap = 2 * (nS / g.capS + 4 * g.P) + 16;
@@ -266,6 +267,7 @@ static int direct_or_lsd(const tbg_config &cfg, const Row *dR, uint64_t nR, cons
     *direct = false;
     RadixGeom g = radix_geometry_msd(nR, nS, rmin, 1, 31, w);
     try_direct(g, cfg, d_rows, cap);
+    g.sample_S = dS;
     const int lg = g.direct_rows ? direct_log2_max_rows(nR) : direct_log2_max(nR);
     // more rows than key values: not distinct
     if (!g.direct || (uint64_t)(rmax - rmin) >= (1ull << lg) || nR > (uint64_t)(rmax - rmin) + 1) return TBG_OK;

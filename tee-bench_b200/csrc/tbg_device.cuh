@@ -54,9 +54,8 @@ __device__ __forceinline__ uint32_t radix_f(const RadixF &rf, uint32_t key) {
 __device__ __forceinline__ uint4 ldg_stream(const uint4 *p) { return __ldcs(p); }
 __device__ __forceinline__ uint2 ldg_stream(const uint2 *p) { return __ldcs(p); }
 
-// One word of the direct join's bit table from L2, not kept in L1 (a line of it is rarely
-// asked for again before it would be replaced).
-__device__ __forceinline__ uint32_t ld_bits(const uint32_t *p) {
+// A read-only word that is not kept in L1.
+__device__ __forceinline__ uint32_t ldg_no_l1(const uint32_t *p) {
     uint32_t v;
     asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;

@@ -48,7 +48,7 @@ struct Ctrl {
     unsigned int direct_inv_min;     // ~(smallest key of R), kept as a maximum so that it starts at 0
     unsigned int direct_max;         // largest key of R
     unsigned int done[4];            // CTA tickets: column scans of R and of S, relations scanned; the bit count
-    unsigned int pad;
+    unsigned int direct_hot;         // a sample of S shows hot keys
 };
 
 // Sums of the CTAs of a small join (small.cu); zero between launches.
@@ -197,9 +197,10 @@ cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *table, int l
                                int nsm, cudaStream_t st);
 cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
                               uint32_t *table, bool payloads, Ctrl *ctrl, cudaStream_t st);
-cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, Ctrl *ctrl, cudaStream_t st);
+cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, Ctrl *ctrl,
+                                 cudaStream_t st);
 cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
-                              const uint32_t *bits, uint64_t nR, Ctrl *ctrl, cudaStream_t st);
+                              const uint32_t *bits, uint64_t nR, int nsm, Ctrl *ctrl, cudaStream_t st);
 
 cudaError_t launch_gen_pk(Row *d, uint64_t n, uint64_t seed, cudaStream_t st);
 cudaError_t launch_gen_fk(Row *d, uint64_t n, uint64_t maxid, uint64_t seed, cudaStream_t st);

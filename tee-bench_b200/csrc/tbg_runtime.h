@@ -97,6 +97,7 @@ struct RadixGeom {
     bool direct_rows = false;      // ... of a materialising join: R's payloads instead of bits,
     tbg_row_out *rows = nullptr;   // ... S's read writes the rows here
     uint64_t rows_cap = 0;
+    const Row *sample_S = nullptr;  // S, when it is there while R is read
 };
 RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int capR, Workspace &w);
 RadixGeom radix_geometry_msd(uint64_t nR, uint64_t nS, uint32_t sub, int B, int lowbits, Workspace &w);

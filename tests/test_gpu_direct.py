@@ -219,3 +219,21 @@ def test_async_join_in_a_captured_graph(tbg, oracle, cuda, nR, materialize):
             got = rows[: 3 * ref].cpu().numpy().view(np.uint32).reshape(-1, 3)
             assert np.array_equal(oracle.sort_rows(got), oracle.sort_rows(ref_rows))
     assert tbg.lib().tbg_sync_status(st.cuda_stream) == 0
+
+
+# |R| around one and two parts of the table in shared memory (P = 2^7 .. 2^9
+# bins beside 55,808 .. 56,192 words of bits) and into L2, with S below one CTA
+# round, with edge rows, and skewed
+@pytest.mark.parametrize("nR", [1780000, 1803000, 3560001, 3610001])
+@pytest.mark.parametrize("nS,z", [(4097, 0), (1000003, 0), (1000003, 1.2)])
+def test_direct_table_parts(tbg, oracle, cuda, nR, nS, z):
+    rng = np.random.default_rng(nR)
+    R, S = relations(oracle, rng, nR, nS, 12345, 1, 0.2)
+    if z:
+        S["key"] = 12345 + np.minimum(rng.zipf(z, nS), nR + 5)
+    want = int(((S["key"].astype(np.int64) >= 12345) & (S["key"].astype(np.int64) < 12345 + nR)).sum())
+    for off in (0, 1):
+        m, _, st = run_join(tbg, cuda, "RHO", R, S, offset=off)
+        assert m == want
+    _, _, st2 = run_join(tbg, cuda, "RHO", R, S, passes=st.passes)
+    assert (st.max_part_R, st.max_part_S, st.work_items) == (st2.max_part_R, st2.max_part_S, st2.work_items)
