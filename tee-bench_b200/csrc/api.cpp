@@ -236,6 +236,7 @@ RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int ca
     g.ch[1] = ((nS + g.G[1] - 1) / g.G[1] + 1) & ~1ull;
     g.n[0] = nR;
     g.n[1] = nS;
+    g.keys = !cfg.materialize;
     // f = (key & (F1 - 1)) << b2 | (key >> b1) & (F2 - 1): pass 1 by the low b1
     // bits, pass 2 by the next b2
     g.rf = g.passes == 1 ? RadixF{(uint32_t)(g.P - 1), 0, 0, 0}
@@ -479,10 +480,11 @@ static PartArgs pass_args(int rel, int which, const RadixGeom &g, const Row *d, 
     a.cnt1 = g.passes == 2 ? (rel ? w.cnt1S : w.cnt1R).as<uint32_t>() : nullptr;
     a.err = &ctrl->error;
     a.skip = &ctrl->direct;
-    Row *part = (rel ? w.partS : w.partR).as<Row>();
-    Row *tmp = g.passes == 2 ? (rel ? w.tmpS : w.tmpR).as<Row>() : part;
+    a.keys = g.keys;
+    void *part = (rel ? w.partS : w.partR).p;
+    void *tmp = g.passes == 2 ? (rel ? w.tmpS : w.tmpR).p : part;
     if (which == 1) {
-        a.in = bypass ? w.sc.as<Row>() : d;
+        a.in = bypass ? w.sc.p : d;
         if (bypass) a.chunk_len = w.kept.as<uint32_t>();
         a.out = tmp;
     } else {

@@ -144,8 +144,8 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
             J.GR = (uint32_t)ceil_div(in.nR, c.chunk);
             J.GS = (uint32_t)ceil_div(in.nS, c.chunk);
             J.item_cap = (uint32_t)(J.P + ceil_div(in.nS, c.capS));
-            o.rp = part_bytes; part_bytes = align_up(part_bytes + in.nR * sizeof(Row));
-            o.sp = part_bytes; part_bytes = align_up(part_bytes + in.nS * sizeof(Row));
+            o.rp = part_bytes; part_bytes = align_up(part_bytes + in.nR * 4);
+            o.sp = part_bytes; part_bytes = align_up(part_bytes + in.nS * 4);
             o.hr = meta2; meta2 = align_up(meta2 + (size_t)J.GR * J.P * 4);
             o.hs = meta2; meta2 = align_up(meta2 + (size_t)J.GS * J.P * 4);
             o.br = meta2; meta2 = align_up(meta2 + (size_t)J.P * 4);
@@ -175,8 +175,8 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
         const Off &o = off[k];
         if (J.bits_log2) J.bits = reinterpret_cast<uint32_t *>(base + meta_off + o.bits);
         if (J.B == 0) continue;
-        J.Rp = reinterpret_cast<Row *>(base + o.rp);
-        J.Sp = reinterpret_cast<Row *>(base + o.sp);
+        J.Rp = reinterpret_cast<uint32_t *>(base + o.rp);
+        J.Sp = reinterpret_cast<uint32_t *>(base + o.sp);
         J.histR = reinterpret_cast<uint32_t *>(base + meta_off + o.hr);
         J.histS = reinterpret_cast<uint32_t *>(base + meta_off + o.hs);
         J.baseR = reinterpret_cast<uint32_t *>(base + meta_off + o.br);

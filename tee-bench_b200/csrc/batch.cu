@@ -392,16 +392,18 @@ __device__ void scatter_chunk(const BatchArgs &a, uint32_t c, BPart &sm, uint64_
     const uint64_t n = rel ? J.nS : J.nR;
     const uint64_t lo = (uint64_t)idx * J.chunk;
     const uint64_t hi = umin64(n, lo + J.chunk);
-    part_tiles<BATCH_THREADS>(in, lo, hi, n, rel ? J.Sp : J.Rp, (uint32_t)n, DigitOp{0u, P - 1}, (int)P, sm, mbar,
-                              kseq, a.err);
+    part_tiles<BATCH_THREADS, uint32_t>(in, lo, hi, n, rel ? J.Sp : J.Rp, (uint32_t)n, DigitOp{0u, P - 1}, sm, mbar,
+                                        kseq, a.err);
     cta_signal(&a.sync[ch.x].scat_done);
 }
 
 // ---------------------------------------------------------------------------
 // join: build/probe
 // ---------------------------------------------------------------------------
-template <bool CG>
-__device__ unsigned long long pair_count(Table &t, CellTable &ct, const Row *R, uint64_t rn, const Row *S, uint64_t sn,
+// R and S: the caller's rows, or (CG, written earlier in the launch)
+// partitions of bare keys.
+template <bool CG, class E>
+__device__ unsigned long long pair_count(Table &t, CellTable &ct, const E *R, uint64_t rn, const E *S, uint64_t sn,
                                          uint32_t capR, uint64_t *scratch) {
     unsigned long long c = 0;
     for (uint64_t r0 = 0; r0 < rn; r0 += capR) {

@@ -31,7 +31,7 @@ constexpr uint32_t BATCH_DCHUNK = 262144;  // S rows per chunk ticket of a direc
 // partitions of the low key bits, then build/probe per partition.
 struct BatchJoin {
     const Row *R, *S;          // caller's relations (device memory, any 8-byte alignment)
-    Row *Rp, *Sp;              // partitioned copies (256-byte aligned regions)
+    uint32_t *Rp, *Sp;         // the keys, partitioned (256-byte aligned regions)
     uint32_t *histR, *histS;   // [GR][P], [GS][P]: per-chunk counts, then per-chunk prefixes
     uint32_t *baseR, *baseS;   // [P] partition starts inside Rp / Sp
     Item *items;               // [item_cap] join work items of this join

@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
     const int tid = threadIdx.x;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
     unsigned long long local = 0;
+    // counting: the partitions hold bare keys
+    const uint32_t *Rk = reinterpret_cast<const uint32_t *>(a.R), *Sk = reinterpret_cast<const uint32_t *>(a.S);
 
     // an item is claimed one step ahead, and its R rows are prefetched into
     // L2 while the current item is probed, so its table build reads L2
@@ -69,12 +71,13 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
             s_item[(iter + 1) & 1] = nx;  // read by all after this item's barriers
             if (nx < nitems) {
                 const Item mn = a.items[nx];
-                prefetch_l2(a.R + mn.r_off, (uint64_t)mn.r_len * sizeof(Row));
+                if (MAT) prefetch_l2(a.R + mn.r_off, (uint64_t)mn.r_len * sizeof(Row));
+                else prefetch_l2(Rk + mn.r_off, (uint64_t)mn.r_len * 4);
             }
         }
         const Item m = a.items[it];
         if (MAT) build_table<JOIN_THREADS>(t, a.R, m.r_off, m.r_len, scan_scratch);
-        else build_cells<JOIN_THREADS>(ct, a.R, m.r_off, m.r_len);
+        else build_cells<JOIN_THREADS>(ct, Rk, m.r_off, m.r_len);
 
         const Row *s = a.S + m.s_off;
         const uint64_t len = m.s_len;
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
         const uint4 *v = reinterpret_cast<const uint4 *>(s + head);
 
         if (!MAT) {
-            local += probe_count<JOIN_THREADS>(ct, s, len);
+            local += stream_sum<JOIN_THREADS>(Sk + m.s_off, len, [&](uint32_t k) { return ct.count(k); });
         } else {
             // block-synchronous rounds: 8 rows per thread, one reservation per round
             const uint64_t per_round = 4ull * JOIN_THREADS;

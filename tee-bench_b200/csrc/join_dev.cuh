@@ -119,14 +119,24 @@ __device__ __forceinline__ uint2 ld_row(const Row *R, uint64_t i) {
     return *p;
 }
 template <bool CG>
+__device__ __forceinline__ uint32_t ld_key(const Row *R, uint64_t i) { return ld_row<CG>(R, i).x; }
+template <bool CG>
+__device__ __forceinline__ uint32_t ld_key(const uint32_t *R, uint64_t i) { return CG ? __ldcg(R + i) : R[i]; }
+
+// A row, or a bare key with no payload.
+template <bool CG>
+__device__ __forceinline__ uint2 ld_elem(const Row *R, uint64_t i) { return ld_row<CG>(R, i); }
+template <bool CG>
+__device__ __forceinline__ uint2 ld_elem(const uint32_t *R, uint64_t i) { return make_uint2(ld_key<CG>(R, i), 0u); }
+template <bool CG>
 __device__ __forceinline__ uint4 ld_pair(const uint4 *p) {
     if (CG) return __ldcg(p);
     return ldg_stream(p);
 }
 
 // Builds the cells of R rows [r_off, r_off + r_len); ends with a barrier.
-template <int THREADS, bool CG = false>
-__device__ __forceinline__ void build_cells(CellTable &t, const Row *__restrict__ R, uint64_t r_off, uint32_t r_len) {
+template <int THREADS, bool CG = false, class E = Row>
+__device__ __forceinline__ void build_cells(CellTable &t, const E *__restrict__ R, uint64_t r_off, uint32_t r_len) {
     const int tid = threadIdx.x;
     const uint32_t least = t.link_bits > t.hs ? 1u << (t.link_bits - t.hs) : 1u;
     const uint32_t N = min(max(next_pow2(r_len), max(least, 4u)), t.hcap);
@@ -136,7 +146,7 @@ __device__ __forceinline__ void build_cells(CellTable &t, const Row *__restrict_
         reinterpret_cast<uint4 *>(t.heads)[i] = make_uint4(CELL_EMPTY, CELL_EMPTY, CELL_EMPTY, CELL_EMPTY);
     __syncthreads();
     for (uint32_t i = tid; i < r_len; i += THREADS) {
-        const uint32_t k = ld_row<CG>(R, r_off + i).x;
+        const uint32_t k = ld_key<CG>(R, r_off + i);
         uint32_t *head = &t.heads[(k >> t.hs) & t.mask];
         const uint32_t tag = t.tag_shift < 32 ? (k >> t.tag_shift) << t.link_bits : 0u;
         uint32_t old = *head;
@@ -150,17 +160,19 @@ __device__ __forceinline__ void build_cells(CellTable &t, const Row *__restrict_
     __syncthreads();
 }
 
-template <int THREADS, bool CG = false>
-__device__ void build_table(Table &t, const Row *__restrict__ R, uint64_t r_off, uint32_t r_len,
+// E: rows, or bare keys (layout 1 without payloads).
+template <int THREADS, bool CG = false, class E = Row>
+__device__ void build_table(Table &t, const E *__restrict__ R, uint64_t r_off, uint32_t r_len,
                             uint64_t *scan_scratch) {
     const int tid = threadIdx.x;
-    if (t.layout == 0) {
+    constexpr bool ROWS = sizeof(E) == sizeof(Row);
+    if (ROWS && t.layout == 0) {
         // next_pow2(|R_p|) buckets as in the reference, at most hcap (a
         // longer average chain when capR is not a power of two)
         const uint32_t N = min(next_pow2(r_len), t.hcap);
         t.mask = N - 1;
         for (uint32_t i = tid; i < r_len; i += THREADS) {
-            uint2 x = ld_row<CG>(R, r_off + i);
+            const uint2 x = ld_elem<CG>(R, r_off + i);
             t.key[i] = x.x;
             t.pay[i] = x.y;
         }
@@ -180,7 +192,7 @@ __device__ void build_table(Table &t, const Row *__restrict__ R, uint64_t r_off,
         for (uint32_t i = tid; i <= Nb; i += THREADS) cnt[i] = 0;
         __syncthreads();
         for (uint32_t i = tid; i < r_len; i += THREADS)
-            atomicAdd(&cnt[t.bucket(ld_row<CG>(R, r_off + i).x)], 1u);
+            atomicAdd(&cnt[t.bucket(ld_elem<CG>(R, r_off + i).x)], 1u);
         __syncthreads();
         // exclusive scan of cnt[0..Nb) in place, cnt[Nb] = r_len
         const uint32_t per = (Nb + THREADS - 1) / THREADS;
@@ -198,10 +210,10 @@ __device__ void build_table(Table &t, const Row *__restrict__ R, uint64_t r_off,
         if (tid == 0) cnt[Nb] = r_len;
         __syncthreads();
         for (uint32_t i = tid; i < r_len; i += THREADS) {
-            uint2 x = ld_row<CG>(R, r_off + i);
+            const uint2 x = ld_elem<CG>(R, r_off + i);
             uint32_t pos = atomicAdd(&cur[t.bucket(x.x)], 1u);
             t.key[pos] = x.x;
-            if (t.pay) t.pay[pos] = x.y;  // counting tables keep keys only
+            if (ROWS && t.pay) t.pay[pos] = x.y;  // counting tables keep keys only
         }
         __syncthreads();
     }
@@ -257,9 +269,43 @@ __device__ __forceinline__ unsigned long long stream_sum(const Row *s, uint64_t 
     return local;
 }
 
+// Sum of fn(key) over the bare keys [0, len) of s (any alignment), this
+// thread's share: 16-byte loads, two in flight while two are looked up.
+template <int THREADS, bool CG = false, class Fn>
+__device__ __forceinline__ unsigned long long stream_sum(const uint32_t *s, uint64_t len, Fn fn) {
+    unsigned long long local = 0;
+    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(s) & 15) / 4;
+    const uint32_t head = mis ? (uint32_t)umin64(4 - mis, len) : 0u;
+    const uint64_t nv = (len - head) / 4;
+    const uint32_t tail = (uint32_t)(len - head) & 3;
+    const uint4 *v = reinterpret_cast<const uint4 *>(s + head);
+    const uint32_t tid = threadIdx.x;
+    if (tid < head) local += fn(ld_key<CG>(s, tid));
+    if (tid < tail) local += fn(ld_key<CG>(s, len - 1 - tid));
+    auto four = [&](const uint4 &x) { local += fn(x.x) + fn(x.y) + fn(x.z) + fn(x.w); };
+    uint64_t i = tid;
+    if (i + THREADS < nv) {
+        uint4 n0 = ld_pair<CG>(v + i), n1 = ld_pair<CG>(v + i + THREADS);
+        for (;;) {
+            const uint4 x0 = n0, x1 = n1;
+            i += 2 * THREADS;
+            const bool more = i + THREADS < nv;
+            if (more) {
+                n0 = ld_pair<CG>(v + i);
+                n1 = ld_pair<CG>(v + i + THREADS);
+            }
+            four(x0);
+            four(x1);
+            if (!more) break;
+        }
+    }
+    for (; i < nv; i += THREADS) four(ld_pair<CG>(v + i));
+    return local;
+}
+
 // Matches of S rows [0, len) against the table, this thread's share.
-template <int THREADS, bool CG = false, class T = Table>
-__device__ __forceinline__ unsigned long long probe_count(const T &t, const Row *s, uint64_t len) {
+template <int THREADS, bool CG = false, class T = Table, class E = Row>
+__device__ __forceinline__ unsigned long long probe_count(const T &t, const E *s, uint64_t len) {
     return stream_sum<THREADS, CG>(s, len, [&](uint32_t k) { return t.count(k); });
 }
 

@@ -73,40 +73,34 @@ __device__ __forceinline__ uint32_t rank_warp(uint32_t *cnt, uint32_t d, bool va
 // ---------------------------------------------------------------------------
 // tile scatter shared by both passes
 // ---------------------------------------------------------------------------
+// The elements of a pass: rows, or (counting joins, which need no payloads)
+// bare keys.  A pass may read rows and write keys.
+__device__ __forceinline__ uint32_t part_key(const Row &r) { return r.key; }
+__device__ __forceinline__ uint32_t part_key(uint32_t k) { return k; }
+__device__ __forceinline__ void part_conv(const Row &r, Row &o) { o = r; }
+__device__ __forceinline__ void part_conv(const Row &r, uint32_t &o) { o = r.key; }
+__device__ __forceinline__ void part_conv(uint32_t k, uint32_t &o) { o = k; }
+
 // Tile buffers per CTA (the default): tile q is loaded and ranked while tile
 // q - 1 is written out and tile q + 1 is being copied in.
 constexpr int PART_NBUF = 3;
 
-// Write-out of a staged tile by bulk stores: every digit run is staged with
-// its shared-memory start in the same 16-byte phase as its global
-// destination (one spare slot per digit), and one thread per digit stores
-// the run's aligned body with one cp.async.bulk store, its edge rows (at most
-// one at each end) with plain stores.  The per-row shared loads and global
-// stores of the write-out leave the SM's load/store pipe.  An output that
-// is not 16-byte aligned takes plain stores for every row.
-#ifndef TBG_BULK_STORE
-#define TBG_BULK_STORE 0
-#endif
-constexpr bool PART_BULK = TBG_BULK_STORE != 0;
 // A third barrier at the end of every tile (the layout before the tile loop
 // was shown not to need it; kept as a build option for A/B timing).
 #ifndef TBG_TILE_END_BARRIER
 #define TBG_TILE_END_BARRIER 0
 #endif
-constexpr int PART_PAD = PART_BULK ? SCATTER_FMAX : 0;  // spare slots per staged tile
 
-template <int THREADS, int NBUF = PART_NBUF>
+template <int THREADS, int NBUF = PART_NBUF, class In_ = Row, int ITEMS_ = PART_ITEMS>
 struct PartSmem {
-    static constexpr int NW = THREADS / 32;
-    static constexpr int T = THREADS * PART_ITEMS;
-    Row buf[NBUF][T + 2 + PART_PAD];            // input tiles (bulk copies), each then staged digit-sorted in place
+    using In = In_;
+    static constexpr int NB = NBUF, ITEMS = ITEMS_;
+    static constexpr int T = THREADS * ITEMS;
+    static constexpr int VEC = 16 / sizeof(In);           // elements per 16 bytes
+    In buf[NBUF][T + (2 * (VEC - 1) + VEC - 1) / VEC * VEC];  // input tiles (bulk copies), each then staged digit-sorted in place
     alignas(16) uint32_t cnt[2][SCATTER_FMAX];  // per-digit counts, then tile offsets, of the two newest tiles
     alignas(16) uint32_t delta[2][SCATTER_FMAX];  // output row - tile slot per digit, of the two newest tiles
     alignas(16) uint32_t cursor[SCATTER_FMAX];  // next output row of each digit
-    // bulk write-out: each digit's staged start and row count, of the two newest tiles
-    alignas(16) uint32_t rstart[PART_BULK ? 2 : 1][PART_BULK ? SCATTER_FMAX : 4];
-    alignas(16) uint32_t rcount[PART_BULK ? 2 : 1][PART_BULK ? SCATTER_FMAX : 4];
-    uint64_t scan[NW + 1];
     uint64_t mbar[NBUF];
 };
 
@@ -125,84 +119,92 @@ struct ShardOp {
     }
 };
 
-// Where tile rows [t, t + cnt) of an n-row array sit in a shared buffer:
-// the bulk copy moves rows [t + c_lo, t + c_hi), a 16-byte aligned span;
-// row r (relative to t) is at buffer index r + off, so the copy's
-// destination is 16-byte aligned too.  When the tile starts or ends 8 bytes
-// past a 16-byte boundary, the copy takes the neighbouring row of the array
-// as well, so the whole tile arrives by the bulk copy; only at the array's
-// own ends, where no neighbour exists, is an edge row left out of the copy
-// (tile rows outside [a_lo, a_hi)) and read from global memory.
+// Where tile elements [t, t + cnt) of an n-element array sit in a shared
+// buffer: the bulk copy moves elements [t + c_lo, t + c_hi), a 16-byte aligned
+// span; element r (relative to t) is at buffer index r + off, so the copy's
+// destination is 16-byte aligned too.  When the tile starts or ends off a
+// 16-byte boundary, the copy takes the neighbouring elements of the array as
+// well, so the whole tile arrives by the bulk copy; only at the array's own
+// ends, where there are not enough neighbours, are edge elements left out of
+// the copy (those outside [a_lo, a_hi)) and read from global memory.
 struct TileGeo {
     uint64_t t;
     uint32_t cnt, a_lo, a_hi, off;
     int32_t c_lo, c_hi;
 };
 
-__device__ __forceinline__ TileGeo tile_geo(const Row *in, uint64_t t, uint32_t cnt, uint64_t n) {
+template <class In>
+__device__ __forceinline__ TileGeo tile_geo(const In *in, uint64_t t, uint32_t cnt, uint64_t n) {
+    constexpr uint32_t VEC = 16 / sizeof(In);
     TileGeo g;
     g.t = t;
     g.cnt = cnt;
     const uintptr_t addr = reinterpret_cast<uintptr_t>(in + t);
-    const bool lo_mis = (addr & 15) != 0;
-    const bool hi_mis = ((addr + (uintptr_t)cnt * 8) & 15) != 0;
-    g.c_lo = lo_mis ? (t >= 1 ? -1 : 1) : 0;
-    g.c_hi = hi_mis ? (t + cnt < n ? (int32_t)cnt + 1 : (int32_t)cnt - 1) : (int32_t)cnt;
-    if (g.c_hi < g.c_lo) g.c_hi = g.c_lo;  // a single row at an array end: no copy
-    g.off = lo_mis ? 1u : 0u;
+    if constexpr (VEC == 2) {
+        const bool lo_mis = (addr & 15) != 0;
+        const bool hi_mis = ((addr + (uintptr_t)cnt * 8) & 15) != 0;
+        g.c_lo = lo_mis ? (t >= 1 ? -1 : 1) : 0;
+        g.c_hi = hi_mis ? (t + cnt < n ? (int32_t)cnt + 1 : (int32_t)cnt - 1) : (int32_t)cnt;
+        g.off = lo_mis ? 1u : 0u;
+    } else {
+        const uint32_t lo_mis = (uint32_t)(addr & 15) / sizeof(In);
+        const uint32_t hi_mis = (uint32_t)((addr + (uintptr_t)cnt * sizeof(In)) & 15) / sizeof(In);
+        g.c_lo = lo_mis ? (t >= lo_mis ? -(int32_t)lo_mis : (int32_t)(VEC - lo_mis)) : 0;
+        g.c_hi = hi_mis ? (t + cnt + (VEC - hi_mis) <= n ? (int32_t)(cnt + VEC - hi_mis) : (int32_t)cnt - (int32_t)hi_mis)
+                        : (int32_t)cnt;
+        g.off = lo_mis;
+    }
+    if (g.c_hi < g.c_lo) g.c_hi = g.c_lo;  // a few elements at an array end: no copy
     g.a_lo = (uint32_t)max(g.c_lo, 0);
-    g.a_hi = (uint32_t)min(g.c_hi, (int32_t)cnt);
+    g.a_hi = (uint32_t)(VEC == 2 ? min(g.c_hi, (int32_t)cnt) : max(min(g.c_hi, (int32_t)cnt), 0));  // pairs: c_hi >= 0
     if (g.a_hi < g.a_lo) g.a_hi = g.a_lo;
     return g;
 }
 
-__device__ __forceinline__ void issue_tile(const Row *in, const TileGeo &g, Row *buf, uint64_t *bar) {
-    const uint32_t bytes = (uint32_t)(g.c_hi - g.c_lo) * 8;
+template <class In>
+__device__ __forceinline__ void issue_tile(const In *in, const TileGeo &g, In *buf, uint64_t *bar) {
+    const uint32_t bytes = (uint32_t)(g.c_hi - g.c_lo) * (uint32_t)sizeof(In);
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(bar, bytes);
     if (bytes) bulk_g2s(buf + g.c_lo + (int32_t)g.off, in + (int64_t)g.t + g.c_lo, bytes, bar);
 }
 
-// A tile's rows are read from its landed buffer and ranked on one shared
+// A tile's elements are read from its landed buffer and ranked on one shared
 // counter per digit (order inside a digit is free: partitions are
 // multisets); one warp prefixes the counts over digits while the other warps
 // write out the previous tile; then the tile is staged digit-sorted into its
 // own buffer, to be written out in slot order (consecutive threads store
-// consecutive rows of each digit's run) during the next tile's prefix.
+// consecutive elements of each digit's run) during the next tile's prefix.
 //
 // Tile q (the CTA's running tile count, continued across ranges so a
 // persistent CTA never re-initialises its barriers) uses buffer q % NB with
 // barrier mbar[q % NB] at phase parity (q / NB) & 1, and counters and deltas
 // q & 1.
 
-// Waits for tile q and ranks its rows on cnt[q & 1].
-template <int THREADS, bool FULL, class Dig, int NB>
-__device__ __forceinline__ void tile_load_rank(const Row *__restrict__ in, const TileGeo &g, uint32_t q, Dig dop,
-                                               PartSmem<THREADS, NB> &sm, uint64_t *mbar, uint2 (&v)[PART_ITEMS],
-                                               uint32_t (&rank)[PART_ITEMS], unsigned *err) {
+// Waits for tile q and ranks its elements on cnt[q & 1].
+template <bool FULL, class Out, class Dig, class Smem>
+__device__ __forceinline__ void tile_load_rank(const typename Smem::In *__restrict__ in, const TileGeo &g, uint32_t q,
+                                               Dig dop, Smem &sm, uint64_t *mbar, Out (&v)[Smem::ITEMS],
+                                               uint32_t (&rank)[Smem::ITEMS], unsigned *err) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t wbase = (uint32_t)w * 32 * PART_ITEMS;
+    const uint32_t wbase = (uint32_t)w * 32 * Smem::ITEMS;
     const uint32_t cnt = g.cnt;
-    const int b = q % NB;
-    if (!mbar_wait(&mbar[b], (q / NB) & 1, SPIN_LIMIT * 16)) atomicCAS(err, 0u, (unsigned)TBG_ERR_TIMEOUT);
+    const int b = q % Smem::NB;
+    if (!mbar_wait(&mbar[b], (q / Smem::NB) & 1, SPIN_LIMIT * 16)) atomicCAS(err, 0u, (unsigned)TBG_ERR_TIMEOUT);
 #pragma unroll
-    for (int i = 0; i < PART_ITEMS; i++) {
+    for (int i = 0; i < Smem::ITEMS; i++) {
         const uint32_t r = wbase + i * 32 + lane;
         if (FULL || r < cnt) {
-            if (r >= g.a_lo && r < g.a_hi) {
-                const Row x = sm.buf[b][r + g.off];
-                v[i] = make_uint2(x.key, x.payload);
-            } else {
-                v[i] = reinterpret_cast<const uint2 *>(in)[g.t + r];
-            }
+            if (r >= g.a_lo && r < g.a_hi) part_conv(sm.buf[b][r + g.off], v[i]);
+            else part_conv(in[g.t + r], v[i]);
         }
     }
     uint32_t *c = sm.cnt[q & 1];
-    const bool dup = warp_has_dups(dop(v[0].x), FULL || wbase + lane < cnt);
+    const bool dup = warp_has_dups(dop(part_key(v[0])), FULL || wbase + lane < cnt);
 #pragma unroll
-    for (int i = 0; i < PART_ITEMS; i++) {
+    for (int i = 0; i < Smem::ITEMS; i++) {
         const bool valid = FULL || wbase + i * 32 + lane < cnt;
-        rank[i] = rank_warp(c, valid ? dop(v[i].x) : 0, valid, dup);
+        rank[i] = rank_warp(c, valid ? dop(part_key(v[i])) : 0, valid, dup);
     }
 }
 
@@ -212,11 +214,10 @@ __device__ __forceinline__ void tile_load_rank(const Row *__restrict__ in, const
 // warp of the write-out that spans a run boundary reads its deltas from
 // different banks.  Lane l owns the 8 consecutive digits [8l, 8l + 8) and
 // moves them with 16-byte accesses (conflict-free).  Every counter of all
-// SCATTER_FMAX digits is kept at zero outside the F digits in use, so those
+// SCATTER_FMAX digits is kept at zero outside the digits in use, so those
 // add nothing.
-template <int THREADS, int NB>
-__device__ __forceinline__ void tile_scan(uint32_t q, int F, PartSmem<THREADS, NB> &sm) {
-    (void)F;
+template <class Smem>
+__device__ __forceinline__ void tile_scan(uint32_t q, Smem &sm) {
     const int lane = threadIdx.x & 31;
     constexpr int PER = SCATTER_FMAX / 32;
     static_assert(PER == 8, "two 16-byte words of counters per lane");
@@ -229,7 +230,6 @@ __device__ __forceinline__ void tile_scan(uint32_t q, int F, PartSmem<THREADS, N
     uint32_t sum = 0;
 #pragma unroll
     for (int i = 0; i < PER; i++) sum += x[i];
-    if (PART_BULK) sum += PER;  // the lane's digits take one spare slot each
     uint32_t inc = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -242,24 +242,10 @@ __device__ __forceinline__ void tile_scan(uint32_t q, int F, PartSmem<THREADS, N
     uint32_t off[PER], dl[PER];
 #pragma unroll
     for (int i = 0; i < PER; i++) {
-        if (PART_BULK) {
-            // one spare slot per digit: the run starts in its destination's 16-byte phase
-            off[i] = run + ((run ^ cur[i]) & 1u);
-            run += x[i] + 1;
-        } else {
-            off[i] = run;
-            run += x[i];
-        }
+        off[i] = run;
+        run += x[i];
         dl[i] = cur[i] - off[i];
         cur[i] += x[i];
-    }
-    if (PART_BULK) {
-        uint4 *s4 = reinterpret_cast<uint4 *>(sm.rstart[q & 1]) + 2 * lane;
-        uint4 *r4 = reinterpret_cast<uint4 *>(sm.rcount[q & 1]) + 2 * lane;
-        s4[0] = make_uint4(off[0], off[1], off[2], off[3]);
-        s4[1] = make_uint4(off[4], off[5], off[6], off[7]);
-        r4[0] = make_uint4(x[0], x[1], x[2], x[3]);
-        r4[1] = make_uint4(x[4], x[5], x[6], x[7]);
     }
     c4[0] = make_uint4(off[0], off[1], off[2], off[3]);
     c4[1] = make_uint4(off[4], off[5], off[6], off[7]);
@@ -271,97 +257,53 @@ __device__ __forceinline__ void tile_scan(uint32_t q, int F, PartSmem<THREADS, N
     n4[1] = make_uint4(0, 0, 0, 0);
 }
 
-// Stages tile q's rows digit-sorted into its own buffer.
-template <int THREADS, bool FULL, class Dig, int NB>
-__device__ __forceinline__ void tile_stage(const TileGeo &g, uint32_t q, Dig dop, PartSmem<THREADS, NB> &sm,
-                                           const uint2 (&v)[PART_ITEMS], const uint32_t (&rank)[PART_ITEMS]) {
+// Stages tile q's elements digit-sorted into its own buffer.
+template <bool FULL, class Out, class Dig, class Smem>
+__device__ __forceinline__ void tile_stage(const TileGeo &g, uint32_t q, Dig dop, Smem &sm, const Out (&v)[Smem::ITEMS],
+                                           const uint32_t (&rank)[Smem::ITEMS]) {
+    static_assert(sizeof(Out) <= sizeof(typename Smem::In), "staged in place");
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t wbase = (uint32_t)w * 32 * PART_ITEMS;
+    const uint32_t wbase = (uint32_t)w * 32 * Smem::ITEMS;
     const uint32_t *c = sm.cnt[q & 1];
-    Row *buf = sm.buf[q % NB];
+    Out *buf = reinterpret_cast<Out *>(sm.buf[q % Smem::NB]);
 #pragma unroll
-    for (int i = 0; i < PART_ITEMS; i++) {
-        if (FULL || wbase + i * 32 + lane < g.cnt) {
-            const uint32_t j = c[dop(v[i].x)] + rank[i];
-            buf[j] = Row{v[i].x, v[i].y};
-        }
-    }
-    if (PART_BULK) fence_proxy_async_smem();  // the staged rows become visible to the bulk stores
+    for (int i = 0; i < Smem::ITEMS; i++)
+        if (FULL || wbase + i * 32 + lane < g.cnt) buf[c[dop(part_key(v[i]))] + rank[i]] = v[i];
 }
 
-// Writes staged tile q (cnt rows) to out, by threads [t0, THREADS).
-template <int THREADS, class Dig, int NB>
-__device__ __forceinline__ void tile_write(uint32_t q, uint32_t cnt, uint2 *__restrict__ out, uint32_t out_n,
-                                           Dig dop, PartSmem<THREADS, NB> &sm, int t0, unsigned *err) {
+// Writes staged tile q (cnt elements) to out, by threads [t0, THREADS).
+template <int THREADS, class Out, class Dig, class Smem>
+__device__ __forceinline__ void tile_write(uint32_t q, uint32_t cnt, Out *__restrict__ out, uint32_t out_n, Dig dop,
+                                           Smem &sm, int t0, unsigned *err) {
     if ((int)threadIdx.x < t0) return;
-    if (PART_BULK) {
-        (void)cnt;
-        (void)dop;
-        const Row *buf = sm.buf[q % NB];
-        const uint32_t *dl = sm.delta[q & 1];
-        const uint32_t *rs = sm.rstart[q & 1], *rc = sm.rcount[q & 1];
-        const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-        bool issued = false;
-        for (int d = (int)threadIdx.x - t0; d < SCATTER_FMAX; d += THREADS - t0) {
-            uint32_t n = rc[d];
-            if (!n) continue;
-            uint32_t s = rs[d];
-            uint32_t gpos = dl[d] + s;
-            if ((uint64_t)gpos + n > out_n) {
-                atomicCAS(err, 0u, (unsigned)TBG_ERR_ARG);
-                continue;
-            }
-            if (!aligned) {
-                for (uint32_t r = 0; r < n; r++) out[gpos + r] = make_uint2(buf[s + r].key, buf[s + r].payload);
-                continue;
-            }
-            if (gpos & 1) {  // head row up to the 16-byte boundary (the staged start shares the phase)
-                out[gpos] = make_uint2(buf[s].key, buf[s].payload);
-                s++;
-                gpos++;
-                n--;
-            }
-            const uint32_t body = n & ~1u;
-            if (body) {
-                bulk_s2g(out + gpos, buf + s, body * 8);
-                issued = true;
-            }
-            if (n & 1) out[gpos + body] = make_uint2(buf[s + body].key, buf[s + body].payload);
-        }
-        if (issued) {
-            bulk_commit();
-            bulk_wait_read();  // the buffer is reloaded after the next barrier
-        }
-        return;
-    }
-    const Row *buf = sm.buf[q % NB];
+    const Out *buf = reinterpret_cast<const Out *>(sm.buf[q % Smem::NB]);
     const uint32_t *dl = sm.delta[q & 1];
 #pragma unroll 4
     for (uint32_t j = threadIdx.x - t0; j < cnt; j += THREADS - t0) {
-        const Row x = buf[j];
-        const uint32_t pos = dl[dop(x.key)] + j;
-        if (pos < out_n) out[pos] = make_uint2(x.key, x.payload);
+        const Out x = buf[j];
+        const uint32_t pos = dl[dop(part_key(x))] + j;
+        if (pos < out_n) out[pos] = x;
         else atomicCAS(err, 0u, (unsigned)TBG_ERR_ARG);
     }
 }
 
-__device__ __forceinline__ TileGeo range_tile(const Row *in, uint64_t lo, uint64_t hi, uint64_t n, int k,
-                                             uint32_t T) {
+template <class In>
+__device__ __forceinline__ TileGeo range_tile(const In *in, uint64_t lo, uint64_t hi, uint64_t n, int k, uint32_t T) {
     const uint64_t t = lo + (uint64_t)k * T;
     return tile_geo(in, t, (uint32_t)umin64(T, hi - t), n);
 }
 
-// Scatters rows [lo, hi) of `in` (in_n rows), digit by digit, to out[sm.cursor[d]...];
-// the caller initialises sm.cursor[0..F) and synchronises.  Two barriers
-// per tile; the bulk copies run NB - 1 tiles ahead.  `kseq` is the CTA's
-// running tile count (see above), and the barriers mbar[0..NB) are
-// initialised once by the caller.
-template <int THREADS, class Dig, int NB>
-__device__ void part_tiles(const Row *__restrict__ in, uint64_t lo, uint64_t hi, uint64_t in_n,
-                           Row *__restrict__ out, uint32_t out_n, Dig dop, int F, PartSmem<THREADS, NB> &sm,
-                           uint64_t *mbar, uint32_t &kseq, unsigned *err) {
-    constexpr uint32_t T = THREADS * PART_ITEMS;
-    uint2 *o = reinterpret_cast<uint2 *>(out);
+// Scatters elements [lo, hi) of `in` (in_n elements), digit by digit, to
+// out[sm.cursor[d]...]; the caller initialises sm.cursor[0..F) and
+// synchronises.  Two barriers per tile; the bulk copies run NB - 1 tiles
+// ahead.  `kseq` is the CTA's running tile count (see above), and the barriers
+// mbar[0..NB) are initialised once by the caller.
+template <int THREADS, class Out, class Dig, class Smem>
+__device__ void part_tiles(const typename Smem::In *__restrict__ in, uint64_t lo, uint64_t hi, uint64_t in_n,
+                           Out *__restrict__ out, uint32_t out_n, Dig dop, Smem &sm, uint64_t *mbar, uint32_t &kseq,
+                           unsigned *err) {
+    constexpr uint32_t T = Smem::T;
+    constexpr int NB = Smem::NB;
     const int ntiles = (int)((hi - lo + T - 1) / T);
     for (int i = threadIdx.x; i < SCATTER_FMAX; i += THREADS) sm.cnt[kseq & 1][i] = 0;
     __syncthreads();
@@ -373,20 +315,20 @@ __device__ void part_tiles(const Row *__restrict__ in, uint64_t lo, uint64_t hi,
     for (int k = 0; k < ntiles; k++) {
         const uint32_t q = kseq + k;
         const TileGeo g = range_tile(in, lo, hi, in_n, k, T);
-        uint2 v[PART_ITEMS];
-        uint32_t rank[PART_ITEMS];
-        if (g.cnt == T) tile_load_rank<THREADS, true, Dig>(in, g, q, dop, sm, mbar, v, rank, err);
-        else tile_load_rank<THREADS, false, Dig>(in, g, q, dop, sm, mbar, v, rank, err);
+        Out v[Smem::ITEMS];
+        uint32_t rank[Smem::ITEMS];
+        if (g.cnt == T) tile_load_rank<true, Out>(in, g, q, dop, sm, mbar, v, rank, err);
+        else tile_load_rank<false, Out>(in, g, q, dop, sm, mbar, v, rank, err);
         __syncthreads();
-        if (threadIdx.x < 32) tile_scan<THREADS>(q, F, sm);
-        else if (k > 0) tile_write<THREADS, Dig>(q - 1, prev_cnt, o, out_n, dop, sm, 32, err);
+        if (threadIdx.x < 32) tile_scan(q, sm);
+        else if (k > 0) tile_write<THREADS, Out>(q - 1, prev_cnt, out, out_n, dop, sm, 32, err);
         __syncthreads();
         // tile q - 1's buffer is free: copy tile k + NB - 1 into it
         if (threadIdx.x == 0 && k + NB - 1 < ntiles)
             issue_tile(in, range_tile(in, lo, hi, in_n, k + NB - 1, T), sm.buf[(q + NB - 1) % NB],
                        &mbar[(q + NB - 1) % NB]);
-        if (g.cnt == T) tile_stage<THREADS, true, Dig>(g, q, dop, sm, v, rank);
-        else tile_stage<THREADS, false, Dig>(g, q, dop, sm, v, rank);
+        if (g.cnt == T) tile_stage<true, Out>(g, q, dop, sm, v, rank);
+        else tile_stage<false, Out>(g, q, dop, sm, v, rank);
         // No barrier here: tile q + 1's load and ranking touch neither tile
         // q's buffer nor its counters, and the next iteration's first barrier
         // orders this staging before tile q's write-out and before the scan
@@ -395,23 +337,21 @@ __device__ void part_tiles(const Row *__restrict__ in, uint64_t lo, uint64_t hi,
         prev_cnt = g.cnt;
     }
     __syncthreads();  // the last tile is staged
-    tile_write<THREADS, Dig>(kseq + ntiles - 1, prev_cnt, o, out_n, dop, sm, 0, err);
-    if (PART_BULK) bulk_wait_all();  // this thread's bulk stores have landed
+    tile_write<THREADS, Out>(kseq + ntiles - 1, prev_cnt, out, out_n, dop, sm, 0, err);
     __syncthreads();  // every buffer is free again
     kseq += ntiles;
 }
 
 // One range per CTA: initialises the barriers held in `sm`.
-template <int THREADS, class Dig, int NB>
-__device__ void part_range(const Row *__restrict__ in, uint64_t lo, uint64_t hi, uint64_t in_n,
-                           Row *__restrict__ out, uint32_t out_n, Dig dop, int F, PartSmem<THREADS, NB> &sm,
-                           unsigned *err) {
+template <int THREADS, class Out, class Dig, class Smem>
+__device__ void part_range(const typename Smem::In *__restrict__ in, uint64_t lo, uint64_t hi, uint64_t in_n,
+                           Out *__restrict__ out, uint32_t out_n, Dig dop, Smem &sm, unsigned *err) {
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NB; i++) mbar_init(&sm.mbar[i], 1);
+        for (int i = 0; i < Smem::NB; i++) mbar_init(&sm.mbar[i], 1);
         fence_mbar_init();
     }
     uint32_t kseq = 0;
-    part_tiles<THREADS, Dig>(in, lo, hi, in_n, out, out_n, dop, F, sm, sm.mbar, kseq, err);
+    part_tiles<THREADS, Out>(in, lo, hi, in_n, out, out_n, dop, sm, sm.mbar, kseq, err);
 }
 
 }  // namespace tbg

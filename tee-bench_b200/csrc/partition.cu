@@ -39,8 +39,8 @@ constexpr int PASS2_THREADS = TBG_PASS2_THREADS;
 #define TBG_PASS_NBUF 3
 #endif
 constexpr int PASS_NBUF = TBG_PASS_NBUF;
-template <int THREADS>
-using PassSmem = PartSmem<THREADS, PASS_NBUF>;
+template <int THREADS, class In = Row>
+using PassSmem = PartSmem<THREADS, PASS_NBUF, In, sizeof(In) == 8 ? PART_ITEMS : PART_KEY_ITEMS>;
 
 // ---------------------------------------------------------------------------
 // K1 per-chunk histogram over the final partition index f
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_plan(PlanArgs a) {
 // Both passes take up to two relations (the second one null for one): S's
 // CTAs come first, and R's, fewer and shorter, fill the last wave.
 // ---------------------------------------------------------------------------
-template <int THREADS>
+template <int THREADS, class Out>
 __device__ __forceinline__ void part_pass1(const PartArgs &a, const int c) {
     if (a.skip && *a.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -415,17 +415,18 @@ __device__ __forceinline__ void part_pass1(const PartArgs &a, const int c) {
     __syncthreads();
     const uint64_t lo = (uint64_t)c * a.chunk;
     const uint64_t hi = a.chunk_len ? lo + a.chunk_len[c] : umin64(a.n, lo + a.chunk);
-    part_range<THREADS>(a.in, lo, hi, a.n, a.out, (uint32_t)a.n, a.d1, F, sm, a.err);
+    part_range<THREADS, Out>(static_cast<const Row *>(a.in), lo, hi, a.n, static_cast<Out *>(a.out), (uint32_t)a.n, a.d1,
+                             sm, a.err);
 }
 
 // ---------------------------------------------------------------------------
 // K5 pass 2: unit (c, s), s-major, scatters by d2 within pass-1 partition s.
 // ---------------------------------------------------------------------------
-template <int THREADS>
+template <int THREADS, class E>
 __device__ __forceinline__ void part_pass2(const PartArgs &a, const unsigned unit) {
     if (a.skip && *a.skip) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    auto &sm = *reinterpret_cast<PassSmem<THREADS> *>(smem_raw);
+    auto &sm = *reinterpret_cast<PassSmem<THREADS, E> *>(smem_raw);
     const int F1 = 1 << a.b1, F2 = 1 << a.b2;
     const int P = F1 * F2;
     const int ngroups = (a.G + a.group - 1) / a.group;
@@ -441,29 +442,31 @@ __device__ __forceinline__ void part_pass2(const PartArgs &a, const unsigned uni
         sm.cursor[d] = (uint32_t)a.base[f] + a.pre[(uint64_t)c0 * P + f];
     }
     __syncthreads();
-    part_range<THREADS>(a.in, lo, hi, a.n, a.out, (uint32_t)a.n, a.d2, F2, sm, a.err);
+    part_range<THREADS, E>(static_cast<const E *>(a.in), lo, hi, a.n, static_cast<E *>(a.out), (uint32_t)a.n, a.d2, sm,
+                           a.err);
 }
 
 // The two relations of a launch take two copies of the pass in the code:
 // reading the arguments through one selected pointer costs registers that the
 // pass does not have (64 of 64 in use; with it the passes ran 5% slower).
-template <int THREADS>
+// E: what the partitions hold, rows or bare keys.
+template <int THREADS, class E>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     k_part_pass1(const __grid_constant__ PartArgs a, const __grid_constant__ PartArgs b) {
     dep_wait();
     dep_trigger();
-    if (blockIdx.x < (unsigned)a.G) part_pass1<THREADS>(a, blockIdx.x);
-    else part_pass1<THREADS>(b, blockIdx.x - a.G);
+    if (blockIdx.x < (unsigned)a.G) part_pass1<THREADS, E>(a, blockIdx.x);
+    else part_pass1<THREADS, E>(b, blockIdx.x - a.G);
 }
 
-template <int THREADS>
+template <int THREADS, class E>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     k_part_pass2(const __grid_constant__ PartArgs a, const __grid_constant__ PartArgs b) {
     dep_wait();
     dep_trigger();
     const unsigned units = (unsigned)((a.G + a.group - 1) / a.group) << a.b1;
-    if (blockIdx.x < units) part_pass2<THREADS>(a, blockIdx.x);
-    else part_pass2<THREADS>(b, blockIdx.x - units);
+    if (blockIdx.x < units) part_pass2<THREADS, E>(a, blockIdx.x);
+    else part_pass2<THREADS, E>(b, blockIdx.x - units);
 }
 
 // ---------------------------------------------------------------------------
@@ -512,20 +515,22 @@ cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st) {
 cudaError_t launch_part_pass1(const PartArgs &a, const PartArgs *b, cudaStream_t st) {
     constexpr int T = PASS1_THREADS;
     const size_t smem = sizeof(PassSmem<T>);
-    cudaError_t e = smem_limit((const void *)k_part_pass1<T>, smem);
+    auto kern = a.keys ? k_part_pass1<T, uint32_t> : k_part_pass1<T, Row>;
+    cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    e = launch_dep(k_part_pass1<T>, a.G + (b ? b->G : 0), T, smem, st, a, b ? *b : a);
+    e = launch_dep(kern, a.G + (b ? b->G : 0), T, smem, st, a, b ? *b : a);
     count_launch();
     return e;
 }
 
 cudaError_t launch_part_pass2(const PartArgs &a, const PartArgs *b, cudaStream_t st) {
     constexpr int T = PASS2_THREADS;
-    const size_t smem = sizeof(PassSmem<T>);
-    cudaError_t e = smem_limit((const void *)k_part_pass2<T>, smem);
+    const size_t smem = a.keys ? sizeof(PassSmem<T, uint32_t>) : sizeof(PassSmem<T>);
+    auto kern = a.keys ? k_part_pass2<T, uint32_t> : k_part_pass2<T, Row>;
+    cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     auto units = [](const PartArgs &p) { return (uint64_t)((p.G + p.group - 1) / p.group) << p.b1; };
-    e = launch_dep(k_part_pass2<T>, (unsigned)(units(a) + (b ? units(*b) : 0)), T, smem, st, a, b ? *b : a);
+    e = launch_dep(kern, (unsigned)(units(a) + (b ? units(*b) : 0)), T, smem, st, a, b ? *b : a);
     count_launch();
     return e;
 }

@@ -174,6 +174,7 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     try_direct(g, cfg, nullptr, 0);
     g.sample_S = dS;
     g.capR = 0x7FFFFFFF;  // counters take any number of R rows
+    g.keys = true;
     g.capS = std::max<uint64_t>(65536, nS / ((uint64_t)w.nsm * 12));
     g.item_cap = 2 * (nS / g.capS + 4 * g.P) + 16;
     int rc = ensure_radix_buffers(g, false, w);

@@ -391,15 +391,15 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm(JoinArgs a) {
 // which leaves room to load the next S tile's keys into registers while the
 // current tile is merged.
 
-// Keys of rows [off, off + n) (n <= THREADS * 8): key[i] is row i * THREADS +
+// Keys [off, off + n) (n <= THREADS * 8): key[i] is key i * THREADS +
 // tid.  All loads are issued before the first use.
 template <int THREADS>
-__device__ __forceinline__ void load_keys(const Row *__restrict__ src, uint64_t off, uint32_t n, uint32_t (&key)[8]) {
-    const uint2 *v = reinterpret_cast<const uint2 *>(src) + off;
+__device__ __forceinline__ void load_keys(const uint32_t *__restrict__ src, uint64_t off, uint32_t n, uint32_t (&key)[8]) {
+    const uint32_t *v = src + off;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const uint32_t e = i * THREADS + threadIdx.x;
-        if (e < n) key[i] = __ldcs(v + e).x;
+        if (e < n) key[i] = __ldcs(v + e);
     }
 }
 
@@ -600,6 +600,7 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm_count(JoinArgs a) {
     dep_wait();
     dep_trigger();
     if (*a.skip) return;
+    const uint32_t *Rp = reinterpret_cast<const uint32_t *>(a.R), *Sp = reinterpret_cast<const uint32_t *>(a.S);
     const int tid = threadIdx.x;
     const int shift = a.hash_shift;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
@@ -620,7 +621,7 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm_count(JoinArgs a) {
             __syncthreads();  // s_item read by every thread before thread 0 rewrites it
             continue;
         }
-        load_keys<RSM_THREADS>(a.R, m.r_off, nr, key);
+        load_keys<RSM_THREADS>(Rp, m.r_off, nr, key);
         uint32_t lo = ~0u, hi = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm_count(JoinArgs a) {
             for (int i = 0; i < 8; i++)
                 if (i * RSM_THREADS + tid < nr) atomicAdd(&h[(key[i] - rmin) >> shift], 1u);
             __syncthreads();
-            local += stream_sum<RSM_THREADS>(a.S + m.s_off, m.s_len, [&](uint32_t k) {
+            local += stream_sum<RSM_THREADS>(Sp + m.s_off, m.s_len, [&](uint32_t k) {
                 const uint32_t d = k - rmin;
                 return d <= rspan ? h[d >> shift] : 0u;
             });
@@ -655,12 +656,12 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm_count(JoinArgs a) {
         __syncthreads();  // red is reused by the sort
         sort_keys<RSM_THREADS>(key, nr, Rk, tmp, bins_cnt, cnt, scan_scratch, red);
         uint32_t ns = (uint32_t)umin64(RSM_STILE, m.s_len);
-        load_keys<RSM_THREADS>(a.S, m.s_off, ns, key);
+        load_keys<RSM_THREADS>(Sp, m.s_off, ns, key);
         for (uint64_t s0 = 0; s0 < m.s_len;) {
             sort_keys<RSM_THREADS>(key, ns, Sk, tmp, bins_cnt, cnt, scan_scratch, red);
             const uint64_t s1 = s0 + ns;
             const uint32_t ns_next = (uint32_t)umin64(RSM_STILE, m.s_len - s1);
-            if (ns_next) load_keys<RSM_THREADS>(a.S, m.s_off + s1, ns_next, key);  // in flight during the merge
+            if (ns_next) load_keys<RSM_THREADS>(Sp, m.s_off + s1, ns_next, key);  // in flight during the merge
             local += merge_count<RSM_THREADS>(Rk, nr, Sk, ns);
             __syncthreads();  // Sk and tmp are rewritten by the next tile
             s0 = s1;
@@ -729,6 +730,7 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
     dep_wait();
     dep_trigger();
     if (*a.skip) return;
+    const uint32_t *Rp = reinterpret_cast<const uint32_t *>(a.R), *Sp = reinterpret_cast<const uint32_t *>(a.S);
     const int tid = threadIdx.x;
     const uint32_t bins = 1u << lowbits;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
@@ -743,7 +745,7 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
             s_item[(iter + 1) & 1] = nx;  // read by all after this item's barriers
             if (nx < nitems) {
                 const Item mn = a.items[nx];
-                prefetch_l2(a.R + mn.r_off, umin64(mn.r_len, 65536) * sizeof(Row));
+                prefetch_l2(Rp + mn.r_off, umin64(mn.r_len, 65536) * 4);
             }
         }
         const Item m = a.items[it];
@@ -751,12 +753,12 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
         for (uint32_t b = tid; b < bins / 4; b += BCOUNT_THREADS)
             reinterpret_cast<uint4 *>(h)[b] = make_uint4(0, 0, 0, 0);
         __syncthreads();
-        stream_sum<BCOUNT_THREADS>(a.R + m.r_off, m.r_len, [&](uint32_t k) {
+        stream_sum<BCOUNT_THREADS>(Rp + m.r_off, m.r_len, [&](uint32_t k) {
             if (k - lo < bins) atomicAdd(&h[k - lo], 1u);
             return 0u;
         });
         __syncthreads();
-        local += stream_sum<BCOUNT_THREADS>(a.S + m.s_off, m.s_len, [&](uint32_t k) {
+        local += stream_sum<BCOUNT_THREADS>(Sp + m.s_off, m.s_len, [&](uint32_t k) {
             const uint32_t d = k - lo;
             return (unsigned long long)(d < bins ? h[d] : 0u);  // a bucket's count may take all 32 bits
         });

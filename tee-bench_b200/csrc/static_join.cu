@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(256) k_static_plan(StaticPlan p) {
         J.chunk = STATIC_CHUNK;
         J.orig = 0;
         if (p.B) {
-            J.Rp = reinterpret_cast<Row *>(b + OFF_ROWS);
-            J.Sp = reinterpret_cast<Row *>(b + OFF_ROWS) + p.rp_rows;
+            J.Rp = reinterpret_cast<uint32_t *>(b + OFF_ROWS);
+            J.Sp = reinterpret_cast<uint32_t *>(b + OFF_ROWS) + p.rp_rows;
             J.histR = reinterpret_cast<uint32_t *>(b + OFF_HIST);
             J.histS = J.histR + (size_t)p.GR * P;
             J.baseR = reinterpret_cast<uint32_t *>(b + OFF_BASE);
@@ -195,7 +195,7 @@ extern "C" TBG_API int tbg_join_count_static(const row_t *dR, uint64_t nR, const
         p.GR = (uint32_t)((nR + STATIC_CHUNK - 1) / STATIC_CHUNK);
         p.GS = (uint32_t)((nS + STATIC_CHUNK - 1) / STATIC_CHUNK);
         p.item_cap = (1u << p.B) + (uint32_t)((nS + p.capS - 1) / p.capS);
-        p.rp_rows = (uint32_t)((nR + 31) & ~uint64_t(31));  // S copy starts 256-byte aligned
+        p.rp_rows = (uint32_t)((nR + 63) & ~uint64_t(63));  // S copy starts 256-byte aligned
         const uint64_t w = std::max<uint64_t>(1, (nR + nS) >> 18);
         p.n_jt = (uint32_t)std::min<uint64_t>(p.item_cap, w);
     }

@@ -10,8 +10,9 @@
 
 namespace tbg {
 
-// 8-byte tuple, the layout of struct row_t (uint32 key, uint32 payload).
-struct Row {
+// 8-byte tuple, the layout of struct row_t (uint32 key, uint32 payload).  Every
+// entry point requires 8-byte aligned relations, so a row moves as one word.
+struct alignas(8) Row {
     uint32_t key;
     uint32_t payload;
 };
@@ -65,6 +66,7 @@ constexpr int SCATTER_FMAX = 256;
 // Rows per thread per tile of the chunked partitioning passes.
 constexpr int PART_THREADS = 512;
 constexpr int PART_ITEMS = 8;
+constexpr int PART_KEY_ITEMS = 16;  // keys per thread per tile of a pass over bare keys
 
 // Shared-memory table capacity of the build/probe kernels (rows of R_p).
 constexpr int JOIN_THREADS = 512;
@@ -106,8 +108,9 @@ struct RelPlan {
 
 // Arguments of the chunked partitioning passes (partition.cu).
 struct PartArgs {
-    const Row *in;
-    Row *out;
+    const void *in;           // pass 1: rows; pass 2: rows or keys
+    void *out;                // rows or keys
+    int keys;                 // 1: the partitions hold bare keys (counting joins)
     uint64_t n;               // rows (< 2^32)
     uint64_t chunk;           // rows per pass-1 chunk
     const uint32_t *chunk_len;  // rows of chunk c (null: full chunks of `chunk` rows)
@@ -126,7 +129,7 @@ struct PartArgs {
 };
 
 struct JoinArgs {
-    const Row *R;
+    const Row *R;              // counting kernels: bare keys (see PartArgs)
     const Row *S;
     const Item *items;
     const unsigned int *nitems;

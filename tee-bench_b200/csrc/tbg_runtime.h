@@ -97,6 +97,7 @@ struct RadixGeom {
     bool direct_rows = false;      // ... of a materialising join: R's payloads instead of bits,
     tbg_row_out *rows = nullptr;   // ... S's read writes the rows here
     uint64_t rows_cap = 0;
+    bool keys = false;             // the partitions hold bare keys (counting joins)
     const Row *sample_S = nullptr;  // S, when it is there while R is read
 };
 RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int capR, Workspace &w);
