@@ -336,7 +336,7 @@ int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &
                                      g.sample_S, g.n[1], ctrl, st);
     } else if (g.direct && g.direct_rows && !bypass) {
         e = launch_hist_emit(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), g.rows,
-                             g.rows_cap, g.s_range_max, ctrl, st);
+                             g.rel, g.rows_cap, g.s_range_max, ctrl, st);
     } else if (g.direct && !bypass) {
         e = launch_hist_probe(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(),
                               g.n[0], w.nsm, ctrl, st);
@@ -534,6 +534,8 @@ int radix_partition(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row
     RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
     try_direct(g, cfg, d_rows, cap);
     g.sample_S = dS;
+    g.rel = run->rel;
+    run->rel_done = g.direct && g.rel;
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;
@@ -672,7 +674,7 @@ int radix_join_phase(const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap, W
 }
 
 // Reads back the control block and fills stats; waits for the stream.
-int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, const JoinRun &run,
+int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, JoinRun &run,
                 uint64_t nR, uint64_t nS, uint64_t cap, uint64_t *matches, tbg_stats *stats) {
     cudaError_t e = run.ctrl_on_host
                         ? cudaSuccess
@@ -680,6 +682,7 @@ int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, const Join
     if (e != cudaSuccess) return cuda_error(e, "readback");
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_error(e, "join");
     const Ctrl &c = *w.host_ctrl;
+    run.rel_done = run.rel_done && c.direct;
     if (matches) *matches = c.matches;
     if (stats) {
         memset(stats, 0, sizeof *stats);

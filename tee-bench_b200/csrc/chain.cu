@@ -31,22 +31,28 @@ cudaError_t launch_rows_to_relation(const tbg_row_out *rows, uint64_t n, Row *ou
     return cudaGetLastError();
 }
 
-// Materialised join R x S into w-owned rows, growing the buffer once if the
-// first guess (|S| rows) was too small.  Returns the rows and their count.
-static int join_rows(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, DevBuf &buf,
-                     cudaStream_t st, tbg_row_out **rows, uint64_t *m) {
+// R x S as a relation of (key, R payload) tuples in w.chain_rel, *m of them.  A
+// direct join writes the relation itself; any other writes rows, which are
+// converted.  The first guess of |S| rows grows once if it was too small.
+static int join_relation(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, Workspace &w,
+                         cudaStream_t st, uint64_t *m) {
     tbg_config c = cfg;
     c.materialize = 1;
     uint64_t cap = std::max<uint64_t>(nS, 1);
     for (int attempt = 0; attempt < 2; attempt++) {
-        cudaError_t e = buf.ensure(cap * sizeof(tbg_row_out));
+        cudaError_t e = w.chain_rows.ensure(cap * sizeof(tbg_row_out));
+        if (e == cudaSuccess) e = w.chain_rel.ensure(cap * sizeof(Row));
         if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (chain rows)");
-        const int rc = tbg_join_device(&c, reinterpret_cast<const row_t *>(dR), nR,
-                                       reinterpret_cast<const row_t *>(dS), nS, buf.as<tbg_row_out>(), cap, m,
-                                       nullptr, st);
+        JoinRun run;
+        run.waits = true;
+        run.rel = w.chain_rel.as<Row>();
+        Workspace *jw = nullptr;
+        int rc = join_device_impl(&c, dR, nR, dS, nS, w.chain_rows.as<tbg_row_out>(), cap, st, &run, &jw);
+        if (rc == TBG_OK) rc = finish_join(c, *jw, st, run, nR, nS, cap, m, nullptr);
         if (rc == TBG_OK) {
-            *rows = buf.as<tbg_row_out>();
-            return TBG_OK;
+            if (run.rel_done) return TBG_OK;
+            e = launch_rows_to_relation(w.chain_rows.as<tbg_row_out>(), *m, w.chain_rel.as<Row>(), w.nsm, st);
+            return e == cudaSuccess ? TBG_OK : cuda_error(e, "to_relation");
         }
         if (rc != TBG_ERR_CAPACITY) return rc;
         cap = std::max<uint64_t>(*m, 1);  // exact count is known now
@@ -80,18 +86,11 @@ TBG_API int tbg_join_three_way(const tbg_config *cfg, const row_t *dR, uint64_t 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Workspace *w = workspace_for(st);
     if (!w) return set_error(TBG_ERR_CUDA, "workspace");
-    // join 1: R x S, materialised on the device
-    tbg_row_out *rows1 = nullptr;
+    // join 1: R x S as (key, R payload) tuples, in HBM
     uint64_t m1 = 0;
-    int rc = join_rows(*cfg, reinterpret_cast<const Row *>(dR), nR, reinterpret_cast<const Row *>(dS), nS,
-                       w->chain_rows, st, &rows1, &m1);
+    int rc = join_relation(*cfg, reinterpret_cast<const Row *>(dR), nR, reinterpret_cast<const Row *>(dS), nS, *w, st, &m1);
     if (rc) return rc;
     *matches1 = m1;
-    // to_relation: (key, R payload) tuples, in HBM
-    cudaError_t e = w->chain_rel.ensure(std::max<uint64_t>(m1, 1) * sizeof(Row));
-    if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (chain relation)");
-    e = launch_rows_to_relation(rows1, m1, w->chain_rel.as<Row>(), w->nsm, st);
-    if (e != cudaSuccess) return cuda_error(e, "to_relation");
     // join 2: T x relation (T on the build side, as the reference calls it)
     tbg_config c2 = *cfg;
     c2.materialize = d_rows2 ? 1 : 0;

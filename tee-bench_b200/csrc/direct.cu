@@ -497,10 +497,14 @@ struct EmitSmem {
     unsigned long long base;
 };
 
+// REL: the output is a relation of (key, R payload) tuples, what a chained join
+// makes of the rows (chain.cu): 8 B a row, and no conversion afterwards.
+template <bool REL>
 __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
     k_hist_emit(const Row *__restrict__ in, uint64_t n, uint64_t chunk, uint32_t *__restrict__ hist, int nbins, RadixF rf,
-                const uint32_t *__restrict__ table, tbg_row_out *__restrict__ out, uint64_t cap, uint32_t range_max,
+                const uint32_t *__restrict__ table, uint32_t *__restrict__ out, uint64_t cap, uint32_t range_max,
                 Ctrl *ctrl) {
+    constexpr uint32_t W = REL ? 2 : 3;  // words per output row
     dep_wait();
     dep_trigger();
     constexpr int T = EMIT_DIRECT_THREADS, NW = T / 32;
@@ -520,8 +524,8 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
     // writes the staged rows out, word by word (coalesced)
     auto flush = [&]() {
         const unsigned long long base = sm.base;
-        const uint32_t words = base < cap ? 3 * (uint32_t)umin64(staged, cap - base) : 0u;
-        uint32_t *g = reinterpret_cast<uint32_t *>(out + base);
+        const uint32_t words = base < cap ? W * (uint32_t)umin64(staged, cap - base) : 0u;
+        uint32_t *g = out + base * W;
 #pragma unroll 4
         for (uint32_t i = tid; i < words; i += T) __stcs(g + i, sm.stage[i]);
     };
@@ -567,10 +571,10 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             if (m[j] >> lane & 1) {
-                uint32_t *q = sm.stage + 3 * (before + __popc(m[j] & lt));
+                uint32_t *q = sm.stage + W * (before + __popc(m[j] & lt));
                 q[0] = k[j];
                 q[1] = r[j];
-                q[2] = p[j];
+                if (!REL) q[2] = p[j];
             }
             before += __popc(m[j]);
         }
@@ -635,14 +639,15 @@ __global__ void __launch_bounds__(EMIT_DIRECT_THREADS, 2)
 }
 
 cudaError_t launch_hist_emit(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
-                             const uint32_t *table, tbg_row_out *out, uint64_t cap, uint32_t range_max, Ctrl *ctrl,
+                             const uint32_t *table, tbg_row_out *out, Row *rel, uint64_t cap, uint32_t range_max, Ctrl *ctrl,
                              cudaStream_t st) {
     const int nbins = 1 << P_log2;
     const size_t smem = sizeof(EmitSmem) + (size_t)nbins * 4;
-    cudaError_t e = smem_limit((const void *)k_hist_emit, smem);
+    auto kern = rel ? k_hist_emit<true> : k_hist_emit<false>;
+    uint32_t *words = rel ? reinterpret_cast<uint32_t *>(rel) : reinterpret_cast<uint32_t *>(out);
+    cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    e = launch_dep(k_hist_emit, G, EMIT_DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, table, out, cap, range_max,
-                   ctrl);
+    e = launch_dep(kern, G, EMIT_DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, table, words, cap, range_max, ctrl);
     count_launch();
     return e;
 }

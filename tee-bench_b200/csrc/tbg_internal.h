@@ -193,7 +193,7 @@ int join_ctas_per_sm(int capR, bool materialize);
 // ---- direct join (direct.cu) ----
 int direct_log2_max(uint64_t nR);
 cudaError_t launch_hist_emit(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
-                             const uint32_t *table, tbg_row_out *out, uint64_t cap, uint32_t range_max, Ctrl *ctrl,
+                             const uint32_t *table, tbg_row_out *out, Row *rel, uint64_t cap, uint32_t range_max, Ctrl *ctrl,
                              cudaStream_t st);
 int direct_log2_max_rows(uint64_t nR);
 cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *table, int log2_max, bool payloads, Ctrl *ctrl,

@@ -57,6 +57,8 @@ struct JoinRun {
     double heavy_pred = 0, heavy_sampled = 0;
     uint64_t launches = 0;
     bool waits = false;         // the caller waits for the result
+    Row *rel = nullptr;         // a direct join may write a relation here instead of its rows (chained joins)
+    bool rel_done = false;      // ... and did (before finish_join: may have)
     bool ctrl_on_host = false;  // the join's last kernel writes host_ctrl itself
 };
 
@@ -69,7 +71,7 @@ int join_capacity(uint64_t nR, bool counting);
 int join_device_impl(const tbg_config *cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
                      tbg_row_out *d_rows, uint64_t rows_cap, cudaStream_t st, JoinRun *run,
                      Workspace **wout);
-int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, const JoinRun &run,
+int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, JoinRun &run,
                 uint64_t nR, uint64_t nS, uint64_t cap, uint64_t *matches, tbg_stats *stats);
 
 // Heavy-key table used by the S histogram of the learned path (device pointers).
@@ -97,6 +99,7 @@ struct RadixGeom {
     bool direct_rows = false;      // ... of a materialising join: R's payloads instead of bits,
     tbg_row_out *rows = nullptr;   // ... S's read writes the rows here
     uint64_t rows_cap = 0;
+    Row *rel = nullptr;            // ... or, when set, a relation of (key, R payload) here (as many)
     bool keys = false;             // the partitions hold bare keys (counting joins)
     const Row *sample_S = nullptr;  // S, when it is there while R is read
 };

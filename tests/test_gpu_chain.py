@@ -66,3 +66,30 @@ def test_three_way_chain_matches_oracle(tbg, oracle, cuda, kind):
     # count only
     m1, m2 = tbg.join_three_way(tbg.config("RHO"), pR, len(R), pS, len(S), pT, len(T))
     assert (m1, m2) == (c1, c2)
+
+
+@pytest.mark.parametrize("nR,nS,nT,step", [(16385, 4095, 7, 1), (16387, 4097, 20000, 3), (20011, 300007, 17001, 1),
+                                           (16385, 70001, 30000, 40)])
+def test_three_way_chain_from_a_direct_join(tbg, oracle, cuda, nR, nS, nT, step):
+    """The first join writes the relation itself when it is direct: output
+    tiles that end unevenly, S rows without a partner, and (step 40) a key
+    range too wide for it, whose rows are converted."""
+    torch = cuda
+    rng = np.random.default_rng(nR + nS)
+    R, S, T = (np.zeros(n, dtype=oracle.ROW) for n in (nR, nS, nT))
+    R["key"] = rng.permutation(100 + step * np.arange(nR))
+    S["key"] = np.where(rng.random(nS) < 0.3, rng.integers(0, step * nR + 200, nS), R["key"][rng.integers(0, nR, nS)])
+    T["key"] = rng.integers(0, step * nR + 200, nT)
+    for rel, kind in ((R, 0), (S, 1), (T, 0)):
+        oracle.fill_payloads(rel, kind)
+    c1, _, c2, rows2 = _oracle_chain(oracle, R, S, T)
+    tR, pR = to_dev(torch, R, 1)
+    tS, pS = to_dev(torch, S)
+    tT, pT = to_dev(torch, T)
+    tO, pO = out_rows(torch, c2 + 16)
+    for algo in ("RHO", "RHT", "PSM"):
+        m1, m2 = tbg.join_three_way(tbg.config(algo), pR, nR, pS, nS, pT, nT, pO, c2 + 16,
+                                    torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert (m1, m2) == (c1, c2), algo
+        assert np.array_equal(oracle.sort_rows(rows_to_host(tO, m2)), oracle.sort_rows(rows2)), algo
