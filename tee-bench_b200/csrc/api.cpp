@@ -330,10 +330,10 @@ int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &
     cudaError_t e;
     if (g.direct && rel == 0 && !bypass) {
         e = launch_hist_build(d, g.n[0], g.ch[0], g.G[0], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(),
-                              g.direct_rows, ctrl, st);
+                              g.direct_rows, g.build_wave, ctrl, st);
         if (e == cudaSuccess)
             e = launch_direct_decide(g.direct_rows ? nullptr : w.direct.as<uint32_t>(), direct_log2_max(g.n[0]), g.n[0],
-                                     g.sample_S, g.n[1], ctrl, st);
+                                     g.sample_S, g.n[1], g.build_wave, ctrl, st);
     } else if (g.direct && g.direct_rows && !bypass) {
         e = launch_hist_emit(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), g.rows,
                              g.rel, g.rows_cap, g.s_range_max, ctrl, st);

@@ -164,7 +164,7 @@ __device__ __forceinline__ void hist_pairs(uint32_t *sh, const RadixF &rf, const
 template <bool PAYLOADS>
 __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__restrict__ in, uint64_t n, uint64_t chunk,
                                                                   uint32_t *__restrict__ hist, int nbins, RadixF rf,
-                                                                  uint32_t *__restrict__ table, Ctrl *ctrl) {
+                                                                  uint32_t *__restrict__ table, Ctrl *ctrl, uint32_t first) {
     dep_wait();
     dep_trigger();
     extern __shared__ uint32_t sh[];
@@ -175,14 +175,15 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
     __syncthreads();
     const unsigned w = ctrl->direct_log2;
     const uint32_t wmask = w ? (uint32_t)((1ull << w) - 1) : 0u;
-    const uint64_t lo = (uint64_t)blockIdx.x * chunk;
+    const uint32_t c = first + blockIdx.x;  // this CTA's chunk
+    const uint64_t lo = (uint64_t)c * chunk;
     const uint64_t hi = umin64(n, lo + chunk);
     volatile unsigned *gave_up = &ctrl->direct_dup;
     bool enter = w != 0;  // the same for all lanes of a warp
     uint32_t kinv = 0, kmax = 0;  // largest ~key (the smallest key) and largest key
     // a sixteenth of the rounds of long chunks, of the chunks when they are short
     const uint32_t rounds16 = (uint32_t)(chunk / (16 * 8 * DIRECT_THREADS));
-    const uint32_t careful = PAYLOADS ? 0xFFFFFFFFu : rounds16 ? rounds16 : (blockIdx.x & 15) == 0 ? 1u : 0u;
+    const uint32_t careful = PAYLOADS ? 0xFFFFFFFFu : rounds16 ? rounds16 : (c & 15) == 0 ? 1u : 0u;
     uint32_t round = 0;
     // enters a row; with ret, true says that the join is not direct
     auto set_bit = [&](uint32_t key, uint32_t payload, bool ret) {
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
         atomicMax(&ctrl->direct_inv_min, s_inv);
         atomicMax(&ctrl->direct_max, s_hi);
     }
-    uint32_t *dst = hist + (uint64_t)blockIdx.x * nbins;
+    uint32_t *dst = hist + (uint64_t)c * nbins;
     for (int i = tid; i < nbins; i += DIRECT_THREADS) dst[i] = sh[i];
 }
 
@@ -486,8 +487,8 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 1)
 // output.  A round's rows leave for memory while the next round's payloads
 // arrive, and the reservation returns while the rows are staged, so a round
 // waits for neither.  Bound by L2 (one sector per row gathered, 12 B out, 8 B
-// in): 16.8 M rows take XXX us, 161 us before the rounds overlapped (then
-// with a bulk store per round).
+// in): 16.8 M rows take 128 us, 161 us before the rounds overlapped (then
+// with a bulk store per round); as a relation (REL) 120 us.
 constexpr int EMIT_DIRECT_THREADS = 512;
 constexpr int EMIT_ROUND = EMIT_DIRECT_THREADS * 8;
 
@@ -662,22 +663,36 @@ cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *table, int l
 }
 
 cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
-                              uint32_t *table, bool payloads, Ctrl *ctrl, cudaStream_t st) {
+                              uint32_t *table, bool payloads, int wave, Ctrl *ctrl, cudaStream_t st) {
     const int nbins = 1 << P_log2;
     const size_t smem = (size_t)nbins * 4;
     auto kern = payloads ? k_hist_build<true> : k_hist_build<false>;
     cudaError_t e = smem_limit((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    e = launch_dep(kern, G, DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, table, ctrl);
-    count_launch();
-    return e;
+    if (!wave || wave >= G) {
+        e = launch_dep(kern, G, DIRECT_THREADS, smem, st, in, n, chunk, hist, nbins, rf, table, ctrl, 0u);
+        count_launch();
+        return e;
+    }
+    // plain launches: a dependent one's CTAs would take the room that the
+    // waves are there to leave
+    for (int c = 0; c < G; c += wave) {
+        kern<<<std::min(wave, G - c), DIRECT_THREADS, smem, st>>>(in, n, chunk, hist, nbins, rf, table, ctrl, (uint32_t)c);
+        count_launch();
+    }
+    return cudaGetLastError();
 }
 
-cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, Ctrl *ctrl,
+cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, int wave, Ctrl *ctrl,
                                  cudaStream_t st) {
     const uint64_t n4 = 1ull << (log2_max - 7);
     // two 16-byte words per thread and CTA at least, one CTA per SM at most
     const unsigned g = bits ? (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), 148)) : 1u;
+    if (wave) {  // no dependent launch, as above
+        k_direct_decide<<<g, DIRECT_THREADS, 0, st>>>(bits, nR, S, nS, ctrl);
+        count_launch();
+        return cudaGetLastError();
+    }
     const cudaError_t e = launch_dep(k_direct_decide, g, DIRECT_THREADS, 0, st, bits, nR, S, nS, ctrl);
     count_launch();
     return e;

@@ -35,15 +35,6 @@ namespace tbg {
 
 static constexpr double kMinHeavyFraction = 0.05;
 
-// 0 (default): R's partitioning is queued before the learning stage's
-// kernels; 1: after them.  Measured at |R| = 2^26, |S| = 2^29, z = 1: 5.41 -
-// 5.49 ms against 5.65 ms.  Queued first, the learning stage ends sooner
-// (0.68 against 0.79 - 0.88 ms) but pushes R's partitioning into S's
-// bandwidth-bound phase; queued after, R's passes use the bandwidth the
-// latency-bound learning kernels leave idle.  A build option for A/B timing.
-#ifndef TBG_LRN_LEARN_FIRST
-#define TBG_LRN_LEARN_FIRST 0
-#endif
 static constexpr unsigned kCandCap = 1u << 20;
 
 int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS,
@@ -84,6 +75,10 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     RadixGeom g = radix_geometry(cfg, nR, nS, capR, w);
     if (!mat) try_direct(g, cfg, nullptr, 0);
     g.sample_S = dS;
+    // One CTA per SM at a time, so that the learning stage's kernels find room
+    // beside R's read; with two, which fill the SMs, they waited for its end
+    // (|R| = 2^26: the decision after 865 us, 744 us with one).
+    g.build_wave = w.nsm;
     run->B = g.B;
     run->passes = g.passes;
     run->P = g.P;
@@ -140,25 +135,21 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     if (timing) cudaEventRecord(w.ev[0], st);
     if ((rc = start_radix_join(g, dR, w, st))) return rc;
     if ((e = cudaEventRecord(w.fork, st)) != cudaSuccess) return cuda_error(e, "event");
-    if (!TBG_LRN_LEARN_FIRST && (rc = partition_r()))
-        return rc;
+    // R's reading is queued before the learning stage: joins that are not
+    // direct then partition R meanwhile (|R| = 2^26, |S| = 2^29, z = 1,
+    // partitioned: 5.41 - 5.49 ms, 5.65 ms queued after)
+    if ((rc = partition_r())) return rc;
 
     // side stream: learn the heavy keys (on the high-priority stream, while
     // R is partitioned)
     if ((e = cudaStreamWaitEvent(s2, w.fork, 0)) != cudaSuccess) return cuda_error(e, "event");
-    if ((e = cudaMemsetAsync(lb.table, 0xFF, (size_t)tslots * 8, s2)) != cudaSuccess ||
-        (e = cudaMemsetAsync(lb.bin_rows, 0, (size_t)CC_BINS * 12, s2)) != cudaSuccess ||
-        (e = cudaMemsetAsync(lb.dec, 0, sizeof(LrnDecision), s2)) != cudaSuccess ||
-        (e = cudaMemsetAsync(hkeys, 0xFF, HEAVY_CAP * 4, s2)) != cudaSuccess ||
-        (e = cudaMemsetAsync(hcnt, 0, HEAVY_CAP * 4 * 4 + 16, s2)) != cudaSuccess)
-        return cuda_error(e, "memset");
     const int steps = cfg.model == TBG_MODEL_MLP ? std::min(std::max(cfg.train_steps, 1), 500) : 0;
     const int use_model = cfg.model == TBG_MODEL_SAMPLE ? 0 : 1;
     // a key must be predicted to hold at least tau_min S rows to be heavy
     const double tau_min = std::max(64.0, (double)nS / (double)(1 << 20));
-    if ((e = launch_sample_blocks(dS, nS, lb.keys, nb, stride, cfg.seed, s2)) != cudaSuccess ||
+    if ((e = launch_learn_start(dS, lb, nb, stride, hkeys, hcnt, cfg.seed, s2)) != cudaSuccess ||
         (e = launch_count_keys(lb, m, s2)) != cudaSuccess || (e = launch_count_stats(lb, s2)) != cudaSuccess ||
-        (e = launch_rank_points(lb, s2)) != cudaSuccess || (e = launch_mlp_init(lb.params, cfg.seed, s2)) != cudaSuccess ||
+        (e = launch_rank_points(lb, s2)) != cudaSuccess ||
         (steps && (e = launch_mlp_train(lb.xs, lb.ys, lb.cw, &lb.dec->npoints, 0, lb.params, steps, 0.03f, cfg.seed, s2)) !=
                       cudaSuccess) ||
         (e = launch_decide(lb, use_model, (double)nS, (double)m, tau_min, kMinHeavyFraction, s2)) != cudaSuccess)
@@ -166,7 +157,6 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     LrnDecision *hd = static_cast<LrnDecision *>(w.host_small);
     if ((e = cudaMemcpyAsync(hd, lb.dec, sizeof(LrnDecision), cudaMemcpyDeviceToHost, s2)) != cudaSuccess)
         return cuda_error(e, "learning stage");
-    if (TBG_LRN_LEARN_FIRST && (rc = partition_r())) return rc;
     if ((e = cudaStreamSynchronize(s2)) != cudaSuccess) return cuda_error(e, "learning stage");
     const LrnDecision dec = *hd;
     run->train_steps = steps;

@@ -19,6 +19,7 @@
 // RHO.  The model only chooses which keys take the heavy path; every row's
 // destination is decided by an exact key comparison, so results are exact
 // whatever the model predicts.
+#include <algorithm>
 #include <cooperative_groups.h>
 
 #include "part_dev.cuh"
@@ -59,221 +60,225 @@ __device__ float mlp_eval(const float *__restrict__ p, float x) {
     return out;
 }
 
-// A batch of MLP_BATCH_CTA samples is processed by MLP_TRAIN_THREADS threads
-// (16 warps).  Forward and backward: warp w serves samples 32 (w / 4) + lane
-// and hidden units [8 (w % 4), 8 (w % 4) + 8) of both layers, so the lanes of
-// a warp read every weight as a broadcast; the four warps of a sample group
-// exchange activations through shared memory under a named barrier.  The
-// per-sample rows have a stride of MLP_H + 1 floats: a warp's lanes (one
-// sample each) touch distinct banks.
-constexpr int RS = MLP_H + 1;
-constexpr int MLP_UNITS_WARP = MLP_H / 4;  // hidden units per warp
-constexpr int GR_SLICES = 8;               // sample slices of the parameter-gradient sums
-static_assert(MLP_TRAIN_THREADS == 4 * MLP_BATCH_CTA, "four warps per 32 samples");
-static_assert(MLP_TRAIN_THREADS == 64 * GR_SLICES && MLP_BATCH_CTA % GR_SLICES == 0, "gradient slices");
+// A batch of MLP_BATCH_CTA samples is processed by MLP_TRAIN_THREADS threads.
+// Warp w serves samples [16w, 16w + 16) through both layers, backwards, and to
+// its share of every gradient sum, so the whole pass runs on warp barriers.
+// Lane (sg, og) = (lane / 8, lane % 8) keeps a register tile of 4 samples
+// (4 sg ..) by 4 hidden units (og + 8r going forward, 4 og + r going back):
+// 16 products per two 16-byte loads.  Activations are stored sample-minor with
+// a row stride of 132 floats and W2 with one of 36: no bank conflicts.  Bound
+// by the bytes the load/store pipe brings to registers (128 a cycle: 5600
+// cycles a step and CTA; the products are 3100): 8800 cycles a step measured,
+// 13900 with a hidden unit per lane, its weights in registers and 16-byte
+// broadcast loads of the activations, which cost as much as distinct ones.
+constexpr int MLP_WARPS = MLP_TRAIN_THREADS / 32;
+constexpr int HS = MLP_BATCH_CTA + 4;   // stride of a unit's samples
+constexpr int W2S = MLP_H + 4;          // stride of W2's rows in shared memory
+static_assert(MLP_H == 32 && MLP_BATCH_CTA == 16 * MLP_WARPS, "a warp serves 16 samples, a lane 4 units");
+
+// Parameters and gradients in shared memory: W2's rows padded to W2S.
+constexpr int S_W1 = 0, S_B1 = MLP_H, S_W2 = 2 * MLP_H, S_B2 = S_W2 + MLP_H * W2S, S_W3 = S_B2 + MLP_H,
+              S_B3 = S_W3 + MLP_H, S_N = S_B3 + 1, S_PAD = (S_N + 3) & ~3;
+__device__ __forceinline__ int s_index(int q) {
+    if (q < P_W2) return q;
+    if (q < P_B2) return S_W2 + ((q - P_W2) / MLP_H) * W2S + (q - P_W2) % MLP_H;
+    return q + (S_B2 - P_B2);
+}
+
+constexpr int DRAW_STEPS = 8;  // steps whose points are drawn at once
 
 struct BatchSmem {
-    float h1[MLP_BATCH_CTA][RS];
-    float h2[MLP_BATCH_CTA][RS];
-    float dz2[MLP_BATCH_CTA][RS];
-    float dz1[MLP_BATCH_CTA][RS];
-    float x[MLP_BATCH_CTA];
-    float dout[MLP_BATCH_CTA];
-    float part[4][MLP_BATCH_CTA];  // output partial of each unit group
-    alignas(16) float red[GR_SLICES][MLP_PARAMS_PAD];  // per-slice gradient partials
+    alignas(16) float h1[MLP_H][HS];
+    alignas(16) float dz2[MLP_H][HS];
+    alignas(16) float x[DRAW_STEPS][MLP_BATCH_CTA], y[DRAW_STEPS][MLP_BATCH_CTA];
+    alignas(16) float red[MLP_WARPS][S_PAD];  // the warps' gradient sums
 };
 
 __device__ __forceinline__ float4 ld4(const float *a) { return *reinterpret_cast<const float4 *>(a); }
-
-// Barrier of the four warps of sample group g (named barriers 1 .. 4, given
-// as immediates so that the kernel reserves only those).
-__device__ __forceinline__ void group_sync(int g) {
-    switch (g) {
-        case 0: asm volatile("bar.sync 1, 128;" ::: "memory"); break;
-        case 1: asm volatile("bar.sync 2, 128;" ::: "memory"); break;
-        case 2: asm volatile("bar.sync 3, 128;" ::: "memory"); break;
-        default: asm volatile("bar.sync 4, 128;" ::: "memory"); break;
-    }
+__device__ __forceinline__ void fma4(float (&acc)[4], float w, const float4 &h) {
+    acc[0] = fmaf(w, h.x, acc[0]);
+    acc[1] = fmaf(w, h.y, acc[1]);
+    acc[2] = fmaf(w, h.z, acc[2]);
+    acc[3] = fmaf(w, h.w, acc[3]);
+}
+__device__ __forceinline__ float dot4(const float4 &a, const float4 &b, float acc) {
+    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+// Sum over the lanes of equal og (the warp's four sample groups).
+__device__ __forceinline__ float sum_sg(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
 }
 
-// Dot product of a 16-byte aligned shared row of MLP_H floats with v
-// (two accumulators).
-__device__ __forceinline__ float dot_row(const float *w, const float (&v)[MLP_H], float acc) {
-    float a0 = acc, a1 = 0.f;
+// Forward and backward of the warp's samples (inputs xs, targets ys, loss
+// weights scale, 0 for a sample that does not count): leaves the warp's sum of
+// every parameter's gradient in b.red[w]; returns the sum of the squared
+// errors of the lane's samples that count.
+__device__ float warp_fwd_bwd(const float *p, BatchSmem &b, const float *xs, const float *ys, const float (&scale)[4]) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sg = lane >> 3, og = lane & 7, s0 = 16 * w + 4 * sg;
+    float *red = b.red[w];
+    const float4 xv = ld4(xs + s0), yv = ld4(ys + s0);
+    const float x[4] = {xv.x, xv.y, xv.z, xv.w}, y[4] = {yv.x, yv.y, yv.z, yv.w};
 #pragma unroll
-    for (int i = 0; i < MLP_H; i += 8) {
-        const float4 x = ld4(w + i), y = ld4(w + i + 4);
-        a0 = fmaf(x.x, v[i], a0);
-        a1 = fmaf(x.y, v[i + 1], a1);
-        a0 = fmaf(x.z, v[i + 2], a0);
-        a1 = fmaf(x.w, v[i + 3], a1);
-        a0 = fmaf(y.x, v[i + 4], a0);
-        a1 = fmaf(y.y, v[i + 5], a1);
-        a0 = fmaf(y.z, v[i + 6], a0);
-        a1 = fmaf(y.w, v[i + 7], a1);
+    for (int r = 0; r < 4; r++) {
+        const int u = og + 8 * r;
+        const float w1 = p[S_W1 + u], b1 = p[S_B1 + u];
+        *reinterpret_cast<float4 *>(&b.h1[u][s0]) =
+            make_float4(tanh_f(w1 * x[0] + b1), tanh_f(w1 * x[1] + b1), tanh_f(w1 * x[2] + b1), tanh_f(w1 * x[3] + b1));
     }
-    return a0 + a1;
-}
-
-// Forward and backward of sample s (input x, target y, loss weight scale) by
-// warp j of its sample group g, which owns hidden units [8j, 8j + 8).
-// Leaves the sample's activations, pre-activation gradients and output
-// gradient in row s; returns the squared error.  Every thread of the group
-// calls it (named barriers).
-__device__ float group_fwd_bwd(const float *p, BatchSmem &b, float x, float y, float scale, int s, int g, int j) {
-    constexpr int U = MLP_UNITS_WARP;
-    const int u0 = U * j;
-    float *h1 = b.h1[s], *h2 = b.h2[s], *dz2 = b.dz2[s], *dz1 = b.dz1[s];
+    __syncwarp();
+    float h2[4][4];
 #pragma unroll
-    for (int t = 0; t < U; t++) h1[u0 + t] = tanh_f(p[P_W1 + u0 + t] * x + p[P_B1 + u0 + t]);
-    group_sync(g);
-    float v[MLP_H];
+    for (int r = 0; r < 4; r++)
 #pragma unroll
-    for (int i = 0; i < MLP_H; i++) v[i] = h1[i];
-    float part = 0.f, g2[U];
+        for (int c = 0; c < 4; c++) h2[r][c] = p[S_B2 + og + 8 * r];
+#pragma unroll 2
+    for (int i = 0; i < MLP_H; i += 4) {
+        const float4 a0 = ld4(&b.h1[i][s0]), a1 = ld4(&b.h1[i + 1][s0]), a2 = ld4(&b.h1[i + 2][s0]),
+                     a3 = ld4(&b.h1[i + 3][s0]);
 #pragma unroll
-    for (int t = 0; t < U; t++) {
-        const int u = u0 + t;
-        const float h = tanh_f(dot_row(p + P_W2 + u * MLP_H, v, p[P_B2 + u]));
-        h2[u] = h;
-        const float w3 = p[P_W3 + u];
-        part = fmaf(w3, h, part);
-        g2[t] = w3 * (1.f - h * h);
+        for (int r = 0; r < 4; r++) {
+            const float4 wv = ld4(p + S_W2 + (og + 8 * r) * W2S + i);
+            fma4(h2[r], wv.x, a0);
+            fma4(h2[r], wv.y, a1);
+            fma4(h2[r], wv.z, a2);
+            fma4(h2[r], wv.w, a3);
+        }
     }
-    b.part[j][s] = part;
-    group_sync(g);
-    const float r = p[P_B3] + ((b.part[0][s] + b.part[1][s]) + (b.part[2][s] + b.part[3][s])) - y;
-    const float dout = 2.f * r * scale;
+    float out[4] = {0.f, 0.f, 0.f, 0.f}, dout[4], loss = 0.f;
 #pragma unroll
-    for (int t = 0; t < U; t++) dz2[u0 + t] = dout * g2[t];
-    group_sync(g);
+    for (int r = 0; r < 4; r++)
 #pragma unroll
-    for (int o = 0; o < MLP_H; o++) v[o] = dz2[o];
-    // dz1[i] = (1 - h1[i]^2) sum_o W2[o][i] dz2[o] for the warp's units i
-    float acc[U];
+        for (int c = 0; c < 4; c++) {
+            h2[r][c] = tanh_f(h2[r][c]);
+            out[c] = fmaf(p[S_W3 + og + 8 * r], h2[r][c], out[c]);
+        }
 #pragma unroll
-    for (int t = 0; t < U; t++) acc[t] = 0.f;
+    for (int c = 0; c < 4; c++) {
+        for (int o = 1; o < 8; o <<= 1) out[c] += __shfl_xor_sync(0xffffffffu, out[c], o);
+        const float e = out[c] + p[S_B3] - y[c];
+        dout[c] = 2.f * e * scale[c];
+        loss += scale[c] != 0.f ? e * e : 0.f;
+    }
+    const float d3 = sum_sg((dout[0] + dout[1]) + (dout[2] + dout[3]));
+    if (lane == 0) red[S_B3] = d3;
 #pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const int u = og + 8 * r;
+        const float w3 = p[S_W3 + u];
+        float d[4], g3 = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            d[c] = dout[c] * (w3 * (1.f - h2[r][c] * h2[r][c]));
+            g3 = fmaf(dout[c], h2[r][c], g3);
+        }
+        *reinterpret_cast<float4 *>(&b.dz2[u][s0]) = make_float4(d[0], d[1], d[2], d[3]);
+        const float g2 = sum_sg((d[0] + d[1]) + (d[2] + d[3]));
+        g3 = sum_sg(g3);
+        if (sg == 0) {
+            red[S_B2 + u] = g2;
+            red[S_W3 + u] = g3;
+        }
+    }
+    __syncwarp();
+    // dz1[i] = (1 - h1[i]^2) sum_o W2[o][i] dz2[o] for units i = 4 og + r
+    float z1[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) z1[r][c] = 0.f;
+#pragma unroll 4
     for (int o = 0; o < MLP_H; o++) {
-        const float4 a = ld4(p + P_W2 + o * MLP_H + u0), c = ld4(p + P_W2 + o * MLP_H + u0 + 4);
-        acc[0] = fmaf(a.x, v[o], acc[0]);
-        acc[1] = fmaf(a.y, v[o], acc[1]);
-        acc[2] = fmaf(a.z, v[o], acc[2]);
-        acc[3] = fmaf(a.w, v[o], acc[3]);
-        acc[4] = fmaf(c.x, v[o], acc[4]);
-        acc[5] = fmaf(c.y, v[o], acc[5]);
-        acc[6] = fmaf(c.z, v[o], acc[6]);
-        acc[7] = fmaf(c.w, v[o], acc[7]);
+        const float4 wv = ld4(p + S_W2 + o * W2S + 4 * og), dv = ld4(&b.dz2[o][s0]);
+        fma4(z1[0], wv.x, dv);
+        fma4(z1[1], wv.y, dv);
+        fma4(z1[2], wv.z, dv);
+        fma4(z1[3], wv.w, dv);
     }
 #pragma unroll
-    for (int t = 0; t < U; t++) {
-        const float a = h1[u0 + t];
-        dz1[u0 + t] = acc[t] * (1.f - a * a);
+    for (int r = 0; r < 4; r++) {
+        const float4 hv = ld4(&b.h1[4 * og + r][s0]);
+        const float h[4] = {hv.x, hv.y, hv.z, hv.w};
+        float g1 = 0.f, gw = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const float d = z1[r][c] * (1.f - h[c] * h[c]);
+            g1 += d;
+            gw = fmaf(d, x[c], gw);
+        }
+        g1 = sum_sg(g1);
+        gw = sum_sg(gw);
+        if (sg == 0) {
+            red[S_B1 + 4 * og + r] = g1;
+            red[S_W1 + 4 * og + r] = gw;
+        }
     }
-    if (j == 0) {
-        b.x[s] = x;
-        b.dout[s] = dout;
+    // W2's gradient over the warp's samples: rows og + 8r, columns sg + 4c
+    float g[4][8];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) g[r][c] = 0.f;
+#pragma unroll 1
+    for (int t = 16 * w; t < 16 * w + 16; t += 4) {
+        float4 d[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) d[r] = ld4(&b.dz2[og + 8 * r][t]);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const float4 h = ld4(&b.h1[sg + 4 * c][t]);
+#pragma unroll
+            for (int r = 0; r < 4; r++) g[r][c] = dot4(d[r], h, g[r][c]);
+        }
     }
-    return r * r;
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 8; c++) red[S_W2 + (og + 8 * r) * W2S + sg + 4 * c] = g[r][c];
+    return loss;
 }
 
-// Gradient of every parameter summed over samples 0 .. nb of the batch, into
-// g[0 .. MLP_PARAMS), by all MLP_TRAIN_THREADS threads (a __syncthreads
-// inside).  Slice k of GR_SLICES takes samples [16k, 16k + 16) on 64
-// threads: each sums one 4 x 4 tile of W2's gradient and two or three of the
-// other parameters over its slice into the slice's partials; then every
-// thread adds the slices' partials of its parameters.
-__device__ void batch_param_grad(BatchSmem &b, int nb, float *g) {
-    constexpr int SPAN = MLP_BATCH_CTA / GR_SLICES;
-    const int tid = threadIdx.x, sl = tid >> 6, t = tid & 63;
-    const int s0 = sl * SPAN, s1 = min(nb, s0 + SPAN);
-    float *red = b.red[sl];
-    {
-        const int o0 = (t >> 3) * 4, i0 = (t & 7) * 4;
-        float acc[4][4];
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) acc[a][c] = 0.f;
-        for (int s = s0; s < s1; s++) {
-            float d[4], h[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                d[k] = b.dz2[s][o0 + k];
-                h[k] = b.h1[s][i0 + k];
-            }
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) acc[a][c] = fmaf(d[a], h[c], acc[a][c]);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-            *reinterpret_cast<float4 *>(red + P_W2 + (o0 + a) * MLP_H + i0) =
-                make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
-    }
-    // the slice's first warp: W1[i] and b2[i]; its second: b1[i] and W3[i];
-    // thread 0 also b3 (i = lane, MLP_H = 32)
-    {
-        static_assert(MLP_H == 32, "one lane per hidden unit");
-        const int i = t & 31;
-        float a = 0.f, c = 0.f;
-        if (t < 32) {
-            for (int s = s0; s < s1; s++) {
-                a = fmaf(b.dz1[s][i], b.x[s], a);
-                c += b.dz2[s][i];
-            }
-            red[P_W1 + i] = a;
-            red[P_B2 + i] = c;
-        } else {
-            for (int s = s0; s < s1; s++) {
-                a += b.dz1[s][i];
-                c = fmaf(b.dout[s], b.h2[s][i], c);
-            }
-            red[P_B1 + i] = a;
-            red[P_W3 + i] = c;
-        }
-        if (t == 0) {
-            float d = 0.f;
-            for (int s = s0; s < s1; s++) d += b.dout[s];
-            red[P_B3] = d;
-        }
-    }
-    __syncthreads();
-    for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) {
+// The batch's gradient (s_index order) into g: the warps' sums added.  Every
+// thread calls it, after a block barrier.
+__device__ void batch_param_grad(const BatchSmem &b, float *g) {
+    for (int q = threadIdx.x; q < S_N; q += MLP_TRAIN_THREADS) {
         float a = 0.f;
 #pragma unroll
-        for (int k = 0; k < GR_SLICES; k++) a += b.red[k][q];
-        g[q] = a;
+        for (int k = 0; k < MLP_WARPS; k++) a += b.red[k][q];
+        g[q] = a;  // W2's row padding sums what no warp wrote; nothing reads it
     }
 }
 
 // Full-batch gradient and loss sum over n samples (tests and the reported
 // training loss): CTAs take MLP_BATCH_CTA samples each and add their partial
 // gradients to grad[] with atomics.
-__global__ void __launch_bounds__(MLP_TRAIN_THREADS, 1) k_mlp_grad(const float *__restrict__ params,
+__global__ void __launch_bounds__(MLP_TRAIN_THREADS, 2) k_mlp_grad(const float *__restrict__ params,
                                                                 const float *__restrict__ xs,
                                                                 const float *__restrict__ ys, uint32_t n,
                                                                 float *grad, float *loss_sum) {
     extern __shared__ __align__(16) unsigned char smem[];
     float *p = reinterpret_cast<float *>(smem);
-    float *gl = p + MLP_PARAMS_PAD;
-    BatchSmem &b = *reinterpret_cast<BatchSmem *>(gl + MLP_PARAMS_PAD);
-    const int tid = threadIdx.x, w = tid >> 5, g = w >> 2, j = w & 3, s = 32 * g + (tid & 31);
-    for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) p[q] = params[q];
-    __syncthreads();
+    float *gl = p + S_PAD;
+    BatchSmem &b = *reinterpret_cast<BatchSmem *>(gl + S_PAD);
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) p[s_index(q)] = params[q];
     const uint32_t s0 = blockIdx.x * MLP_BATCH_CTA;
     const int nb = (int)min((uint32_t)MLP_BATCH_CTA, n - s0);
-    const bool ok = s < nb;
-    // every group runs (named barriers); samples past n add nothing
-    const float l = group_fwd_bwd(p, b, ok ? xs[s0 + s] : 0.f, ok ? ys[s0 + s] : 0.f, 1.f / (float)n, s, g, j);
+    for (int s = tid; s < MLP_BATCH_CTA; s += MLP_TRAIN_THREADS) {
+        b.x[0][s] = s < nb ? xs[s0 + s] : 0.f;
+        b.y[0][s] = s < nb ? ys[s0 + s] : 0.f;
+    }
     __syncthreads();
-    batch_param_grad(b, nb, gl);
+    float scale[4];  // samples past n add nothing
+#pragma unroll
+    for (int c = 0; c < 4; c++) scale[c] = 16 * (tid >> 5) + 4 * (lane >> 3) + c < nb ? 1.f / (float)n : 0.f;
+    float lw = warp_fwd_bwd(p, b, b.x[0], b.y[0], scale);
     __syncthreads();
-    for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) atomicAdd(&grad[q], gl[q]);
-    float lw = (ok && j == 0) ? l : 0.f;
-    for (int o = 16; o > 0; o >>= 1) lw += __shfl_xor_sync(0xffffffffu, lw, o);
-    if ((tid & 31) == 0) atomicAdd(loss_sum, lw);
+    batch_param_grad(b, gl);
+    __syncthreads();
+    for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) atomicAdd(&grad[q], gl[s_index(q)]);
+    lw = sum_sg(lw);  // the eight lanes of a sample group hold the same errors
+    if (lane == 0) atomicAdd(loss_sum, lw);
 }
 
 // Training points staged in the trainer's shared memory (larger point sets
@@ -281,13 +286,16 @@ __global__ void __launch_bounds__(MLP_TRAIN_THREADS, 1) k_mlp_grad(const float *
 constexpr int MLP_STAGE = CC_BINS;
 
 // Trainer: one cluster of MLP_CLUSTER CTAs, persistent over all steps.  Each
-// step every CTA draws MLP_BATCH_CTA seeded random training points (uniformly,
+// step every CTA takes MLP_BATCH_CTA seeded random training points (uniformly,
 // or in proportion to their weights), runs their forward and backward passes
 // and its partial parameter gradient; after a
 // cluster barrier CTA r sums the partials of its parameter slice from every
 // CTA's shared memory, applies Adam, and writes the new values into every
-// CTA's parameter copy; a second barrier ends the step.
-__global__ void __cluster_dims__(MLP_CLUSTER, 1, 1) __launch_bounds__(MLP_TRAIN_THREADS)
+// CTA's parameter copy; a second barrier ends the step.  Each warp draws its
+// own next points while a first barrier is on its way.  128 registers at most,
+// so that a CTA fits beside one of k_hist_build's.  30 steps: 190 us, 235 us
+// with 512 threads, a sample per lane and the draws between the steps.
+__global__ void __cluster_dims__(MLP_CLUSTER, 1, 1) __launch_bounds__(MLP_TRAIN_THREADS, 2)
     k_mlp_train(const float *__restrict__ xs, const float *__restrict__ ys, const float *__restrict__ cw,
                 const unsigned *n_dev, uint32_t n_host, float *params, int steps, float lr0, uint64_t seed) {
     cg::cluster_group cl = cg::this_cluster();
@@ -298,15 +306,12 @@ __global__ void __cluster_dims__(MLP_CLUSTER, 1, 1) __launch_bounds__(MLP_TRAIN_
     if (n == 0) return;
     extern __shared__ __align__(16) unsigned char smem[];
     float *p = reinterpret_cast<float *>(smem);
-    float *gpart = p + MLP_PARAMS_PAD;
-    float *am = gpart + MLP_PARAMS_PAD;  // Adam moments of this CTA's slice
-    float *av = am + MLP_SLICE;
-    BatchSmem &b = *reinterpret_cast<BatchSmem *>(av + MLP_SLICE);
+    float *gpart = p + S_PAD;
+    BatchSmem &b = *reinterpret_cast<BatchSmem *>(gpart + S_PAD);
     float *sx = reinterpret_cast<float *>(&b + 1), *sy = sx + MLP_STAGE, *scw = sy + MLP_STAGE;
-    const int tid = threadIdx.x, w = tid >> 5, g = w >> 2, j = w & 3, s = 32 * g + (tid & 31);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const bool staged = n <= (uint32_t)MLP_STAGE;
-    for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) p[q] = params[q];
-    for (int q = tid; q < MLP_SLICE; q += MLP_TRAIN_THREADS) am[q] = av[q] = 0.f;
+    for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) p[s_index(q)] = params[q];
     if (staged)
         for (uint32_t q = tid; q < n; q += MLP_TRAIN_THREADS) {
             sx[q] = xs[q];
@@ -316,75 +321,102 @@ __global__ void __cluster_dims__(MLP_CLUSTER, 1, 1) __launch_bounds__(MLP_TRAIN_
     const float *px = staged ? sx : xs, *py = staged ? sy : ys, *pw = staged ? scw : cw;
     cl.sync();
     const float b1c = 0.9f, b2c = 0.999f, eps = 1e-8f;
-    const float scale = 1.f / (float)(MLP_BATCH_CTA * MLP_CLUSTER);
-    const int q0 = rank * MLP_SLICE, q1 = min(MLP_PARAMS, q0 + MLP_SLICE);
+    const float sc = 1.f / (float)(MLP_BATCH_CTA * MLP_CLUSTER);
+    const float scale[4] = {sc, sc, sc, sc};
+    // this thread's parameter of the CTA's slice and its Adam moments
+    static_assert(MLP_SLICE <= MLP_TRAIN_THREADS, "one parameter per thread");
+    const int q = rank * MLP_SLICE + tid;
+    const bool mine = tid < MLP_SLICE && q < MLP_PARAMS;
+    const int qs = mine ? s_index(q) : 0;
+    float am = 0.f, av = 0.f;
     const float wtot = cw ? pw[n - 1] : 0.f;
     float pow1 = 1.f, pow2 = 1.f;
-    for (int step = 0; step < steps; step++) {
-        // sample s: the group's first warp draws the point, the other three
-        // read it after the group barrier
-        if (j == 0) {
-            const uint64_t hsh = mix64(seed ^ mix64(((uint64_t)step << 20) | (uint64_t)(rank * MLP_BATCH_CTA + s)));
-            uint32_t i;
-            if (cw) {  // the first point whose cumulative weight exceeds u * total
-                const float u = (float)((hsh >> 40) * (1.0 / 16777216.0)) * wtot;
-                uint32_t lo = 0, hi = n - 1;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (pw[mid] > u) hi = mid;
-                    else lo = mid + 1;
-                }
-                i = lo;
-            } else {
-                i = (uint32_t)(hsh % n);
-            }
-            b.x[s] = px[i];
-            b.dout[s] = py[i];  // the target, until the backward pass overwrites it
+    // the warp's points of steps step .. step + DRAW_STEPS - 1: four at a time
+    // per lane, since each is a chain of loads (a binary search); one step's
+    // on half the lanes took 1630 cycles
+    auto draw = [&](int step) {
+        constexpr int PER = DRAW_STEPS / 2;
+        uint32_t lo[PER], hi[PER];
+        float u[PER];
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const int st = step + 2 * k + (lane >> 4), s = 16 * w + (lane & 15);
+            const uint64_t hsh = mix64(seed ^ mix64(((uint64_t)st << 20) | (uint64_t)(rank * MLP_BATCH_CTA + s)));
+            u[k] = (float)((hsh >> 40) * (1.0 / 16777216.0)) * wtot;
+            lo[k] = cw ? 0u : (uint32_t)(hsh % n);
+            hi[k] = n - 1;
         }
-        group_sync(g);
-        group_fwd_bwd(p, b, b.x[s], b.dout[s], scale, s, g, j);
+        if (cw)  // the first point whose cumulative weight exceeds u * total
+            for (uint32_t left = n; left > 1; left = left / 2 + (left & 1))
+#pragma unroll
+                for (int k = 0; k < PER; k++)
+                    if (lo[k] < hi[k]) {
+                        const uint32_t mid = (lo[k] + hi[k]) >> 1;
+                        const bool above = pw[mid] > u[k];
+                        hi[k] = above ? mid : hi[k];
+                        lo[k] = above ? lo[k] : mid + 1;
+                    }
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const int j = 2 * k + (lane >> 4), s = 16 * w + (lane & 15);
+            b.x[j][s] = px[lo[k]];
+            b.y[j][s] = py[lo[k]];
+        }
+        __syncwarp();
+    };
+    draw(0);
+    for (int step = 0; step < steps; step++) {
+        const int j = step % DRAW_STEPS;
+        warp_fwd_bwd(p, b, b.x[j], b.y[j], scale);
         __syncthreads();
-        batch_param_grad(b, MLP_BATCH_CTA, gpart);
-        cl.sync();
+        batch_param_grad(b, gpart);
+        cl.barrier_arrive();
+        if (j == DRAW_STEPS - 1 && step + 1 < steps) draw(step + 1);
         pow1 *= b1c;
         pow2 *= b2c;
         // cosine decay from lr0 to lr0 / 10
         const float lr = lr0 * (0.55f + 0.45f * cospif((float)step / (float)(steps > 1 ? steps - 1 : 1)));
-        for (int q = q0 + tid; q < q1; q += MLP_TRAIN_THREADS) {
-            float gs = 0.f;
-            for (int r = 0; r < MLP_CLUSTER; r++) gs += cl.map_shared_rank(gpart, r)[q];
-            const int k = q - q0;
-            am[k] = b1c * am[k] + (1.f - b1c) * gs;
-            av[k] = b2c * av[k] + (1.f - b2c) * gs * gs;
-            const float mh = am[k] / (1.f - pow1), vh = av[k] / (1.f - pow2);
-            const float np = p[q] - lr * mh / (sqrtf(vh) + eps);
-            for (int r = 0; r < MLP_CLUSTER; r++) cl.map_shared_rank(p, r)[q] = np;
+        cl.barrier_wait();
+        if (mine) {
+            float part[MLP_CLUSTER], gs = 0.f;
+#pragma unroll
+            for (int r = 0; r < MLP_CLUSTER; r++) part[r] = cl.map_shared_rank(gpart, r)[qs];
+#pragma unroll
+            for (int r = 0; r < MLP_CLUSTER; r++) gs += part[r];
+            am = b1c * am + (1.f - b1c) * gs;
+            av = b2c * av + (1.f - b2c) * gs * gs;
+            const float mh = am / (1.f - pow1), vh = av / (1.f - pow2);
+            const float np = p[qs] - lr * mh / (sqrtf(vh) + eps);
+#pragma unroll
+            for (int r = 0; r < MLP_CLUSTER; r++) cl.map_shared_rank(p, r)[qs] = np;
         }
         cl.sync();
     }
     if (rank == 0)
-        for (int q = tid; q < MLP_PARAMS; q += MLP_TRAIN_THREADS) params[q] = p[q];
+        for (int i = tid; i < MLP_PARAMS; i += MLP_TRAIN_THREADS) params[i] = p[s_index(i)];
 }
 
-// Seeded initialisation (uniform Glorot ranges) written to params.
+// Seeded initialisation (uniform Glorot ranges) of parameter q.
+__device__ float mlp_init_param(int q, uint64_t seed) {
+    const double u = (double)(mix64(seed ^ mix64(0xC0FFEE + q)) >> 11) * (1.0 / 9007199254740992.0);
+    float a;
+    if (q < MLP_H) a = sqrtf(6.f / (1 + MLP_H)) * 4.f;                     // W1: spread over the rank range
+    else if (q < 2 * MLP_H) a = 1.f;                                        // b1
+    else if (q < 2 * MLP_H + MLP_H * MLP_H) a = sqrtf(6.f / (2 * MLP_H));  // W2
+    else if (q < 3 * MLP_H + MLP_H * MLP_H) a = 0.1f;                       // b2
+    else if (q < 4 * MLP_H + MLP_H * MLP_H) a = sqrtf(6.f / (MLP_H + 1));  // W3
+    else a = 0.f;                                                           // b3
+    return (float)((2.0 * u - 1.0) * a);
+}
+
 __global__ void k_mlp_init(float *params, uint64_t seed) {
-    for (int q = threadIdx.x; q < MLP_PARAMS; q += blockDim.x) {
-        const double u = (double)(mix64(seed ^ mix64(0xC0FFEE + q)) >> 11) * (1.0 / 9007199254740992.0);
-        float a;
-        if (q < MLP_H) a = sqrtf(6.f / (1 + MLP_H)) * 4.f;                     // W1: spread over the rank range
-        else if (q < 2 * MLP_H) a = 1.f;                                        // b1
-        else if (q < 2 * MLP_H + MLP_H * MLP_H) a = sqrtf(6.f / (2 * MLP_H));  // W2
-        else if (q < 3 * MLP_H + MLP_H * MLP_H) a = 0.1f;                       // b2
-        else if (q < 4 * MLP_H + MLP_H * MLP_H) a = sqrtf(6.f / (MLP_H + 1));  // W3
-        else a = 0.f;                                                           // b3
-        params[q] = (float)((2.0 * u - 1.0) * a);
-    }
+    for (int q = threadIdx.x; q < MLP_PARAMS; q += blockDim.x) params[q] = mlp_init_param(q, seed);
 }
 
 size_t mlp_train_smem() {
-    return (size_t)(2 * MLP_PARAMS_PAD + 2 * MLP_SLICE) * 4 + sizeof(BatchSmem) + (size_t)3 * MLP_STAGE * 4;
+    return (size_t)2 * S_PAD * 4 + sizeof(BatchSmem) + (size_t)3 * MLP_STAGE * 4;
 }
-size_t mlp_grad_smem() { return (size_t)2 * MLP_PARAMS_PAD * 4 + sizeof(BatchSmem); }
+size_t mlp_grad_smem() { return (size_t)2 * S_PAD * 4 + sizeof(BatchSmem); }
 
 cudaError_t launch_mlp_init(float *params, uint64_t seed, cudaStream_t st) {
     k_mlp_init<<<1, 256, 0, st>>>(params, seed);
@@ -424,26 +456,39 @@ cudaError_t launch_mlp_train(const float *xs, const float *ys, const float *cw, 
 // from the stride-sized stretch j of S at a seeded offset (a stratified 1%
 // sample read with coalesced loads).  One warp per block; every block lies
 // inside S (stride * nblocks <= nS / SAMPLE_BLOCK).
-__global__ void k_sample_blocks(const Row *__restrict__ S, uint32_t *__restrict__ keys, uint64_t nblocks,
-                                uint64_t stride, uint64_t seed) {
+// The same launch sets up what the learning stage's kernels add to (the count
+// table, the bins, the decision, the heavy table) and the model's initial
+// parameters: six launches less on the path to the decision, and the 134 MB
+// table of |S| = 2^29 is cleared while the sample is read (92 + 36 us apart).
+__global__ void __launch_bounds__(256) k_learn_start(const Row *__restrict__ S, LearnBufs b, uint64_t nblocks,
+                                                     uint64_t stride, uint32_t *hkeys, unsigned *hcnt, uint64_t seed) {
     const int lane = threadIdx.x & 31;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t j = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < nblocks; j += nw) {
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
+    auto fill = [&](void *at, size_t bytes, uint32_t v) {
+        for (uint64_t i = tid; i < bytes / 4; i += nt) reinterpret_cast<uint32_t *>(at)[i] = v;
+    };
+    static_assert(sizeof(LrnDecision) % 4 == 0, "cleared by words");
+    for (uint64_t i = tid; i < ((uint64_t)b.tmask + 1) / 2; i += nt)
+        reinterpret_cast<ulonglong2 *>(b.table)[i] = make_ulonglong2(~0ull, ~0ull);  // CNT_EMPTY
+    fill(b.bin_rows, (size_t)CC_BINS * 12, 0);  // and bin_keys, which follow them
+    fill(b.dec, sizeof(LrnDecision), 0);
+    fill(hkeys, (size_t)HEAVY_CAP * 4, EMPTY_KEY);
+    fill(hcnt, (size_t)HEAVY_CAP * 16 + 16, 0);
+    for (uint64_t q = tid; q < MLP_PARAMS; q += nt) b.params[q] = mlp_init_param((int)q, seed);
+    for (uint64_t j = tid >> 5; j < nblocks; j += nt >> 5) {
         const uint64_t sb = j * stride + (stride > 1 ? mix64(seed ^ mix64(j + 0x51ED)) % stride : 0);
         const Row *src = S + sb * SAMPLE_BLOCK;
-        const uint2 a = ldg_stream(reinterpret_cast<const uint2 *>(src) + lane);
-        const uint2 b = ldg_stream(reinterpret_cast<const uint2 *>(src) + lane + 32);
-        keys[j * SAMPLE_BLOCK + lane] = a.x;
-        keys[j * SAMPLE_BLOCK + lane + 32] = b.x;
+        const uint2 x = ldg_stream(reinterpret_cast<const uint2 *>(src) + lane);
+        const uint2 y = ldg_stream(reinterpret_cast<const uint2 *>(src) + lane + 32);
+        b.keys[j * SAMPLE_BLOCK + lane] = x.x;
+        b.keys[j * SAMPLE_BLOCK + lane + 32] = y.x;
     }
 }
 
-cudaError_t launch_sample_blocks(const Row *S, uint64_t nS, uint32_t *keys, uint64_t nblocks, uint64_t stride,
-                                 uint64_t seed, cudaStream_t st) {
-    (void)nS;
-    if (!nblocks) return cudaSuccess;
-    const unsigned g = (unsigned)umin64((nblocks * 32 + 255) / 256, 148 * 16);
-    k_sample_blocks<<<g, 256, 0, st>>>(S, keys, nblocks, stride, seed);
+cudaError_t launch_learn_start(const Row *S, const LearnBufs &b, uint64_t nblocks, uint64_t stride, uint32_t *hkeys,
+                               unsigned *hcnt, uint64_t seed, cudaStream_t st) {
+    const uint64_t work = std::max<uint64_t>(nblocks * 32, HEAVY_CAP);
+    k_learn_start<<<(unsigned)umin64((work + 255) / 256, 148 * 16), 256, 0, st>>>(S, b, nblocks, stride, hkeys, hcnt, seed);
     count_launch();
     return cudaGetLastError();
 }
@@ -684,7 +729,7 @@ cudaError_t launch_count_stats(const LearnBufs &b, cudaStream_t st) {
 // spread over the points (so the network starts at the curve's mean and
 // learns its shape).  One block; writes the point count and the
 // normalisation to dec.
-__global__ void __launch_bounds__(1024) k_rank_points(const unsigned *__restrict__ bin_keys,
+__global__ void __launch_bounds__(1024, 2) k_rank_points(const unsigned *__restrict__ bin_keys,
                                                      const unsigned long long *__restrict__ bin_rows, float *xs,
                                                      float *ys, float *cw, LrnDecision *dec) {
     constexpr int PER = (CC_BINS + 1023) / 1024;
@@ -826,7 +871,7 @@ __global__ void __launch_bounds__(EVAL_THREADS) k_model_eval(const float *__rest
 constexpr int DECIDE_THREADS = 1024;
 constexpr int DECIDE_PER = (CC_BINS + DECIDE_THREADS - 1) / DECIDE_THREADS;
 
-__global__ void __launch_bounds__(DECIDE_THREADS) k_decide(int use_model, const unsigned *__restrict__ bin_keys,
+__global__ void __launch_bounds__(DECIDE_THREADS, 2) k_decide(int use_model, const unsigned *__restrict__ bin_keys,
                                                           const unsigned long long *__restrict__ bin_rows,
                                                           const float *__restrict__ lpred_model, double rows_scale,
                                                           double nS, double tau_min, double min_frac,
@@ -1282,24 +1327,55 @@ __global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass(BypassArgs a) {
 // bin and looked up in the bit table (L2); a heavy row is counted, and matches
 // when its key's bit is set, which the CTA looks up once per heavy key.  The
 // bypass saves the heavy rows' L2 lookups, one L1 line per clock and SM each.
-__global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass_direct(BypassArgs a) {
+//
+// The bound is the SM's load/store data path, so heavy keys are looked up in
+// the buckets (two 8-byte loads and one of the bit: 14 wavefronts a warp) only
+// where the key filter cannot tell: one word per hash slot, found by a
+// multiplication modulo 2^32.  That is a bijection, so slot and the remaining
+// hash bits identify a key, and the word has room for flags: the slot is
+// taken, R holds its key, more keys share the slot (the one case that goes to
+// the buckets; 6% of the heavy keys with the table full and 2^15 slots).
+// |S| = 2^29 at z = 1: 1.53 ms, 1.79 ms without the filter.  The rows it leaves
+// are looked up after the round's others, a lane at a time: tested in turn with
+// the others they cost more than the filter saved.
+constexpr uint32_t HF_USED = 1u << 31, HF_MATCH = 1u << 30, HF_MORE = 1u << 29;
+constexpr uint32_t HF_MUL = 0x9E3779B1u;  // odd
+
+__global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass_direct(BypassArgs a, int filter_log2) {
     if (!a.ctrl->direct) return;
     extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t *hkeys = reinterpret_cast<uint32_t *>(smem);  // 8-byte aligned buckets
-    uint32_t *hist = hkeys + HEAVY_CAP;
+    uint32_t *filter = reinterpret_cast<uint32_t *>(smem);
+    uint32_t *hist = filter + (1u << filter_log2);
     __shared__ uint32_t hbit[HEAVY_CAP / 32];  // the heavy keys that R holds
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t kmin = ~a.ctrl->direct_inv_min, span = a.ctrl->direct_max - kmin;
     const uint32_t wordmask = (uint32_t)((1ull << (a.ctrl->direct_log2 - 5)) - 1);
     auto word = [&](uint32_t key) { return key - kmin <= span ? ldg_no_l1(a.bits + ((key >> 5) & wordmask)) : 0u; };
+    const int fshift = 32 - filter_log2;
+    const uint32_t fmask = (1u << fshift) - 1;  // the key's hash bits beside its slot (below 2^29)
     for (int i = tid; i < a.nbins; i += BYP_THREADS) hist[i] = 0;
+    for (int i = tid; i < 1 << filter_log2; i += BYP_THREADS) filter[i] = 0;
+    __syncthreads();
     for (int i = tid; i < HEAVY_CAP; i += BYP_THREADS) {
         const uint32_t k = a.hkeys[i];
-        hkeys[i] = k;
-        const unsigned b = __ballot_sync(0xffffffffu, k != EMPTY_KEY && ((word(k) >> (k & 31)) & 1u));
+        const bool hit = k != EMPTY_KEY && ((word(k) >> (k & 31)) & 1u);
+        const unsigned b = __ballot_sync(0xffffffffu, hit);
         if (lane == 0) hbit[i >> 5] = b;
+        if (k != EMPTY_KEY) {
+            const uint32_t h = k * HF_MUL;
+            uint32_t *f = &filter[h >> fshift];
+            if (atomicCAS(f, 0u, HF_USED | (hit ? HF_MATCH : 0u) | (h & fmask)) != 0u) atomicOr(f, HF_MORE);
+        }
     }
     __syncthreads();
+    // bit 0: the key is heavy, bit 1: and R holds it
+    auto heavy_key = [&](uint32_t key) -> unsigned {
+        const uint32_t h = key * HF_MUL, f = filter[h >> fshift];
+        if ((f & (HF_USED | fmask)) == (HF_USED | (h & fmask))) return f & HF_MATCH ? 3u : 1u;
+        if (!(f & HF_MORE)) return 0u;
+        const int slot = heavy_lookup(a.hkeys, key);
+        return slot < 0 ? 0u : 1u | ((hbit[slot >> 5] >> (slot & 31)) & 1u) << 1;
+    };
     const uint64_t lo = (uint64_t)blockIdx.x * a.chunk;
     const uint64_t hi = umin64(a.n, lo + a.chunk);
     const uint32_t len = hi > lo ? (uint32_t)(hi - lo) : 0u;  // a chunk holds < 2^32 rows
@@ -1330,15 +1406,31 @@ __global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass_direct(BypassArg
         }
         load_round(base + ROUND);  // the next round's loads go out before this round's work
         uint32_t bw[2 * BYP_U];
-        unsigned hm = 0;
+        unsigned hm = 0, more = 0;  // heavy rows; rows the filter leaves to the buckets
 #pragma unroll
         for (int j = 0; j < 2 * BYP_U; j++) {
-            const int slot = heavy_lookup(hkeys, k[j]);
-            const bool heavy = slot >= 0 && (valid >> j & 1);
-            hm |= heavy ? 1u << j : 0u;
-            matches += heavy ? (hbit[slot >> 5] >> (slot & 31)) & 1u : 0u;
-            bw[j] = (valid >> j & 1) && !heavy ? word(k[j]) : 0u;
+            const uint32_t h = k[j] * HF_MUL, f = filter[h >> fshift];
+            const bool same = (f & (HF_USED | fmask)) == (HF_USED | (h & fmask));
+            hm |= same ? 1u << j : 0u;
+            matches += same && (valid >> j & 1) ? f >> 30 & 1u : 0u;
+            more |= !same && (f & HF_MORE) ? 1u << j : 0u;
         }
+        // few rows, so each lane takes its next one: one or two turns a warp
+        for (more &= valid; __any_sync(0xffffffffu, more); more &= more - 1) {
+            const int j = __ffs(more) - 1;
+            uint32_t key = EMPTY_KEY;  // never heavy
+#pragma unroll
+            for (int i = 0; i < 2 * BYP_U; i++) key = i == j ? k[i] : key;
+            if (j < 0) continue;
+            const int slot = heavy_lookup(a.hkeys, key);
+            if (slot >= 0) {
+                hm |= 1u << j;
+                matches += (hbit[slot >> 5] >> (slot & 31)) & 1u;
+            }
+        }
+        hm &= valid;
+#pragma unroll
+        for (int j = 0; j < 2 * BYP_U; j++) bw[j] = (valid & ~hm) >> j & 1 ? word(k[j]) : 0u;
         heavy_rows += __popc(hm);
         const unsigned km = valid & ~hm;
         const bool dup = warp_has_dups(radix_f(a.rf, k[0]), km & 1u);
@@ -1349,10 +1441,10 @@ __global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass_direct(BypassArg
     }
     if (tid == 0) {
         auto edge = [&](uint32_t key) {
-            const int slot = heavy_lookup(hkeys, key);
-            if (slot >= 0) {
+            const unsigned hk = heavy_key(key);
+            if (hk) {
                 heavy_rows++;
-                matches += (hbit[slot >> 5] >> (slot & 31)) & 1u;
+                matches += hk >> 1;
             } else {
                 atomicAdd(&hist[radix_f(a.rf, key)], 1u);
                 matches += (word(key) >> (key & 31)) & 1u;
@@ -1508,9 +1600,13 @@ cudaError_t launch_hist_bypass(const BypassArgs &a, bool mat, cudaStream_t st) {
     kern<<<a.G, BYP_THREADS, smem, st>>>(a);
     count_launch();
     if (!mat && a.bits) {
-        const size_t smem_d = (size_t)HEAVY_CAP * 4 + (size_t)a.nbins * 4;
+        // The filter as large as keeps it and the bins within 160 KB: the L1
+        // holds the lines of the light rows' lookups in flight, and at 192 KB
+        // |S| = 2^29 with its 8 MB bit table took 3.20 ms in place of 2.67.
+        const int flog = a.nbins <= 1 << 13 ? 15 : a.nbins <= 1 << 14 ? 14 : 13;
+        const size_t smem_d = ((size_t)4 << flog) + (size_t)a.nbins * 4;
         if ((e = smem_limit((const void *)k_hist_bypass_direct, smem_d)) != cudaSuccess) return e;
-        k_hist_bypass_direct<<<a.G, BYP_THREADS, smem_d, st>>>(a);
+        k_hist_bypass_direct<<<a.G, BYP_THREADS, smem_d, st>>>(a, flog);
         count_launch();
     }
     return cudaGetLastError();

@@ -16,7 +16,7 @@ constexpr int MLP_PARAMS = 2 * MLP_H + MLP_H * MLP_H + 2 * MLP_H + 1;
 constexpr int MLP_PARAMS_PAD = 1184;  // stride of parameter-sized arrays (>= MLP_PARAMS)
 constexpr int MLP_CLUSTER = 8;        // CTAs of the training cluster
 constexpr int MLP_BATCH_CTA = 128;    // samples per CTA per step
-constexpr int MLP_TRAIN_THREADS = 512;  // trainer threads per CTA (the gradient sums are spread over them)
+constexpr int MLP_TRAIN_THREADS = 256;  // trainer threads per CTA
 constexpr int MLP_SLICE = 152;        // parameters updated by each CTA
 static_assert(MLP_PARAMS <= MLP_PARAMS_PAD, "parameter stride");
 static_assert(MLP_SLICE * MLP_CLUSTER >= MLP_PARAMS, "every parameter belongs to a slice");
@@ -143,8 +143,8 @@ struct LearnBufs {
     LrnDecision *dec;
     unsigned *err;
 };
-cudaError_t launch_sample_blocks(const Row *S, uint64_t nS, uint32_t *keys, uint64_t nblocks, uint64_t stride,
-                                 uint64_t seed, cudaStream_t st);
+cudaError_t launch_learn_start(const Row *S, const LearnBufs &b, uint64_t nblocks, uint64_t stride, uint32_t *hkeys,
+                               unsigned *hcnt, uint64_t seed, cudaStream_t st);
 cudaError_t launch_count_keys(const LearnBufs &b, uint64_t m, cudaStream_t st);
 cudaError_t launch_count_stats(const LearnBufs &b, cudaStream_t st);
 cudaError_t launch_rank_points(const LearnBufs &b, cudaStream_t st);

@@ -99,6 +99,7 @@ struct RadixGeom {
     bool direct_rows = false;      // ... of a materialising join: R's payloads instead of bits,
     tbg_row_out *rows = nullptr;   // ... S's read writes the rows here
     uint64_t rows_cap = 0;
+    int build_wave = 0;            // CTAs per launch of R's read into the table (0: all)
     Row *rel = nullptr;            // ... or, when set, a relation of (key, R payload) here (as many)
     bool keys = false;             // the partitions hold bare keys (counting joins)
     const Row *sample_S = nullptr;  // S, when it is there while R is read

@@ -222,3 +222,29 @@ def test_full_size_c3_configs(tbg, cuda, z, scatter):
         assert st1.used_fallback == 1 and st1.heavy_rows_S == 0
     else:  # the heavy keys leave partitioning: about half of S at z = 1, nearly all at z = 1.5
         assert st1.used_fallback == 0 and st1.heavy_rows_S > (0.4 if z == 1.0 else 0.9) * nS
+
+
+@pytest.mark.parametrize("hot,held,off", [(1, 1.0, 0), (60, 0.5, 1), (3000, 0.0, 0), (3500, 0.7, 1)])
+def test_direct_counting_bypass(tbg, oracle, cuda, hot, held, off):
+    """The heavy keys' filter of the direct counting join: from one key to a
+    table so full that keys share filter slots, keys of which R holds all,
+    some or none, and rows of the padding key; against the oracle and the
+    partitioned join's statistics."""
+    rng = np.random.default_rng(hot)
+    nR, nS = 300001, 1 << 22
+    keys = rng.permutation(np.arange(5, 5 + 2 * nR, dtype=np.int64))
+    inner, outer = keys[:nR], keys[nR:]
+    R, S = np.zeros(nR, dtype=oracle.ROW), np.zeros(nS + 1, dtype=oracle.ROW)
+    R["key"] = inner
+    n_in = int(round(hot * held))
+    hk = np.concatenate([inner[:n_in], outer[:hot - n_in]])
+    S["key"] = np.where(rng.random(nS + 1) < 0.6, hk[rng.integers(0, hot, nS + 1)], keys[rng.integers(0, 2 * nR, nS + 1)])
+    S["key"][:7] = 0xFFFFFFFF
+    oracle.fill_payloads(R, 0)
+    oracle.fill_payloads(S, 1)
+    ref = oracle.rho(R, S)
+    m, _, st = run_join(tbg, cuda, "LRN", R, S, offset=off)
+    m2, _, st2 = run_join(tbg, cuda, "LRN", R, S, offset=off, passes=st.passes)  # the partitioned join
+    assert m == m2 == ref
+    for f in ("heavy_keys", "heavy_rows_S", "used_fallback", "max_part_R", "max_part_S", "partitions"):
+        assert getattr(st, f) == getattr(st2, f), f
