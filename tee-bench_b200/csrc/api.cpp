@@ -172,7 +172,8 @@ void mark(Workspace &w, bool timing, int i, cudaStream_t st) {
 //   Counting joins, |R| <= 2^28: JOIN_CAPR_WIDE, so the radix geometry is the
 //   one whose average R partition fills a JOIN_CAPR_FIT-row table (14 bits,
 //   7 + 7, at |R| = 2^27, where half-full 5120-row tables need 15 bits,
-//   7 + 8).  The join then launches a JOIN_CAPR_FIT-row table kernel and a
+//   7 + 8); both figures are of the tables with payload-sized cells, whose
+//   kernels held 8192 rows.  The join then launches a JOIN_CAPR_FIT-row table kernel and a
 //   JOIN_CAPR_WIDE one, each gated on the largest R partition (device
 //   memory).  Measured at 2^27 x 2^30: 11.41 ms against 12.28 ms; the
 //   8-bit fan-out of the second pass costs more than the bigger tables.

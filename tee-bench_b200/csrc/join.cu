@@ -7,6 +7,8 @@
 //   layout 1  histogram_join (Joins/radix_join.c:374-440, RHT): bucket counts
 //             over max(next_pow2(|R_p|)/4, 4) slots, prefix sum, R_p reordered
 //             by bucket, probe scans the bucket's range.
+// These are the materialising tables.  Counting joins of both layouts build a
+// CellTable (join_dev.cuh: 32-bit heads and cells) over partitions of bare keys.
 // Counting uses per-thread counters folded once per CTA; materialisation
 // reserves output rows once per CTA round (one global atomic for up to
 // JOIN_THREADS * 8 probe rows) and places them in (row slot, lane) order, so

@@ -19,7 +19,8 @@
 //
 // One histogram read gives every cursor of both passes, so the traffic is
 // 8 (hist) + 16 (pass 1) + 16 (pass 2) bytes per row, and no CTA ever waits
-// for another.  Each pass stages a tile digit-sorted in shared memory and
+// for another.  A counting join needs no payloads: its pass 1 writes bare keys
+// and pass 2 moves those, 8 + 12 + 8 bytes per row.  Each pass stages a tile digit-sorted in shared memory and
 // writes runs with consecutive threads on consecutive addresses (coalesced).
 #include "part_dev.cuh"
 
