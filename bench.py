@@ -623,8 +623,9 @@ def main():
             del pR, pS
 
     peak, peak_kind = read_peaks()
-    # algorithmic bytes: histogram reads 8 B/row; each partitioning pass
-    # reads and writes 8 B/row; build/probe reads 8 B/row
+    # algorithmic bytes: the histogram reads 8 B/row; a counting join's first
+    # pass reads rows and writes keys (12 B/row), its second moves keys (8) and
+    # build/probe reads keys (4); a materialising join moves whole rows
     rows = nR + nS
     K = args.steps
     passes = st.passes or 2
@@ -644,37 +645,29 @@ def main():
                                    "the lookups in the L2-resident table, not by HBM",
                     "timing": "CUDA events around the timed joins on their stream"}
     elif algo in ("RHO", "RHT") and not mat:
-        scat_bytes = 16 * rows * passes
+        scat_bytes = (12 + 8 * (passes - 1)) * rows
         achieved = scat_bytes / (scat_ms / 1e3) / 1e9 if scat_ms > 0 else None
-        traffic, traffic_source = None, None
-        tp = os.path.join(ROOT, "profiles", "ncu_traffic.json")
-        geom = (f"B{st.radix_bits}_{st.radix_bits // 2}+{st.radix_bits - st.radix_bits // 2}" if passes == 2
-                else f"B{st.radix_bits}")
-        if os.path.exists(tp):
-            with open(tp) as f:
-                tt = json.load(f)
-            k = tt.get("k_part_pass", {}).get(geom)
-            if k:  # DRAM bytes per row moved at this radix geometry, from one ncu capture
-                traffic = k["dram_bytes_per_row"] * rows * passes
-                traffic_source = f"profiles/ncu_traffic.json [{geom}]: {k['source']}"
-        total_bytes = (8 + 16 * passes + 8) * rows
+        total_bytes = 8 * rows + scat_bytes + 4 * rows
         roofline = {"bound": "hbm",
-                    "kernel": f"k_part_pass1 + k_part_pass2 ({passes} partitioning passes over R and S, "
-                              f"{2 * passes} launches per join)",
+                    "kernel": f"k_part_pass1 + k_part_pass2 ({passes} partitioning passes over R and S, bare keys)",
                     "achieved": achieved, "peak": peak, "unit": "GB/s",
-                    "frac": achieved / peak if achieved else None, "traffic": traffic,
-                    "traffic_source": traffic_source or f"no ncu capture at radix geometry {geom}",
+                    "frac": achieved / peak if achieved else None, "traffic": None,
                     "peak_source": peak_source,
-                    "algorithmic_bytes_per_row_per_pass": 16,
+                    "algorithmic_bytes_per_row": 12 + 8 * (passes - 1),
                     "timing": "library CUDA events on the join stream around each pass, summed over "
                               "the timed steps",
-                    "pipeline": {"bytes_per_row": 8 + 16 * passes + 8,
+                    "pipeline": {"bytes_per_row": 12 + 12 + 8 * (passes - 1),
                                  "achieved_gbs": total_bytes / (pipe_ms / 1e3) / 1e9,
                                  "frac": total_bytes / (pipe_ms / 1e3) / 1e9 / peak}}
     else:
         # whole join: LRN's learning and bypass run on two streams and PSM's
         # sort passes are not radix passes, so the pipeline is the unit
-        if algo == "PSM" and st.partitions:
+        if not mat or (algo != "LRN" and scat_ms < 0.05 * pipe_ms):
+            # what the join cannot do without, whichever way it went (direct,
+            # or partitioned and counted)
+            alg = 8 * rows
+            model = "every row of R and S read once (8 B)"
+        elif algo == "PSM" and st.partitions:
             # MSD sort: R's key range, histogram (it checks S's keys against
             # R's range), radix passes by the top bits, one bucket-sort pass
             # (its re-reads of a bucket come from L2), merge
@@ -907,20 +900,12 @@ def sharded_main(args, rank, world, local):
 
 
 # ------------------------------------------------------------------ batch
-def batch_algorithmic_bytes(dj, desc):
-    """Bytes each join must move under the plan's choices: partitioned joins
-    8 (histogram) + 16 (scatter) + 8 (build/probe) per row; direct joins read
-    S once and R once per S slice."""
-    choice = {c["log2_R"]: c for c in desc["classes"]}
+def batch_algorithmic_bytes(dj):
+    """Bytes each join cannot do without: every row read once."""
     total = 0
     for (_, nR, _, nS) in dj:
-        if not nR or not nS:
-            continue
-        c = choice[int(nR).bit_length() - 1]
-        if c["bits"] > 0:
-            total += 32 * (nR + nS)
-        else:
-            total += 8 * nS + 8 * nR * (-(-nS // c["capS"]))
+        if nR and nS:
+            total += 8 * (nR + nS)
     return total
 
 
@@ -1034,7 +1019,7 @@ def batch_main(args, rank, world, local):
     K = args.steps
     value = job_mtuples(world, rows, K, ms / 1e3)
     peak, peak_kind = read_peaks()
-    alg = batch_algorithmic_bytes(dj, desc)
+    alg = batch_algorithmic_bytes(dj)
     achieved = alg / (ms / K / 1e3) / 1e9
 
     # e2e through the public batch API: each step copies every join's inputs
