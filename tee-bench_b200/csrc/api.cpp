@@ -438,15 +438,18 @@ void try_direct(RadixGeom &g, const tbg_config &cfg, tbg_row_out *d_rows, uint64
 }
 
 // Start of a join: the control block cleared, and with g.direct
-// the table sized and cleared (dR is read).
-int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st) {
+// the table sized and cleared (dR is read).  Without memory for the table the
+// join is not direct.
+int start_radix_join(RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st) {
+    const int lg = g.direct_rows ? direct_log2_max_rows(g.n[0]) : direct_log2_max(g.n[0]);
+    if (g.direct && w.direct.ensure((size_t)1 << (g.direct_rows ? lg + 2 : lg - 3)) != cudaSuccess) {
+        cudaGetLastError();
+        g.direct = false;
+    }
     cudaError_t e;
     if (!g.direct) {
         e = cudaMemsetAsync(w.ctrl.p, 0, sizeof(Ctrl), st);
     } else {
-        const int lg = g.direct_rows ? direct_log2_max_rows(g.n[0]) : direct_log2_max(g.n[0]);
-        if ((e = w.direct.ensure((size_t)1 << (g.direct_rows ? lg + 2 : lg - 3))) != cudaSuccess)
-            return cuda_error(e, "cudaMalloc");
         e = launch_direct_prep(dR, g.n[0], w.direct.as<uint32_t>(), lg, g.direct_rows, w.ctrl.as<Ctrl>(), w.nsm, st);
     }
     return e == cudaSuccess ? TBG_OK : cuda_error(e, "start of the join");
@@ -609,6 +612,7 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
         const Row *d = dS + s_lo[k];
         RadixGeom g = radix_geometry(cfg, nR, n, capR, w);
         try_direct(g, cfg, d_rows, cap);
+        g.direct = gmax.direct;
         if ((e = cudaStreamWaitEvent(st, s_ready[k], 0)) != cudaSuccess) return cuda_error(e, "sliced join: wait");
         if ((rc = part_hist_read(1, g, d, cfg, w, st, nullptr))) return rc;
         if ((rc = part_hist_plan(2, true, g, w, st))) return rc;

@@ -41,16 +41,19 @@ static int join_relation(const tbg_config &cfg, const Row *dR, uint64_t nR, cons
     uint64_t cap = std::max<uint64_t>(nS, 1);
     for (int attempt = 0; attempt < 2; attempt++) {
         cudaError_t e = w.chain_rows.ensure(cap * sizeof(tbg_row_out));
-        if (e == cudaSuccess) e = w.chain_rel.ensure(cap * sizeof(Row));
         if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (chain rows)");
         JoinRun run;
         run.waits = true;
-        run.rel = w.chain_rel.as<Row>();
+        // no room for |S| tuples: rows, and a relation of as many as there are
+        if (w.chain_rel.ensure(cap * sizeof(Row)) == cudaSuccess) run.rel = w.chain_rel.as<Row>();
+        else cudaGetLastError();
         Workspace *jw = nullptr;
         int rc = join_device_impl(&c, dR, nR, dS, nS, w.chain_rows.as<tbg_row_out>(), cap, st, &run, &jw);
         if (rc == TBG_OK) rc = finish_join(c, *jw, st, run, nR, nS, cap, m, nullptr);
         if (rc == TBG_OK) {
             if (run.rel_done) return TBG_OK;
+            e = w.chain_rel.ensure(std::max<uint64_t>(*m, 1) * sizeof(Row));
+            if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (chain relation)");
             e = launch_rows_to_relation(w.chain_rows.as<tbg_row_out>(), *m, w.chain_rel.as<Row>(), w.nsm, st);
             return e == cudaSuccess ? TBG_OK : cuda_error(e, "to_relation");
         }

@@ -1350,7 +1350,11 @@ __global__ void __launch_bounds__(BYP_THREADS, 1) k_hist_bypass_direct(BypassArg
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t kmin = ~a.ctrl->direct_inv_min, span = a.ctrl->direct_max - kmin;
     const uint32_t wordmask = (uint32_t)((1ull << (a.ctrl->direct_log2 - 5)) - 1);
-    auto word = [&](uint32_t key) { return key - kmin <= span ? ldg_no_l1(a.bits + ((key >> 5) & wordmask)) : 0u; };
+    // Through the L1: the light rows' most frequent keys may be neighbours, a few
+    // lines of the table that all SMs would ask of the same L2 slices (2^26 x
+    // 2^29, z = 1, rank = key: 5.04 ms past the L1, 2.28 through it; ranks
+    // scattered over the keys: 2.40 and 2.43).
+    auto word = [&](uint32_t key) { return key - kmin <= span ? __ldg(a.bits + ((key >> 5) & wordmask)) : 0u; };
     const int fshift = 32 - filter_log2;
     const uint32_t fmask = (1u << fshift) - 1;  // the key's hash bits beside its slot (below 2^29)
     for (int i = tid; i < a.nbins; i += BYP_THREADS) hist[i] = 0;

@@ -109,7 +109,7 @@ RadixGeom radix_geometry_msd(uint64_t nR, uint64_t nS, uint32_t sub, int B, int 
 int ensure_radix_buffers(const RadixGeom &g, bool bypass, Workspace &w);
 bool automatic_plan(const tbg_config &cfg);
 void try_direct(RadixGeom &g, const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap);
-int start_radix_join(const RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st);
+int start_radix_join(RadixGeom &g, const Row *dR, Workspace &w, cudaStream_t st);
 int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &cfg, Workspace &w, cudaStream_t st,
                    const SBypass *bypass);
 int part_hist_plan(int rels, bool items, const RadixGeom &g, Workspace &w, cudaStream_t st);
