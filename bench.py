@@ -633,7 +633,7 @@ def main():
     peak_source = (f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                    else "fallback 6650 GB/s")
     scat_ms = (phase["ms_pass1"] + phase["ms_pass2"]) / K
-    if algo in ("RHO", "RHT") and not mat and scat_ms < 0.05 * pipe_ms:
+    if algo in ("RHO", "RHT") and not mat and st.path == tbg.PATH_DIRECT:
         # the direct counting join: S is joined in its histogram read, nothing
         # is partitioned
         achieved = 8 * rows / (pipe_ms / 1e3) / 1e9
@@ -662,7 +662,7 @@ def main():
     else:
         # whole join: LRN's learning and bypass run on two streams and PSM's
         # sort passes are not radix passes, so the pipeline is the unit
-        if not mat or (algo != "LRN" and scat_ms < 0.05 * pipe_ms):
+        if not mat or st.path == tbg.PATH_DIRECT:
             # what the join cannot do without, whichever way it went (direct,
             # or partitioned and counted)
             alg = 8 * rows

@@ -187,6 +187,14 @@ typedef struct tbg_row_out { /* one materialised row, 12 bytes */
     uint32_t Spayload;
 } tbg_row_out;
 
+/* how a join was done (tbg_stats.path) */
+enum {
+    TBG_PATH_PARTITIONED = 0, /* partitioning or sorting passes, then build/probe or merge   */
+    TBG_PATH_DIRECT = 1,      /* R's distinct keys in a table by key value, S joined as it is
+                                 read; the statistics are those of the passes not taken      */
+    TBG_PATH_SMALL = 2        /* R's table whole in every CTA, one launch; likewise          */
+};
+
 typedef struct tbg_stats {
     uint64_t matches;
     uint64_t partitions;        /* final partitions                          */
@@ -197,6 +205,7 @@ typedef struct tbg_stats {
     double predicted_imbalance; /* LRN: the model's own estimate            */
     int radix_bits, passes;
     int used_fallback;          /* LRN fell back to radix partitioning       */
+    int path;                   /* TBG_PATH_*                                */
     uint64_t heavy_keys;        /* LRN: keys joined by the heavy path        */
     uint64_t heavy_rows_S;      /* LRN: S rows that skipped partitioning     */
     int train_steps;
@@ -314,8 +323,9 @@ TBG_API int tbg_batch_run(tbg_batch *b, uint64_t *d_counts, void *stream);
 /* Waits for the last run; returns its device status (TBG_ERR_TIMEOUT if a
  * bounded wait inside the kernel gave up). */
 TBG_API int tbg_batch_sync(tbg_batch *b);
-/* JSON summary of the plan (grid, tickets, per-size-class choices and tuned
- * times) into buf[cap]; returns the full length. */
+/* JSON summary of the plan (grid, tickets, joins with a bit table,
+ * per-size-class choices and tuned times) into buf[cap]; returns the full
+ * length. */
 TBG_API int tbg_batch_describe(const tbg_batch *b, char *buf, size_t cap);
 TBG_API void tbg_batch_destroy(tbg_batch *b);
 

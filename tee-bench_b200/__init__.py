@@ -29,6 +29,7 @@ OUT_ROW = np.dtype([("key", "<u4"), ("Rpayload", "<u4"), ("Spayload", "<u4")])
 OK, ERR_ARG, ERR_CUDA, ERR_OOM, ERR_TIMEOUT, ERR_CAPACITY, ERR_UNKNOWN_ALGO, ERR_NO_DEVICE = range(8)
 RHO_ID, RHT_ID, RSM_ID, PSM_ID, LRN_ID = range(5)
 ALGO_IDS = {"RHO": RHO_ID, "RHT": RHT_ID, "RSM": RSM_ID, "PSM": PSM_ID, "LRN": LRN_ID}
+PATH_PARTITIONED, PATH_DIRECT, PATH_SMALL = range(3)
 MODEL_MLP, MODEL_SAMPLE, MODEL_UNTRAINED, MODEL_UNIFORM = range(4)
 ERRMODE_EXIT, ERRMODE_RETURN = 0, 1
 
@@ -81,7 +82,7 @@ class Stats(C.Structure):
                 ("mean_part_R", C.c_double), ("mean_part_S", C.c_double),
                 ("imbalance", C.c_double), ("predicted_imbalance", C.c_double),
                 ("radix_bits", C.c_int), ("passes", C.c_int), ("used_fallback", C.c_int),
-                ("heavy_keys", C.c_uint64), ("heavy_rows_S", C.c_uint64),
+                ("path", C.c_int), ("heavy_keys", C.c_uint64), ("heavy_rows_S", C.c_uint64),
                 ("train_steps", C.c_int), ("train_loss", C.c_float),
                 ("kernel_launches", C.c_uint32),
                 ("ms_hist", C.c_float), ("ms_pass1", C.c_float), ("ms_pass2", C.c_float),

@@ -706,6 +706,7 @@ int finish_join(const tbg_config &cfg, Workspace &w, cudaStream_t st, JoinRun &r
         stats->heavy_keys = c.heavy_keys;
         stats->heavy_rows_S = c.heavy_rows_S;
         stats->used_fallback = run.used_fallback;
+        stats->path = run.small ? TBG_PATH_SMALL : c.direct ? TBG_PATH_DIRECT : TBG_PATH_PARTITIONED;
         stats->predicted_imbalance = run.predicted_imbalance;
         stats->train_steps = run.train_steps;
         stats->train_loss = run.train_loss;

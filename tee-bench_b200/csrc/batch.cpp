@@ -70,6 +70,7 @@ struct Plan {
     uint64_t rows = 0;  // input rows covered by the plan
     uint32_t tickets = 0;
     std::vector<int> order;  // caller's index of each join of the plan
+    int bit_tables = 0;      // joins with a bit table
 };
 
 int validate(const tbg_batch_join *joins, int njoins) {
@@ -241,7 +242,11 @@ int build_plan(const tbg_batch_join *joins, int njoins, const std::vector<int> &
     p.njoins = njoins;
     p.rows = rows;
     p.order.clear();
-    for (const BatchJoin &J : bj) p.order.push_back((int)J.orig);
+    p.bit_tables = 0;
+    for (const BatchJoin &J : bj) {
+        p.order.push_back((int)J.orig);
+        p.bit_tables += J.bits_log2 != 0;
+    }
     p.tickets = a.n_builds + a.n_dchunks + 2 * a.n_chunks + a.n_scans + a.n_jt;
     return TBG_OK;
 }
@@ -545,6 +550,7 @@ TBG_API int tbg_batch_describe(const tbg_batch *b, char *buf, size_t cap) {
     if (!b) return set_error(TBG_ERR_ARG, "tbg_batch_describe: NULL batch");
     std::string s = "{\"grid\": " + std::to_string(b->plan.grid) + ", \"tickets\": " +
                     std::to_string(b->plan.tickets) + ", \"chunks\": " + std::to_string(b->plan.args.n_chunks) +
+                    ", \"bit_tables\": " + std::to_string(b->plan.bit_tables) +
                     ", \"rows\": " + std::to_string(b->plan.rows) + ", \"tune_ms\": " +
                     std::to_string(b->tune_ms) + ", \"classes\": [";
     bool first = true;

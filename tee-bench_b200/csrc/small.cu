@@ -284,6 +284,7 @@ int run_small_join(const tbg_config &cfg, const RadixGeom &g, const Row *dR, con
     run->passes = g.passes;
     run->P = g.P;
     run->ctrl_on_host = run->waits;
+    run->small = true;
     return TBG_OK;
 }
 

@@ -60,6 +60,7 @@ struct JoinRun {
     Row *rel = nullptr;         // a direct join may write a relation here instead of its rows (chained joins)
     bool rel_done = false;      // ... and did (before finish_join: may have)
     bool ctrl_on_host = false;  // the join's last kernel writes host_ctrl itself
+    bool small = false;         // one launch (small.cu)
 };
 
 Workspace *workspace_for(cudaStream_t st);
