@@ -149,12 +149,15 @@ static bool msd_bits(int span, int *B, int *lowbits) {
     return *B >= 1 && *lowbits <= kLowBitsMax;
 }
 
-cudaError_t launch_bucket_count(const JoinArgs &a, uint32_t sub, int lowbits, int nsm, cudaStream_t st);
+uint64_t heavy_bucket_rows(uint64_t nR, int nsm);
+cudaError_t launch_bucket_count(const JoinArgs &a, const HeavyBuckets &hv, uint32_t sub, int lowbits, int nsm,
+                                cudaStream_t st);
 
 // Count-only PSM on MSD buckets: both relations partitioned by the top bits of
 // key - sub (sub: R's smallest key), then k_bucket_count.  Nothing waits, and
 // neither S's keys outside R's range nor heavy keys (S's buckets are split over
-// CTAs by the planner) need another plan.
+// CTAs by the planner, R's rows of a large bucket counted once) need another
+// plan.
 // lsd_passes > 0: the range has no bits above the low ones, where the sort
 // would be an LSD sort of that many passes; the buckets do for it too.
 static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, uint32_t sub, int B,
@@ -193,7 +196,19 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     ja.matches = &ctrl->matches;
     ja.err = &ctrl->error;
     ja.skip = &ctrl->direct;
-    const cudaError_t e = launch_bucket_count(ja, sub, lowbits, w.nsm, st);
+    HeavyBuckets hv;
+    hv.rows = heavy_bucket_rows(nR, w.nsm);
+    if (nR <= hv.rows) {
+        hv.rows = 0;  // no bucket can be
+    } else if (w.aux[5].ensure(((nR / hv.rows + 1) << lowbits) * 4) != cudaSuccess) {
+        cudaGetLastError();
+        hv.rows = 0;  // no memory for the counters: every item counts its bucket's rows
+    }
+    hv.nR = nR;
+    hv.counters = w.aux[5].as<uint32_t>();
+    hv.base = w.baseR.as<uint64_t>();
+    hv.max_part = &ctrl->max_part_R;
+    const cudaError_t e = launch_bucket_count(ja, hv, sub, lowbits, w.nsm, st);
     if (e != cudaSuccess) return cuda_error(e, "bucket count");
     mark_ev(w, cfg.timing != 0, 4, st);
     run->B = lsd_passes ? 8 : B;

@@ -723,7 +723,82 @@ cudaError_t launch_join_rsm(const JoinArgs &a, bool materialize, int grid, cudaS
 // ---------------------------------------------------------------------------
 constexpr int BCOUNT_THREADS = 512;
 
-__global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, uint32_t sub, int lowbits) {
+// Buckets with more than HeavyBuckets::rows R rows (a hot key, or few distinct
+// ones) are counted once, by k_heavy_count, into counters in device memory that
+// every item of the bucket copies: an item that counted its bucket's R rows
+// again would read them once per S slice.  Bucket f's counters are at slot
+// base[f] / rows, its own since such buckets start more than `rows` apart.
+// 2^24 x 2^26 rows, R's keys 3000 values (two buckets): the count takes 104 us,
+// 5751 us with the rows counted per item; a quarter of both sides on one key:
+// 124 and 944 us.  Below the line an item's own count is the cheaper one: it
+// costs less than the item's S slice of 65,536 rows or more.
+__device__ __forceinline__ bool heavy_none(const JoinArgs &a, const HeavyBuckets &hv) {
+    return *a.skip || *a.err || *hv.max_part <= hv.rows;
+}
+
+__global__ void __launch_bounds__(BCOUNT_THREADS) k_heavy_clear(JoinArgs a, HeavyBuckets hv, uint64_t n4) {
+    dep_wait();
+    dep_trigger();
+    if (heavy_none(a, hv)) return;
+    uint4 *c4 = reinterpret_cast<uint4 *>(hv.counters);
+    for (uint64_t i = (uint64_t)blockIdx.x * BCOUNT_THREADS + threadIdx.x; i < n4; i += (uint64_t)gridDim.x * BCOUNT_THREADS)
+        c4[i] = make_uint4(0, 0, 0, 0);
+}
+
+// CTA c counts the heavy buckets' rows among R's rows [c * chunk, ...), which
+// the passes left in bucket order; a chunk holds parts of few heavy buckets
+// (each has more than half a chunk's rows).
+constexpr int HEAVY_PER_CHUNK = 8;
+
+__global__ void __launch_bounds__(BCOUNT_THREADS) k_heavy_count(JoinArgs a, HeavyBuckets hv, uint32_t sub, int lowbits,
+                                                                uint64_t chunk) {
+    extern __shared__ __align__(16) uint32_t hc_smem[];
+    __shared__ uint32_t list[HEAVY_PER_CHUNK], nlist;
+    dep_wait();
+    dep_trigger();
+    if (heavy_none(a, hv)) return;
+    constexpr int T = BCOUNT_THREADS;
+    const uint32_t *Rp = reinterpret_cast<const uint32_t *>(a.R);
+    const int tid = threadIdx.x;
+    const uint32_t bins = 1u << lowbits;
+    const uint64_t lo = (uint64_t)blockIdx.x * chunk, hi = umin64(hv.nR, lo + chunk);
+    if (lo >= hi) return;
+    if (tid == 0) nlist = 0;
+    __syncthreads();
+    const uint32_t f0 = (Rp[lo] - sub) >> lowbits, f1 = (Rp[hi - 1] - sub) >> lowbits;
+    for (uint32_t f = f0 + tid; f <= f1; f += T)
+        if (hv.base[f + 1] - hv.base[f] > hv.rows) {
+            const uint32_t at = atomicAdd(&nlist, 1u);
+            if (at < HEAVY_PER_CHUNK) list[at] = f;
+        }
+    __syncthreads();
+    for (uint32_t i = 0; i < min(nlist, (uint32_t)HEAVY_PER_CHUNK); i++) {
+        const uint32_t f = list[i], klo = sub + (f << lowbits);
+        const uint64_t b0 = hv.base[f] > lo ? hv.base[f] : lo, b1 = umin64(hv.base[f + 1], hi);
+        for (uint32_t b = tid; b < bins; b += T) hc_smem[b] = 0;
+        __syncthreads();
+        for (uint64_t at = b0; at < b1; at += 8 * T) {
+            uint32_t d[8];
+            bool ok[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const uint64_t q = at + u * T + tid;
+                d[u] = q < b1 ? __ldcs(Rp + q) - klo : ~0u;
+                ok[u] = d[u] < bins;
+            }
+            const bool dup = warp_has_dups(d[0], ok[0]);
+#pragma unroll
+            for (int u = 0; u < 8; u++) hist_add_warp(hc_smem, d[u], ok[u], dup);
+        }
+        __syncthreads();
+        uint32_t *dst = hv.counters + hv.base[f] / hv.rows * bins;
+        for (uint32_t b = tid; b < bins; b += T)
+            if (hc_smem[b]) atomicAdd(dst + b, hc_smem[b]);
+        __syncthreads();  // the counters are rewritten by the next bucket
+    }
+}
+
+__global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, HeavyBuckets hv, uint32_t sub, int lowbits) {
     extern __shared__ __align__(16) uint32_t bc_smem[];
     uint32_t *h = bc_smem;
     __shared__ uint32_t s_item[2];
@@ -734,6 +809,7 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
     const int tid = threadIdx.x;
     const uint32_t bins = 1u << lowbits;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
+    const bool heavy = hv.rows && *hv.max_part > hv.rows;
     unsigned long long local = 0;
     if (tid == 0) s_item[0] = atomicAdd(a.item_ctr, 1u);
     __syncthreads();
@@ -750,15 +826,24 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
         }
         const Item m = a.items[it];
         const uint32_t lo = sub + (m.part << lowbits);
-        for (uint32_t b = tid; b < bins / 4; b += BCOUNT_THREADS)
-            reinterpret_cast<uint4 *>(h)[b] = make_uint4(0, 0, 0, 0);
+        uint64_t s_len = m.s_len;
+        if (heavy && hv.base[m.part + 1] - hv.base[m.part] > hv.rows) {
+            // the bucket's counters, whole: with its first item of R rows (a
+            // bucket of more rows than one item takes has two)
+            if (m.r_off != hv.base[m.part]) s_len = 0;
+            const uint4 *src = reinterpret_cast<const uint4 *>(hv.counters + hv.base[m.part] / hv.rows * bins);
+            for (uint32_t b = tid; b < bins / 4; b += BCOUNT_THREADS) reinterpret_cast<uint4 *>(h)[b] = __ldcg(src + b);
+        } else {
+            for (uint32_t b = tid; b < bins / 4; b += BCOUNT_THREADS)
+                reinterpret_cast<uint4 *>(h)[b] = make_uint4(0, 0, 0, 0);
+            __syncthreads();
+            stream_sum<BCOUNT_THREADS>(Rp + m.r_off, m.r_len, [&](uint32_t k) {
+                if (k - lo < bins) atomicAdd(&h[k - lo], 1u);
+                return 0u;
+            });
+        }
         __syncthreads();
-        stream_sum<BCOUNT_THREADS>(Rp + m.r_off, m.r_len, [&](uint32_t k) {
-            if (k - lo < bins) atomicAdd(&h[k - lo], 1u);
-            return 0u;
-        });
-        __syncthreads();
-        local += stream_sum<BCOUNT_THREADS>(Sp + m.s_off, m.s_len, [&](uint32_t k) {
+        local += stream_sum<BCOUNT_THREADS>(Sp + m.s_off, s_len, [&](uint32_t k) {
             const uint32_t d = k - lo;
             return (unsigned long long)(d < bins ? h[d] : 0u);  // a bucket's count may take all 32 bits
         });
@@ -770,12 +855,27 @@ __global__ void __launch_bounds__(BCOUNT_THREADS, 3) k_bucket_count(JoinArgs a, 
 
 constexpr int BCOUNT_CTAS = 3;  // resident per SM (the launch bound; up to 64 KB of counters each)
 
-cudaError_t launch_bucket_count(const JoinArgs &a, uint32_t sub, int lowbits, int nsm, cudaStream_t st) {
+// R rows from which a bucket is counted once: a share of R that a CTA counts in
+// passing, and as many as half of the smallest S slice.  The counters take
+// (nR / heavy_bucket_rows + 1) << lowbits words, 19 MB at most.
+uint64_t heavy_bucket_rows(uint64_t nR, int nsm) { return std::max<uint64_t>(32768, nR / ((uint64_t)nsm * 4)); }
+
+cudaError_t launch_bucket_count(const JoinArgs &a, const HeavyBuckets &hv, uint32_t sub, int lowbits, int nsm,
+                                cudaStream_t st) {
     if (lowbits < 2 || lowbits > 14) return cudaErrorInvalidValue;
     const size_t smem = (size_t)4 << lowbits;
     cudaError_t e = smem_limit((const void *)k_bucket_count, smem);
+    if (e == cudaSuccess) e = smem_limit((const void *)k_heavy_count, smem);
     if (e != cudaSuccess) return e;
-    e = launch_dep(k_bucket_count, nsm * BCOUNT_CTAS, BCOUNT_THREADS, smem, st, a, sub, lowbits);
+    if (hv.rows) {
+        const uint64_t n4 = (hv.nR / hv.rows + 1) << (lowbits - 2);
+        if ((e = launch_dep(k_heavy_clear, nsm, BCOUNT_THREADS, 0, st, a, hv, n4)) != cudaSuccess) return e;
+        const uint64_t chunk = (hv.nR + 2 * nsm - 1) / (2 * nsm);
+        e = launch_dep(k_heavy_count, 2 * nsm, BCOUNT_THREADS, smem, st, a, hv, sub, lowbits, chunk);
+        if (e != cudaSuccess) return e;
+        count_launch(2);
+    }
+    e = launch_dep(k_bucket_count, nsm * BCOUNT_CTAS, BCOUNT_THREADS, smem, st, a, hv, sub, lowbits);
     count_launch();
     return e;
 }

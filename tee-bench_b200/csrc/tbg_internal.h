@@ -150,6 +150,15 @@ struct JoinArgs {
     unsigned int *err;
 };
 
+// Buckets of a counting PSM whose R rows are counted once (sortmerge.cu).
+struct HeavyBuckets {
+    uint64_t rows = 0;         // buckets with more R rows than this; 0: none
+    uint64_t nR = 0;
+    uint32_t *counters = nullptr;  // [nR / rows + 1][2^lowbits]
+    const uint64_t *base = nullptr;  // [P + 1] R's bucket starts
+    const unsigned long long *max_part = nullptr;  // the largest bucket of R
+};
+
 struct PlanArgs {
     RelPlan r, s;
     uint64_t nR, nS;
