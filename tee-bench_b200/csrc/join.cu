@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "join_dev.cuh"
 
@@ -26,8 +27,14 @@ namespace tbg {
 // table or less, see join_capacity).
 __host__ __device__ __forceinline__ uint32_t count_heads(int capR) { return floor_pow2((uint32_t)capR); }
 
+// S keys against a table with long runs (a function of its own, so that the
+// plain probe's registers are its own).
+__device__ __noinline__ unsigned long long probe_runs(const CellTable t, const uint32_t *s, uint64_t len) {
+    return stream_sum<JOIN_THREADS>(s, len, [&](uint32_t k) { return t.count<true>(k); });
+}
+
 template <bool MAT>
-__global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
+__global__ void __launch_bounds__(JOIN_THREADS, MAT ? 2 : 3) k_join(JoinArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_item[2];
     __shared__ uint64_t scan_scratch[JOIN_THREADS / 32 + 1];
@@ -40,6 +47,7 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
     }
     Table t;
     CellTable ct;
+    __shared__ std::conditional_t<MAT, uint32_t, LongRuns> runs;
     if (MAT) {
         t.key = reinterpret_cast<uint32_t *>(smem);
         t.pay = t.key + a.capR;
@@ -54,6 +62,7 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
         ct.cells = ct.heads + ct.hcap;
         ct.hs = a.hash_shift;
         ct.link_bits = cell_link_bits((uint32_t)a.capR);
+        ct.runs = reinterpret_cast<LongRuns *>(&runs);
     }
     const int tid = threadIdx.x;
     const unsigned nitems = *a.err ? 0u : *a.nitems;  // a planner error leaves the item list unusable
@@ -79,7 +88,7 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
         }
         const Item m = a.items[it];
         if (MAT) build_table<JOIN_THREADS>(t, a.R, m.r_off, m.r_len, scan_scratch);
-        else build_cells<JOIN_THREADS>(ct, Rk, m.r_off, m.r_len);
+        else build_cells<JOIN_THREADS, false, true>(ct, Rk, m.r_off, m.r_len);
 
         const Row *s = a.S + m.s_off;
         const uint64_t len = m.s_len;
@@ -90,7 +99,8 @@ __global__ void __launch_bounds__(JOIN_THREADS) k_join(JoinArgs a) {
         const uint4 *v = reinterpret_cast<const uint4 *>(s + head);
 
         if (!MAT) {
-            local += stream_sum<JOIN_THREADS>(Sk + m.s_off, len, [&](uint32_t k) { return ct.count(k); });
+            if (!ct.has_runs) local += probe_count<JOIN_THREADS>(ct, Sk + m.s_off, len);
+            else local += probe_runs(ct, Sk + m.s_off, len);
         } else {
             // block-synchronous rounds: 8 rows per thread, one reservation per round
             const uint64_t per_round = 4ull * JOIN_THREADS;

@@ -67,6 +67,42 @@ struct Table {
 };
 
 
+// Long runs of one key in a table of R rows: the buckets with chains of
+// RUN_ROWS cells or more, and how many rows each key in them has.  A lookup
+// then reads one count where the chain costs a dependent load per row.
+constexpr uint32_t RUN_ROWS = 128;  // a table of 16384 rows holds at most RUN_BUCKETS such runs
+constexpr uint32_t RUN_BUCKETS = 128, RUN_KEYS = 256;
+constexpr uint32_t RUN_NONE = 0xFFFFFFFFu;
+struct LongRuns {
+    uint32_t bucket[RUN_BUCKETS];       // hashed set, RUN_NONE: free
+    uint32_t key[RUN_KEYS];             // hashed, RUN_NONE: free
+    uint32_t rows[RUN_KEYS];            // R rows of the key
+    uint32_t full;                      // no room: the chains stay
+
+    __device__ __forceinline__ static uint32_t hash(uint32_t x, uint32_t n) { return (x * 0x9E3779B1u >> 16) & (n - 1); }
+    // Slot of x in set[n], or (not there) the first free slot after its hash,
+    // or n.
+    __device__ __forceinline__ static uint32_t find(const uint32_t *set, uint32_t n, uint32_t x) {
+        uint32_t h = hash(x, n);
+        for (uint32_t t = 0; t < n; t++, h = (h + 1) & (n - 1))
+            if (set[h] == x || set[h] == RUN_NONE) return h;
+        return n;
+    }
+    // The same, entering x where it is not there.
+    __device__ __forceinline__ static uint32_t enter(uint32_t *set, uint32_t n, uint32_t x) {
+        uint32_t h = hash(x, n);
+        for (uint32_t t = 0; t < n; t++, h = (h + 1) & (n - 1)) {
+            const uint32_t seen = set[h] == x ? x : atomicCAS(&set[h], RUN_NONE, x);
+            if (seen == RUN_NONE || seen == x) return h;
+        }
+        return n;
+    }
+    __device__ __forceinline__ uint32_t count(uint32_t k) const {
+        const uint32_t h = find(key, RUN_KEYS, k);
+        return h < RUN_KEYS && key[h] == k && k != RUN_NONE ? rows[h] : 0u;
+    }
+};
+
 // Count-only bucket chains of 32-bit cells.  With q = key >> hs, row i's
 // bucket is q mod N and its tag the bits of q above that, which with the
 // bucket and the low hs bits (shared by all rows of the join's partition)
@@ -78,7 +114,17 @@ struct Table {
 // and links in arrays of their own (112 KB at 8192 rows, two CTAs per SM) a
 // lookup reads one 4-byte word instead of 8 bytes, and 10240 rows take 72 KB,
 // three CTAs per SM.
-constexpr uint32_t CELL_EMPTY = 0xFFFFFFFFu;  // its link is past any row
+//
+// With `runs` set, buckets with long chains are counted per key instead
+// (LongRuns), and CELL_RUN is their head; has_runs says that there are any (the
+// same for all threads), for which the probe has a loop of its own: the test in
+// every lookup took 2% of a 16 M x 134 M join.  2^20 x 2^24 rows with 4096 rows
+// a key take 0.22 ms, 46 ms along the chains; with 256 rows a key 0.21 and 3.0;
+// with 1% of R on one key (2^20 x 2^22) 0.13 and 3.3, most of it the swaps in
+// build_cells.  Counting RHO and RHT take it, the batch (whose plan has the
+// histogram table to choose) does not.
+constexpr uint32_t CELL_EMPTY = 0xFFFFFFFFu;  // the links of these two are past any row
+constexpr uint32_t CELL_RUN = 0xFFFFFFFEu;
 
 struct CellTable {
     uint32_t *heads;  // [N <= hcap]
@@ -87,10 +133,13 @@ struct CellTable {
     int hs, link_bits;
     uint32_t mask;    // N - 1
     int tag_shift;    // hs + log2 N
+    LongRuns *runs = nullptr;
+    bool has_runs = false;
 
+    template <bool RUNS = false>
     __device__ __forceinline__ uint32_t count(uint32_t k) const {
         uint32_t c = heads[(k >> hs) & mask];
-        if (c == CELL_EMPTY) return 0;
+        if (c >= (RUNS ? CELL_RUN : CELL_EMPTY)) return RUNS && c == CELL_RUN ? runs->count(k) : 0u;
         const uint32_t tag = tag_shift < 32 ? k >> tag_shift : 0u;
         const uint32_t lmask = (1u << link_bits) - 1;
         uint32_t n = 0;
@@ -103,10 +152,10 @@ struct CellTable {
     }
 };
 
-// Link bits of a table of `rows` rows: links 0 .. rows, and one value more.
+// Link bits of a table of `rows` rows: links 0 .. rows, and two values more.
 __host__ __device__ __forceinline__ int cell_link_bits(uint32_t rows) {
     int b = 1;
-    while ((1u << b) < rows + 2) b++;
+    while ((1u << b) < rows + 3) b++;
     return b;
 }
 
@@ -134,8 +183,53 @@ __device__ __forceinline__ uint4 ld_pair(const uint4 *p) {
     return ldg_stream(p);
 }
 
-// Builds the cells of R rows [r_off, r_off + r_len); ends with a barrier.
-template <int THREADS, bool CG = false, class E = Row>
+// Finds the long chains of a built table and counts their keys' rows (see
+// LongRuns); true when there are any.  The caller has a barrier before, and
+// this ends with one.  The first THREADS rows look along their chains: a run of
+// RUN_ROWS among 10240 rows has one of 512 of them but once in 600 tables, and
+// then stays a chain.
+template <int THREADS, bool CG, class E>
+__device__ __noinline__ bool collapse_runs(uint32_t *heads, const uint32_t *cells, uint32_t mask, int hs, int link_bits,
+                                           const E *__restrict__ R, uint32_t r_len, LongRuns *lr) {
+    const uint32_t tid = threadIdx.x, lmask = (1u << link_bits) - 1;
+    for (uint32_t i = tid; i < RUN_KEYS; i += THREADS) {
+        lr->key[i] = RUN_NONE;
+        lr->rows[i] = 0;
+        if (i < RUN_BUCKETS) lr->bucket[i] = RUN_NONE;
+    }
+    if (tid == 0) lr->full = 0;
+    __syncthreads();
+    bool found = false;
+    if (tid < r_len) {
+        const uint32_t b = (ld_key<CG>(R, tid) >> hs) & mask;
+        uint32_t n = 1;
+        for (uint32_t c = heads[b]; n < RUN_ROWS && (c & lmask); n++) c = cells[(c & lmask) - 1];
+        found = n == RUN_ROWS;
+        if (found) LongRuns::enter(lr->bucket, RUN_BUCKETS, b);
+    }
+    if (!__syncthreads_or(found)) return false;
+    for (uint32_t i = tid; i < r_len; i += THREADS) {
+        const uint32_t k = ld_key<CG>(R, i), b = (k >> hs) & mask;
+        const uint32_t q = LongRuns::find(lr->bucket, RUN_BUCKETS, b);
+        if (q == RUN_BUCKETS || lr->bucket[q] != b) continue;
+        const uint32_t h = k == RUN_NONE ? RUN_KEYS : LongRuns::enter(lr->key, RUN_KEYS, k);
+        if (h < RUN_KEYS) atomicAdd(&lr->rows[h], 1u);
+        else lr->full = 1;
+    }
+    __syncthreads();
+    if (lr->full) return false;
+    if (tid < RUN_BUCKETS && lr->bucket[tid] != RUN_NONE) heads[lr->bucket[tid]] = CELL_RUN;
+    __syncthreads();
+    return true;
+}
+
+// Builds the cells of R rows [r_off, r_off + r_len); ends with a barrier.  A
+// row whose swap fails finds another row's cell at the head, never the empty
+// one, so it exchanges its cell for whatever is there and does not try again
+// (in a loop of swaps 10,000 rows of one key took 3 ms).
+// RUNS: a row that displaces a cell of its own tag says that there may be long
+// runs (or a key twice: a look at 512 chains finds those short).
+template <int THREADS, bool CG = false, bool RUNS = false, class E = Row>
 __device__ __forceinline__ void build_cells(CellTable &t, const E *__restrict__ R, uint64_t r_off, uint32_t r_len) {
     const int tid = threadIdx.x;
     const uint32_t least = t.link_bits > t.hs ? 1u << (t.link_bits - t.hs) : 1u;
@@ -145,19 +239,21 @@ __device__ __forceinline__ void build_cells(CellTable &t, const E *__restrict__ 
     for (uint32_t i = tid; i < N / 4; i += THREADS)
         reinterpret_cast<uint4 *>(t.heads)[i] = make_uint4(CELL_EMPTY, CELL_EMPTY, CELL_EMPTY, CELL_EMPTY);
     __syncthreads();
+    bool run = false;
     for (uint32_t i = tid; i < r_len; i += THREADS) {
         const uint32_t k = ld_key<CG>(R, r_off + i);
         uint32_t *head = &t.heads[(k >> t.hs) & t.mask];
         const uint32_t tag = t.tag_shift < 32 ? (k >> t.tag_shift) << t.link_bits : 0u;
         uint32_t old = *head;
-        for (;;) {  // ends: each failed swap means another row entered this chain
-            const uint32_t seen = atomicCAS(head, old, old == CELL_EMPTY ? tag : tag | (i + 1));
-            if (seen == old) break;
-            old = seen;
+        if (atomicCAS(head, old, old == CELL_EMPTY ? tag : tag | (i + 1)) != old) old = atomicExch(head, tag | (i + 1));
+        if (old != CELL_EMPTY) {
+            t.cells[i] = old;
+            if (RUNS) run |= (old ^ tag) >> t.link_bits == 0;
         }
-        if (old != CELL_EMPTY) t.cells[i] = old;
     }
-    __syncthreads();
+    if (!RUNS) __syncthreads();
+    else t.has_runs = __syncthreads_or(run) && collapse_runs<THREADS, CG>(t.heads, t.cells, t.mask, t.hs, t.link_bits,
+                                                                                  R + r_off, r_len, t.runs);
 }
 
 // E: rows, or bare keys (layout 1 without payloads).

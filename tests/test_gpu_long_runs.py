@@ -1,0 +1,99 @@
+"""Counting joins whose R holds long runs of one key: their rows are counted
+once per table, not walked by every S row.  Whole numbers: exact."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from gpu_util import run_join
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(oracle, keys, kind):
+    t = np.zeros(len(keys), dtype=oracle.ROW)
+    t["key"] = np.asarray(keys, dtype=np.uint64) & 0xFFFFFFFF
+    oracle.fill_payloads(t, kind)
+    return t
+
+
+def count(R, S):
+    """The equi-join's rows (numpy: the oracle walks a run for every match)."""
+    k, n = np.unique(R["key"], return_counts=True)
+    at = np.minimum(np.searchsorted(k, S["key"]), len(k) - 1)
+    return int(n[at][k[at] == S["key"]].sum())
+
+
+def check(tbg, oracle, cuda, algo, r, s, **cfg):
+    R, S = rel(oracle, r, 0), rel(oracle, s, 1)
+    for off in (0, 1):
+        m, _, st = run_join(tbg, cuda, algo, R, S, offset=off, **cfg)
+        assert m == count(R, S)
+    return st
+
+
+# one run around the line (128 rows), a whole table (10240 rows) and several,
+# among rows that fill the 4096-, the 10240- and the 16384-row table
+@pytest.mark.parametrize("algo", ["RHO", "RHT"])
+@pytest.mark.parametrize("run", [2, 127, 128, 129, 3000, 10240, 40001])
+@pytest.mark.parametrize("per_part", [3000, 8000, 12000])
+def test_one_run(tbg, oracle, cuda, algo, run, per_part):
+    rng = np.random.default_rng(run + per_part)
+    spread = rng.choice(1 << 32, 4 * per_part, replace=False)
+    hot = spread[11]
+    r = rng.permutation(np.concatenate([spread, np.full(run, hot)]))
+    s = rng.permutation(np.concatenate([spread[rng.integers(0, len(spread), 60013)], np.full(2003, hot),
+                                        hot ^ (1 << rng.integers(0, 32, 999))]))
+    check(tbg, oracle, cuda, algo, r, s, radix_bits=2, passes=1)
+
+
+# many runs in every table, up to more of them than their list holds
+@pytest.mark.parametrize("run", [64, 128, 200, 4000])
+@pytest.mark.parametrize("stride", [1, 3, 40503, 1 << 13])
+def test_many_runs(tbg, oracle, cuda, run, stride):
+    rng = np.random.default_rng(run)
+    n = 80001
+    r = rng.permutation(np.arange(n) // run) * stride + 5
+    s = rng.integers(0, n // run + 9, 50021) * stride + 5
+    check(tbg, oracle, cuda, "RHT", r, s)
+
+
+# the top key value (the mark of a free place in the list), and a long chain
+# of distinct keys (more than the list holds)
+@pytest.mark.parametrize("case", ["top", "chain"])
+def test_chains_that_stay(tbg, oracle, cuda, case):
+    rng = np.random.default_rng(5)
+    if case == "top":
+        r = np.concatenate([rng.integers(0, 1 << 32, 30001), np.full(5000, 0xFFFFFFFF), np.full(700, 12345)])
+    else:
+        r = np.concatenate([np.arange(2000) << 20, rng.integers(0, 1 << 32, 20001), np.full(700, 1 << 20)])
+    r = rng.permutation(r)
+    s = np.concatenate([r[rng.integers(0, len(r), 9001)], [0xFFFFFFFF, 0xFFFFFFFE, 0, 1], np.arange(4000) << 20])
+    check(tbg, oracle, cuda, "RHO", r, s, radix_bits=2, passes=1)
+
+
+@pytest.mark.parametrize("algo", ["RHO", "RHT"])
+def test_hot_key_takes_no_longer(tbg, cuda, algo):
+    """A hundredth of R's rows on one key: within five times the join of rows
+    that all come twice (1.4 times is measured; with the swap loop 33)."""
+    torch = cuda
+    nR, nS = 1 << 20, 1 << 22
+    g = torch.Generator("cuda").manual_seed(1)
+    cfg, st = tbg.config(algo), torch.cuda.current_stream().cuda_stream
+    rows = lambda k: k | (torch.arange(len(k), device="cuda") << 32)  # noqa: E731
+    S = rows(torch.randint(0, nR, (nS,), device="cuda", generator=g))
+
+    def ms(k):
+        R, best = rows(k[torch.randperm(nR, device="cuda", generator=g)]), 1e9
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            tbg.join_device(cfg, R.data_ptr(), nR, S.data_ptr(), nS, stream=st)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    hot = torch.arange(nR, device="cuda")
+    hot[: nR // 100] = 7
+    assert ms(hot) <= 5 * ms(torch.arange(nR, device="cuda") // 2)
