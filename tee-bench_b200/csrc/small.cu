@@ -8,12 +8,15 @@
 //
 // Counting, the table is one bit per key value when R's keys are distinct and
 // their range fits shared memory (as in direct.cu), else the bucket chains of
-// the partitioned join (join_dev.cuh; Joins/radix_join.c:187-244).
+// the partitioned join (join_dev.cuh; Joins/radix_join.c:187-244), long runs of
+// one key counted: 4000 rows of one key x 1 M rows take 43 us, 4.7 ms along the
+// chain (RSM's sorted merge, the other plan for it, 155 us).
 // Materialising joins use bucket chains with payloads.  The last CTA to finish
 // fills the control block, with the partition sizes and work items that the
 // partitioned join would have had (a few partitions: 2 to 8), in device memory
 // and in the caller's pinned mirror, so that no copy follows either.
 #include <algorithm>
+#include <type_traits>
 
 #include "join_dev.cuh"
 #include "tbg_runtime.h"
@@ -21,7 +24,7 @@
 namespace tbg {
 
 constexpr int SMALL_THREADS = 1024;
-constexpr size_t SMALL_SMEM_MAX = 226 * 1024;
+constexpr size_t SMALL_SMEM_MAX = 223 * 1024;
 
 struct SmallArgs {
     const Row *R, *S;
@@ -38,8 +41,8 @@ struct SmallArgs {
     uint64_t cap;
 };
 
-// Heads of the count-only table: two to four per row (the tag needs 2^15 of
-// them at 16384 rows, 2^14 below).
+// Heads of the count-only table: two per row (2^13 at 4096 rows, 2^14, 2^15),
+// as many as the tag needs.
 __host__ __device__ __forceinline__ uint32_t small_heads(uint32_t table_rows) {
     return 1u << cell_link_bits(table_rows);
 }
@@ -75,6 +78,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
     // R's table
     Table t;
     CellTable ct;
+    __shared__ std::conditional_t<MAT, uint32_t, LongRuns> runs;
     if (MAT) {
         t.key = reinterpret_cast<uint32_t *>(smem);
         t.hs = a.B;
@@ -89,6 +93,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
         ct.cells = ct.heads + ct.hcap;
         ct.hs = 0;  // nothing is partitioned: keys differ in every bit
         ct.link_bits = cell_link_bits(a.table_rows);
+        ct.runs = reinterpret_cast<LongRuns *>(&runs);
     }
     uint32_t *bits = reinterpret_cast<uint32_t *>(smem);
     uint32_t kmin = 0, span = 0;
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
         }
     }
     if (MAT) build_table<T>(t, a.R, 0, a.nR, scratch);
-    else if (!by_bits) build_cells<T>(ct, a.R, 0, a.nR);
+    else if (!by_bits) build_cells<T, false, true>(ct, a.R, 0, a.nR);
 
     // this CTA's slice of S
     const uint64_t s0 = (uint64_t)blockIdx.x * a.slice;
@@ -138,10 +143,15 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
                 const uint32_t d = k - kmin;
                 return d <= span ? (bits[d >> 5] >> (d & 31)) & 1u : 0u;
             });
-        } else {
+        } else if (!ct.has_runs) {
             local = stream_sum<T>(s, len, [&](uint32_t k) {
                 odd += k & 1;
                 return ct.count(k);
+            });
+        } else {
+            local = stream_sum<T>(s, len, [&](uint32_t k) {
+                odd += k & 1;
+                return ct.count<true>(k);
             });
         }
         odd = __reduce_add_sync(0xffffffffu, odd);

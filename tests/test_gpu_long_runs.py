@@ -97,3 +97,43 @@ def test_hot_key_takes_no_longer(tbg, cuda, algo):
     hot = torch.arange(nR, device="cuda")
     hot[: nR // 100] = 7
     assert ms(hot) <= 5 * ms(torch.arange(nR, device="cuda") // 2)
+
+
+# R in one table (at most 16384 rows), one launch: every algorithm that takes it
+@pytest.mark.parametrize("algo", ["RHO", "RSM"])
+@pytest.mark.parametrize("nR", [127, 128, 4000, 4096, 16384])
+@pytest.mark.parametrize("values", [1, 2, 30, 129])
+@pytest.mark.parametrize("stride", [1, 99991])
+def test_small_joins(tbg, oracle, cuda, algo, nR, values, stride):
+    rng = np.random.default_rng(nR + values)
+    r = rng.permutation(np.arange(nR) % values) * stride + 3
+    s = np.concatenate([rng.integers(0, values + 3, 30011) * stride + 3, [0xFFFFFFFF, 0]])
+    st = check(tbg, oracle, cuda, algo, r, s)
+    if algo == "RHO" or nR <= 4096:  # RSM takes more than two partitions above
+        assert st.path == tbg.PATH_SMALL
+
+
+@pytest.mark.parametrize("algo", ["RSM", "RHO"])
+def test_small_hot_key_takes_no_longer(tbg, cuda, algo):
+    """4000 rows of one key: within four times the join of distinct keys (1.2 to
+    1.4 measured; every S row walking the run: 100)."""
+    torch = cuda
+    nR, nS = 4000, 1 << 20
+    g = torch.Generator("cuda").manual_seed(1)
+    cfg, st = tbg.config(algo), torch.cuda.current_stream().cuda_stream
+    rows = lambda k: k | (torch.arange(len(k), device="cuda") << 32)  # noqa: E731
+    S = rows(torch.randint(0, nR, (nS,), device="cuda", generator=g))
+
+    def ms(R, S):
+        best = 1e9
+        for _ in range(9):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            tbg.join_device(cfg, R.data_ptr(), nR, S.data_ptr(), nS, stream=st)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    one = ms(rows(torch.full((nR,), 7, device="cuda")), rows(torch.full((nS,), 7, device="cuda")))
+    assert one <= 4 * ms(rows(torch.arange(nR, device="cuda")), S)
