@@ -154,14 +154,14 @@ cudaError_t launch_bucket_count(const JoinArgs &a, const HeavyBuckets &hv, uint3
                                 cudaStream_t st);
 
 // Count-only PSM on MSD buckets: both relations partitioned by the top bits of
-// key - sub (sub: R's smallest key), then k_bucket_count.  Nothing waits, and
+// key - sub (sub, rmax: R's key range), then k_bucket_count.  Nothing waits, and
 // neither S's keys outside R's range nor heavy keys (S's buckets are split over
 // CTAs by the planner, R's rows of a large bucket counted once) need another
 // plan.
 // lsd_passes > 0: the range has no bits above the low ones, where the sort
 // would be an LSD sort of that many passes; the buckets do for it too.
-static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, uint32_t sub, int B,
-                     int lowbits, int lsd_passes, Workspace &w, cudaStream_t st, JoinRun *run) {
+static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *dS, uint64_t nS, uint32_t sub,
+                     uint32_t rmax, int B, int lowbits, int lsd_passes, Workspace &w, cudaStream_t st, JoinRun *run) {
     if (lsd_passes) {  // a range of at most kLowBits bits: two buckets
         B = 1;
         lowbits = std::max(lowbits - 1, 2);
@@ -175,6 +175,7 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     }
     RadixGeom g = radix_geometry_msd(nR, nS, sub, B, lowbits, w);
     try_direct(g, cfg, nullptr, 0);
+    if (nR > (uint64_t)(rmax - sub) + 1) g.direct = false;  // more rows than key values: not distinct
     g.sample_S = dS;
     g.capR = 0x7FFFFFFF;  // counters take any number of R rows
     g.keys = true;
@@ -339,10 +340,10 @@ int run_psm_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Row *d
     int B = 0, lowbits = 0;
     if (!cfg.materialize && nR && nS) {
         if (msd_bits(span_of(rmin, rmax), &B, &lowbits))
-            return msd_count(cfg, dR, nR, dS, nS, rmin, B, lowbits, 0, w, st, run);
+            return msd_count(cfg, dR, nR, dS, nS, rmin, rmax, B, lowbits, 0, w, st, run);
         if (span_of(rmin, rmax) <= kLowBits)
-            return msd_count(cfg, dR, nR, dS, nS, rmin, 1, lowbits, std::max<int>(1, (int)sort_plan(rmin, rmax).size()), w,
-                             st, run);
+            return msd_count(cfg, dR, nR, dS, nS, rmin, rmax, 1, lowbits,
+                             std::max<int>(1, (int)sort_plan(rmin, rmax).size()), w, st, run);
     }
     bool direct = false;
     run->B = 8;

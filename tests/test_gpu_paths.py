@@ -90,3 +90,20 @@ def test_batch_reports_its_bit_tables(tbg, oracle, cuda, kind, tables):
         assert b.describe()["bit_tables"] == tables
     finally:
         b.close()
+
+
+def test_more_rows_than_key_values(tbg, oracle, cuda):
+    """PSM knows R's range: more rows than key values are not tried (building
+    their table took 8 of 79 us), as many distinct rows are."""
+    launches = {}
+    for nR, path in ((40000, tbg.PATH_DIRECT), (40001, tbg.PATH_PARTITIONED)):
+        rng = np.random.default_rng(4)
+        R = np.zeros(nR, dtype=oracle.ROW)
+        S = np.zeros(60001, dtype=oracle.ROW)
+        R["key"] = 77 + rng.permutation(nR) % 40000
+        S["key"] = 77 + rng.integers(0, 40100, len(S))
+        m, _, st = run_join(tbg, cuda, "PSM", R, S)
+        assert m == oracle.rho(R, S) and st.path == path
+        launches[nR] = st.kernel_launches
+    # without the table's launches (clear, decide, one of two probes)
+    assert launches[40001] == launches[40000] - 3
