@@ -152,15 +152,19 @@ __device__ __forceinline__ void hist_pairs(uint32_t *sh, const RadixF &rf, const
     }
 }
 
-// R: chunk histograms, key range, bits.  A sixteenth of the rows is entered
-// first with a returning atomic, which gives up (for the whole grid, through
-// ctrl->direct_dup) at the first key already there: a relation with many
-// duplicates costs little before it takes the passes.  The other rows use
-// atomics without a result, and a duplicate there shows in the count of set
-// bits.  Bound by the L2's atomics: 2^27 rows take 0.80 ms
+// R: chunk histograms, key range, bits.  Three things end the attempt before
+// all of R is entered; the CTA that sees one tells the grid through
+// ctrl->direct_dup, which every CTA looks at once a round:
+//   - two equal keys among a warp's neighbouring rows (no atomic needed), which
+//     shows sorted and hot keys before they queue at one word: 2^22 x 2^23 rows,
+//     R's last quarter one key, RSM 0.52 ms against 1.18;
+//   - a key already there in a careful round, whose atomics return: a sixteenth
+//     of the rounds of long chunks, else one round of every sixteenth chunk;
+//   - a payload already there (PAYLOADS: every row exchanges its payload with
+//     the key's entry, 2^22 rows: 37 us).
+// The other rows use atomics without a result, and a duplicate there shows in
+// the count of set bits.  Bound by the L2's atomics: 2^27 rows take 0.80 ms
 // without results against 1.17 ms with; the histogram read alone 0.16 ms.
-// PAYLOADS: every row exchanges its payload with the key's entry (2^22 rows:
-// 37 us), so a duplicate shows at once.
 template <bool PAYLOADS>
 __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__restrict__ in, uint64_t n, uint64_t chunk,
                                                                   uint32_t *__restrict__ hist, int nbins, RadixF rf,
@@ -169,9 +173,10 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
     dep_trigger();
     extern __shared__ uint32_t sh[];
     __shared__ uint32_t s_inv, s_hi;
+    __shared__ volatile unsigned s_off;  // as *gave_up of an earlier round
     const int tid = threadIdx.x;
     for (int i = tid; i < nbins; i += DIRECT_THREADS) sh[i] = 0;
-    if (tid == 0) s_inv = s_hi = 0;
+    if (tid == 0) s_inv = s_hi = s_off = 0;
     __syncthreads();
     const unsigned w = ctrl->direct_log2;
     const uint32_t wmask = w ? (uint32_t)((1ull << w) - 1) : 0u;
@@ -200,6 +205,18 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
     stream_pairs(
         in, lo, hi,
         [&](const uint4(&x)[4], const bool(&ok)[4]) {
+            if (enter) {
+                if (tid == 0 && *gave_up) s_off = 1;
+                // rows side by side (u), or in the next lane's pair, with one key
+                bool same = s_off != 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint32_t before = __shfl_up_sync(0xffffffffu, x[u].z, 1);
+                    same |= ok[u] && (x[u].x == x[u].z || (x[u].x == before && (tid & 31) != 0));
+                }
+                enter = !__any_sync(0xffffffffu, same);
+                if (!enter && (tid & 31) == 0 && !*gave_up) *gave_up = 1;
+            }
             if (enter) {
                 if (round < careful) {
                     bool dup = false;

@@ -192,6 +192,15 @@ template <int THREADS, bool CG, class E>
 __device__ __noinline__ bool collapse_runs(uint32_t *heads, const uint32_t *cells, uint32_t mask, int hs, int link_bits,
                                            const E *__restrict__ R, uint32_t r_len, LongRuns *lr) {
     const uint32_t tid = threadIdx.x, lmask = (1u << link_bits) - 1;
+    bool found = false;
+    uint32_t b0 = 0;
+    if (tid < r_len) {
+        b0 = (ld_key<CG>(R, tid) >> hs) & mask;
+        uint32_t n = 1;
+        for (uint32_t c = heads[b0]; n < RUN_ROWS && (c & lmask); n++) c = cells[(c & lmask) - 1];
+        found = n == RUN_ROWS;
+    }
+    if (!__syncthreads_or(found)) return false;
     for (uint32_t i = tid; i < RUN_KEYS; i += THREADS) {
         lr->key[i] = RUN_NONE;
         lr->rows[i] = 0;
@@ -199,15 +208,8 @@ __device__ __noinline__ bool collapse_runs(uint32_t *heads, const uint32_t *cell
     }
     if (tid == 0) lr->full = 0;
     __syncthreads();
-    bool found = false;
-    if (tid < r_len) {
-        const uint32_t b = (ld_key<CG>(R, tid) >> hs) & mask;
-        uint32_t n = 1;
-        for (uint32_t c = heads[b]; n < RUN_ROWS && (c & lmask); n++) c = cells[(c & lmask) - 1];
-        found = n == RUN_ROWS;
-        if (found) LongRuns::enter(lr->bucket, RUN_BUCKETS, b);
-    }
-    if (!__syncthreads_or(found)) return false;
+    if (found) LongRuns::enter(lr->bucket, RUN_BUCKETS, b0);
+    __syncthreads();
     for (uint32_t i = tid; i < r_len; i += THREADS) {
         const uint32_t k = ld_key<CG>(R, i), b = (k >> hs) & mask;
         const uint32_t q = LongRuns::find(lr->bucket, RUN_BUCKETS, b);
