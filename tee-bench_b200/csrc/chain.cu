@@ -31,6 +31,14 @@ cudaError_t launch_rows_to_relation(const tbg_row_out *rows, uint64_t n, Row *ou
     return cudaGetLastError();
 }
 
+// Whether the join may write the relation itself: the direct join of RHO, RHT
+// and RSM can (api.cpp, radix_partition), with an R past the one-launch joins
+// that the payload table may hold.
+static bool may_write_relation(const tbg_config &cfg, uint64_t nR) {
+    return (cfg.algo == TBG_RHO || cfg.algo == TBG_RHT || cfg.algo == TBG_RSM) && automatic_plan(cfg) && nR > SMALL_R &&
+           nR <= (1ull << direct_log2_max_rows(nR));
+}
+
 // R x S as a relation of (key, R payload) tuples in w.chain_rel, *m of them.  A
 // direct join writes the relation itself; any other writes rows, which are
 // converted.  The first guess of |S| rows grows once if it was too small.
@@ -39,16 +47,30 @@ static int join_relation(const tbg_config &cfg, const Row *dR, uint64_t nR, cons
     tbg_config c = cfg;
     c.materialize = 1;
     uint64_t cap = std::max<uint64_t>(nS, 1);
-    for (int attempt = 0; attempt < 2; attempt++) {
+    bool direct_rel = may_write_relation(c, nR);
+    for (int grown = 0; grown < 2;) {
         cudaError_t e = w.chain_rows.ensure(cap * sizeof(tbg_row_out));
+        if (e == cudaErrorMemoryAllocation && w.chain_rel.p) {
+            cudaGetLastError();
+            w.chain_rel.release();
+            e = w.chain_rows.ensure(cap * sizeof(tbg_row_out));
+        }
         if (e != cudaSuccess) return cuda_error(e, "cudaMalloc (chain rows)");
         JoinRun run;
         run.waits = true;
         // no room for |S| tuples: rows, and a relation of as many as there are
-        if (w.chain_rel.ensure(cap * sizeof(Row)) == cudaSuccess) run.rel = w.chain_rel.as<Row>();
-        else cudaGetLastError();
+        if (direct_rel) {
+            if (w.chain_rel.ensure(cap * sizeof(Row)) == cudaSuccess) run.rel = w.chain_rel.as<Row>();
+            else cudaGetLastError();
+        }
         Workspace *jw = nullptr;
         int rc = join_device_impl(&c, dR, nR, dS, nS, w.chain_rows.as<tbg_row_out>(), cap, st, &run, &jw);
+        if (rc == TBG_ERR_OOM && w.chain_rel.p) {  // the join needs the memory more
+            cudaGetLastError();
+            w.chain_rel.release();
+            direct_rel = false;
+            continue;
+        }
         if (rc == TBG_OK) rc = finish_join(c, *jw, st, run, nR, nS, cap, m, nullptr);
         if (rc == TBG_OK) {
             if (run.rel_done) return TBG_OK;
@@ -59,6 +81,7 @@ static int join_relation(const tbg_config &cfg, const Row *dR, uint64_t nR, cons
         }
         if (rc != TBG_ERR_CAPACITY) return rc;
         cap = std::max<uint64_t>(*m, 1);  // exact count is known now
+        grown++;
     }
     return set_error(TBG_ERR_CAPACITY, "chained join: output grew between attempts");
 }

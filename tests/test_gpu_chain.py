@@ -93,3 +93,29 @@ def test_three_way_chain_from_a_direct_join(tbg, oracle, cuda, nR, nS, nT, step)
         torch.cuda.synchronize()
         assert (m1, m2) == (c1, c2), algo
         assert np.array_equal(oracle.sort_rows(rows_to_host(tO, m2)), oracle.sort_rows(rows2)), algo
+
+
+@pytest.mark.parametrize("nR", [1 << 20, 5000])
+def test_chain_near_the_memory_limit(tbg, oracle, cuda, nR):
+    """A selective chain whose first join's rows and passes fit, but not with
+    room for |S| tuples beside them (which only a direct join could use)."""
+    torch = cuda
+    nS, nT = 1 << 25, 3001
+    st = torch.cuda.Stream()
+    S = torch.arange(nS, device="cuda") + (1 << 21) | (torch.arange(nS, device="cuda") << 32)
+    S[-2000:] = torch.arange(2000, device="cuda") * 2 + 1
+    R = torch.randperm(nR, device="cuda") | (torch.arange(nR, device="cuda") << 32)
+    T = torch.arange(nT, device="cuda") | (torch.arange(nT, device="cuda") << 32)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    # 12 B a row, two copies of S for the passes, R's, histograms and T x the
+    # relation; each buffer with an eighth more where there is room, and no
+    # room for the 8 B a row of |S| tuples (256 MB)
+    need = nS * (12 + 16) + (96 << 20)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - need - need // 8, dtype=torch.uint8, device="cuda")
+    try:
+        got = tbg.join_three_way(tbg.config("RHO"), R.data_ptr(), nR, S.data_ptr(), nS, T.data_ptr(), nT, stream=st.cuda_stream)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert tuple(got) == (2000, 1500)  # T holds the odd keys up to 2999
