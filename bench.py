@@ -368,7 +368,7 @@ def reference_main(args, metric, base_config, world, mat, scaling="weak"):
 LVR_CASES = [("z1", 1.0, 0), ("z1_scattered", 1.0, 1)]
 # RHO partitioned (fixed passes) with and without the split, and under the
 # automatic plan (the direct counting join)
-LVR_VARIANTS = [("lrn", "LRN", {}), ("rho_skew_split", "RHO", {"passes": 2}),
+LVR_VARIANTS = [("lrn", "LRN", {}), ("rho_partitioned_split", "RHO", {"passes": 2}),
                 ("rho_plain", "RHO", {"skew_split": 0}), ("rho_automatic", "RHO", {})]
 
 
@@ -417,7 +417,7 @@ def learned_vs_radix(tbg, torch, dev, stream, steps, warmup, lr=26, ls=29, cases
         counts = {entry[n]["matches"] for n, _, _ in LVR_VARIANTS}
         entry["identical_counts"] = len(counts) == 1 and counts == {nS}
         entry["lrn_speedup_vs_plain"] = entry["rho_plain"]["ms"] / entry["lrn"]["ms"]
-        entry["lrn_speedup_vs_skew_split"] = entry["rho_skew_split"]["ms"] / entry["lrn"]["ms"]
+        entry["lrn_speedup_vs_partitioned_split"] = entry["rho_partitioned_split"]["ms"] / entry["lrn"]["ms"]
         out["cases"][label] = entry
     del tR, tS
     return out
@@ -757,6 +757,16 @@ def cpu_baseline_line(host_rows, algo, mat):
 
 
 # ------------------------------------------------------------------ sharded
+def sharded_bytes(own_rows, joined_rows, world, partitioned):
+    """HBM bytes of one rank's split and count-only join, and what they are."""
+    split = 8 + 16 if world > 1 else 0
+    join = 8 + 12 + 8 + 4 if partitioned else 8
+    model = ("split: histogram 8 + scatter 16 B per own row; " if split else "") + (
+        "join: histogram 8, passes over bare keys 12 + 8, build/probe 4 B per received row" if partitioned
+        else "join (direct): 8 B per received row")
+    return split * own_rows + join * joined_rows, model
+
+
 def sharded_main(args, rank, world, local):
     """One |R| = 2^27, |S| = 2^30 uniform FK join spread over the ranks (strong
     scaling): rank r holds rows shard_rows(n, world, r) of R and of S.  Each
@@ -808,7 +818,9 @@ def sharded_main(args, rank, world, local):
 
     def join(Rt, St):
         moved["joined"] = Rt.numel() + St.numel()
-        return tbg.join_device(cfg, Rt.data_ptr(), Rt.numel(), St.data_ptr(), St.numel(), stream=sh)[1]
+        _, m, st = tbg.join_device(cfg, Rt.data_ptr(), Rt.numel(), St.data_ptr(), St.numel(), stream=sh)
+        moved["partitioned"] = st.path == tbg.PATH_PARTITIONED
+        return m
 
     def new_rows(n):
         return torch.empty(max(n, 1), dtype=torch.int64, device=dev)[:n]
@@ -863,10 +875,7 @@ def sharded_main(args, rank, world, local):
                       "each rank's rows copied from pinned host memory each step", "count": int(m)}
     peak, peak_kind = read_peaks()
     local_rows = tR.numel() + tS.numel()
-    joined = moved.get("joined", local_rows)
-    # this rank's HBM bytes: split 8 (histogram) + 16 (scatter) per own row when
-    # world > 1, the join 48 per received row (histogram 8, 2 passes x 16, build/probe 8)
-    alg = (24 * local_rows if world > 1 else 0) + 48 * joined
+    alg, bytes_model = sharded_bytes(local_rows, moved["joined"], world, moved["partitioned"])
     line = {
         "metric": metric, "value": value, "unit": "Mtuples/s", "n_gpus": world, "steps": K,
         "warmup": args.warmup, "ms_per_step": ms / K, "higher_is_better": True, "scaling": "strong",
@@ -883,8 +892,7 @@ def sharded_main(args, rank, world, local):
                      "frac": alg / (ms / K / 1e3) / 1e9 / peak, "traffic": None, "peak_source": peak_kind,
                      "algorithmic_bytes_per_rank": alg,
                      "nvlink_bytes_per_rank": sent_rows * 8,
-                     "bytes_model": "split: histogram 8 + scatter 16 B per own row (world > 1); join: 48 B per "
-                                    "received row"},
+                     "bytes_model": bytes_model},
         "clocks": clocks.summary(),
         "matches": int(m),
     }
