@@ -334,7 +334,7 @@ int part_hist_read(int rel, const RadixGeom &g, const Row *d, const tbg_config &
                               g.direct_rows, g.build_wave, ctrl, st);
         if (e == cudaSuccess)
             e = launch_direct_decide(g.direct_rows ? nullptr : w.direct.as<uint32_t>(), direct_log2_max(g.n[0]), g.n[0],
-                                     g.sample_S, g.n[1], g.build_wave, ctrl, st);
+                                     g.sample_S, g.n[1], g.build_wave, w.nsm, ctrl, st);
     } else if (g.direct && g.direct_rows && !bypass) {
         e = launch_hist_emit(d, g.n[1], g.ch[1], g.G[1], hist.as<uint32_t>(), g.B, g.rf, w.direct.as<uint32_t>(), g.rows,
                              g.rel, g.rows_cap, g.s_range_max, ctrl, st);

@@ -700,11 +700,11 @@ cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, int wave, Ctrl *ctrl,
-                                 cudaStream_t st) {
+cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, int wave, int nsm,
+                                 Ctrl *ctrl, cudaStream_t st) {
     const uint64_t n4 = 1ull << (log2_max - 7);
     // two 16-byte words per thread and CTA at least, one CTA per SM at most
-    const unsigned g = bits ? (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), 148)) : 1u;
+    const unsigned g = bits ? (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n4 / (DIRECT_THREADS * 2), (uint64_t)nsm)) : 1u;
     if (wave) {  // no dependent launch, as above
         k_direct_decide<<<g, DIRECT_THREADS, 0, st>>>(bits, nR, S, nS, ctrl);
         count_launch();

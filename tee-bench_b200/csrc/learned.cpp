@@ -147,7 +147,7 @@ int run_learned_join(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     const int use_model = cfg.model == TBG_MODEL_SAMPLE ? 0 : 1;
     // a key must be predicted to hold at least tau_min S rows to be heavy
     const double tau_min = std::max(64.0, (double)nS / (double)(1 << 20));
-    if ((e = launch_learn_start(dS, lb, nb, stride, hkeys, hcnt, cfg.seed, s2)) != cudaSuccess ||
+    if ((e = launch_learn_start(dS, lb, nb, stride, hkeys, hcnt, cfg.seed, w.nsm, s2)) != cudaSuccess ||
         (e = launch_count_keys(lb, m, s2)) != cudaSuccess || (e = launch_count_stats(lb, s2)) != cudaSuccess ||
         (e = launch_rank_points(lb, s2)) != cudaSuccess ||
         (steps && (e = launch_mlp_train(lb.xs, lb.ys, lb.cw, &lb.dec->npoints, 0, lb.params, steps, 0.03f, cfg.seed, s2)) !=

@@ -486,9 +486,9 @@ __global__ void __launch_bounds__(256) k_learn_start(const Row *__restrict__ S, 
 }
 
 cudaError_t launch_learn_start(const Row *S, const LearnBufs &b, uint64_t nblocks, uint64_t stride, uint32_t *hkeys,
-                               unsigned *hcnt, uint64_t seed, cudaStream_t st) {
+                               unsigned *hcnt, uint64_t seed, int nsm, cudaStream_t st) {
     const uint64_t work = std::max<uint64_t>(nblocks * 32, HEAVY_CAP);
-    k_learn_start<<<(unsigned)umin64((work + 255) / 256, 148 * 16), 256, 0, st>>>(S, b, nblocks, stride, hkeys, hcnt, seed);
+    k_learn_start<<<(unsigned)umin64((work + 255) / 256, (uint64_t)nsm * 16), 256, 0, st>>>(S, b, nblocks, stride, hkeys, hcnt, seed);
     count_launch();
     return cudaGetLastError();
 }

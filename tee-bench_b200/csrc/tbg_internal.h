@@ -209,8 +209,8 @@ cudaError_t launch_direct_prep(const Row *R, uint64_t nR, uint32_t *table, int l
                                int nsm, cudaStream_t st);
 cudaError_t launch_hist_build(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
                               uint32_t *table, bool payloads, int wave, Ctrl *ctrl, cudaStream_t st);
-cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, int wave, Ctrl *ctrl,
-                                 cudaStream_t st);
+cudaError_t launch_direct_decide(const uint32_t *bits, int log2_max, uint64_t nR, const Row *S, uint64_t nS, int wave, int nsm,
+                                 Ctrl *ctrl, cudaStream_t st);
 cudaError_t launch_hist_probe(const Row *in, uint64_t n, uint64_t chunk, int G, uint32_t *hist, int P_log2, RadixF rf,
                               const uint32_t *bits, uint64_t nR, int nsm, Ctrl *ctrl, cudaStream_t st);
 

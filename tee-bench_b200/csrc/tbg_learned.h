@@ -144,7 +144,7 @@ struct LearnBufs {
     unsigned *err;
 };
 cudaError_t launch_learn_start(const Row *S, const LearnBufs &b, uint64_t nblocks, uint64_t stride, uint32_t *hkeys,
-                               unsigned *hcnt, uint64_t seed, cudaStream_t st);
+                               unsigned *hcnt, uint64_t seed, int nsm, cudaStream_t st);
 cudaError_t launch_count_keys(const LearnBufs &b, uint64_t m, cudaStream_t st);
 cudaError_t launch_count_stats(const LearnBufs &b, cudaStream_t st);
 cudaError_t launch_rank_points(const LearnBufs &b, cudaStream_t st);
