@@ -4,9 +4,9 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--workload rho_c2|rho_c2_sel50|rsm_c2|lrn_c3_z1|radix_c3_z1|...]
 
-One step = one full join (histogram, partitioning passes, build/probe) of a
-device-resident synthetic |R| = 2^27, |S| = 2^30 uniform foreign-key workload,
-count only (the headline configuration).  On N > 1 GPUs (torchrun) the same
+One step = one full join (as the library does it: direct, or histogram,
+partitioning passes and build/probe) of a device-resident synthetic |R| = 2^27,
+|S| = 2^30 uniform foreign-key workload, count only (the headline configuration).  On N > 1 GPUs (torchrun) the same
 join is spread over the ranks: each holds 1/N of R and S, splits its rows by
 key hash, an NCCL all-to-all exchanges the pieces, every rank joins its share
 and the counts are all-reduced (strong scaling).  Prints ONE JSON line on
@@ -17,11 +17,11 @@ rank 0.
 * e2e        the same metric through the drop-in RHO(table_t*, table_t*, int)
              with pinned host buffers: H2D of R and S, the join and the result
              read-back inside each timed step;
-* roofline   the dominant kernel (the partitioning scatter) against the
+* roofline   the direct join's bytes, or the partitioning passes', against the
              measured HBM copy bandwidth, from per-phase CUDA events recorded
              by the library on the join stream during the timed steps;
-* learned_vs_radix  LRN against RHO with and without its skew split on the
-             skewed configuration (2^26 / 2^29 Zipf z = 1), same process,
+* learned_vs_radix  LRN against RHO partitioned, with and without its
+             skew split, and RHO as it comes, on the skewed configuration (2^26 / 2^29 Zipf z = 1), same process,
              clocks sampled;
 * cpu_baseline  the reference's own RHO (oracle/_ref, built from the
              reference sources) on this host's cores, on the workload's own

@@ -304,7 +304,7 @@ typedef struct tbg_batch tbg_batch; /* opaque plan: tuned, graph-captured */
 
 /* Plans njoins joins.  cfg (NULL = defaults): algo TBG_RHO or TBG_RHT (RHT
  * fixes the histogram table layout), count only; radix_bits 0 autotunes the
- * partitioning (direct or 1..8 radix bits), table layout, S rows per work
+ * partitioning (none or 1..8 radix bits), table layout, S rows per work
  * item and chunk size per size class by timing the batch's own joins;
  * radix_bits > 0 partitions every join with that many bits (one pass, <= 8);
  * radix_bits < 0 uses the built-in heuristic without timing.  The whole

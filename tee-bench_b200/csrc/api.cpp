@@ -164,19 +164,16 @@ void mark(Workspace &w, bool timing, int i, cudaStream_t st) {
     if (timing) cudaEventRecord(w.ev[i], st);
 }
 
-// Geometry of the chunked radix partitioning of R and S into 2^B final
-// partitions (shared by RHO, RHT, RSM and LRN).
 // R rows per shared-memory join table that the planner plans with (R
 // partitions larger than that are joined in chunks).  choose_radix aims the
 // average R partition at half of it.
-//   Counting joins, |R| <= 2^28: JOIN_CAPR_WIDE, so the radix geometry is the
-//   one whose average R partition fills a JOIN_CAPR_FIT-row table (14 bits,
-//   7 + 7, at |R| = 2^27, where half-full 5120-row tables need 15 bits,
-//   7 + 8); both figures are of the tables with payload-sized cells, whose
-//   kernels held 8192 rows.  The join then launches a JOIN_CAPR_FIT-row table kernel and a
-//   JOIN_CAPR_WIDE one, each gated on the largest R partition (device
-//   memory).  Measured at 2^27 x 2^30: 11.41 ms against 12.28 ms; the
-//   8-bit fan-out of the second pass costs more than the bigger tables.
+//   Counting joins, |R| <= 2^28: JOIN_CAPR_WIDE, so the average R partition
+//   has 8192 rows (14 bits, 7 + 7, at |R| = 2^27, where half-full 5120-row
+//   tables need 15 bits, 7 + 8).  The join then launches a JOIN_CAPR_FIT-row
+//   table kernel (10240, room for uneven partitions) and a JOIN_CAPR_WIDE one,
+//   each gated on the largest R partition (device memory).  Measured at 2^27 x
+//   2^30, with 8192-row tables and partitions of rows: 11.41 ms against 12.28
+//   ms; the 8-bit fan-out of the second pass costs more than the bigger tables.
 //   Otherwise: JOIN_CAPR_DEFAULT (three CTAs per SM) while R's partitions at
 //   the largest radix (15 bits) fit it, else the next power of two, up to
 //   16384 (one CTA per SM), so a partition of R is built once and S is not
@@ -193,6 +190,8 @@ int join_capacity(uint64_t nR, bool counting) {
     return (int)c;
 }
 
+// Geometry of the chunked radix partitioning of R and S into 2^B final
+// partitions (shared by RHO, RHT, RSM and LRN).
 RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int capR, Workspace &w) {
     RadixGeom g;
     choose_radix(cfg, nR, capR, &g.B, &g.passes);
@@ -222,7 +221,7 @@ RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int ca
     // room for every R chunk of a partition to split its S side (k_plan
     // keeps oversized S sides whole if a skewed input still overflows this)
     g.item_cap = 2 * (nR / capR + (g.capS ? nS / g.capS : 0) + 2 * g.P) + 16;
-    // four chunks per SM (two resident partitioning CTAs each).  A chunk's
+    // two chunks per SM, as many as partitioning CTAs are resident.  A chunk's
     // CTA reads its row of the per-chunk prefix (2^B counters) to set up its
     // cursors, so a chunk holds at least max(4096, 2^B) rows: at 15 bits 32K
     // rows, while small joins still get enough chunks to fill the GPU.
@@ -654,7 +653,7 @@ int radix_join_phase(const tbg_config &cfg, tbg_row_out *d_rows, uint64_t cap, W
     // known on the device only (the planner's max_part_R).  So both table
     // sizes are launched, each gated on it: one does the join, the other
     // returns at once, and no host read-back is needed.  The geometry of
-    // JOIN_CAPR_WIDE plans aims R's partitions at JOIN_CAPR_FIT rows.
+    // JOIN_CAPR_WIDE plans aims R's partitions at 8192 rows.
     const int small_cap = cfg.materialize ? 0
                           : capR == JOIN_CAPR_WIDE    ? JOIN_CAPR_FIT
                           : capR == JOIN_CAPR_DEFAULT ? JOIN_CAPR_SMALL

@@ -1,6 +1,6 @@
 // Batched joins: planner, autotuner and CUDA graph behind tbg_batch_*.
 //
-// A plan fixes, per join, the partitioning (direct, or one radix pass of B
+// A plan fixes, per join, the partitioning (none, or one radix pass of B
 // bits), the table layout, the S rows per work item (capS) and the rows per
 // histogram/scatter chunk; lays out every partitioned copy, histogram, base
 // array and item list in one device allocation (256-byte aligned regions, so
@@ -38,9 +38,9 @@ uint64_t ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 int size_class(uint64_t nR) { return nR <= 1 ? 0 : 63 - __builtin_clzll(nR); }
 
 struct Choice {
-    int B = 0;               // 0: direct join, > 0: radix bits of the single pass
+    int B = 0;               // 0: unpartitioned, > 0: radix bits of the single pass
     int layout = 0;          // table layout: 0 bucket chain, 1 histogram
-    uint32_t capS = 65536;   // S rows per work item / direct slice
+    uint32_t capS = 65536;   // S rows per work item / slice of an unpartitioned join
     uint32_t chunk = 262144;  // rows per histogram and scatter chunk
     double ms = 0;           // tuned time of the class sample (0: not tuned)
     int joins = 0;           // joins of the batch in this class
@@ -48,7 +48,7 @@ struct Choice {
 };
 
 // Partitions of about capR / 2 rows for the largest |R| of the class;
-// classes whose R fits one table are joined directly.
+// classes whose R fits one table are not partitioned.
 Choice heuristic(int cls) {
     Choice c;
     const uint64_t rmax = (2ull << cls) - 1;
@@ -354,7 +354,7 @@ static void batch_free(tbg_batch *b) {
 
 // Picks the choice of every size class present in the batch by timing
 // candidates on up to ~2^25 rows of that class's own joins: first the
-// partitioning (direct or B bits), then the table layout, the S rows per
+// partitioning (none or B bits), then the table layout, the S rows per
 // item and the chunk size, keeping each winner.
 static int autotune(tbg_batch *b, const tbg_batch_join *joins, int njoins, int grid, int force_layout) {
     std::vector<int> members[NCLASS];
@@ -390,7 +390,7 @@ static int autotune(tbg_batch *b, const tbg_batch_join *joins, int njoins, int g
         const Choice h = heuristic(c);
         std::vector<int> bits;
         const uint64_t rmax = (2ull << c) - 1;
-        if (rmax <= 4ull * BATCH_CAPR) bits.push_back(0);  // direct: R re-read at most 4 times
+        if (rmax <= 4ull * BATCH_CAPR) bits.push_back(0);  // unpartitioned: R re-read at most 4 times
         const int b0 = std::max(1, h.B);
         for (int B = b0 - 1; B <= b0 + 2; B++)
             if (B >= 1 && B <= 8 && (rmax >> B) <= 4ull * BATCH_CAPR) bits.push_back(B);

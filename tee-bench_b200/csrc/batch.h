@@ -25,7 +25,7 @@ constexpr int BATCH_BITS_MAX_LOG2 = 20;
 constexpr int BATCH_PART_LOG2 = 19;
 constexpr uint32_t BATCH_DCHUNK = 262144;  // S rows per chunk ticket of a direct join
 
-// One join of the batch, in plan order.  B == 0: direct join (no
+// One join of the batch, in plan order.  B == 0: unpartitioned (no
 // partitioning; R is loaded into shared memory capR rows at a time and S is
 // probed in slices of capS rows).  B > 0: one radix pass over P = 2^B
 // partitions of the low key bits, then build/probe per partition.

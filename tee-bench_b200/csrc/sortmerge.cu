@@ -582,7 +582,7 @@ size_t rsm_count_smem_bytes() { return (size_t)RSM_COUNT_WORDS * 4; }
 // are the sorted R chunk as (key, run length) pairs, and the merge with S's
 // rows is one counter read per S row, in any order.  S is read once, where
 // sorting it in tiles read it twice and then merged: the kernel took 4.39 ms
-// at 2^27 x 2^30 and takes the time of one 8 B/row stream now.
+// at 2^27 x 2^30 reading rows; it reads 4 B keys once now.
 // Sort path, wider spans: the chunk's keys are sorted (sort_keys) and S tiles
 // of RSM_STILE keys are sorted too and merged, tile k + 1's keys loading while
 // tile k merges.

@@ -10,7 +10,7 @@
 // holds it until the process exits.
 //
 // The join is the batched persistent kernel (k_batch) run on a plan of one
-// join, count only: a direct shared-memory join when |R| fits one table
+// join, count only: an unpartitioned shared-memory join when |R| fits one table
 // (8192 rows), otherwise one radix pass of B = clamp(log2 |R| - 11, 1, 8)
 // bits, then build/probe per partition.  A one-block prologue kernel writes
 // the plan into the array and clears what must start at zero (progress
