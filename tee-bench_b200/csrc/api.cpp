@@ -206,21 +206,29 @@ RadixGeom radix_geometry(const tbg_config &cfg, uint64_t nR, uint64_t nS, int ca
     g.F1 = 1ull << g.b1;
     g.capR = capR;
     g.join_grid = w.nsm * join_ctas_per_sm(capR, cfg.materialize != 0);
-    g.capS = 0;
     if (cfg.skew_split) {
         // 64K rows an item; with fewer partitions than SMs two items per SM (of
         // at least twice the R rows that each builds): 16 partitions of 62K S
         // rows kept 132 of 148 SMs idle (100000 x 1M rows: 104 against 82 us)
-        g.capS = 65536;
+        const uint64_t spread = nS / ((uint64_t)g.join_grid * 4);
+        g.split.rows = g.split.wide = std::max<uint64_t>(65536, spread);
         if (g.P < (uint64_t)w.nsm) {
             const uint64_t fill = std::max<uint64_t>(nS / ((uint64_t)w.nsm * 2), 2 * nR / g.P);
-            g.capS = std::min<uint64_t>(g.capS, std::max<uint64_t>(fill, 4096));
+            g.split.rows = std::max<uint64_t>(spread, std::min<uint64_t>(65536, std::max(fill, SplitRule::LEAST)));
+            g.split.ctas = cfg.algo == TBG_RSM ? (uint64_t)w.nsm * rsm_ctas_per_sm(capR, cfg.materialize != 0) : g.join_grid;
         }
-        g.capS = std::max<uint64_t>(g.capS, nS / ((uint64_t)g.join_grid * 4));
     }
     // room for every R chunk of a partition to split its S side (k_plan
     // keeps oversized S sides whole if a skewed input still overflows this)
-    g.item_cap = 2 * (nR / capR + (g.capS ? nS / g.capS : 0) + 2 * g.P) + 16;
+    const uint64_t srows = g.split.rows, rchunks = nR / capR;
+    g.item_cap = 2 * (rchunks + (srows ? nS / srows : 0) + 2 * g.P) + 16;
+    // with fewer partitions than SMs, room for it whatever partitions the rows
+    // are in: without it one partition of several R chunks kept its S whole and
+    // filled as many SMs (keys 2^13 apart, 2^16 x 2^20: RHO 90.9 ms, 2.7 split;
+    // 2^16 apart, 2^16 x 2^18: RSM 0.73 and 0.15)
+    if (g.split.ctas)
+        g.item_cap = std::max<uint64_t>(g.item_cap, (rchunks + g.P) * (nS / g.split.wide + 1) +
+                                                        std::min(g.P, rchunks) * g.split.ctas + nS / srows + g.P + 16);
     // two chunks per SM, as many as partitioning CTAs are resident.  A chunk's
     // CTA reads its row of the per-chunk prefix (2^B counters) to set up its
     // cursors, so a chunk holds at least max(4096, 2^B) rows: at 15 bits 32K
@@ -261,7 +269,6 @@ RadixGeom radix_geometry_msd(uint64_t nR, uint64_t nS, uint32_t sub, int B, int 
     g.F1 = 1ull << g.b1;
     g.capR = 0;
     g.join_grid = 0;
-    g.capS = 0;
     g.item_cap = 16;
     const uint64_t min_chunk = std::max<uint64_t>(4096, g.P);
     auto chunks = [&](uint64_t n) {
@@ -382,7 +389,7 @@ static PlanArgs plan_args(const RadixGeom &g, Workspace &w) {
     pa.b2 = g.b2;
     pa.passes = g.passes;
     pa.capR = g.capR;
-    pa.capS = g.capS;
+    pa.split = g.split;
     pa.items = w.items.as<Item>();
     pa.item_cap = g.item_cap;
     pa.ctrl = w.ctrl.as<Ctrl>();
@@ -612,6 +619,7 @@ int run_radix_join_sliced(const tbg_config &cfg, const Row *dR, uint64_t nR, con
         RadixGeom g = radix_geometry(cfg, nR, n, capR, w);
         try_direct(g, cfg, d_rows, cap);
         g.direct = gmax.direct;
+        g.item_cap = std::min(g.item_cap, gmax.item_cap);  // the buffer is the longest slice's (rounding)
         if ((e = cudaStreamWaitEvent(st, s_ready[k], 0)) != cudaSuccess) return cuda_error(e, "sliced join: wait");
         if ((rc = part_hist_read(1, g, d, cfg, w, st, nullptr))) return rc;
         if ((rc = part_hist_plan(2, true, g, w, st))) return rc;

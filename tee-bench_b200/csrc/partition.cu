@@ -240,12 +240,11 @@ __device__ void plan_bases(const uint32_t *tot, uint64_t *base, int P, unsigned 
 // sorted by partition.
 __device__ void plan_block(const PlanArgs &a, int block, int tid, uint64_t *scratch) {
     const int P = 1 << a.P_log2;
-    // S sides larger than capS are split (skew) for every R chunk of the
+    // large S sides are split (skew) for every R chunk of the
     // partition; if that would overflow the item buffer, partitions whose R
     // side needs several chunks keep S whole
     auto s_chunks = [&](uint32_t hs, uint64_t nrc, bool split_all) -> uint64_t {
-        if (!a.capS || (nrc > 1 && !split_all)) return 1;
-        return (hs + a.capS - 1) / a.capS;
+        return nrc > 1 && !split_all ? 1 : a.split.items(hs, nrc);
     };
     const int f = block * PLAN_THREADS + tid;
     const uint32_t hr = f < P ? __ldcg(a.r.hist + f) : 0, hs = f < P ? __ldcg(a.s.hist + f) : 0;

@@ -32,7 +32,8 @@ struct SmallArgs {
     uint32_t nR;
     int B;                    // radix bits of the statistics (P = 2^B <= 8)
     int capR;                 // rows of R per work item (statistics)
-    uint64_t capS, item_cap;
+    SplitRule split;
+    uint64_t item_cap;
     uint32_t table_rows;      // shared-memory table size
     uint32_t bit_words;       // words of shared memory for bits
     SmallCtl *sc;
@@ -221,8 +222,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
                 const uint32_t hr = cnt[f];
                 if (!hr || !hs[f]) continue;
                 const uint64_t nrc = (hr + (uint64_t)a.capR - 1) / a.capR;
-                const bool whole = !a.capS || (pass && nrc > 1 && all > a.item_cap);
-                n += nrc * (whole ? 1 : (hs[f] + a.capS - 1) / a.capS);
+                n += nrc * (pass && nrc > 1 && all > a.item_cap ? 1 : a.split.items(hs[f], nrc));
             }
             (pass ? items : all) = n;
         }
@@ -273,7 +273,7 @@ int run_small_join(const tbg_config &cfg, const RadixGeom &g, const Row *dR, con
     a.slice = std::max<uint64_t>(mat ? 8 : 2048, (nS + w.nsm - 1) / w.nsm);
     a.B = g.B;
     a.capR = g.capR;
-    a.capS = g.capS;
+    a.split = g.split;
     a.item_cap = g.item_cap;
     a.table_rows = nR <= 4096 ? 4096 : nR <= 8192 ? 8192 : 16384;
     a.sc = w.small.as<SmallCtl>();

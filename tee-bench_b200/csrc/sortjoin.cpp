@@ -19,7 +19,6 @@
 namespace tbg {
 
 cudaError_t launch_join_rsm(const JoinArgs &a, bool materialize, int grid, cudaStream_t st);
-int rsm_ctas_per_sm(int capR, bool materialize);
 cudaError_t launch_merge_join(const Row *R, uint64_t nr, const Row *S, uint64_t ns, uint64_t *splits,
                               unsigned long long *matches, unsigned long long *rows_ctr, tbg_row_out *out,
                               uint64_t cap, bool mat, cudaStream_t st);
@@ -179,8 +178,8 @@ static int msd_count(const tbg_config &cfg, const Row *dR, uint64_t nR, const Ro
     g.sample_S = dS;
     g.capR = 0x7FFFFFFF;  // counters take any number of R rows
     g.keys = true;
-    g.capS = std::max<uint64_t>(65536, nS / ((uint64_t)w.nsm * 12));
-    g.item_cap = 2 * (nS / g.capS + 4 * g.P) + 16;
+    g.split.rows = g.split.wide = std::max<uint64_t>(65536, nS / ((uint64_t)w.nsm * 12));
+    g.item_cap = 2 * (nS / g.split.rows + 4 * g.P) + 16;
     int rc = ensure_radix_buffers(g, false, w);
     if (rc) return rc;
     if ((rc = start_radix_join(g, dR, w, st)) || (rc = part_hist_read(0, g, dR, cfg, w, st, nullptr)) || (rc = part_hist_read(1, g, dS, cfg, w, st, nullptr)) ||

@@ -23,6 +23,8 @@
 // unbounded inner loops and a stale S cursor that miscount duplicates and
 // misses; these merges count exactly the equi-join.
 #include <algorithm>
+#include <map>
+#include <mutex>
 
 #include "join_dev.cuh"
 #include "part_dev.cuh"
@@ -672,21 +674,34 @@ __global__ void __launch_bounds__(RSM_THREADS, 2) k_join_rsm_count(JoinArgs a) {
     if ((tid & 31) == 0 && ws) atomicAdd(a.matches, ws);
 }
 
-// Resident CTAs per SM of the RSM join kernel a launch would use.
+// Resident CTAs per SM of the RSM join kernel a launch would use, cached per
+// (device, capR, materialize) as join_ctas_per_sm.
 // RSM's planner caps R chunks at RSM_STILE rows, so counting joins always
 // take the bare-key kernel and k_join_rsm runs materialising only.
 int rsm_ctas_per_sm(int capR, bool materialize) {
-    int n = 0;
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, int> cache;
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> g(mu);
+    const auto key = std::make_pair(dev, capR * 2 + (materialize ? 1 : 0));
+    const auto it = cache.find(key);
+    if (it != cache.end()) return it->second;
+    cudaError_t e;
     if (!materialize) {
         const size_t smem = rsm_count_smem_bytes();
-        smem_limit((const void *)k_join_rsm_count, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_join_rsm_count, RSM_THREADS, smem);
+        if ((e = smem_limit((const void *)k_join_rsm_count, smem)) == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_join_rsm_count, RSM_THREADS, smem);
     } else {
         const size_t smem = rsm_smem_bytes(capR);
-        smem_limit((const void *)k_join_rsm<true>, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_join_rsm<true>, RSM_THREADS, smem);
+        if ((e = smem_limit((const void *)k_join_rsm<true>, smem)) == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_join_rsm<true>, RSM_THREADS, smem);
     }
-    return n < 1 ? 1 : n;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return 1;  // not cached: a later call retries
+    }
+    return cache[key] = n < 1 ? 1 : n;
 }
 
 cudaError_t launch_join_rsm(const JoinArgs &a, bool materialize, int grid, cudaStream_t st) {

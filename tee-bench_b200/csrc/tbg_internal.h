@@ -159,12 +159,32 @@ struct HeavyBuckets {
     const unsigned long long *max_part = nullptr;  // the largest bucket of R
 };
 
+// How the planner splits the S rows of a partition into work items.
+struct SplitRule {
+    uint64_t rows = 0;  // S rows per item (0: no split)
+    // partitions of several R chunks, one of which every item builds: as many
+    // items as the join has CTAs, of LEAST to `wide` rows
+    uint64_t wide = 0;
+    uint64_t ctas = 0;
+    static constexpr uint64_t LEAST = 4096;
+    // Items for each of nrc R chunks of a partition with hs S rows.
+#ifdef __CUDACC__
+    __host__ __device__
+#endif
+    uint64_t items(uint64_t hs, uint64_t nrc) const {
+        if (!rows) return 1;
+        if (nrc <= 1) return (hs + rows - 1) / rows;
+        const uint64_t few = (hs + wide - 1) / wide, many = (hs + LEAST - 1) / LEAST, wave = ctas / nrc;
+        return wave < few ? few : wave < many ? wave : many;
+    }
+};
+
 struct PlanArgs {
     RelPlan r, s;
     uint64_t nR, nS;
     int P_log2, b1, b2, passes;
     int capR;
-    uint64_t capS;            // S rows per work item when splitting (0: no split)
+    SplitRule split;
     Item *items;
     uint64_t item_cap;
     Ctrl *ctrl;
@@ -198,6 +218,7 @@ cudaError_t launch_join(const JoinArgs &a, bool materialize, int grid, cudaStrea
 size_t join_smem_bytes(int capR);
 size_t join_launch_smem(int capR, bool materialize);
 int join_ctas_per_sm(int capR, bool materialize);
+int rsm_ctas_per_sm(int capR, bool materialize);
 
 // ---- direct join (direct.cu) ----
 int direct_log2_max(uint64_t nR);

@@ -87,7 +87,8 @@ struct RadixGeom {
     int B, passes, b1, b2;
     uint64_t P, F1;
     int capR, join_grid;
-    uint64_t capS, item_cap;
+    SplitRule split;
+    uint64_t item_cap;
     int G[2];          // chunks of R, S
     uint64_t ch[2];    // rows per chunk
     uint64_t n[2];     // rows of R, S
