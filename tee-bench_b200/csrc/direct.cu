@@ -154,7 +154,8 @@ __device__ __forceinline__ void hist_pairs(uint32_t *sh, const RadixF &rf, const
 
 // R: chunk histograms, key range, bits.  Three things end the attempt before
 // all of R is entered; the CTA that sees one tells the grid through
-// ctrl->direct_dup, which every CTA looks at once a round:
+// ctrl->direct_dup, which every CTA looks at once a round (PAYLOADS: every warp,
+// with its exchanges):
 //   - two equal keys among a warp's neighbouring rows (no atomic needed), which
 //     shows sorted and hot keys before they queue at one word: 2^22 x 2^23 rows,
 //     R's last quarter one key, RSM 0.52 ms against 1.18;
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) k_hist_build(const Row *__r
         in, lo, hi,
         [&](const uint4(&x)[4], const bool(&ok)[4]) {
             if (enter) {
-                if (tid == 0 && *gave_up) s_off = 1;
+                if (!PAYLOADS && tid == 0 && round && *gave_up) s_off = 1;
                 // rows side by side (u), or in the next lane's pair, with one key
                 bool same = s_off != 0;
 #pragma unroll
