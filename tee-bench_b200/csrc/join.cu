@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(JOIN_THREADS, MAT ? 0 : 3) k_join(JoinArgs a) 
         const uint32_t it = s_item[iter & 1];
         if (it >= nitems) break;
         if (MAT) build_table<JOIN_THREADS>(t, a.R, a.items[it].r_off, a.items[it].r_len, scan_scratch);
-        else build_cells<JOIN_THREADS, false, true>(ct, Rk, a.items[it].r_off, a.items[it].r_len);
+        else build_cells<JOIN_THREADS, false, RUNS_CALL>(ct, Rk, a.items[it].r_off, a.items[it].r_len);
         if (tid == 0) {
             const uint32_t nx = atomicAdd(a.item_ctr, 1u);
             s_item[(iter + 1) & 1] = nx;  // read by all after this item's barriers

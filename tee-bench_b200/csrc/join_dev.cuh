@@ -189,7 +189,7 @@ __device__ __forceinline__ uint4 ld_pair(const uint4 *p) {
 // RUN_ROWS among 10240 rows has one of 512 of them but once in 600 tables, and
 // then stays a chain.
 template <int THREADS, bool CG, class E>
-__device__ __noinline__ bool collapse_runs(uint32_t *heads, const uint32_t *cells, uint32_t mask, int hs, int link_bits,
+__device__ __forceinline__ bool collapse_runs(uint32_t *heads, const uint32_t *cells, uint32_t mask, int hs, int link_bits,
                                            const E *__restrict__ R, uint32_t r_len, LongRuns *lr) {
     const uint32_t tid = threadIdx.x, lmask = (1u << link_bits) - 1;
     bool found = false;
@@ -225,13 +225,22 @@ __device__ __noinline__ bool collapse_runs(uint32_t *heads, const uint32_t *cell
     return true;
 }
 
+// The same as a function: k_join's probe keeps its registers. (The one-launch
+// join has registers to spare, and a function cost it 0.2 of 26 us.)
+template <int THREADS, bool CG, class E>
+__device__ __noinline__ bool collapse_runs_call(uint32_t *heads, const uint32_t *cells, uint32_t mask, int hs, int link_bits,
+                                                const E *__restrict__ R, uint32_t r_len, LongRuns *lr) {
+    return collapse_runs<THREADS, CG>(heads, cells, mask, hs, link_bits, R, r_len, lr);
+}
+enum Runs { RUNS_NONE, RUNS_CALL, RUNS_INLINE };  // whether, and how, a build looks for long runs
+
 // Builds the cells of R rows [r_off, r_off + r_len); ends with a barrier.  A
 // row whose swap fails finds another row's cell at the head, never the empty
 // one, so it exchanges its cell for whatever is there and does not try again
 // (in a loop of swaps 10,000 rows of one key took 3 ms).
 // RUNS: a row that displaces a cell of its own tag says that there may be long
 // runs (or a key twice: a look at 512 chains finds those short).
-template <int THREADS, bool CG = false, bool RUNS = false, class E = Row>
+template <int THREADS, bool CG = false, Runs RUNS = RUNS_NONE, class E = Row>
 __device__ __forceinline__ void build_cells(CellTable &t, const E *__restrict__ R, uint64_t r_off, uint32_t r_len) {
     const int tid = threadIdx.x;
     const uint32_t least = t.link_bits > t.hs ? 1u << (t.link_bits - t.hs) : 1u;
@@ -253,9 +262,14 @@ __device__ __forceinline__ void build_cells(CellTable &t, const E *__restrict__ 
             if (RUNS) run |= (old ^ tag) >> t.link_bits == 0;
         }
     }
-    if (!RUNS) __syncthreads();
-    else t.has_runs = __syncthreads_or(run) && collapse_runs<THREADS, CG>(t.heads, t.cells, t.mask, t.hs, t.link_bits,
-                                                                                  R + r_off, r_len, t.runs);
+    if (RUNS == RUNS_NONE) {
+        __syncthreads();
+    } else if (__syncthreads_or(run)) {
+        auto look = RUNS == RUNS_CALL ? collapse_runs_call<THREADS, CG, E> : collapse_runs<THREADS, CG, E>;
+        t.has_runs = look(t.heads, t.cells, t.mask, t.hs, t.link_bits, R + r_off, r_len, t.runs);
+    } else {
+        t.has_runs = false;
+    }
 }
 
 // E: rows, or bare keys (layout 1 without payloads).

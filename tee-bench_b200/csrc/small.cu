@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 1) k_small(SmallArgs a) {
         }
     }
     if (MAT) build_table<T>(t, a.R, 0, a.nR, scratch);
-    else if (!by_bits) build_cells<T, false, true>(ct, a.R, 0, a.nR);
+    else if (!by_bits) build_cells<T, false, RUNS_INLINE>(ct, a.R, 0, a.nR);
 
     // this CTA's slice of S
     const uint64_t s0 = (uint64_t)blockIdx.x * a.slice;
