@@ -119,7 +119,7 @@ struct LongRuns {
 // (LongRuns), and CELL_RUN is their head; has_runs says that there are any (the
 // same for all threads), for which the probe has a loop of its own: the test in
 // every lookup took 2% of a 16 M x 134 M join.  2^20 x 2^24 rows with 4096 rows
-// a key take 0.22 ms, 46 ms along the chains; with 256 rows a key 0.21 and 3.0;
+// a key take 0.20 ms, 46 ms along the chains; with 256 rows a key 0.19 and 3.0;
 // with 1% of R on one key (2^20 x 2^22) 0.13 and 3.3, most of it the swaps in
 // build_cells.  Counting RHO and RHT take it, the batch (whose plan has the
 // histogram table to choose) does not.
